@@ -21,6 +21,7 @@
 //    Negative or NaN weights run the reference's Jacobi rounds (min-plus SpMV).
 #include <vector>
 
+#include "gg_queue.cuh"
 #include "gg_semiring.cuh"
 #include "gg_tma.cuh"
 
@@ -419,28 +420,10 @@ struct Counters {
 
 // Frontier vertices with more than kPushHub out-edges are not walked by one warp:
 // the push kernels defer them to a hub queue, and the hub kernels split each one into
-// pieces of kPushPiece edges spread over all warps.
-static const int kPushHub = 2048;
-static const int kPushPiece = 1024;
-
-// warp-aggregated append of the lanes with `want` into q (full warp must call)
-__device__ __forceinline__ void warp_append(bool want, int32_t v, int32_t deg, int32_t* q,
-                                            Counters* ctr) {
-  const int lane = threadIdx.x & 31;
-  const unsigned b = __ballot_sync(kFullG, want);
-  if (!b) return;
-  int32_t d = want ? deg : 0;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) d += __shfl_xor_sync(kFullG, d, o);
-  const int leader = __ffs(b) - 1;
-  unsigned long long base = 0;
-  if (lane == leader) {
-    base = atomicAdd(&ctr->nf, (unsigned long long)__popc(b));
-    atomicAdd(&ctr->mf, (unsigned long long)d);
-  }
-  base = __shfl_sync(kFullG, base, leader);
-  if (want) q[base + __popc(b & ((1u << lane) - 1u))] = v;
-}
+// pieces of kPushPiece edges spread over all warps.  A piece is four steps of a warp
+// (bfs_push_range); with 2048 / 1024 one vertex below the line held its warp for 67 us.
+static const int kPushHub = 512;
+static const int kPushPiece = 512;
 
 __global__ void k_bfs_init(int32_t s, unsigned* visited, int32_t* dist, int32_t* q) {
   visited[s >> 5] |= 1u << (s & 31);
@@ -448,36 +431,60 @@ __global__ void k_bfs_init(int32_t s, unsigned* visited, int32_t* dist, int32_t*
   q[0] = s;
 }
 
+// out-edges [kb, ke) of one frontier vertex, the whole warp: 128 edges per step, so the
+// columns and then the visited words of four lines are in flight together (one line at
+// a time a warp walking 2048 edges took 64 chains of three L2 round trips, 67 us)
+static const int kPushStep = 4;
+
+__device__ __forceinline__ void bfs_push_range(const int32_t* __restrict__ prow,
+                                               const int32_t* __restrict__ pcol, int32_t kb,
+                                               int32_t ke, int32_t level, unsigned* visited,
+                                               int32_t* dist, WarpQueue& wq,
+                                               unsigned long long& edges) {
+  const int lane = threadIdx.x & 31;
+  for (int32_t base = kb; base < ke; base += 32 * kPushStep) {
+    int32_t w[kPushStep];
+    unsigned seen[kPushStep];
+#pragma unroll
+    for (int t = 0; t < kPushStep; ++t) {
+      const int32_t k = base + t * 32 + lane;
+      w[t] = k < ke ? __ldg(pcol + k) : -1;
+    }
+#pragma unroll
+    for (int t = 0; t < kPushStep; ++t) seen[t] = w[t] >= 0 ? __ldcg(visited + (w[t] >> 5)) : ~0u;
+#pragma unroll
+    for (int t = 0; t < kPushStep; ++t) {
+      const unsigned bit = 1u << (w[t] & 31);
+      const bool claim = !(seen[t] & bit) && !(atomicOr(visited + (w[t] >> 5), bit) & bit);
+      if (claim) {
+        dist[w[t]] = level;
+        edges += (unsigned long long)(__ldg(prow + w[t] + 1) - __ldg(prow + w[t]));
+      }
+      wq.push(claim, w[t]);
+    }
+  }
+}
+
 // top-down level: warp per frontier vertex, lanes over its out-edges
 __global__ void __launch_bounds__(256)
     k_bfs_push(const int32_t* __restrict__ prow, const int32_t* __restrict__ pcol,
                const int32_t* __restrict__ q, int64_t nf, int32_t level, unsigned* visited,
                int32_t* dist, int32_t* qn, Counters* ctr, int32_t* hq) {
-  const int lane = threadIdx.x & 31;
+  __shared__ int32_t stage[8][WarpQueue::kCap];
+  WarpQueue wq(stage[threadIdx.x >> 5], qn, &ctr->nf);
+  unsigned long long edges = 0;
   for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < nf;
        i += ((int64_t)gridDim.x * blockDim.x) >> 5) {
     const int32_t u = q[i];
     const int32_t k0 = prow[u], k1 = prow[u + 1];
     if (hq && k1 - k0 > kPushHub) {  // left to k_bfs_push_hub
-      if (lane == 0) hq[atomicAdd(&ctr->nh, 1ull)] = u;
+      if ((threadIdx.x & 31) == 0) hq[atomicAdd(&ctr->nh, 1ull)] = u;
       continue;
     }
-    for (int32_t base = k0; base < k1; base += 32) {
-      const int32_t k = base + lane;
-      bool claim = false;
-      int32_t w = 0, deg = 0;
-      if (k < k1) {
-        w = __ldg(pcol + k);
-        const unsigned bit = 1u << (w & 31);
-        if (!(__ldcg(visited + (w >> 5)) & bit)) claim = !(atomicOr(visited + (w >> 5), bit) & bit);
-        if (claim) {
-          dist[w] = level;
-          deg = prow[w + 1] - prow[w];
-        }
-      }
-      warp_append(claim, w, deg, qn, ctr);
-    }
+    bfs_push_range(prow, pcol, k0, k1, level, visited, dist, wq, edges);
   }
+  wq.flush();
+  warp_add(edges, &ctr->mf);
 }
 
 // pieces of the deferred frontier hubs: piece p of hub h has the global index
@@ -525,72 +532,106 @@ __global__ void __launch_bounds__(256)
                    const int32_t* __restrict__ hq, int32_t level, unsigned* visited,
                    int32_t* dist, int32_t* qn, Counters* ctr, const Counters* hctr,
                    const int32_t* __restrict__ hoff) {
-  const int lane = threadIdx.x & 31;
+  __shared__ int32_t stage[8][WarpQueue::kCap];
   const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
   const int64_t nh = (int64_t)*((volatile const unsigned long long*)&hctr->nh);
   if (nh == 0) return;
   const int64_t npieces = hoff[nh];
+  WarpQueue wq(stage[threadIdx.x >> 5], qn, &ctr->nf);
+  unsigned long long edges = 0;
   int64_t h = 0;
   for (int64_t q = gw; q < npieces; q += nw) {
     h = hub_of(hoff, nh, q, h);
-    {
-      const int32_t u = hq[h];
-      const int32_t k0 = prow[u], k1 = prow[u + 1];
-      const int64_t p = q - hoff[h];
-      const int32_t kb = k0 + (int32_t)p * kPushPiece;
-      const int32_t ke = kb + kPushPiece < k1 ? kb + kPushPiece : k1;
-      for (int32_t base = kb; base < ke; base += 32) {
-        const int32_t k = base + lane;
-        bool claim = false;
-        int32_t w = 0, deg = 0;
-        if (k < ke) {
-          w = __ldg(pcol + k);
-          const unsigned bit = 1u << (w & 31);
-          if (!(__ldcg(visited + (w >> 5)) & bit)) claim = !(atomicOr(visited + (w >> 5), bit) & bit);
-          if (claim) {
-            dist[w] = level;
-            deg = prow[w + 1] - prow[w];
-          }
-        }
-        warp_append(claim, w, deg, qn, ctr);
-      }
-    }
+    const int32_t u = hq[h];
+    const int32_t k1 = prow[u + 1];
+    const int32_t kb = prow[u] + (int32_t)(q - hoff[h]) * kPushPiece;
+    const int32_t ke = kb + kPushPiece < k1 ? kb + kPushPiece : k1;
+    bfs_push_range(prow, pcol, kb, ke, level, visited, dist, wq, edges);
   }
+  wq.flush();
+  warp_add(edges, &ctr->mf);
 }
 
 // bottom-up level: thread per vertex; an unvisited vertex joins when one of its
-// in-neighbours (A_T row) is in the frontier bitmap over an active edge
+// in-neighbours (A_T row) is in the frontier bitmap over an active edge.  In-edges are
+// tested four at a time (one 32-byte sector of columns, then four bitmap words, in
+// flight together).  Only the frontier's size and out-edges are counted, once per
+// block: the next level reads the bitmap, and the queue a push level needs is made from
+// it then (k_bitmap_to_queue).  With a queue written by every level (two same-address
+// atomics per warp, a million in one level of R-MAT scale 24) and one in-edge at a time
+// the three pull levels of a scale-24 search took 2130 us; the whole search went from
+// 3.00 to 0.66 ms.
 template <bool kOddOnly>
 __global__ void __launch_bounds__(256)
     k_bfs_pull(int64_t n, const int32_t* __restrict__ rp, const int32_t* __restrict__ cv,
                const void* nz, int tv, const unsigned* __restrict__ fb, unsigned* visited,
-               int32_t* dist, int32_t level, unsigned* fbn, int32_t* qn, Counters* ctr,
+               int32_t* dist, int32_t level, unsigned* fbn, Counters* ctr,
                const int32_t* __restrict__ prow) {
+  __shared__ unsigned long long s_nf, s_mf;
+  if (threadIdx.x == 0) s_nf = s_mf = 0;
+  __syncthreads();
   const int lane = threadIdx.x & 31;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  unsigned long long joined = 0, edges = 0;
   for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < n; base += stride) {
     const int64_t v = base + threadIdx.x;
     bool found = false;
     const unsigned vw = (v < n) ? visited[v >> 5] : ~0u;
     if (v < n && !((vw >> (v & 31)) & 1u)) {
       const int32_t k1 = rp[v + 1] - 1;
-      for (int32_t k = rp[v] - 1; k < k1; ++k) {
-        const int32_t u = __ldg(cv + k) - 1;
-        if (bit_of(fb, u) && (!kOddOnly || value_odd(nz, tv, k))) {
-          found = true;
-          break;
-        }
+      for (int32_t k = rp[v] - 1; k < k1 && !found; k += 4) {
+        int32_t u[4];
+        bool hit[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) u[t] = k + t < k1 ? __ldg(cv + k + t) - 1 : -1;
+#pragma unroll
+        for (int t = 0; t < 4; ++t) hit[t] = u[t] >= 0 && bit_of(fb, u[t]);
+#pragma unroll
+        for (int t = 0; t < 4; ++t) found |= hit[t] && (!kOddOnly || value_odd(nz, tv, k + t));
       }
     }
     const unsigned bal = __ballot_sync(kFullG, found);
-    if (found) dist[v] = level;
+    if (found) {
+      dist[v] = level;
+      ++joined;
+      edges += (unsigned long long)(prow[v + 1] - prow[v]);
+    }
     if (lane == 0 && bal) {
       const int64_t word = v >> 5;  // the warp's 32 vertices share one bitmap word
       visited[word] = vw | bal;
       fbn[word] = bal;
     }
-    warp_append(found, (int32_t)v, found ? prow[v + 1] - prow[v] : 0, qn, ctr);
+  }
+  warp_add(joined, &s_nf);
+  warp_add(edges, &s_mf);
+  __syncthreads();
+  if (threadIdx.x == 0 && s_nf) {
+    atomicAdd(&ctr->nf, s_nf);
+    atomicAdd(&ctr->mf, s_mf);
+  }
+}
+
+// the vertices of a frontier bitmap as a queue (a thread per word; one atomic per warp)
+__global__ void k_bitmap_to_queue(const unsigned* __restrict__ bm, int64_t nwords, int32_t* q,
+                                  unsigned long long* len) {
+  const int lane = threadIdx.x & 31;
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x - lane; i0 < nwords; i0 += stride) {
+    const int64_t i = i0 + lane;
+    unsigned w = i < nwords ? bm[i] : 0u;
+    int incl = __popc(w);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(kFullG, incl, o);
+      if (lane >= o) incl += t;
+    }
+    const int total = __shfl_sync(kFullG, incl, 31);
+    if (total == 0) continue;
+    unsigned long long at = 0;
+    if (lane == 31) at = atomicAdd(len, (unsigned long long)total);
+    at = __shfl_sync(kFullG, at, 31) + (unsigned long long)(incl - __popc(w));
+    for (; w; w &= w - 1) q[at++] = (int32_t)(i * 32 + __ffs(w) - 1);
   }
 }
 
@@ -1127,7 +1168,7 @@ static int bfs_run(gg_ctx* ctx, gg_mat* A, int32_t s, int which, int32_t* dist,
   Counters* h = reinterpret_cast<Counters*>(ctx->h_flags);
   int64_t nf = 1, level = 0, mf = 0, explored = 0;
   int cur = 0;
-  bool frontier_is_bitmap = false, pull = false;
+  bool frontier_is_bitmap = false, pull = false;  // a pull level leaves a bitmap, no queue
   const int64_t total_edges = P.nnz;
   // hub-free graphs (grids, meshes) run medium frontiers in the persistent kernel
   const bool coop_ok = P.max_deg <= kCoopMaxDeg && n >= (1 << 16);
@@ -1231,13 +1272,18 @@ static int bfs_run(gg_ctx* ctx, gg_mat* A, int32_t s, int which, int32_t* dist,
       if (odd_only)
         k_bfs_pull<true><<<gridsz(ctx, n), 256, 0, ctx->stream>>>(
             n, g->vrowptr, g->vcolval, g->vnz, A->dtype, sc.fb[cur], sc.visited, dist,
-            (int32_t)level, sc.fb[cur ^ 1], sc.q[cur ^ 1], sc.ctr, P.rowptr);
+            (int32_t)level, sc.fb[cur ^ 1], sc.ctr, P.rowptr);
       else
         k_bfs_pull<false><<<gridsz(ctx, n), 256, 0, ctx->stream>>>(
             n, g->vrowptr, g->vcolval, g->vnz, A->dtype, sc.fb[cur], sc.visited, dist,
-            (int32_t)level, sc.fb[cur ^ 1], sc.q[cur ^ 1], sc.ctr, P.rowptr);
+            (int32_t)level, sc.fb[cur ^ 1], sc.ctr, P.rowptr);
       frontier_is_bitmap = true;
     } else {
+      if (frontier_is_bitmap) {
+        const int64_t nwords = (n + 31) / 32;
+        k_bitmap_to_queue<<<gridsz(ctx, nwords), 256, 0, ctx->stream>>>(sc.fb[cur], nwords, sc.q[cur],
+                                                                        &sc.ctr->pad[0]);
+      }
       const bool hubs = P.max_deg > kPushHub;
       k_bfs_push<<<gridsz(ctx, nf * 32), 256, 0, ctx->stream>>>(
           P.rowptr, P.colval, sc.q[cur], nf, (int32_t)level, sc.visited, dist, sc.q[cur ^ 1], sc.ctr,
@@ -1256,7 +1302,7 @@ static int bfs_run(gg_ctx* ctx, gg_mat* A, int32_t s, int which, int32_t* dist,
     nf = (int64_t)h->nf;
     mf = (int64_t)h->mf;
     explored += mf;
-    cur ^= 1;  // the queue of the new frontier is always written; its bitmap only by pull levels
+    cur ^= 1;
   }
   if (levels_out) *levels_out = level;
   return GG_OK;
@@ -1334,13 +1380,49 @@ template <typename T> __device__ __forceinline__ T relax_add(T w, T d) {
   return (w == Lim<T>::max() || d == Lim<T>::max()) ? Lim<T>::max() : w_add(w, d);
 }
 
-// relax the out-edges of frontier vertices; improved targets join the next frontier
-// once (bitmap inq); the frontier vertex's own bit in inq_cur is cleared
+// relax the out-edges [kb, ke) of one frontier vertex at distance du, the whole warp:
+// 128 edges per step with their columns, weights and then distances in flight together;
+// improved targets join the next frontier once (bitmap inq_next)
+template <typename T>
+__device__ __forceinline__ void sssp_push_range(const int32_t* __restrict__ prow,
+                                                const int32_t* __restrict__ pcol,
+                                                const T* __restrict__ pw, int32_t kb, int32_t ke,
+                                                T du, T* dist, unsigned* inq_next, WarpQueue& wq,
+                                                unsigned long long& edges) {
+  const int lane = threadIdx.x & 31;
+  for (int32_t base = kb; base < ke; base += 32 * kPushStep) {
+    int32_t w[kPushStep];
+    T cand[kPushStep], dw[kPushStep];
+#pragma unroll
+    for (int t = 0; t < kPushStep; ++t) {
+      const int32_t k = base + t * 32 + lane;
+      w[t] = k < ke ? __ldg(pcol + k) : -1;
+      cand[t] = k < ke ? relax_add(__ldg(pw + k), du) : Lim<T>::max();
+    }
+#pragma unroll
+    for (int t = 0; t < kPushStep; ++t) dw[t] = w[t] >= 0 ? ld_cg(dist + w[t]) : Lim<T>::min();
+#pragma unroll
+    for (int t = 0; t < kPushStep; ++t) {
+      bool add = false;
+      if (cand[t] < dw[t] && cand[t] < atomic_min_t(dist + w[t], cand[t])) {
+        const unsigned bit = 1u << (w[t] & 31);
+        add = !(atomicOr(inq_next + (w[t] >> 5), bit) & bit);
+        if (add) edges += (unsigned long long)(__ldg(prow + w[t] + 1) - __ldg(prow + w[t]));
+      }
+      wq.push(add, w[t]);
+    }
+  }
+}
+
+// push round: warp per frontier vertex; the vertex's own bit in inq_cur is cleared
 template <typename T>
 __global__ void __launch_bounds__(256)
     k_sssp_push(const int32_t* __restrict__ prow, const int32_t* __restrict__ pcol,
                 const T* __restrict__ pw, const int32_t* __restrict__ q, int64_t nf, T* dist,
                 unsigned* inq_cur, unsigned* inq_next, int32_t* qn, Counters* ctr, int32_t* hq) {
+  __shared__ int32_t stage[8][WarpQueue::kCap];
+  WarpQueue wq(stage[threadIdx.x >> 5], qn, &ctr->nf);
+  unsigned long long edges = 0;
   const int lane = threadIdx.x & 31;
   for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < nf;
        i += ((int64_t)gridDim.x * blockDim.x) >> 5) {
@@ -1351,25 +1433,10 @@ __global__ void __launch_bounds__(256)
       if (lane == 0) hq[atomicAdd(&ctr->nh, 1ull)] = u;
       continue;
     }
-    const T du = ld_cg(dist + u);
-    for (int32_t base = k0; base < k1; base += 32) {
-      const int32_t k = base + lane;
-      bool add = false;
-      int32_t w = 0;
-      if (k < k1) {
-        w = __ldg(pcol + k);
-        const T cand = relax_add(__ldg(pw + k), du);
-        if (cand < ld_cg(dist + w)) {
-          const T old = atomic_min_t(dist + w, cand);
-          if (cand < old) {
-            const unsigned bit = 1u << (w & 31);
-            add = !(atomicOr(inq_next + (w >> 5), bit) & bit);
-          }
-        }
-      }
-      warp_append(add, w, add ? prow[w + 1] - prow[w] : 0, qn, ctr);
-    }
+    sssp_push_range<T>(prow, pcol, pw, k0, k1, ld_cg(dist + u), dist, inq_next, wq, edges);
   }
+  wq.flush();
+  warp_add(edges, &ctr->mf);
 }
 
 template <typename T>
@@ -1378,41 +1445,25 @@ __global__ void __launch_bounds__(256)
                     const T* __restrict__ pw, const int32_t* __restrict__ hq, T* dist,
                     unsigned* inq_next, int32_t* qn, Counters* ctr, const Counters* hctr,
                     const int32_t* __restrict__ hoff) {
-  const int lane = threadIdx.x & 31;
+  __shared__ int32_t stage[8][WarpQueue::kCap];
   const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
   const int64_t nh = (int64_t)*((volatile const unsigned long long*)&hctr->nh);
   if (nh == 0) return;
   const int64_t npieces = hoff[nh];
+  WarpQueue wq(stage[threadIdx.x >> 5], qn, &ctr->nf);
+  unsigned long long edges = 0;
   int64_t h = 0;
   for (int64_t q = gw; q < npieces; q += nw) {
     h = hub_of(hoff, nh, q, h);
     const int32_t u = hq[h];
-    const int32_t k0 = prow[u], k1 = prow[u + 1];
-    const T du = ld_cg(dist + u);
-    {
-      const int64_t p = q - hoff[h];
-      const int32_t kb = k0 + (int32_t)p * kPushPiece;
-      const int32_t ke = kb + kPushPiece < k1 ? kb + kPushPiece : k1;
-      for (int32_t base = kb; base < ke; base += 32) {
-        const int32_t k = base + lane;
-        bool add = false;
-        int32_t w = 0;
-        if (k < ke) {
-          w = __ldg(pcol + k);
-          const T cand = relax_add(__ldg(pw + k), du);
-          if (cand < ld_cg(dist + w)) {
-            const T old = atomic_min_t(dist + w, cand);
-            if (cand < old) {
-              const unsigned bit = 1u << (w & 31);
-              add = !(atomicOr(inq_next + (w >> 5), bit) & bit);
-            }
-          }
-        }
-        warp_append(add, w, add ? prow[w + 1] - prow[w] : 0, qn, ctr);
-      }
-    }
+    const int32_t k1 = prow[u + 1];
+    const int32_t kb = prow[u] + (int32_t)(q - hoff[h]) * kPushPiece;
+    const int32_t ke = kb + kPushPiece < k1 ? kb + kPushPiece : k1;
+    sssp_push_range<T>(prow, pcol, pw, kb, ke, ld_cg(dist + u), dist, inq_next, wq, edges);
   }
+  wq.flush();
+  warp_add(edges, &ctr->mf);
 }
 
 // single-CTA rounds while the frontier is small (mirror of k_bfs_small)
@@ -1565,15 +1616,18 @@ __global__ void __launch_bounds__(1024)
 
 // frontier = every vertex whose start distance is finite
 template <typename T>
-__global__ void k_sssp_seed(int64_t n, const T* dist, unsigned* inq, int32_t* q, Counters* ctr) {
+__global__ void __launch_bounds__(256) k_sssp_seed(int64_t n, const T* dist, unsigned* inq, int32_t* q, Counters* ctr) {
+  __shared__ int32_t stage[8][WarpQueue::kCap];
+  WarpQueue wq(stage[threadIdx.x >> 5], q, &ctr->nf);
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < n; base += stride) {
     const int64_t v = base + threadIdx.x;
     const bool fin = v < n && dist[v] != Lim<T>::max();
     const unsigned bal = __ballot_sync(kFullG, fin);
     if ((threadIdx.x & 31) == 0 && bal) inq[v >> 5] = bal;
-    warp_append(fin, (int32_t)v, 0, q, ctr);
+    wq.push(fin, (int32_t)v);
   }
+  wq.flush();
 }
 
 template <typename T>
@@ -1866,6 +1920,9 @@ __global__ void __launch_bounds__(256)
     k_sssp_pull(int64_t n, const int32_t* __restrict__ rp, const int32_t* __restrict__ cv,
                 const void* nz, int tv, const unsigned* __restrict__ chg, T* dist,
                 unsigned* chg_next, int32_t* qn, Counters* ctr, const int32_t* __restrict__ prow) {
+  __shared__ int32_t stage[8][WarpQueue::kCap];
+  WarpQueue wq(stage[threadIdx.x >> 5], qn, &ctr->nf);
+  unsigned long long edges = 0;
   const int lane = threadIdx.x & 31;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < n; base += stride) {
@@ -1905,8 +1962,11 @@ __global__ void __launch_bounds__(256)
     }
     const unsigned word = __ballot_sync(kFullG, changed);
     if (lane == 0 && base + threadIdx.x - lane < n) chg_next[v >> 5] = word;
-    warp_append(changed, (int32_t)v, changed ? prow[v + 1] - prow[v] : 0, qn, ctr);
+    if (changed) edges += (unsigned long long)(prow[v + 1] - prow[v]);
+    wq.push(changed, (int32_t)v);
   }
+  wq.flush();
+  warp_add(edges, &ctr->mf);
 }
 
 // rows of 33..kHubDegB in-edges of a pull round (the hub plan's mid list, longest
@@ -1919,6 +1979,9 @@ __global__ void __launch_bounds__(256)
                     int tv, const unsigned* __restrict__ chg, T* dist, unsigned* chg_next,
                     int32_t* qn, Counters* ctr, const int32_t* __restrict__ prow,
                     const int32_t* __restrict__ mid, int64_t nmid) {
+  __shared__ int32_t stage[8][WarpQueue::kCap];
+  WarpQueue wq(stage[threadIdx.x >> 5], qn, &ctr->nf);
+  unsigned long long edges = 0;
   const int lane = threadIdx.x & 31;
   // warps numbered block-major: the longest groups go to different SMs
   const int64_t gw = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
@@ -2010,8 +2073,11 @@ __global__ void __launch_bounds__(256)
       changed = true;
       atomicOr(chg_next + (myv >> 5), 1u << (myv & 31));
     }
-    warp_append(changed, myv, changed ? prow[myv + 1] - prow[myv] : 0, qn, ctr);
+    if (changed) edges += (unsigned long long)(prow[myv + 1] - prow[myv]);
+    wq.push(changed, myv);
   }
+  wq.flush();
+  warp_add(edges, &ctr->mf);
 }
 
 // hub rows of the pull round: one warp per piece of the matrix's hub plan (rows of
@@ -2070,22 +2136,20 @@ static const int64_t kPullSellDiv = GG_PULL_SELL_DIV;
 
 template <typename T>
 __device__ __forceinline__ void pull_lower(int64_t srow, int64_t m, const int32_t* __restrict__ perm,
-                                           T cand, T* dist, unsigned* inq_next, int32_t* qn,
-                                           Counters* ctr, const int32_t* __restrict__ prow) {
+                                           T cand, T* dist, unsigned* inq_next, WarpQueue& wq,
+                                           unsigned long long& edges,
+                                           const int32_t* __restrict__ prow) {
   bool improved = false;
-  int32_t v = 0, deg = 0;
+  int32_t v = 0;
   if (srow < m && cand != Lim<T>::max()) {
     v = __ldg(perm + srow) - 1;
-    if (cand < ld_cg(dist + v)) {
-      const T old = atomic_min_t(dist + v, cand);
-      if (cand < old) {
-        const unsigned bit = 1u << (v & 31);
-        improved = !(atomicOr(inq_next + (v >> 5), bit) & bit);
-        if (improved) deg = __ldg(prow + v + 1) - __ldg(prow + v);
-      }
+    if (cand < ld_cg(dist + v) && cand < atomic_min_t(dist + v, cand)) {
+      const unsigned bit = 1u << (v & 31);
+      improved = !(atomicOr(inq_next + (v >> 5), bit) & bit);
+      if (improved) edges += (unsigned long long)(__ldg(prow + v + 1) - __ldg(prow + v));
     }
   }
-  warp_append(improved, v, deg, qn, ctr);
+  wq.push(improved, v);
 }
 
 template <typename T>
@@ -2094,6 +2158,9 @@ __global__ void __launch_bounds__(kPullSellThreads)
                      const int32_t* __restrict__ perm, int64_t m, const int4* __restrict__ pitems,
                      int64_t nitems, T* dist, unsigned* inq_next, int32_t* qn, Counters* ctr,
                      const int32_t* __restrict__ prow) {
+  __shared__ int32_t stage[kPullSellThreads / 32][WarpQueue::kCap];
+  WarpQueue wq(stage[threadIdx.x >> 5], qn, &ctr->nf);
+  unsigned long long edges = 0;
   const int lane = threadIdx.x & 31;
   const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -2125,7 +2192,7 @@ __global__ void __launch_bounds__(kPullSellThreads)
         for (int u = 0; u < kNarrowCols; ++u)
           if (u >= u0 && u < u0 + w && c[u] < best) best = c[u];
         u0 += w;
-        pull_lower(d.y + t * 32 + lane, m, perm, best, dist, inq_next, qn, ctr, prow);
+        pull_lower(d.y + t * 32 + lane, m, perm, best, dist, inq_next, wq, edges, prow);
       }
       continue;
     }
@@ -2166,8 +2233,10 @@ __global__ void __launch_bounds__(kPullSellThreads)
         }
       }
     }
-    pull_lower(srow, m, perm, best, dist, inq_next, qn, ctr, prow);
+    pull_lower(srow, m, perm, best, dist, inq_next, wq, edges, prow);
   }
+  wq.flush();
+  warp_add(edges, &ctr->mf);
 }
 
 // the SELL-32 copy (rows sorted by length) and its work plan, built on first use
