@@ -822,42 +822,40 @@ __global__ void __launch_bounds__(1024)
 static const int kCoopMaxDeg = 64;
 static const int kCoopLo = 1024;   // the single-CTA kernel takes smaller frontiers
 static const int kCoopThreads = 1024;
+#ifndef GG_NF_THREADS
+#define GG_NF_THREADS 512
+#endif
+static const int kNfThreads = GG_NF_THREADS;  // near-far searches
 static const double kNearFarScale = 32.0;  // near-far band width = this x the mean weight
 
 struct CoopCtl {
   unsigned long long cnt[3];
-  unsigned bar[4];  // arrivals, generation, error, poll limit of the barrier's waits
+  unsigned bar[4];  // arrivals, unused, error, poll limit of the barrier's waits
   long long nf_out;
   int level_out;    // last completed level / round (relative for SSSP)
   int which_out;    // queue holding the remaining frontier: 0 = first, 1 = second
 };
 
-__device__ __forceinline__ bool coop_grid_sync(unsigned* bar, unsigned nblocks) {
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    volatile unsigned* vgen = bar + 1;
-    volatile unsigned* verr = bar + 2;
-    const unsigned gen = *vgen;
-    const unsigned long long limit = bar[3];  // set by the control block's init kernel
-    __threadfence();
-    if (atomicAdd(bar, 1u) == nblocks - 1) {
-      bar[0] = 0;
-      __threadfence();
-      atomicAdd(bar + 1, 1u);
-    } else {
-      unsigned long long polls = 0;
-      while (*vgen == gen && *verr == 0) {
-        if (++polls > limit) {
-          atomicExch(bar + 2, 1u);
-          break;
-        }
-        __nanosleep(100);
-      }
+// Grid barrier, the part of thread 0 of every block (between two block barriers): the
+// arrival counter bar[0] only grows and `target` is its value once every block arrived
+// (blocks x barriers so far, compared modulo 2^32), so one arrival and the polls of one
+// word are all the traffic.  The wait is bounded by `limit` polls; running out sets the
+// error word bar[2], which the waiting blocks look at every 16 polls.
+__device__ __forceinline__ bool coop_leader_sync(unsigned* bar, unsigned target,
+                                                 unsigned long long limit) {
+  __threadfence();
+  atomicAdd(bar, 1u);
+  unsigned long long polls = 0;
+  for (;;) {
+    unsigned a;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(a) : "l"(bar) : "memory");
+    if ((int)(a - target) >= 0) return true;
+    if (++polls > limit) {
+      atomicExch(bar + 2, 1u);
+      return false;
     }
-    __threadfence();
+    if ((polls & 15) == 0 && *((volatile unsigned*)(bar + 2))) return false;
   }
-  __syncthreads();
-  return *((volatile unsigned*)(bar + 2)) == 0;
 }
 
 __global__ void k_coop_init(CoopCtl* cc, long long nf0, unsigned polls) {
@@ -865,39 +863,93 @@ __global__ void k_coop_init(CoopCtl* cc, long long nf0, unsigned polls) {
   cc->cnt[1] = 0;
   cc->cnt[2] = (unsigned long long)nf0;
   cc->bar[0] = cc->bar[1] = cc->bar[2] = 0;
-  cc->bar[3] = polls;
+  cc->bar[3] = polls;  // poll limit of the barrier's waits
   cc->nf_out = 0;
   cc->level_out = 0;
   cc->which_out = 0;
 }
 
-// warp-aggregated append to a queue counted by *cnt (full warp must call)
-__device__ __forceinline__ void coop_append(bool want, int32_t v, int32_t* q,
+// What a block appends to the two lists of a persistent step (the next frontier and,
+// for near-far searches, the far list) is staged in shared memory, so a step costs one
+// atomic per list and block on the lists' lengths; entries past kStepStage go to the
+// list directly (one atomic per warp).
+static const int kStepStage = 2048;
+
+struct StepLists {
+  int32_t buf[2][kStepStage];
+  int n[2];
+  unsigned long long base[2];
+  long long len;   // length of the list the next step reads
+  long long flen;  // far list length (near-far)
+  int ok;
+};
+
+// the whole warp calls
+__device__ __forceinline__ void step_append(StepLists& S, int list, bool want, int32_t v, int32_t* q,
                                             unsigned long long* cnt) {
   const int lane = threadIdx.x & 31;
   const unsigned b = __ballot_sync(kFullG, want);
   if (!b) return;
   const int leader = __ffs(b) - 1;
-  unsigned long long base = 0;
-  if (lane == leader) base = atomicAdd(cnt, (unsigned long long)__popc(b));
-  base = __shfl_sync(kFullG, base, leader);
-  if (want) q[base + __popc(b & ((1u << lane) - 1u))] = v;
+  int at = 0;
+  if (lane == leader) at = atomicAdd(&S.n[list], __popc(b));
+  at = __shfl_sync(kFullG, at, leader) + __popc(b & ((1u << lane) - 1u));
+  if (want && at < kStepStage) S.buf[list][at] = v;
+  const unsigned over = __ballot_sync(kFullG, want && at >= kStepStage);
+  if (!over) return;
+  const int l2 = __ffs(over) - 1;
+  unsigned long long g = 0;
+  if (lane == l2) g = atomicAdd(cnt, (unsigned long long)__popc(over));
+  g = __shfl_sync(kFullG, g, l2);
+  if (want && at >= kStepStage) q[g + __popc(over & ((1u << lane) - 1u))] = v;
 }
 
-// BFS levels, thread per frontier vertex; exits when the frontier is empty, at most
-// lo, or above hi
+// writes the staged entries out; the whole block calls, a block barrier comes after
+__device__ __forceinline__ void step_flush(StepLists& S, int32_t* q0, unsigned long long* cnt0,
+                                           int32_t* q1, unsigned long long* cnt1) {
+  __syncthreads();
+  const int n0 = S.n[0] < kStepStage ? S.n[0] : kStepStage;
+  const int n1 = S.n[1] < kStepStage ? S.n[1] : kStepStage;
+  if (threadIdx.x == 0 && n0) S.base[0] = atomicAdd(cnt0, (unsigned long long)n0);
+  if (threadIdx.x == 32 && n1) S.base[1] = atomicAdd(cnt1, (unsigned long long)n1);
+  __syncthreads();
+  for (int i = threadIdx.x; i < n0; i += blockDim.x) q0[S.base[0] + i] = S.buf[0][i];
+  for (int i = threadIdx.x; i < n1; i += blockDim.x) q1[S.base[1] + i] = S.buf[1][i];
+  __syncthreads();
+  if (threadIdx.x == 0) S.n[0] = S.n[1] = 0;
+}
+
+// Frontier vertices are taken kLanesPerVertex lanes each (grid and mesh vertices have 4
+// to 8 edges): a step's chain of dependent L2 round trips is walked once instead of
+// once per edge.  Warps are numbered across the blocks first, so a frontier of a few
+// thousand vertices keeps every SM busy rather than the first four blocks.  With a
+// thread per vertex, one edge after another, queue atomics per warp and a sleeping
+// generation barrier, a near-far search of the 2048 x 2048 Float32 grid took 46.3 ms
+// (about 11 us a step); this way 14.9 ms (3.6 us), bound by the step's ten dependent
+// L2 round trips.
+static const int kLanesPerVertex = 4;
+static const int kVerticesPerWarp = 32 / kLanesPerVertex;
+
+// BFS levels; exits when the frontier is empty, at most lo, or above hi
 __global__ void __launch_bounds__(kCoopThreads, 1)
     k_bfs_coop(const int32_t* __restrict__ prow, const int32_t* __restrict__ pcol, int32_t* qa,
                int32_t* qb, unsigned* visited, int32_t* dist, CoopCtl* cc, int32_t level0,
                long long lo, long long hi) {
+  __shared__ StepLists S;
   const int lane = threadIdx.x & 31;
-  const int64_t gt = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t nt = (int64_t)gridDim.x * blockDim.x;
+  const int64_t gw = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+  const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
+  const unsigned long long limit = cc->bar[3];
   int32_t* cur = qa;
   int32_t* nxt = qb;
+  if (threadIdx.x == 0) {
+    S.n[0] = S.n[1] = 0;
+    S.len = (long long)*((volatile unsigned long long*)&cc->cnt[2]);
+  }
+  __syncthreads();
   for (int st = 0;; ++st) {
     const int r = st % 3;
-    const long long nf = (long long)*((volatile unsigned long long*)&cc->cnt[(r + 2) % 3]);
+    const long long nf = S.len;
     if (nf == 0 || nf <= lo || nf > hi) {
       if (blockIdx.x == 0 && threadIdx.x == 0) {
         cc->nf_out = nf;
@@ -908,33 +960,34 @@ __global__ void __launch_bounds__(kCoopThreads, 1)
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) cc->cnt[(r + 1) % 3] = 0;
     const int32_t level = level0 + st + 1;
-    for (int64_t i0 = gt - lane; i0 < nf; i0 += nt) {  // warp-uniform trip count
-      const int64_t i = i0 + lane;
-      int32_t k0 = 0, k1 = 0;
+    for (int64_t i0 = gw * kVerticesPerWarp; i0 < nf; i0 += nw * kVerticesPerWarp) {
+      const int64_t i = i0 + lane / kLanesPerVertex;
+      int32_t k = 0, k1 = 0;
       if (i < nf) {
-        const int32_t u = cur[i];
-        k0 = __ldg(prow + u);
+        const int32_t u = __ldcg(cur + i);
+        k = __ldg(prow + u) + lane % kLanesPerVertex;
         k1 = __ldg(prow + u + 1);
       }
-      int32_t dmax = k1 - k0;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const int32_t t = __shfl_xor_sync(kFullG, dmax, o);
-        dmax = t > dmax ? t : dmax;
-      }
-      for (int32_t j = 0; j < dmax; ++j) {
+      while (__any_sync(kFullG, k < k1)) {
         bool claim = false;
         int32_t w = 0;
-        if (k0 + j < k1) {
-          w = __ldg(pcol + k0 + j);
+        if (k < k1) {
+          w = __ldg(pcol + k);
           const unsigned bit = 1u << (w & 31);
-          if (!(__ldcg(visited + (w >> 5)) & bit)) claim = !(atomicOr(visited + (w >> 5), bit) & bit);
+          claim = !(__ldcg(visited + (w >> 5)) & bit) && !(atomicOr(visited + (w >> 5), bit) & bit);
           if (claim) dist[w] = level;
         }
-        coop_append(claim, w, nxt, &cc->cnt[r]);
+        step_append(S, 0, claim, w, nxt, &cc->cnt[r]);
+        k += kLanesPerVertex;
       }
     }
-    if (!coop_grid_sync(cc->bar, gridDim.x)) return;
+    step_flush(S, nxt, &cc->cnt[r], nullptr, nullptr);
+    if (threadIdx.x == 0) {
+      S.ok = coop_leader_sync(cc->bar, (unsigned)(st + 1) * gridDim.x, limit);
+      S.len = (long long)*((volatile unsigned long long*)&cc->cnt[r]);
+    }
+    __syncthreads();
+    if (!S.ok) return;
     int32_t* t = cur;
     cur = nxt;
     nxt = t;
@@ -1010,6 +1063,8 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kCoopThre
   __shared__ int s_spill;
   const int rank = blockIdx.x;  // the grid is one cluster
   const int lane = threadIdx.x & 31;
+  const int64_t gw = (int64_t)(threadIdx.x >> 5) * kClusterCtas + rank;
+  const int64_t nw = (int64_t)kClusterCtas * (blockDim.x >> 5);
   const int64_t gt = (int64_t)rank * blockDim.x + threadIdx.x;
   const int64_t nt = (int64_t)kClusterCtas * blockDim.x;
   {  // an even share of the starting frontier (at most kClusterCap) per CTA
@@ -1056,33 +1111,28 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kCoopThre
     }
     const int32_t level = level0 + st + 1;
     int32_t* nxt = sq[p ^ 1];
-    for (int64_t i0 = gt - lane; i0 < nf; i0 += nt) {
-      const int64_t i = i0 + lane;
-      int32_t k0 = 0, k1 = 0;
+    for (int64_t i0 = gw * kVerticesPerWarp; i0 < nf; i0 += nw * kVerticesPerWarp) {
+      const int64_t i = i0 + lane / kLanesPerVertex;
+      int32_t k = 0, k1 = 0;
       if (i < nf) {
         int r = 0;
         while (r + 1 < kClusterCtas && s_pre[r + 1] <= i) ++r;
         const int32_t u = dsmem_ld(dsmem_addr(&sq[p][i - s_pre[r]], (uint32_t)r));
-        k0 = __ldg(prow + u);
+        k = __ldg(prow + u) + lane % kLanesPerVertex;
         k1 = __ldg(prow + u + 1);
       }
-      int32_t dmax = k1 - k0;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const int32_t t = __shfl_xor_sync(kFullG, dmax, o);
-        dmax = t > dmax ? t : dmax;
-      }
-      for (int32_t j = 0; j < dmax; ++j) {
+      while (__any_sync(kFullG, k < k1)) {
         bool claim = false;
         int32_t w = 0;
-        if (k0 + j < k1) {
-          w = __ldg(pcol + k0 + j);
+        if (k < k1) {
+          w = __ldg(pcol + k);
           const unsigned bit = 1u << (w & 31);
           // claimed by the atomic alone: one L2 round trip on this level's critical path
           claim = !(atomicOr(visited + (w >> 5), bit) & bit);
           if (claim) dist[w] = level;
         }
         stage_append(claim, w, nxt, &s_cnt[p ^ 1], qb, &cc->cnt[1]);
+        k += kLanesPerVertex;
       }
     }
     cluster_barrier();
@@ -1656,75 +1706,6 @@ __global__ void k_changed_copy(int64_t n, const T* next, T* dist, unsigned* flag
   if (ch) atomicOr(flag, 1u);
 }
 
-// Bellman-Ford rounds (push, atomic min, membership bitmaps), thread per frontier vertex
-template <typename T>
-__global__ void __launch_bounds__(kCoopThreads, 1)
-    k_sssp_coop(const int32_t* __restrict__ prow, const int32_t* __restrict__ pcol,
-                const T* __restrict__ pw, int32_t* qa, int32_t* qb, T* dist, unsigned* inq_a,
-                unsigned* inq_b, CoopCtl* cc, long long lo, long long hi, long long max_rounds) {
-  const int lane = threadIdx.x & 31;
-  const int64_t gt = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t nt = (int64_t)gridDim.x * blockDim.x;
-  int32_t* cur = qa;
-  int32_t* nxt = qb;
-  unsigned* icur = inq_a;
-  unsigned* inxt = inq_b;
-  for (int st = 0;; ++st) {
-    const int r = st % 3;
-    const long long nf = (long long)*((volatile unsigned long long*)&cc->cnt[(r + 2) % 3]);
-    if (nf == 0 || nf <= lo || nf > hi || st >= max_rounds) {
-      if (blockIdx.x == 0 && threadIdx.x == 0) {
-        cc->nf_out = nf;
-        cc->level_out = st;
-        cc->which_out = st & 1;
-      }
-      return;
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) cc->cnt[(r + 1) % 3] = 0;
-    for (int64_t i0 = gt - lane; i0 < nf; i0 += nt) {
-      const int64_t i = i0 + lane;
-      int32_t k0 = 0, k1 = 0;
-      T du = T(0);
-      if (i < nf) {
-        const int32_t u = cur[i];
-        atomicAnd(icur + (u >> 5), ~(1u << (u & 31)));
-        k0 = __ldg(prow + u);
-        k1 = __ldg(prow + u + 1);
-        du = ld_cg(dist + u);
-      }
-      int32_t dmax = k1 - k0;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const int32_t t = __shfl_xor_sync(kFullG, dmax, o);
-        dmax = t > dmax ? t : dmax;
-      }
-      for (int32_t j = 0; j < dmax; ++j) {
-        bool add = false;
-        int32_t w = 0;
-        if (k0 + j < k1) {
-          w = __ldg(pcol + k0 + j);
-          const T cand = relax_add(__ldg(pw + k0 + j), du);
-          if (cand < ld_cg(dist + w)) {
-            const T old = atomic_min_t(dist + w, cand);
-            if (cand < old) {
-              const unsigned bit = 1u << (w & 31);
-              add = !(atomicOr(inxt + (w >> 5), bit) & bit);
-            }
-          }
-        }
-        coop_append(add, w, nxt, &cc->cnt[r]);
-      }
-    }
-    if (!coop_grid_sync(cc->bar, gridDim.x)) return;
-    int32_t* t = cur;
-    cur = nxt;
-    nxt = t;
-    unsigned* tb = icur;
-    icur = inxt;
-    inxt = tb;
-  }
-}
-
 // Whole shortest-path search for hub-free graphs in one persistent cooperative
 // launch, near-far ordered: only vertices whose tentative distance is below the
 // threshold thr are relaxed ("near"); improved vertices at or above it wait in the far
@@ -1732,7 +1713,7 @@ __global__ void __launch_bounds__(kCoopThreads, 1)
 // On high-diameter graphs with spread weights this avoids most of the repeated
 // relaxations of plain rounds.  The fixpoint is the same (min over paths of the
 // left-folded sums; every improved vertex is relaxed again eventually).  Grid
-// barriers are bounded (coop_grid_sync); the number of steps is bounded by max_steps.
+// barriers are bounded (coop_leader_sync); the number of steps is bounded by max_steps.
 struct NfCtl {
   unsigned long long cnt[3];  // near queue lengths, rotating as in CoopCtl
   unsigned long long fcnt[3];  // far list lengths (three lists in rotation)
@@ -1753,14 +1734,16 @@ __global__ void k_nf_init(NfCtl* cc, long long nf0, unsigned polls) {
 }
 
 template <typename T>
-__global__ void __launch_bounds__(kCoopThreads, 1)
+__global__ void __launch_bounds__(kNfThreads, 1)
     k_sssp_nearfar(const int32_t* __restrict__ prow, const int32_t* __restrict__ pcol,
                    const T* __restrict__ pw, int32_t* qa, int32_t* qb, int32_t* fa, int32_t* fb,
                    int32_t* fz, T* dist, unsigned* inq_a, unsigned* inq_b, unsigned* infar,
                    NfCtl* cc, T delta, long long max_steps) {
+  __shared__ StepLists S;
   const int lane = threadIdx.x & 31;
-  const int64_t gt = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t nt = (int64_t)gridDim.x * blockDim.x;
+  const int64_t gw = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+  const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
+  const unsigned long long limit = cc->bar[3];
   int32_t* cur = qa;
   int32_t* nxt = qb;
   unsigned* icur = inq_a;
@@ -1771,40 +1754,39 @@ __global__ void __launch_bounds__(kCoopThreads, 1)
   int32_t* const fl[3] = {fa, fb, fz};
   int fc = 0;
   T thr = delta;
+  if (threadIdx.x == 0) {
+    S.n[0] = S.n[1] = 0;
+    S.len = (long long)*((volatile unsigned long long*)&cc->cnt[2]);
+    S.flen = 0;
+  }
+  __syncthreads();
   for (long long st = 0;; ++st) {
     const int r = (int)(st % 3);
-    const long long nf = (long long)*((volatile unsigned long long*)&cc->cnt[(r + 2) % 3]);
-    if (st >= max_steps) {
+    const long long nf = S.len, nfar = S.flen;
+    const int fn = fc == 2 ? 0 : fc + 1;
+    const bool band = nf == 0;
+    if (st >= max_steps || (band && nfar == 0)) {
       if (blockIdx.x == 0 && threadIdx.x == 0) {
         cc->steps_out = st;
-        cc->status = 2;
+        cc->status = st >= max_steps ? 2 : 1;
       }
       return;
     }
-    if (nf == 0) {
-      const long long nfar = (long long)*((volatile unsigned long long*)&cc->fcnt[fc]);
-      const int fn = fc == 2 ? 0 : fc + 1;
-      if (nfar == 0) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
-          cc->steps_out = st;
-          cc->status = 1;
-        }
-        return;
-      }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      cc->cnt[(r + 1) % 3] = 0;
+      cc->fcnt[(fc + 2) % 3] = 0;
+    }
+    if (band) {
       // next distance band: far vertices below the new threshold become the next
       // frontier (counted and marked like a normal step's output), the others move to
-      // the other far list
+      // the next far list
       thr = thr > Lim<T>::max() - delta ? Lim<T>::max() : w_add(thr, delta);
-      if (blockIdx.x == 0 && threadIdx.x == 0) {
-        cc->cnt[(r + 1) % 3] = 0;
-        cc->fcnt[(fc + 2) % 3] = 0;
-      }
-      for (int64_t i0 = gt - lane; i0 < nfar; i0 += nt) {
+      for (int64_t i0 = gw * 32; i0 < nfar; i0 += nw * 32) {
         const int64_t i = i0 + lane;
         bool to_near = false, to_far = false;
         int32_t v = 0;
         if (i < nfar) {
-          v = fl[fc][i];
+          v = __ldcg(fl[fc] + i);
           if (ld_cg(dist + v) < thr) {
             atomicAnd(infar + (v >> 5), ~(1u << (v & 31)));
             const unsigned bit = 1u << (v & 31);
@@ -1813,60 +1795,49 @@ __global__ void __launch_bounds__(kCoopThreads, 1)
             to_far = true;
           }
         }
-        coop_append(to_near, v, nxt, &cc->cnt[r]);
-        coop_append(to_far, v, fl[fn], &cc->fcnt[fn]);
+        step_append(S, 0, to_near, v, nxt, &cc->cnt[r]);
+        step_append(S, 1, to_far, v, fl[fn], &cc->fcnt[fn]);
       }
-      if (!coop_grid_sync(cc->bar, gridDim.x)) return;
-      int32_t* t = cur;
-      cur = nxt;
-      nxt = t;
-      unsigned* tb = icur;
-      icur = inxt;
-      inxt = tb;
       fc = fn;
-      continue;
-    }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-      cc->cnt[(r + 1) % 3] = 0;
-      cc->fcnt[(fc + 2) % 3] = 0;
-    }
-    for (int64_t i0 = gt - lane; i0 < nf; i0 += nt) {
-      const int64_t i = i0 + lane;
-      int32_t k0 = 0, k1 = 0;
-      T du = T(0);
-      if (i < nf) {
-        const int32_t u = cur[i];
-        atomicAnd(icur + (u >> 5), ~(1u << (u & 31)));
-        k0 = __ldg(prow + u);
-        k1 = __ldg(prow + u + 1);
-        du = ld_cg(dist + u);
-      }
-      int32_t dmax = k1 - k0;
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        const int32_t t = __shfl_xor_sync(kFullG, dmax, o);
-        dmax = t > dmax ? t : dmax;
-      }
-      for (int32_t j = 0; j < dmax; ++j) {
-        bool near_add = false, far_add = false;
-        int32_t w = 0;
-        if (k0 + j < k1) {
-          w = __ldg(pcol + k0 + j);
-          const T cand = relax_add(__ldg(pw + k0 + j), du);
-          if (cand < ld_cg(dist + w)) {
-            const T old = atomic_min_t(dist + w, cand);
-            if (cand < old) {
+    } else {
+      for (int64_t i0 = gw * kVerticesPerWarp; i0 < nf; i0 += nw * kVerticesPerWarp) {
+        const int64_t i = i0 + lane / kLanesPerVertex;
+        int32_t k = 0, k1 = 0;
+        T du = T(0);
+        if (i < nf) {
+          const int32_t u = __ldcg(cur + i);
+          if (lane % kLanesPerVertex == 0) atomicAnd(icur + (u >> 5), ~(1u << (u & 31)));
+          k = __ldg(prow + u) + lane % kLanesPerVertex;
+          k1 = __ldg(prow + u + 1);
+          du = ld_cg(dist + u);
+        }
+        while (__any_sync(kFullG, k < k1)) {
+          bool near_add = false, far_add = false;
+          int32_t w = 0;
+          if (k < k1) {
+            w = __ldg(pcol + k);
+            const T cand = relax_add(__ldg(pw + k), du);
+            // lowered by the atomic alone: one L2 round trip on the step's critical path
+            if (cand < atomic_min_t(dist + w, cand)) {
               const unsigned bit = 1u << (w & 31);
               if (cand < thr) near_add = !(atomicOr(inxt + (w >> 5), bit) & bit);
               else far_add = !(atomicOr(infar + (w >> 5), bit) & bit);
             }
           }
+          step_append(S, 0, near_add, w, nxt, &cc->cnt[r]);
+          step_append(S, 1, far_add, w, fl[fc], &cc->fcnt[fc]);
+          k += kLanesPerVertex;
         }
-        coop_append(near_add, w, nxt, &cc->cnt[r]);
-        coop_append(far_add, w, fl[fc], &cc->fcnt[fc]);
       }
     }
-    if (!coop_grid_sync(cc->bar, gridDim.x)) return;
+    step_flush(S, nxt, &cc->cnt[r], fl[fc], &cc->fcnt[fc]);
+    if (threadIdx.x == 0) {
+      S.ok = coop_leader_sync(cc->bar, (unsigned)(st + 1) * gridDim.x, limit);
+      S.len = (long long)*((volatile unsigned long long*)&cc->cnt[r]);
+      S.flen = (long long)*((volatile unsigned long long*)&cc->fcnt[fc]);
+    }
+    __syncthreads();
+    if (!S.ok) return;
     int32_t* t = cur;
     cur = nxt;
     nxt = t;
@@ -2348,7 +2319,7 @@ static int sssp_fixpoint(gg_ctx* ctx, gg_mat* A, T* d, int64_t* rounds_out) {
     void* args[] = {&P.rowptr, &P.colval, &pw, &qa, &qb, &sc.hq, &sc.q2, &sc.q3, &d, &ia, &ib,
                     &sc.visited, &ncc, &delta, &max_steps};
     GG_CUDA(cudaLaunchCooperativeKernel((const void*)k_sssp_nearfar<T>, dim3(ctx->num_sms),
-                                        dim3(kCoopThreads), args, 0, ctx->stream));
+                                        dim3(kNfThreads), args, 0, ctx->stream));
     NfCtl hn;
     GG_CUDA(cudaMemcpyAsync(&hn, ncc, sizeof(NfCtl), cudaMemcpyDeviceToHost, ctx->stream));
     GG_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -2357,36 +2328,11 @@ static int sssp_fixpoint(gg_ctx* ctx, gg_mat* A, T* d, int64_t* rounds_out) {
     if (rounds_out) *rounds_out += hn.steps_out;
     return GG_OK;
   }
-  const int32_t small_cap = coop_ok ? kCoopLo : kSmallCap;
-  const long long coop_hi = n / 8 > kCoopLo ? n / 8 : kCoopLo;
+  const int32_t small_cap = kSmallCap;
   // large CSR handles pull over a SELL-32 copy (built at the first pull round)
   const bool sell_pull = A->format == GG_FMT_CSR && n >= (1 << 16);
   while (nf > 0) {
     if (rounds > max_rounds) return set_error(GG_ERR_NOT_CONVERGED, "shortest_path did not converge");
-    if (coop_ok && nf > small_cap && nf <= coop_hi && mf * 8 <= P.nnz) {
-      k_coop_init<<<1, 1, 0, ctx->stream>>>(sc.cc, nf, barrier_polls(ctx));
-      int32_t* qa = sc.q[cur];
-      int32_t* qb = sc.q[cur ^ 1];
-      unsigned* ia = sc.fb[cur];
-      unsigned* ib = sc.fb[cur ^ 1];
-      const T* pw = static_cast<const T*>(P.w);
-      long long lo = kCoopLo / 2, hi = coop_hi, mr = max_rounds - rounds + 1;
-      void* args[] = {&P.rowptr, &P.colval, &pw, &qa, &qb, &d, &ia, &ib, &sc.cc, &lo, &hi, &mr};
-      CoopCtl* hc = reinterpret_cast<CoopCtl*>(ctx->h_flags);
-      GG_CHECK(coop_launch(ctx, (const void*)k_sssp_coop<T>, args, sc.cc, hc));
-      nf = hc->nf_out;
-      rounds += hc->level_out;
-      if (hc->which_out) cur ^= 1;
-      mf = 0;
-      if (nf > 0) {
-        GG_CUDA(cudaMemsetAsync(sc.ctr, 0, sizeof(Counters), ctx->stream));
-        k_queue_degree<<<gridsz(ctx, nf), 256, 0, ctx->stream>>>(P.rowptr, sc.q[cur], nf, sc.ctr);
-        GG_CUDA(cudaMemcpyAsync(h, sc.ctr, sizeof(Counters), cudaMemcpyDeviceToHost, ctx->stream));
-        GG_CUDA(cudaStreamSynchronize(ctx->stream));
-        mf = (int64_t)h->mf;
-      }
-      continue;
-    }
     if (nf <= small_cap && mf <= (int64_t)kSmallEdges) {
       GG_CUDA(cudaMemsetAsync(sc.ctr, 0, sizeof(Counters), ctx->stream));
       k_sssp_small<T><<<1, kSmallThreads, kSmallSmem, ctx->stream>>>(

@@ -57,3 +57,15 @@ def test_dense_core_then_paths(core, tail):
     n = core + 33 * tail
     _check(n, *_graph(n, r[keep], c[keep], np.int32, seed=tail), 1 + int(r[keep][0]))
     _check(n, *_graph(n, r[keep], c[keep], np.float32, seed=tail), n)
+
+
+@pytest.mark.parametrize("n,deg", [(65536, 3), (80001, 12), (1000003, 5)])
+def test_hub_free_persistent_steps(n, deg):
+    """Hub-free graphs (degrees of 1 to ~40): the persistent BFS / near-far kernels with
+    vertices of more than 4 edges, and steps that append more than a block stages."""
+    rng = np.random.default_rng(n)
+    r, c = rng.integers(0, n, deg * n), rng.integers(0, n, deg * n)
+    keep = r != c
+    rp, cv, nz = _graph(n, r[keep], c[keep], np.float32, seed=deg)
+    assert np.diff(rp).max() <= 64
+    _check(n, rp, cv, nz, 1 + int(r[keep][0]))
