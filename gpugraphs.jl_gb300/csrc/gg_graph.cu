@@ -836,28 +836,6 @@ struct CoopCtl {
   int which_out;    // queue holding the remaining frontier: 0 = first, 1 = second
 };
 
-// Grid barrier, the part of thread 0 of every block (between two block barriers): the
-// arrival counter bar[0] only grows and `target` is its value once every block arrived
-// (blocks x barriers so far, compared modulo 2^32), so one arrival and the polls of one
-// word are all the traffic.  The wait is bounded by `limit` polls; running out sets the
-// error word bar[2], which the waiting blocks look at every 16 polls.
-__device__ __forceinline__ bool coop_leader_sync(unsigned* bar, unsigned target,
-                                                 unsigned long long limit) {
-  __threadfence();
-  atomicAdd(bar, 1u);
-  unsigned long long polls = 0;
-  for (;;) {
-    unsigned a;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(a) : "l"(bar) : "memory");
-    if ((int)(a - target) >= 0) return true;
-    if (++polls > limit) {
-      atomicExch(bar + 2, 1u);
-      return false;
-    }
-    if ((polls & 15) == 0 && *((volatile unsigned*)(bar + 2))) return false;
-  }
-}
-
 __global__ void k_coop_init(CoopCtl* cc, long long nf0, unsigned polls) {
   cc->cnt[0] = 0;
   cc->cnt[1] = 0;
@@ -1753,7 +1731,8 @@ __global__ void __launch_bounds__(kNfThreads, 1)
   // fc + 2, which nobody touches before it is next written
   int32_t* const fl[3] = {fa, fb, fz};
   int fc = 0;
-  T thr = delta;
+  T thr = delta, width = delta;
+  bool was_change = false;
   if (threadIdx.x == 0) {
     S.n[0] = S.n[1] = 0;
     S.len = (long long)*((volatile unsigned long long*)&cc->cnt[2]);
@@ -1780,7 +1759,10 @@ __global__ void __launch_bounds__(kNfThreads, 1)
       // next distance band: far vertices below the new threshold become the next
       // frontier (counted and marked like a normal step's output), the others move to
       // the next far list
-      thr = thr > Lim<T>::max() - delta ? Lim<T>::max() : w_add(thr, delta);
+      // (an empty band doubles the next one, so gaps between the distances cost few steps)
+      width = !was_change ? delta : (width < Lim<T>::max() / 2 ? w_add(width, width) : width);
+      was_change = true;
+      thr = thr > Lim<T>::max() - width ? Lim<T>::max() : w_add(thr, width);
       for (int64_t i0 = gw * 32; i0 < nfar; i0 += nw * 32) {
         const int64_t i = i0 + lane;
         bool to_near = false, to_far = false;
@@ -1800,6 +1782,7 @@ __global__ void __launch_bounds__(kNfThreads, 1)
       }
       fc = fn;
     } else {
+      was_change = false;
       for (int64_t i0 = gw * kVerticesPerWarp; i0 < nf; i0 += nw * kVerticesPerWarp) {
         const int64_t i = i0 + lane / kLanesPerVertex;
         int32_t k = 0, k1 = 0;

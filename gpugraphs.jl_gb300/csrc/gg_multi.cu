@@ -13,8 +13,10 @@
 //    call reports GG_ERR_TIMEOUT.  The launch (with its resets) is captured once in
 //    a CUDA graph and replayed by later calls.
 //  * gg_multigraph_sssp: one single-source shortest-path search per graph in one
-//    persistent cooperative launch (frontier Bellman-Ford, atomic min, bounded grid
-//    barrier), captured in a CUDA graph the same way.
+//    persistent cooperative launch (near-far ordered relaxation, atomic min, bounded
+//    grid barrier), captured in a CUDA graph the same way.
+//  The captured launches read the result pointer from device memory (the word after the
+//  sources), so a call with another result vector replays the same CUDA graph.
 // Levels follow bfs_distances (src/algorithms/bfs.jl:1-73): edges with odd / true
 // stored values (every stored entry of a floating-point graph, i.e. its Bool
 // pattern), dist = hop level, typemax(Int32) when unreached.  Distances follow
@@ -24,6 +26,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "gg_queue.cuh"
 #include "gg_semiring.cuh"
 
 struct gg_multigraph {
@@ -40,16 +43,18 @@ struct gg_multigraph {
   // persistent BFS state
   unsigned* visited = nullptr;
   int32_t* q[2] = {nullptr, nullptr};
-  unsigned long long* ctr = nullptr;  // [3] rotating queue counters
-  unsigned* bar = nullptr;  // [8] barrier count, generation, error, levels, poll limit
-  int64_t* d_src = nullptr;           // [G] global source ids
-  int32_t* dist_bound = nullptr;      // dist pointer captured in the graph
+  unsigned long long* ctr = nullptr;  // [3] rotating queue counters, [3] of the far lists
+  unsigned* bar = nullptr;  // [8] barrier arrivals, unused, error, levels, poll limit
+  int64_t* d_src = nullptr;           // [G + 1] global source ids, address of the results
   unsigned polls_set = 0;  // poll limit last written to bar[4] (0: none yet)
   cudaGraphExec_t gexec = nullptr;
   int grid = 0;
   // persistent shortest-path state (allocated on first use)
-  unsigned* inq[2] = {nullptr, nullptr};
-  void* sssp_dist_bound = nullptr;
+  unsigned* inq[2] = {nullptr, nullptr};  // queued vertices of this / the next step
+  unsigned* infar = nullptr;              // vertices in the far list
+  int32_t* qf[2] = {nullptr, nullptr};    // far lists
+  void* sssp_mem = nullptr;               // one allocation behind the five
+  double sum_w = 0.0;                     // sum of the stored values (finite ones)
   cudaGraphExec_t sssp_gexec = nullptr;
   int nonneg = -1;  // all stored values >= 0 (and not NaN)? -1: not yet checked
 };
@@ -69,15 +74,6 @@ static int mg_set_polls(gg_ctx* ctx, gg_multigraph* M) {
 namespace gg {
 
 static const unsigned kFullM = 0xffffffffu;
-
-__device__ __forceinline__ int graph_of(const int64_t* __restrict__ off, int64_t G, int64_t v) {
-  int64_t lo = 0, hi = G - 1;  // largest g with off[g] <= v
-  while (lo < hi) {
-    const int64_t mid = (lo + hi + 1) >> 1;
-    if (off[mid] <= v) lo = mid; else hi = mid - 1;
-  }
-  return (int)lo;
-}
 
 // 8 lanes per row over all graphs' rows (global column ids: no per-row graph lookup)
 __global__ void __launch_bounds__(256)
@@ -106,39 +102,49 @@ __device__ __forceinline__ bool mg_odd(const void* nz, int tv, int64_t k) {
   return false;
 }
 
-// grid-wide barrier for a cooperative launch; the wait gives up after bar[4] polls
-// (the context's limit, gg_set_wait_limit) and records an error so that every block
-// can return.  bar: arrivals, generation, error, levels / rounds done, poll limit.
-__device__ __forceinline__ bool mg_grid_sync(unsigned* bar, unsigned nblocks) {
+// Persistent launches: kMgThreads per block; a frontier vertex gets kMgLanes lanes, so a
+// warp keeps four vertices' edge loads in flight (a warp per vertex left 13 of 32 lanes
+// idle at a mean degree of 19, waited on one vertex's chain at a time, and did one
+// atomic on the queue's length for nearly every vertex).  128 random graphs of 1000 to
+// 200000 vertices (93 M entries), Int32 shortest paths: 14.4 -> 3.3 ms, together with
+// the near-far order; bound by the chain of dependent L2 round trips of its 133 steps
+// (48 warps an SM, 24% issue, L2 29%).  4 / 8 / 16 lanes a vertex: 3.7 / 3.25 / 3.4 ms;
+// 32 / 48 / 64 warps an SM: 3.7 / 3.25 / 3.3 ms.
+static const int kMgThreads = 512;
+static const int kMgLanes = 8;
+static const int kMgVerts = 32 / kMgLanes;
+static const int kMgStep = 2;  // edges in flight per lane
+
+// end of a step: every block's appends are in, the leader waits for all blocks and
+// reads the length of the list the next step takes (bar: arrivals, unused, error,
+// levels / steps done, poll limit)
+struct MgStep {
+  long long len, flen;
+  int ok;
+};
+__device__ __forceinline__ bool mg_step_end(MgStep& S, unsigned* bar, unsigned target,
+                                            unsigned long long limit, unsigned long long* len,
+                                            unsigned long long* flen) {
   __syncthreads();
   if (threadIdx.x == 0) {
-    volatile unsigned* vgen = bar + 1;
-    volatile unsigned* verr = bar + 2;
-    const unsigned gen = *vgen;
-    const unsigned long long limit = bar[4];  // written by the host before each launch
-    __threadfence();
-    if (atomicAdd(bar, 1u) == nblocks - 1) {
-      bar[0] = 0;
-      __threadfence();
-      atomicAdd(bar + 1, 1u);
-    } else {
-      unsigned long long polls = 0;
-      while (*vgen == gen && *verr == 0) {
-        if (++polls > limit) {
-          atomicExch(bar + 2, 1u);
-          break;
-        }
-        __nanosleep(100);
-      }
-    }
-    __threadfence();
+    S.ok = coop_leader_sync(bar, target, limit);
+    S.len = (long long)*((volatile unsigned long long*)len);
+    if (flen) S.flen = (long long)*((volatile unsigned long long*)flen);
   }
   __syncthreads();
-  return *((volatile unsigned*)(bar + 2)) == 0;
+  return S.ok;
 }
 
-__global__ void k_mg_bfs_init(int64_t G, const int64_t* src, unsigned* visited, int32_t* dist,
-                              int32_t* q, unsigned long long* ctr) {
+__global__ void k_mg_fill(const int64_t* src, int64_t G, int64_t n, int32_t v) {
+  int32_t* d = reinterpret_cast<int32_t*>(src[G]);
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+       i += (int64_t)gridDim.x * blockDim.x)
+    d[i] = v;
+}
+
+__global__ void k_mg_bfs_init(int64_t G, const int64_t* src, unsigned* visited, int32_t* q,
+                              unsigned long long* ctr) {
+  int32_t* dist = reinterpret_cast<int32_t*>(src[G]);
   for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < G;
        g += (int64_t)gridDim.x * blockDim.x) {
     const int64_t v = src[g];
@@ -153,51 +159,61 @@ __global__ void k_mg_bfs_init(int64_t G, const int64_t* src, unsigned* visited, 
   }
 }
 
-// all graphs' BFS levels in one persistent launch (warp per frontier vertex)
-__global__ void __launch_bounds__(256)
-    k_mg_bfs(int64_t G, const int64_t* __restrict__ row_off, const int64_t* __restrict__ rp,
+// all graphs' BFS levels in one persistent launch
+__global__ void __launch_bounds__(kMgThreads, 3)
+    k_mg_bfs(int64_t G, const int64_t* __restrict__ src, const int64_t* __restrict__ rp,
              const int32_t* __restrict__ colval, const void* nz, int tv, int odd_only,
-             unsigned* visited, int32_t* dist, int32_t* qa, int32_t* qb,
-             unsigned long long* ctr, unsigned* bar) {
+             unsigned* visited, int32_t* qa, int32_t* qb, unsigned long long* ctr, unsigned* bar) {
+  __shared__ int32_t stage[kMgThreads / 32][WarpQueue::kCap];
+  __shared__ MgStep S;
+  int32_t* dist = reinterpret_cast<int32_t*>(src[G]);
+  const unsigned long long limit = bar[4];  // written by the host before each launch
   const int lane = threadIdx.x & 31;
-  const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  const int64_t gw = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+  const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
   int32_t* cur = qa;
   int32_t* nxt = qb;
+  long long nf = (long long)*((volatile unsigned long long*)ctr);
   for (int32_t level = 1;; ++level) {
     const int r = level % 3;
-    const int64_t nf = (int64_t)*((volatile unsigned long long*)(ctr + (r + 2) % 3));
     if (nf == 0) {
       if (blockIdx.x == 0 && threadIdx.x == 0) bar[3] = (unsigned)(level - 1);
       return;
     }
     // counter for this level's appends was zeroed two levels ago; zero the next one
     if (blockIdx.x == 0 && threadIdx.x == 0) ctr[(r + 1) % 3] = 0;
-    for (int64_t i = gw; i < nf; i += nw) {
-      const int64_t v = cur[i];
-      const int64_t k0 = rp[v], k1 = rp[v + 1];
-      for (int64_t kb = k0; kb < k1; kb += 32) {
-        const int64_t k = kb + lane;
-        bool claim = false;
-        int64_t w = 0;
-        if (k < k1 && (!odd_only || mg_odd(nz, tv, k))) {
-          w = __ldg(colval + k);
-          const unsigned bit = 1u << (w & 31);
-          if (!(__ldcg(visited + (w >> 5)) & bit))
-            claim = !(atomicOr(visited + (w >> 5), bit) & bit);
-          if (claim) dist[w] = level;
+    WarpQueue wq(stage[threadIdx.x >> 5], nxt, ctr + r);
+    for (int64_t i0 = gw * kMgVerts; i0 < nf; i0 += nw * kMgVerts) {
+      const int64_t i = i0 + lane / kMgLanes;
+      int64_t k = 0, k1 = 0;
+      if (i < nf) {
+        const int64_t v = __ldcg(cur + i);
+        k = rp[v] + lane % kMgLanes;
+        k1 = rp[v + 1];
+      }
+      while (__any_sync(kFullM, k < k1)) {
+        int32_t w[kMgStep];
+        unsigned seen[kMgStep];
+#pragma unroll
+        for (int t = 0; t < kMgStep; ++t) {
+          const int64_t kk = k + t * kMgLanes;
+          w[t] = kk < k1 && (!odd_only || mg_odd(nz, tv, kk)) ? __ldg(colval + kk) : -1;
         }
-        const unsigned b = __ballot_sync(kFullM, claim);
-        if (b) {
-          const int leader = __ffs(b) - 1;
-          unsigned long long pos = 0;
-          if (lane == leader) pos = atomicAdd(ctr + r, (unsigned long long)__popc(b));
-          pos = __shfl_sync(kFullM, pos, leader);
-          if (claim) nxt[pos + __popc(b & ((1u << lane) - 1u))] = (int32_t)w;
+#pragma unroll
+        for (int t = 0; t < kMgStep; ++t) seen[t] = w[t] >= 0 ? __ldcg(visited + (w[t] >> 5)) : ~0u;
+#pragma unroll
+        for (int t = 0; t < kMgStep; ++t) {
+          const unsigned bit = 1u << (w[t] & 31);
+          const bool claim = !(seen[t] & bit) && !(atomicOr(visited + (w[t] >> 5), bit) & bit);
+          if (claim) dist[w[t]] = level;
+          wq.push(claim, w[t]);
         }
+        k += kMgStep * kMgLanes;
       }
     }
-    if (!mg_grid_sync(bar, gridDim.x)) return;
+    wq.flush();
+    if (!mg_step_end(S, bar, (unsigned)level * gridDim.x, limit, ctr + r, nullptr)) return;
+    nf = S.len;
     int32_t* t = cur;
     cur = nxt;
     nxt = t;
@@ -231,15 +247,17 @@ __device__ __forceinline__ T mg_weight(const void* nz, int tv, int64_t k) {
 }
 
 template <typename T>
-__global__ void k_mg_fill_t(T* d, int64_t n, T v) {
+__global__ void k_mg_fill_t(const int64_t* src, int64_t G, int64_t n, T v) {
+  T* d = reinterpret_cast<T*>(src[G]);
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (int64_t)gridDim.x * blockDim.x)
     d[i] = v;
 }
 
 template <typename T>
-__global__ void k_mg_sssp_seed(int64_t G, const int64_t* src, T* dist, unsigned* inq, int32_t* q,
+__global__ void k_mg_sssp_seed(int64_t G, const int64_t* src, unsigned* inq, int32_t* q,
                                unsigned long long* ctr) {
+  T* dist = reinterpret_cast<T*>(src[G]);
   for (int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; g < G;
        g += (int64_t)gridDim.x * blockDim.x) {
     const int64_t v = src[g];
@@ -249,69 +267,133 @@ __global__ void k_mg_sssp_seed(int64_t G, const int64_t* src, T* dist, unsigned*
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     ctr[0] = (unsigned long long)G;
-    ctr[1] = 0;
-    ctr[2] = 0;
+    for (int i = 1; i < 6; ++i) ctr[i] = 0;
   }
 }
 
-// all graphs' Bellman-Ford rounds in one persistent launch (warp per frontier
-// vertex, push over its row); inq_cur / inq_next mark queued vertices
+// All graphs' shortest paths in one persistent launch, near-far ordered over all graphs
+// together: vertices below the distance threshold thr are relaxed, improved vertices at
+// or above it wait in a far list, and when no near vertex is left thr grows by delta and
+// the far list is split.  The fixpoint is the same (every improved vertex is relaxed
+// again, and distances only fall), but a vertex is relaxed little more than once instead
+// of once per improvement.  icur / inxt mark queued vertices, infar the waiting ones.
+// Band b appends to far list b mod 2 counted in fctr[b mod 3]; every step zeroes the
+// counter that the band after next will use.
 template <typename T>
-__global__ void __launch_bounds__(256)
-    k_mg_sssp(int64_t G, const int64_t* __restrict__ row_off, const int64_t* __restrict__ rp,
-              const int32_t* __restrict__ colval, const void* nz, int tv, T* dist, unsigned* inq_a,
-              unsigned* inq_b, int32_t* qa, int32_t* qb, unsigned long long* ctr, unsigned* bar,
-              int64_t max_rounds) {
-  const int lane = threadIdx.x & 31;
-  const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+__global__ void __launch_bounds__(kMgThreads, 3)
+    k_mg_sssp(int64_t G, const int64_t* __restrict__ src, const int64_t* __restrict__ rp,
+              const int32_t* __restrict__ colval, const void* nz, int tv, unsigned* inq_a,
+              unsigned* inq_b, unsigned* infar, int32_t* qa, int32_t* qb, int32_t* fa, int32_t* fb,
+              unsigned long long* ctr, unsigned* bar, T delta, int64_t max_steps) {
+  __shared__ int32_t stage[2][kMgThreads / 32][WarpQueue::kCap];
+  __shared__ MgStep S;
+  T* dist = reinterpret_cast<T*>(src[G]);
+  unsigned long long* fctr = ctr + 3;
+  const unsigned long long limit = bar[4];  // written by the host before each launch
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t gw = (int64_t)warp * gridDim.x + blockIdx.x;
+  const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
   int32_t* cur = qa;
   int32_t* nxt = qb;
   unsigned* icur = inq_a;
   unsigned* inxt = inq_b;
-  for (int64_t round = 1;; ++round) {
-    const int r = (int)(round % 3);
-    const int64_t nf = (int64_t)*((volatile unsigned long long*)(ctr + (r + 2) % 3));
-    if (nf == 0 || round > max_rounds) {
+  T thr = delta, width = delta;
+  int64_t band = 0;
+  bool was_change = false;
+  long long nf = (long long)*((volatile unsigned long long*)ctr), nfar = 0;
+  for (int64_t step = 1;; ++step) {
+    const int r = (int)(step % 3);
+    if ((nf == 0 && nfar == 0) || step > max_steps) {
       if (blockIdx.x == 0 && threadIdx.x == 0) {
-        bar[3] = (unsigned)(round - 1);
-        if (nf != 0) atomicExch(bar + 2, 2u);  // still improving after max_rounds
+        bar[3] = (unsigned)(step - 1);
+        if (step > max_steps) atomicExch(bar + 2, 2u);  // still improving
       }
       return;
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) ctr[(r + 1) % 3] = 0;
-    for (int64_t i = gw; i < nf; i += nw) {
-      const int64_t u = cur[i];
-      if (lane == 0) atomicAnd(icur + (u >> 5), ~(1u << (u & 31)));
-      const T du = __ldcg(dist + u);
-      const int64_t k0 = rp[u], k1 = rp[u + 1];
-      for (int64_t kb = k0; kb < k1; kb += 32) {
-        const int64_t k = kb + lane;
-        bool add = false;
-        int64_t v = 0;
-        if (k < k1) {
-          v = __ldg(colval + k);
-          const T w = mg_weight<T>(nz, tv, k);
-          const T cand = (w == Lim<T>::max() || du == Lim<T>::max()) ? Lim<T>::max() : w_add(w, du);
-          if (cand < __ldcg(dist + v)) {
-            const T old = mg_atomic_min<T>(dist + v, cand);
-            if (cand < old) {
-              const unsigned bit = 1u << (v & 31);
-              add = !(atomicOr(inxt + (v >> 5), bit) & bit);
-            }
+    int fc = (int)(band % 3);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      ctr[(r + 1) % 3] = 0;
+      fctr[(fc + 2) % 3] = 0;
+    }
+    WarpQueue wn(stage[0][warp], nxt, ctr + r);
+    if (nf == 0) {
+      const int32_t* from = band % 2 ? fb : fa;
+      ++band;
+      fc = (int)(band % 3);
+      WarpQueue wf(stage[1][warp], band % 2 ? fb : fa, fctr + fc);
+      // an empty band doubles the next one: gaps between the distances (or a width below
+      // a large threshold's rounding) cost a logarithmic number of steps
+      width = !was_change ? delta : (width < Lim<T>::max() / 2 ? w_add(width, width) : width);
+      was_change = true;
+      thr = thr > Lim<T>::max() - width ? Lim<T>::max() : w_add(thr, width);
+      for (int64_t i0 = gw * 32; i0 < nfar; i0 += nw * 32) {
+        const int64_t i = i0 + lane;
+        bool to_near = false, to_far = false;
+        int32_t v = 0;
+        if (i < nfar) {
+          v = __ldcg(from + i);
+          if (__ldcg(dist + v) < thr) {
+            const unsigned bit = 1u << (v & 31);
+            atomicAnd(infar + (v >> 5), ~bit);
+            to_near = !(atomicOr(inxt + (v >> 5), bit) & bit);
+          } else {
+            to_far = true;
           }
         }
-        const unsigned b = __ballot_sync(kFullM, add);
-        if (b) {
-          const int leader = __ffs(b) - 1;
-          unsigned long long pos = 0;
-          if (lane == leader) pos = atomicAdd(ctr + r, (unsigned long long)__popc(b));
-          pos = __shfl_sync(kFullM, pos, leader);
-          if (add) nxt[pos + __popc(b & ((1u << lane) - 1u))] = (int32_t)v;
+        wn.push(to_near, v);
+        wf.push(to_far, v);
+      }
+      wf.flush();
+    } else {
+      was_change = false;
+      WarpQueue wf(stage[1][warp], band % 2 ? fb : fa, fctr + fc);
+      for (int64_t i0 = gw * kMgVerts; i0 < nf; i0 += nw * kMgVerts) {
+        const int64_t i = i0 + lane / kMgLanes;
+        int64_t k = 0, k1 = 0;
+        T du = T(0);
+        if (i < nf) {
+          const int64_t u = __ldcg(cur + i);
+          if (lane % kMgLanes == 0) atomicAnd(icur + (u >> 5), ~(1u << (u & 31)));
+          k = rp[u] + lane % kMgLanes;
+          k1 = rp[u + 1];
+          du = __ldcg(dist + u);
+        }
+        while (__any_sync(kFullM, k < k1)) {
+          int32_t v[kMgStep];
+          T cand[kMgStep], dv[kMgStep];
+#pragma unroll
+          for (int t = 0; t < kMgStep; ++t) {
+            const int64_t kk = k + t * kMgLanes;
+            v[t] = kk < k1 ? __ldg(colval + kk) : -1;
+            const T w = kk < k1 ? mg_weight<T>(nz, tv, kk) : Lim<T>::max();
+            cand[t] = (w == Lim<T>::max() || du == Lim<T>::max()) ? Lim<T>::max() : w_add(w, du);
+          }
+#pragma unroll
+          for (int t = 0; t < kMgStep; ++t) dv[t] = v[t] >= 0 ? __ldcg(dist + v[t]) : Lim<T>::min();
+          unsigned near_add = 0, far_add = 0;  // bit t
+#pragma unroll
+          for (int t = 0; t < kMgStep; ++t)
+            if (cand[t] < dv[t] && cand[t] < mg_atomic_min<T>(dist + v[t], cand[t])) {
+              const unsigned bit = 1u << (v[t] & 31);
+              if (cand[t] < thr) near_add |= !(atomicOr(inxt + (v[t] >> 5), bit) & bit) ? 1u << t : 0u;
+              else far_add |= !(atomicOr(infar + (v[t] >> 5), bit) & bit) ? 1u << t : 0u;
+            }
+          if (__any_sync(kFullM, near_add | far_add)) {
+#pragma unroll
+            for (int t = 0; t < kMgStep; ++t) {
+              wn.push((near_add >> t) & 1u, v[t]);
+              wf.push((far_add >> t) & 1u, v[t]);
+            }
+          }
+          k += kMgStep * kMgLanes;
         }
       }
+      wf.flush();
     }
-    if (!mg_grid_sync(bar, gridDim.x)) return;
+    wn.flush();
+    if (!mg_step_end(S, bar, (unsigned)step * gridDim.x, limit, ctr + r, fctr + fc)) return;
+    nf = S.len;
+    nfar = S.flen;
     int32_t* t = cur;
     cur = nxt;
     nxt = t;
@@ -321,25 +403,20 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-__global__ void k_mg_nonneg(const void* nz, int tv, int64_t nnz, unsigned* bad) {
+// stored values: any negative or NaN one (*bad), and the sum of the finite ones
+__global__ void k_mg_values(const void* nz, int tv, int64_t nnz, unsigned* bad, double* sum) {
   unsigned b = 0;
+  double s = 0.0;
   for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < nnz;
        k += (int64_t)gridDim.x * blockDim.x) {
-    switch (tv) {
-      case GG_INT32: b |= static_cast<const int32_t*>(nz)[k] < 0; break;
-      case GG_INT64: b |= static_cast<const int64_t*>(nz)[k] < 0; break;
-      case GG_FLOAT32: { const float w = static_cast<const float*>(nz)[k]; b |= !(w >= 0.0f); break; }
-      case GG_FLOAT64: { const double w = static_cast<const double*>(nz)[k]; b |= !(w >= 0.0); break; }
-      default: break;
-    }
+    const double w = mg_weight<double>(nz, tv, k);
+    b |= !(w >= 0.0);
+    if (w <= 1.7976931348623157e308) s += w;
   }
   if (__syncthreads_or(b) && threadIdx.x == 0) atomicOr(bad, 1u);
-}
-
-__global__ void k_mg_fill(int32_t* d, int64_t n, int32_t v) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x)
-    d[i] = v;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(kFullM, s, o);
+  if ((threadIdx.x & 31) == 0) atomicAdd(sum, s);
 }
 
 // global 0-based column ids: colval_g (1-based within graph g) + row_off[g] - 1
@@ -366,6 +443,23 @@ static int mg_grid(int num_sms, int64_t work) {
 }  // namespace gg
 
 using namespace gg;
+
+// checks the sources and puts their global ids, then the address of the results, into
+// the words the captured launches read
+static int mg_upload_sources(gg_ctx* ctx, gg_multigraph* M, const int64_t* sources, void* dist) {
+  std::vector<int64_t> gsrc(M->ngraphs + 1);
+  for (int64_t g = 0; g < M->ngraphs; ++g) {
+    const int64_t n = M->h_row_off[g + 1] - M->h_row_off[g];
+    if (sources[g] < 1 || sources[g] > n)
+      return set_error(GG_ERR_BOUNDS, "source %lld of graph %lld out of 1:%lld", (long long)sources[g],
+                       (long long)g, (long long)n);
+    gsrc[g] = M->h_row_off[g] + sources[g] - 1;
+  }
+  gsrc[M->ngraphs] = (int64_t)(uintptr_t)dist;
+  GG_CUDA(cudaMemcpyAsync(M->d_src, gsrc.data(), gsrc.size() * sizeof(int64_t),
+                          cudaMemcpyHostToDevice, ctx->stream));
+  return GG_OK;
+}
 
 extern "C" {
 
@@ -419,10 +513,10 @@ int gg_multigraph_create(gg_ctx* ctx, const gg_mat* const* graphs, int64_t ngrap
   if (e == cudaSuccess) e = cudaMalloc((void**)&M->visited, nw * sizeof(unsigned));
   if (e == cudaSuccess) e = cudaMalloc((void**)&M->q[0], (M->total_n + 1) * sizeof(int32_t));
   if (e == cudaSuccess) e = cudaMalloc((void**)&M->q[1], (M->total_n + 1) * sizeof(int32_t));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&M->ctr, 4 * sizeof(unsigned long long));
+  if (e == cudaSuccess) e = cudaMalloc((void**)&M->ctr, 8 * sizeof(unsigned long long));
   if (e == cudaSuccess) e = cudaMalloc((void**)&M->bar, 8 * sizeof(unsigned));
   if (e == cudaSuccess) e = cudaMemset(M->bar, 0, 8 * sizeof(unsigned));
-  if (e == cudaSuccess) e = cudaMalloc((void**)&M->d_src, ngraphs * sizeof(int64_t));
+  if (e == cudaSuccess) e = cudaMalloc((void**)&M->d_src, (ngraphs + 1) * sizeof(int64_t));
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
   if (e != cudaSuccess) {
     gg_multigraph_destroy(M);
@@ -441,8 +535,7 @@ int gg_multigraph_destroy(gg_multigraph* M) {
   cudaSetDevice(M->device);
   if (M->gexec) cudaGraphExecDestroy(M->gexec);
   if (M->sssp_gexec) cudaGraphExecDestroy(M->sssp_gexec);
-  cudaFree(M->inq[0]);
-  cudaFree(M->inq[1]);
+  cudaFree(M->sssp_mem);
   cudaFree(M->row_off);
   cudaFree(M->rp64);
   cudaFree(M->colval);
@@ -482,23 +575,10 @@ int gg_multigraph_bfs(gg_ctx* ctx, gg_multigraph* M, const int64_t* sources, int
                       int64_t* levels_out) {
   if (!ctx || !M || !sources || !dist) return set_error(GG_ERR_ARGUMENT, "NULL argument");
   GG_CUDA(cudaSetDevice(ctx->device));
-  std::vector<int64_t> gsrc(M->ngraphs);
-  for (int64_t g = 0; g < M->ngraphs; ++g) {
-    const int64_t n = M->h_row_off[g + 1] - M->h_row_off[g];
-    if (sources[g] < 1 || sources[g] > n)
-      return set_error(GG_ERR_BOUNDS, "source %lld of graph %lld out of 1:%lld", (long long)sources[g],
-                       (long long)g, (long long)n);
-    gsrc[g] = M->h_row_off[g] + sources[g] - 1;
-  }
-  GG_CUDA(cudaMemcpyAsync(M->d_src, gsrc.data(), M->ngraphs * sizeof(int64_t),
-                          cudaMemcpyHostToDevice, ctx->stream));
-  if (!M->gexec || M->dist_bound != dist) {
-    if (M->gexec) {
-      cudaGraphExecDestroy(M->gexec);
-      M->gexec = nullptr;
-    }
+  GG_CHECK(mg_upload_sources(ctx, M, sources, dist));
+  if (!M->gexec) {
     int per_sm = 0;
-    GG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_mg_bfs, 256, 0));
+    GG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_mg_bfs, kMgThreads, 0));
     if (per_sm < 1) return set_error(GG_ERR_CUDA, "k_mg_bfs cannot be resident");
     M->grid = ctx->num_sms * per_sm;  // every block resident: the cooperative barrier is safe
     cudaStream_t cs = nullptr;
@@ -511,16 +591,16 @@ int gg_multigraph_bfs(gg_ctx* ctx, gg_multigraph* M, const int64_t* sources, int
     if (e == cudaSuccess) e = cudaMemsetAsync(M->visited, 0, nw * sizeof(unsigned), cs);
     if (e == cudaSuccess) e = cudaMemsetAsync(M->bar, 0, 4 * sizeof(unsigned), cs);
     if (e == cudaSuccess) {
-      k_mg_fill<<<mg_grid(ctx->num_sms, M->total_n), 256, 0, cs>>>(dist, M->total_n, INT32_MAX);
-      k_mg_bfs_init<<<mg_grid(ctx->num_sms, G), 256, 0, cs>>>(G, M->d_src, M->visited, dist, M->q[0],
-                                                              M->ctr);
+      k_mg_fill<<<mg_grid(ctx->num_sms, M->total_n), 256, 0, cs>>>(M->d_src, G, M->total_n, INT32_MAX);
+      k_mg_bfs_init<<<mg_grid(ctx->num_sms, G), 256, 0, cs>>>(G, M->d_src, M->visited, M->q[0], M->ctr);
       e = cudaGetLastError();
     }
     if (e == cudaSuccess) {
       int tv = M->dtype;
-      void* args[] = {&G, &M->row_off, &M->rp64, &M->colval, &M->nzval, &tv,
-                      (void*)&odd_only, &M->visited, &dist, &M->q[0], &M->q[1], &M->ctr, &M->bar};
-      e = cudaLaunchCooperativeKernel((const void*)k_mg_bfs, dim3(M->grid), dim3(256), args, 0, cs);
+      void* args[] = {&G, &M->d_src, &M->rp64, &M->colval, &M->nzval, &tv, (void*)&odd_only,
+                      &M->visited, &M->q[0], &M->q[1], &M->ctr, &M->bar};
+      e = cudaLaunchCooperativeKernel((const void*)k_mg_bfs, dim3(M->grid), dim3(kMgThreads), args, 0,
+                                      cs);
     }
     cudaError_t e2 = cudaStreamEndCapture(cs, &graph);
     if (e == cudaSuccess) e = e2;
@@ -528,7 +608,6 @@ int gg_multigraph_bfs(gg_ctx* ctx, gg_multigraph* M, const int64_t* sources, int
     if (graph) cudaGraphDestroy(graph);
     cudaStreamDestroy(cs);
     if (e != cudaSuccess) return cuda_error(e, "multigraph BFS graph capture");
-    M->dist_bound = dist;
   }
   GG_CHECK(mg_set_polls(ctx, M));
   GG_CUDA(cudaGraphLaunch(M->gexec, ctx->stream));
@@ -542,33 +621,53 @@ int gg_multigraph_bfs(gg_ctx* ctx, gg_multigraph* M, const int64_t* sources, int
 
 }  // extern "C"
 
+// Near-far band: this multiple of the mean weight over the mean degree (the distances of
+// random graphs go as that), and at least 1 for whole-number weights.  Narrow bands cost
+// steps, wide ones repeat relaxations: 2 / 8 / 16 / 32 / 64 gave 476 / 201 / 133 / 91 / -
+// steps and 5.0 / 3.5 / 3.25 / 4.1 / 4.6 ms on the 128 graphs above.  Fewer entries than
+// kMgBandNnz run as plain rounds (one band): repeated relaxations of a small frontier
+// fit the same latency-bound step.  Bands / plain rounds, ms: 0.30 M entries 0.43 / 0.22,
+// 3 M 0.71 / 0.42, 8 M 1.22 / 0.99, 15 M 1.15 / 0.86, 93 M 3.25 / 4.40.
+static const double kMgBand = 16.0;
+static const int64_t kMgBandNnz = 1 << 25;
+
 template <typename T>
-static int mg_sssp_capture(gg_ctx* ctx, gg_multigraph* M, T* dist) {
+static int mg_sssp_capture(gg_ctx* ctx, gg_multigraph* M) {
   int per_sm = 0;
-  GG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_mg_sssp<T>, 256, 0));
+  GG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_mg_sssp<T>, kMgThreads, 0));
   if (per_sm < 1) return set_error(GG_ERR_CUDA, "k_mg_sssp cannot be resident");
   const int grid = ctx->num_sms * per_sm;  // every block resident: the barrier is safe
+  const double nnz = M->total_nnz > 0 ? (double)M->total_nnz : 1.0;
+  double dd = kMgBand * (M->sum_w / nnz) / (nnz / (double)(M->total_n > 0 ? M->total_n : 1));
+  if (!(dd > 0.0)) dd = 1.0;
+  if (dd > (double)Lim<T>::max() / 4) dd = (double)Lim<T>::max() / 4;
+  T delta = static_cast<T>(dd);
+  if (!(delta > T(0))) delta = T(1);
+  if (M->total_nnz < kMgBandNnz) delta = Lim<T>::max();
   cudaStream_t cs = nullptr;
   GG_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));
   cudaGraph_t graph = nullptr;
   cudaError_t e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeThreadLocal);
   const int64_t nw = M->total_n / 32 + 2;
   int64_t G = M->ngraphs;
-  int64_t max_rounds = M->total_n + 1;
+  int64_t max_steps = 8 * M->total_n + 1024;
   if (e == cudaSuccess) e = cudaMemsetAsync(M->inq[0], 0, nw * sizeof(unsigned), cs);
   if (e == cudaSuccess) e = cudaMemsetAsync(M->inq[1], 0, nw * sizeof(unsigned), cs);
+  if (e == cudaSuccess) e = cudaMemsetAsync(M->infar, 0, nw * sizeof(unsigned), cs);
   if (e == cudaSuccess) e = cudaMemsetAsync(M->bar, 0, 4 * sizeof(unsigned), cs);
   if (e == cudaSuccess) {
-    k_mg_fill_t<T><<<mg_grid(ctx->num_sms, M->total_n), 256, 0, cs>>>(dist, M->total_n, Lim<T>::max());
-    k_mg_sssp_seed<T><<<mg_grid(ctx->num_sms, G), 256, 0, cs>>>(G, M->d_src, dist, M->inq[0],
-                                                                M->q[0], M->ctr);
+    k_mg_fill_t<T><<<mg_grid(ctx->num_sms, M->total_n), 256, 0, cs>>>(M->d_src, G, M->total_n,
+                                                                      Lim<T>::max());
+    k_mg_sssp_seed<T><<<mg_grid(ctx->num_sms, G), 256, 0, cs>>>(G, M->d_src, M->inq[0], M->q[0], M->ctr);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) {
     int tv = M->dtype;
-    void* args[] = {&G, &M->row_off, &M->rp64, &M->colval, &M->nzval, &tv, &dist, &M->inq[0],
-                    &M->inq[1], &M->q[0], &M->q[1], &M->ctr, &M->bar, &max_rounds};
-    e = cudaLaunchCooperativeKernel((const void*)k_mg_sssp<T>, dim3(grid), dim3(256), args, 0, cs);
+    void* args[] = {&G, &M->d_src, &M->rp64, &M->colval, &M->nzval, &tv, &M->inq[0], &M->inq[1],
+                    &M->infar, &M->q[0], &M->q[1], &M->qf[0], &M->qf[1], &M->ctr, &M->bar, &delta,
+                    &max_steps};
+    e = cudaLaunchCooperativeKernel((const void*)k_mg_sssp<T>, dim3(grid), dim3(kMgThreads), args, 0,
+                                    cs);
   }
   cudaError_t e2 = cudaStreamEndCapture(cs, &graph);
   if (e == cudaSuccess) e = e2;
@@ -576,7 +675,6 @@ static int mg_sssp_capture(gg_ctx* ctx, gg_multigraph* M, T* dist) {
   if (graph) cudaGraphDestroy(graph);
   cudaStreamDestroy(cs);
   if (e != cudaSuccess) return cuda_error(e, "multigraph shortest-path graph capture");
-  M->sssp_dist_bound = dist;
   return GG_OK;
 }
 
@@ -590,42 +688,38 @@ int gg_multigraph_sssp(gg_ctx* ctx, gg_multigraph* M, const int64_t* sources, vo
     return set_error(GG_ERR_TYPE, "dist element type must be Int32 for Bool graphs, else the graphs' type");
   GG_CUDA(cudaSetDevice(ctx->device));
   if (M->nonneg < 0) {
-    GG_CUDA(cudaMemsetAsync(ctx->d_flags, 0, sizeof(unsigned), ctx->stream));
-    k_mg_nonneg<<<mg_grid(ctx->num_sms, M->total_nnz), 256, 0, ctx->stream>>>(
-        M->nzval, M->dtype, M->total_nnz, ctx->d_flags);
+    double* dsum = reinterpret_cast<double*>(ctx->d_flags + 2);
+    GG_CUDA(cudaMemsetAsync(ctx->d_flags, 0, 4 * sizeof(unsigned), ctx->stream));
+    k_mg_values<<<mg_grid(ctx->num_sms, M->total_nnz), 256, 0, ctx->stream>>>(
+        M->nzval, M->dtype, M->total_nnz, ctx->d_flags, dsum);
     GG_CUDA(cudaGetLastError());
-    GG_CUDA(cudaMemcpyAsync(ctx->h_flags, ctx->d_flags, sizeof(unsigned), cudaMemcpyDeviceToHost,
+    GG_CUDA(cudaMemcpyAsync(ctx->h_flags, ctx->d_flags, 4 * sizeof(unsigned), cudaMemcpyDeviceToHost,
                             ctx->stream));
     GG_CUDA(cudaStreamSynchronize(ctx->stream));
     M->nonneg = ctx->h_flags[0] ? 0 : 1;
+    M->sum_w = *reinterpret_cast<const double*>(ctx->h_flags + 2);
   }
   if (!M->nonneg)
     return set_error(GG_ERR_UNSUPPORTED, "multigraph shortest paths need non-negative weights");
-  std::vector<int64_t> gsrc(M->ngraphs);
-  for (int64_t g = 0; g < M->ngraphs; ++g) {
-    const int64_t n = M->h_row_off[g + 1] - M->h_row_off[g];
-    if (sources[g] < 1 || sources[g] > n)
-      return set_error(GG_ERR_BOUNDS, "source %lld of graph %lld out of 1:%lld", (long long)sources[g],
-                       (long long)g, (long long)n);
-    gsrc[g] = M->h_row_off[g] + sources[g] - 1;
-  }
   const int64_t nw = M->total_n / 32 + 2;
-  if (!M->inq[0]) {
-    GG_CUDA(cudaMalloc((void**)&M->inq[0], nw * sizeof(unsigned)));
-    GG_CUDA(cudaMalloc((void**)&M->inq[1], nw * sizeof(unsigned)));
+  if (!M->sssp_mem) {
+    const size_t bm = ((size_t)nw * sizeof(unsigned) + 255) & ~(size_t)255;
+    const size_t qb = ((size_t)(M->total_n + 1) * sizeof(int32_t) + 255) & ~(size_t)255;
+    GG_CUDA(cudaMalloc(&M->sssp_mem, 3 * bm + 2 * qb));
+    char* p = static_cast<char*>(M->sssp_mem);
+    M->inq[0] = (unsigned*)p;
+    M->inq[1] = (unsigned*)(p + bm);
+    M->infar = (unsigned*)(p + 2 * bm);
+    M->qf[0] = (int32_t*)(p + 3 * bm);
+    M->qf[1] = (int32_t*)(p + 3 * bm + qb);
   }
-  GG_CUDA(cudaMemcpyAsync(M->d_src, gsrc.data(), M->ngraphs * sizeof(int64_t),
-                          cudaMemcpyHostToDevice, ctx->stream));
-  if (!M->sssp_gexec || M->sssp_dist_bound != dist) {
-    if (M->sssp_gexec) {
-      cudaGraphExecDestroy(M->sssp_gexec);
-      M->sssp_gexec = nullptr;
-    }
+  GG_CHECK(mg_upload_sources(ctx, M, sources, dist));
+  if (!M->sssp_gexec) {
     switch (dist_dtype) {
-      case GG_INT32: GG_CHECK(mg_sssp_capture<int32_t>(ctx, M, static_cast<int32_t*>(dist))); break;
-      case GG_INT64: GG_CHECK(mg_sssp_capture<int64_t>(ctx, M, static_cast<int64_t*>(dist))); break;
-      case GG_FLOAT32: GG_CHECK(mg_sssp_capture<float>(ctx, M, static_cast<float*>(dist))); break;
-      default: GG_CHECK(mg_sssp_capture<double>(ctx, M, static_cast<double*>(dist))); break;
+      case GG_INT32: GG_CHECK(mg_sssp_capture<int32_t>(ctx, M)); break;
+      case GG_INT64: GG_CHECK(mg_sssp_capture<int64_t>(ctx, M)); break;
+      case GG_FLOAT32: GG_CHECK(mg_sssp_capture<float>(ctx, M)); break;
+      default: GG_CHECK(mg_sssp_capture<double>(ctx, M)); break;
     }
   }
   GG_CHECK(mg_set_polls(ctx, M));

@@ -1,4 +1,4 @@
-// gg_queue.cuh -- queue appends of the searches.
+// gg_queue.cuh -- queue appends of the searches, grid barrier of the persistent ones.
 //
 // A frontier queue has one length counter, and atomics on one address pass L2 one after
 // another (about 0.5 ns each on GB300).  One atomic per warp instruction that appends
@@ -52,6 +52,28 @@ __device__ __forceinline__ void warp_add(unsigned long long v, unsigned long lon
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   if ((threadIdx.x & 31) == 0 && v) atomicAdd(out, v);
+}
+
+// Grid barrier, the part of thread 0 of every block (between two block barriers): the
+// arrival counter bar[0] only grows and `target` is its value once every block arrived
+// (blocks x barriers so far, compared modulo 2^32), so one arrival and the polls of one
+// word are all the traffic.  The wait is bounded by `limit` polls; running out sets the
+// error word bar[2], which the waiting blocks look at every 16 polls.
+__device__ __forceinline__ bool coop_leader_sync(unsigned* bar, unsigned target,
+                                                 unsigned long long limit) {
+  __threadfence();
+  atomicAdd(bar, 1u);
+  unsigned long long polls = 0;
+  for (;;) {
+    unsigned a;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(a) : "l"(bar) : "memory");
+    if ((int)(a - target) >= 0) return true;
+    if (++polls > limit) {
+      atomicExch(bar + 2, 1u);
+      return false;
+    }
+    if ((polls & 15) == 0 && *((volatile unsigned*)(bar + 2))) return false;
+  }
 }
 
 }  // namespace gg

@@ -69,3 +69,60 @@ def test_hub_free_persistent_steps(n, deg):
     rp, cv, nz = _graph(n, r[keep], c[keep], np.float32, seed=deg)
     assert np.diff(rp).max() <= 64
     _check(n, rp, cv, nz, 1 + int(r[keep][0]))
+
+
+@pytest.mark.parametrize("dtype", [np.bool_, np.int32, np.int64, np.float32, np.float64])
+@pytest.mark.parametrize("sizes", [(2, 33, 700, 1500), (1, 1, 40000)])
+def test_many_graphs_uneven_weights(dtype, sizes):
+    """Several graphs at once: weights spread over nine decades, a vertex of 600 edges,
+    isolated vertices, and result vectors that change between calls."""
+    from gpugraphs.multigraph import MultiGraph
+    gs, src, ref = [], [], []
+    for i, n in enumerate(sizes):
+        rng = np.random.default_rng(n + i)
+        r, c = rng.integers(0, n, 3 * n), rng.integers(0, n, 3 * n)
+        r, c = np.concatenate([r, np.zeros(min(n, 600), np.int64)]), np.concatenate([c, np.arange(min(n, 600))])
+        r, c = r[r != c], c[r != c]
+        lo, hi = np.minimum(r, c), np.maximum(r, c)
+        key = np.unique(lo * n + hi) if len(lo) else np.zeros(0, np.int64)
+        w = np.floor(10.0 ** rng.uniform(0, 6 if dtype == np.int32 else 9, len(key)))
+        lo, hi = key // n, key % n
+        A = sp.coo_matrix((np.concatenate([w, w]), (np.concatenate([lo, hi]), np.concatenate([hi, lo]))),
+                          shape=(n, n)).tocsr()
+        rp, cv, nz = csr_from_scipy(A.astype(dtype))
+        gs.append(G.SparseGPUMatrixCSR(n, n, rp, cv, nz))
+        src.append(n // 2 + 1)
+        ref.append(G.shortest_path(gs[-1], n // 2 + 1).cpu().numpy())
+        if dtype in (np.bool_, np.int32, np.float32):
+            d = O.sssp_dijkstra(n, rp, cv, nz, n // 2 + 1, symmetric=True)
+            assert (ref[-1] == d).all()
+    mg = MultiGraph(gs)
+    keep = []
+    for _ in range(3):
+        keep.append(mg.sssp(src))
+        lev = mg.bfs(src) if dtype != np.float64 else None
+        keep.append(lev)
+    for out in keep[::2]:
+        for got, want in zip(mg.split(out), ref):
+            assert (got.cpu().numpy() == want).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.int32, torch.float32])
+def test_many_graphs_in_bands(dtype):
+    """More than 2^25 entries: near-far bands over all graphs, with weights of nine decades
+    in one of them (empty bands, a band below the threshold's rounding)."""
+    from gpugraphs import generators as gen
+    from gpugraphs.multigraph import MultiGraph
+    gs = []
+    for i, n in enumerate((1100000, 3001, 50000)):
+        A = gen.erdos_renyi(n, 16, seed=i + 3, symmetric=True, wkind=gen.W_INT_1_255)
+        w = A.nzval.to(torch.float64)
+        if i == 1:
+            w = torch.floor(w ** (2.0 if dtype == torch.int32 else 3.7))
+        gs.append(G.SparseGPUMatrixCSR(n, n, A.rowptr, A.colval, w.to(dtype)))
+    assert sum(g.nnz() for g in gs) > 1 << 25
+    src = [5, 3001, 7]
+    mg = MultiGraph(gs)
+    for _ in range(2):
+        for got, A, s in zip(mg.split(mg.sssp(src)), gs, src):
+            assert torch.equal(got, G.shortest_path(A, s))
