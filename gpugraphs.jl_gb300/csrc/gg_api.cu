@@ -9,7 +9,6 @@
 #include <string.h>
 
 #include <algorithm>
-#include <numeric>
 #include <vector>
 
 #include "gg_common.cuh"
@@ -119,35 +118,6 @@ __global__ void k_validate_csr(int64_t m, int64_t n, int64_t nnz, const int32_t*
     if (c < 1 || (int64_t)c > n) bad |= 4u;
   }
   if (bad) atomicOr(flags, bad);
-}
-
-// one thread per stored SELL row: copy its entries into the slice-column-major layout
-__global__ void k_sell_fill(int64_t m, int64_t C, const int32_t* rowptr, const int32_t* colval,
-                            const char* nzval, int esz, const int32_t* perm,
-                            const int32_t* slice_ptr, int32_t* s_colval, char* s_nzval) {
-  const int64_t total = ((m + C - 1) / C) * C;
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total;
-       t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t s = t / C, o = t - s * C;
-    const int64_t base = (int64_t)slice_ptr[s] - 1;
-    const int64_t mx = ((int64_t)slice_ptr[s + 1] - slice_ptr[s]) / C;
-    int64_t start = 0, len = 0;
-    if (t < m) {
-      const int64_t r = (int64_t)perm[t] - 1;
-      start = (int64_t)rowptr[r] - 1;
-      len = (int64_t)rowptr[r + 1] - rowptr[r];
-    }
-    for (int64_t j = 0; j < mx; ++j) {
-      const int64_t dst = base + j * C + o;
-      if (j < len) {
-        s_colval[dst] = colval[start + j];
-        for (int b = 0; b < esz; ++b) s_nzval[dst * esz + b] = nzval[(start + j) * esz + b];
-      } else {
-        s_colval[dst] = -1;
-        for (int b = 0; b < esz; ++b) s_nzval[dst * esz + b] = 0;
-      }
-    }
-  }
 }
 
 __global__ void k_invert_perm(int64_t m, const int32_t* perm, int32_t* iperm) {
@@ -415,34 +385,37 @@ int gg_sell_create(gg_ctx* ctx, const gg_mat* csr, int64_t slice_size, int64_t s
   if (sigma < 1) return set_error(GG_ERR_ARGUMENT, "sigma must be >= 1");
   GG_CUDA(cudaSetDevice(ctx->device));
   const int64_t m = csr->m;
-  std::vector<int32_t> rp(m + 1);
-  GG_CUDA(cudaMemcpyAsync(rp.data(), csr->rowptr, (m + 1) * sizeof(int32_t), cudaMemcpyDeviceToHost,
-                          ctx->stream));
-  GG_CUDA(cudaStreamSynchronize(ctx->stream));
   // slice height clamped to m (src/storage/SELL.jl:108)
   const int64_t C = slice_size < m ? slice_size : m;
   const int64_t ns = C > 0 ? (m + C - 1) / C : 0;
-  std::vector<int32_t> perm(m);
-  std::iota(perm.begin(), perm.end(), 1);
-  if (sigma > 1) {
-    for (int64_t w0 = 0; w0 < m; w0 += sigma) {
-      const int64_t w1 = std::min<int64_t>(w0 + sigma, m);
-      std::stable_sort(perm.begin() + w0, perm.begin() + w1, [&](int32_t a, int32_t b) {
-        return (rp[a] - rp[a - 1]) > (rp[b] - rp[b - 1]);
-      });
-    }
+  // row order and slice widths on the device; the slices' offsets (64 bits, checked
+  // against the Int32 range) here
+  int32_t *perm = nullptr, *d_width = nullptr;
+  std::vector<int32_t> width(ns), sp(ns + 1);
+  cudaError_t e = cudaMalloc((void**)&perm, (m > 0 ? m : 1) * sizeof(int32_t));
+  if (e != cudaSuccess) return cuda_error(e, "gg_sell_create");
+  int rc = sort_rows_by_length(ctx, csr->rowptr, m, sigma, perm);
+  if (rc == GG_OK) {
+    e = cudaMallocAsync((void**)&d_width, (ns > 0 ? ns : 1) * sizeof(int32_t), ctx->stream);
+    if (e == cudaSuccess) rc = sell_slice_widths(ctx, csr->rowptr, perm, m, C, ns, d_width);
+    if (e == cudaSuccess && rc == GG_OK && ns > 0)
+      e = cudaMemcpyAsync(width.data(), d_width, ns * sizeof(int32_t), cudaMemcpyDeviceToHost,
+                          ctx->stream);
+    cudaFreeAsync(d_width, ctx->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    if (e != cudaSuccess && rc == GG_OK) rc = cuda_error(e, "gg_sell_create");
   }
-  std::vector<int32_t> sp(ns + 1);
   sp[0] = 1;
   int64_t acc = 1;
-  for (int64_t s = 0; s < ns; ++s) {
-    int64_t mx = 0;
-    for (int64_t r = s * C; r < std::min<int64_t>((s + 1) * C, m); ++r)
-      mx = std::max<int64_t>(mx, rp[perm[r]] - rp[perm[r] - 1]);
-    acc += mx * C;
+  for (int64_t s = 0; s < ns && rc == GG_OK; ++s) {
+    acc += (int64_t)width[s] * C;
     if (acc > (int64_t)INT32_MAX - 4096)  // kernels step Int32 positions past the end
-      return set_error(GG_ERR_ARGUMENT, "SELL n_stored exceeds the Int32 index range (use a larger sigma)");
+      rc = set_error(GG_ERR_ARGUMENT, "SELL n_stored exceeds the Int32 index range (use a larger sigma)");
     sp[s + 1] = (int32_t)acc;
+  }
+  if (rc != GG_OK) {
+    cudaFree(perm);
+    return rc;
   }
   gg_mat* S = new gg_mat();
   S->format = GG_FMT_SELL;
@@ -457,31 +430,24 @@ int gg_sell_create(gg_ctx* ctx, const gg_mat* csr, int64_t slice_size, int64_t s
   S->sigma = sigma;
   const size_t esz = dtype_size(csr->dtype);
   const int64_t nst = S->n_stored;
-  cudaError_t e = cudaMalloc((void**)&S->slice_ptr, (ns + 1) * sizeof(int32_t));
+  S->perm = perm;
+  e = cudaMalloc((void**)&S->slice_ptr, (ns + 1) * sizeof(int32_t));
   if (e == cudaSuccess) e = cudaMalloc((void**)&S->colval, (nst > 0 ? nst : 1) * sizeof(int32_t));
   if (e == cudaSuccess) e = cudaMalloc(&S->nzval, (nst > 0 ? nst : 1) * esz);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&S->perm, (m > 0 ? m : 1) * sizeof(int32_t));
   if (e == cudaSuccess) e = cudaMalloc((void**)&S->iperm, (m > 0 ? m : 1) * sizeof(int32_t));
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(S->slice_ptr, sp.data(), (ns + 1) * sizeof(int32_t), cudaMemcpyHostToDevice,
                         ctx->stream);
-  if (e == cudaSuccess && m > 0)
-    e = cudaMemcpyAsync(S->perm, perm.data(), m * sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream);
-  if (e == cudaSuccess && ns > 0) {
-    k_sell_fill<<<blocks_for(ctx, ns * C), 256, 0, ctx->stream>>>(
-        m, C, csr->rowptr, csr->colval, static_cast<const char*>(csr->nzval), (int)esz, S->perm,
-        S->slice_ptr, S->colval, static_cast<char*>(S->nzval));
-    e = cudaGetLastError();
-  }
+  if (e == cudaSuccess) rc = sell_fill(ctx, csr, S);
   if (e == cudaSuccess && m > 0) {
     k_invert_perm<<<blocks_for(ctx, m), 256, 0, ctx->stream>>>(m, S->perm, S->iperm);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-  if (e != cudaSuccess) {
+  if (e != cudaSuccess || rc != GG_OK) {
     free_mat_storage(S);
     delete S;
-    return cuda_error(e, "gg_sell_create");
+    return rc != GG_OK ? rc : cuda_error(e, "gg_sell_create");
   }
   *out = S;
   return GG_OK;

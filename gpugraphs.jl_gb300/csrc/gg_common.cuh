@@ -621,4 +621,11 @@ void free_spv_plan(gg_mat* A);  // gg_spmspv.cu
 // out[0..n] = base + exclusive prefix sums of cnt (gg_graph.cu; synchronises the stream)
 int scan_counts(gg_ctx* ctx, const int32_t* cnt, int64_t n, int32_t* out, int32_t base);
 int row_stats(gg_ctx* ctx, gg_mat* A);
+// orders and fills of the derived layouts (gg_layout.cu)
+int sort_rows_by_length(gg_ctx* ctx, const int32_t* rowptr, int64_t m, int64_t sigma, int32_t* perm);
+int sell_slice_widths(gg_ctx* ctx, const int32_t* rowptr, const int32_t* perm, int64_t m, int64_t C,
+                      int64_t ns, int32_t* width);
+int sell_fill(gg_ctx* ctx, const gg_mat* csr, gg_mat* S);
+int rank_columns(gg_ctx* ctx, const int32_t* cnt, int64_t n, int64_t top, int32_t* inv,
+                 int32_t* rank, int64_t* top_sum);
 }  // namespace gg

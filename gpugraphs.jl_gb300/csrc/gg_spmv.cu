@@ -902,52 +902,38 @@ static int build_colperm(gg_ctx* ctx, gg_mat* A) {
   const int64_t n = A->n;
   const int64_t len = A->format == GG_FMT_CSR ? A->nnz : A->n_stored;
   if (n < (1 << 16) || A->nnz == 0) return GG_OK;
-  int32_t* cnt = nullptr;
-  GG_CUDA(cudaMalloc((void**)&cnt, n * sizeof(int32_t)));
-  GG_CUDA(cudaMemsetAsync(cnt, 0, n * sizeof(int32_t), ctx->stream));
-  k_col_count<<<grid_for(ctx, len, 256), 256, 0, ctx->stream>>>(A->colval, len, cnt);
-  std::vector<int32_t> hc(n);
-  cudaError_t e = cudaMemcpyAsync(hc.data(), cnt, n * sizeof(int32_t), cudaMemcpyDeviceToHost,
-                                  ctx->stream);
-  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-  if (e != cudaSuccess) {
-    cudaFree(cnt);
-    return cuda_error(e, "column counts");
-  }
-  std::vector<uint64_t> key(n);
-  for (int64_t c = 0; c < n; ++c) key[c] = ((uint64_t)(uint32_t)(~(uint32_t)hc[c]) << 32) | (uint64_t)c;
-  std::sort(key.begin(), key.end());
-  int64_t top = 0;
-  const int64_t ntop = n / 100;
-  for (int64_t i = 0; i < ntop; ++i) top += hc[key[i] & 0xffffffffu];
-  if (top * 4 <= A->nnz) {  // not skewed: keep the natural column order
-    cudaFree(cnt);
-    return GG_OK;
-  }
-  std::vector<int32_t> inv(n), rank(n);
-  for (int64_t i = 0; i < n; ++i) {
-    inv[i] = (int32_t)(key[i] & 0xffffffffu);
-    rank[inv[i]] = (int32_t)i;
-  }
-  e = cudaMemcpyAsync(cnt, rank.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&P->colval_r, (len > 0 ? len : 1) * sizeof(int32_t));
+  int32_t *cnt = nullptr, *rank = nullptr;
+  cudaError_t e = cudaMallocAsync((void**)&cnt, n * sizeof(int32_t), ctx->stream);
+  if (e == cudaSuccess) e = cudaMallocAsync((void**)&rank, n * sizeof(int32_t), ctx->stream);
   if (e == cudaSuccess) e = cudaMalloc((void**)&P->inv, n * sizeof(int32_t));
-  // xr padded with zeros to whole column windows (the bulk copies of gg_spmv_hub.cu
-  // read complete windows)
-  const int64_t npad = (n + kHwCols - 1) / kHwCols * kHwCols;
-  if (e == cudaSuccess) e = cudaMalloc((void**)&P->xr, npad * sizeof(float));
-  if (e == cudaSuccess && npad > n)
-    e = cudaMemsetAsync(P->xr + n, 0, (npad - n) * sizeof(float), ctx->stream);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(P->inv, inv.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream);
+  if (e == cudaSuccess) e = cudaMemsetAsync(cnt, 0, n * sizeof(int32_t), ctx->stream);
+  int rc = GG_OK;
+  bool skewed = false;
   if (e == cudaSuccess) {
-    k_col_relabel<<<grid_for(ctx, len, 256), 256, 0, ctx->stream>>>(A->colval, len, cnt, P->colval_r);
-    e = cudaGetLastError();
+    k_col_count<<<grid_for(ctx, len, 256), 256, 0, ctx->stream>>>(A->colval, len, cnt);
+    int64_t top = 0;
+    rc = rank_columns(ctx, cnt, n, n / 100, P->inv, rank, &top);
+    skewed = rc == GG_OK && top * 4 > A->nnz;
   }
+  if (skewed) {
+    e = cudaMalloc((void**)&P->colval_r, (len > 0 ? len : 1) * sizeof(int32_t));
+    // xr padded with zeros to whole column windows (the bulk copies of gg_spmv_hub.cu
+    // read complete windows)
+    const int64_t npad = (n + kHwCols - 1) / kHwCols * kHwCols;
+    if (e == cudaSuccess) e = cudaMalloc((void**)&P->xr, npad * sizeof(float));
+    if (e == cudaSuccess && npad > n)
+      e = cudaMemsetAsync(P->xr + n, 0, (npad - n) * sizeof(float), ctx->stream);
+    if (e == cudaSuccess) {
+      k_col_relabel<<<grid_for(ctx, len, 256), 256, 0, ctx->stream>>>(A->colval, len, rank, P->colval_r);
+      e = cudaGetLastError();
+    }
+  }
+  cudaFreeAsync(cnt, ctx->stream);
+  cudaFreeAsync(rank, ctx->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-  cudaFree(cnt);
   if (e != cudaSuccess) return cuda_error(e, "column relabelling");
-  P->enabled = true;
+  GG_CHECK(rc);
+  P->enabled = skewed;
   return GG_OK;
 }
 
