@@ -146,6 +146,7 @@ static void free_derived(gg_mat* A) {
     delete A->sell_copy;
     A->sell_copy = nullptr;
   }
+  A->no_sell_copy = false;
   if (A->tr_copy) {
     free_mat_storage(A->tr_copy);
     delete A->tr_copy;

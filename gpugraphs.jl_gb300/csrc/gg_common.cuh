@@ -409,7 +409,7 @@ struct ColPerm {
   bool enabled = false;
   int32_t* colval_r = nullptr;
   int32_t* inv = nullptr;
-  float* xr = nullptr;
+  float* xr = nullptr;  // room for n values of the matrix's element type (4 bytes at least)
 };
 
 // Column-window tiles of a large CSR for the plus-times Float32 SpMV (gg_spmv_win.cu).
@@ -576,7 +576,10 @@ struct gg_mat {
   gg::WinPlan* winplan = nullptr;
   gg::HubWinPlan* hubwin = nullptr;  // SELL-32 copies: hub rows from column windows
   gg::SpvPlan* spv = nullptr;
-  gg_mat* sell_copy = nullptr;  // CSR handles: SELL-32 copy (rows sorted by length) for plus-times
+  // SELL-32 copy (rows sorted by length) for SpMV: large CSR handles, and SELL handles
+  // whose own slices are mostly padding
+  gg_mat* sell_copy = nullptr;
+  bool no_sell_copy = false;  // the copy could not be made (memory, index range)
   gg_mat* tr_copy = nullptr;    // CSR handles: CSR storage of the transpose (gg_spmv_t)
   int64_t max_row_len = -1;
   // tuned choices (gg_tune): plus-times SpMV kernel (0 = built-in rule, 1 = CSR row
@@ -601,6 +604,11 @@ int compute_type(int tv, int tx, int mul);
 int check_semiring(int tv, int tx, int ty, int mul, int add, int accum, int* tc_out);
 int spmv_dispatch(gg_ctx* ctx, gg_mat* A, int tc, int mul, int add, int accum, void* y, int ty,
                   const void* x, int tx, const void* mask, int tmask, int64_t lo, int64_t hi);
+// the SELL matrix a product of SELL handle A runs on: its sorted copy or A (gg_spmv.cu)
+gg_mat* sell_for_spmv(gg_ctx* ctx, gg_mat* A);
+// products of the common semirings with fixed operators and type (gg_spmv_typed.cu)
+int spmv_typed(gg_ctx* ctx, gg_mat* A, int tc, int mul, int add, int accum, void* y, int ty,
+               const void* x, int tx, const void* mask, int tmask, int64_t lo, int64_t hi, bool* done);
 int build_row_blocks(gg_ctx* ctx, gg_mat* A);
 int build_sell_plan(gg_ctx* ctx, gg_mat* A);
 int launch_col1_sell(gg_ctx* ctx, gg_mat* A, const float* x, float* y);  // gg_spmv.cu
@@ -626,6 +634,7 @@ int sort_rows_by_length(gg_ctx* ctx, const int32_t* rowptr, int64_t m, int64_t s
 int sell_slice_widths(gg_ctx* ctx, const int32_t* rowptr, const int32_t* perm, int64_t m, int64_t C,
                       int64_t ns, int32_t* width);
 int sell_fill(gg_ctx* ctx, const gg_mat* csr, gg_mat* S);
+int sell_resorted(gg_ctx* ctx, const gg_mat* A, gg_mat** out);
 int rank_columns(gg_ctx* ctx, const int32_t* cnt, int64_t n, int64_t top, int32_t* inv,
                  int32_t* rank, int64_t* top_sum);
 }  // namespace gg

@@ -3,6 +3,8 @@
 //  * sort_rows_by_length: the row order of SELL-C-sigma (rows by decreasing length
 //    within windows of sigma rows, equal lengths in row order).
 //  * sell_fill: a CSR matrix's entries into the slice-column-major SELL arrays.
+//  * sell_resorted: a SELL matrix again as SELL-32 with its rows sorted over the whole
+//    matrix.
 //  * rank_columns: columns by decreasing number of entries (equal counts by column).
 //
 // The first call on a matrix pays for these.  On the host (std::stable_sort over the
@@ -11,6 +13,8 @@
 // product's time.  Radix sorts are stable, so the orders are the same ones.  First call on
 // new matrices: Float32 product on R-MAT scale 22 437 -> 6.2 ms, Int32 shortest paths on
 // R-MAT scale 22 324 -> 81 ms.
+#include <vector>
+
 #include <cub/device/device_radix_sort.cuh>
 
 #include "gg_semiring.cuh"
@@ -192,6 +196,134 @@ int sell_fill(gg_ctx* ctx, const gg_mat* csr, gg_mat* S) {
     default: launch_fill<uint64_t>(ctx, csr, S); break;
   }
   GG_CUDA(cudaGetLastError());
+  return GG_OK;
+}
+
+// entries of original row r of a SELL matrix: the place of its first padding column
+// (entries come first), by bisection -- a hub row walked entry by entry is a chain of
+// 10^4 loads
+__global__ void k_sell_lengths(int64_t m, int32_t C, const int32_t* __restrict__ slice_ptr,
+                               const int32_t* __restrict__ colval, const int32_t* __restrict__ iperm,
+                               int32_t* len) {
+  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < m;
+       r += (int64_t)gridDim.x * blockDim.x) {
+    const int32_t t = iperm[r], s = t / C, o = t - s * C;
+    const int64_t base = (int64_t)slice_ptr[s] - 1 + o;
+    int32_t lo = 0, hi = (slice_ptr[s + 1] - slice_ptr[s]) / C;
+    while (lo < hi) {
+      const int32_t mid = (lo + hi) >> 1;
+      if (colval[base + (int64_t)mid * C] != -1) lo = mid + 1; else hi = mid;
+    }
+    len[r] = lo;
+  }
+}
+
+// the entries of SELL matrix A (C, perm inverse iperm) at the places of SELL-32 matrix S
+template <typename V>
+__global__ void __launch_bounds__(256)
+    k_sell_refill(int64_t m, int64_t ns, int64_t nst, const int32_t* __restrict__ perm,
+                  const int32_t* __restrict__ slice_ptr, int32_t* s_colval, V* s_nz, int32_t C,
+                  const int32_t* __restrict__ a_iperm, const int32_t* __restrict__ a_slice_ptr,
+                  const int32_t* __restrict__ a_colval, const V* __restrict__ a_nz) {
+  // a warp per slice of S, lane = row: the row's place in A is found once
+  const int lane = threadIdx.x & 31;
+  for (int64_t it = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; it < ns * 8;
+       it += ((int64_t)gridDim.x * blockDim.x) >> 5) {
+    const int64_t s = it >> 3, part = it & 7;  // 8 warps share a slice's columns
+    const int64_t t = s * 32 + lane, base = (int64_t)slice_ptr[s] - 1 + lane;
+    const int32_t width = (slice_ptr[s + 1] - slice_ptr[s]) / 32;
+    int64_t from = 0;
+    int32_t wide = 0;
+    if (t < m) {
+      const int32_t at = a_iperm[perm[t] - 1], as = at / C;
+      from = (int64_t)a_slice_ptr[as] - 1 + (at - as * C);
+      wide = (a_slice_ptr[as + 1] - a_slice_ptr[as]) / C;
+    }
+#pragma unroll 4
+    for (int32_t j = (int32_t)part; j < width; j += 8) {
+      int32_t c = -1;
+      V v = V(0);
+      if (j < wide) {
+        c = a_colval[from + (int64_t)j * C];
+        v = a_nz[from + (int64_t)j * C];
+      }
+      s_colval[base + (int64_t)j * 32] = c;
+      s_nz[base + (int64_t)j * 32] = v;
+    }
+  }
+}
+
+template <typename V>
+static void launch_refill(gg_ctx* ctx, const gg_mat* A, gg_mat* S) {
+  k_sell_refill<V><<<grid_of(ctx, S->nslices * 256), 256, 0, ctx->stream>>>(
+      S->m, S->nslices, S->n_stored, S->perm, S->slice_ptr, S->colval, static_cast<V*>(S->nzval),
+      (int32_t)A->slice_size, A->iperm, A->slice_ptr, A->colval, static_cast<const V*>(A->nzval));
+}
+
+// SELL-32 copy of SELL matrix A with rows sorted by length over the whole matrix
+int sell_resorted(gg_ctx* ctx, const gg_mat* A, gg_mat** out) {
+  *out = nullptr;
+  const int64_t m = A->m, ns = (m + 31) / 32;
+  const int esz = dtype_size(A->dtype);
+  cudaStream_t st = ctx->stream;
+  gg_mat* S = new gg_mat();
+  S->format = GG_FMT_SELL;
+  S->m = m;
+  S->n = A->n;
+  S->nnz = A->nnz;
+  S->dtype = A->dtype;
+  S->device = ctx->device;
+  S->slice_size = 32;
+  S->nslices = ns;
+  S->sigma = m;
+  int32_t *len = nullptr, *rp = nullptr, *width = nullptr;
+  std::vector<int32_t> w(ns), sp(ns + 1);
+  cudaError_t e = cudaMallocAsync((void**)&len, m * sizeof(int32_t), st);
+  if (e == cudaSuccess) e = cudaMallocAsync((void**)&rp, (m + 1) * sizeof(int32_t), st);
+  if (e == cudaSuccess) e = cudaMallocAsync((void**)&width, ns * sizeof(int32_t), st);
+  if (e == cudaSuccess) e = cudaMalloc((void**)&S->perm, m * sizeof(int32_t));
+  if (e == cudaSuccess) e = cudaMalloc((void**)&S->slice_ptr, (ns + 1) * sizeof(int32_t));
+  int rc = GG_OK;
+  if (e == cudaSuccess) {
+    k_sell_lengths<<<grid_of(ctx, m), 256, 0, st>>>(m, (int32_t)A->slice_size, A->slice_ptr, A->colval,
+                                                    A->iperm, len);
+    rc = scan_counts(ctx, len, m, rp, 1);
+    if (rc == GG_OK) rc = sort_rows_by_length(ctx, rp, m, m, S->perm);
+    if (rc == GG_OK) rc = sell_slice_widths(ctx, rp, S->perm, m, 32, ns, width);
+    if (rc == GG_OK) e = cudaMemcpyAsync(w.data(), width, ns * sizeof(int32_t), cudaMemcpyDeviceToHost, st);
+    if (rc == GG_OK && e == cudaSuccess) e = cudaStreamSynchronize(st);
+  }
+  cudaFreeAsync(len, st);
+  cudaFreeAsync(rp, st);
+  cudaFreeAsync(width, st);
+  int64_t acc = 1;
+  sp[0] = 1;
+  for (int64_t s = 0; s < ns && rc == GG_OK && e == cudaSuccess; ++s) {
+    acc += (int64_t)w[s] * 32;
+    if (acc > (int64_t)INT32_MAX - 4096) rc = set_error(GG_ERR_ARGUMENT, "SELL n_stored exceeds the Int32 index range");
+    sp[s + 1] = (int32_t)acc;
+  }
+  S->n_stored = acc - 1;
+  const int64_t nst = S->n_stored > 0 ? S->n_stored : 1;
+  if (rc == GG_OK && e == cudaSuccess) e = cudaMalloc((void**)&S->colval, nst * sizeof(int32_t));
+  if (rc == GG_OK && e == cudaSuccess) e = cudaMalloc(&S->nzval, nst * esz);
+  if (rc == GG_OK && e == cudaSuccess)
+    e = cudaMemcpyAsync(S->slice_ptr, sp.data(), (ns + 1) * sizeof(int32_t), cudaMemcpyHostToDevice, st);
+  if (rc == GG_OK && e == cudaSuccess) {
+    switch (esz) {
+      case 1: launch_refill<uint8_t>(ctx, A, S); break;
+      case 4: launch_refill<uint32_t>(ctx, A, S); break;
+      default: launch_refill<uint64_t>(ctx, A, S); break;
+    }
+    e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  }
+  if (rc == GG_OK && e != cudaSuccess) rc = cuda_error(e, "sorted SELL copy");
+  if (rc != GG_OK) {
+    gg_mat_destroy(S);
+    return rc;
+  }
+  *out = S;
   return GG_OK;
 }
 

@@ -26,13 +26,18 @@ __device__ __forceinline__ void accum_store_t(void* y, int64_t idx, typename CTy
   else r.i = static_cast<int64_t>(acc);
   Y a = raw_to<TY>(r, TC);
   Y* yp = static_cast<Y*>(y);
+  if (accum == GG_OP_SECOND) {  // nothing of the old value is wanted: not read
+    if (TY == GG_BOOL) a = (a != Y(0)) ? Y(1) : Y(0);
+    __stcs(yp + idx, a);
+    return;
+  }
   Y old = yp[idx];
   Raw ar;
   ar.i = 0;
   ar.d = 0;
   if (dtype_is_float(TY)) ar.d = static_cast<double>(a);
   else ar.i = static_cast<int64_t>(a);
-  Y v = (accum == GG_OP_SECOND) ? a : apply_op<TY>(accum, old, a, ar, TY, ai, aj, bi, bj);
+  Y v = apply_op<TY>(accum, old, a, ar, TY, ai, aj, bi, bj);
   if (TY == GG_BOOL) v = (v != Y(0)) ? Y(1) : Y(0);
   yp[idx] = v;
 }
