@@ -71,7 +71,9 @@ struct SRGen {
   const void* x;
   void* y;
   int64_t ldb, ldc;
-  int layout;
+  int layout;           // of B
+  int layout_c = GG_COL_MAJOR;
+  int64_t col0 = 0;     // columns of C (and ids of the index operators) before x's first
 
   __device__ __forceinline__ T neutral() const { return neutral_v; }
   __device__ __forceinline__ bool is_absorb(T a) const { return has_absorb && a == absorb_v; }
@@ -79,13 +81,14 @@ struct SRGen {
     return layout == GG_COL_MAJOR ? (int64_t)(col1 - 1) + j * ldb : (int64_t)(col1 - 1) * ldb + j;
   }
   __device__ __forceinline__ int64_t cidx(int64_t row0, int64_t j) const {
-    return layout == GG_COL_MAJOR ? row0 + j * ldc : row0 * ldc + j;
+    return layout_c == GG_COL_MAJOR ? row0 + j * ldc : row0 * ldc + j;
   }
   // mul(A[k], B[col, j], row, col, col, j+1); row1 is the 1-based row
   __device__ __forceinline__ T mulk(int64_t k, int32_t col1, int64_t row1, int64_t j = 0) const {
     Raw a = load_raw(nz, tv, k);
     Raw b = load_raw(x, tx, bidx(col1, j));
-    return apply_op<TC>(mul, raw_to<TC>(a, tv), raw_to<TC>(b, tx), b, tx, row1, col1, col1, j + 1);
+    return apply_op<TC>(mul, raw_to<TC>(a, tv), raw_to<TC>(b, tx), b, tx, row1, col1, col1,
+                        col0 + j + 1);
   }
   __device__ __forceinline__ T addv(T acc, T v) const {
     Raw z;
@@ -99,7 +102,8 @@ struct SRGen {
   }
   // SpMM epilogue: accum(C[row, j], acc, row, j, row, j)
   __device__ __forceinline__ void write_mm(int64_t row0, int64_t j, T acc) const {
-    accum_store<TC>(y, ty, cidx(row0, j), acc, accum, row0 + 1, j + 1, row0 + 1, j + 1);
+    accum_store<TC>(y, ty, cidx(row0, col0 + j), acc, accum, row0 + 1, col0 + j + 1, row0 + 1,
+                    col0 + j + 1);
   }
 };
 

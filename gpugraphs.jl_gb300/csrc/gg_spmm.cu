@@ -10,7 +10,10 @@
 // folded by separate warps and combined in order by a second pass: exact for every
 // associative monoid, within rounding for Float32/Float64 sums.
 // With a row-major dense operand (the batched-query layout) each gathered B row is
-// one contiguous 128-byte read.
+// one contiguous 128-byte read.  Column-major operands (Julia's arrays) are transposed
+// into the context's scratch first, 32-column tiles through shared memory: gathered
+// where they lie, every lane's value is a 32-byte sector of its own.  Row-major Float32
+// rows that are not whole 16-byte groups are padded there for the float4 kernels.
 #include <algorithm>
 #include <vector>
 
@@ -628,22 +631,29 @@ static int col1_sell(gg_ctx* ctx, gg_mat* A, const SRPlusTimesF32MM& sr) {
   return launch_col1_sell(ctx, A, sr.x, sr.y);
 }
 
+// scratch the pieces of long rows take for k columns: their columns per pass and bytes
+static size_t mm_partial_bytes(const MMPlan* P, size_t esz, int64_t k, int64_t* jwin) {
+  *jwin = k;
+  if (P->nseg == 0) return 0;
+  const int64_t per_col = P->nseg * (int64_t)esz;
+  const int64_t cap = kMMPartialBytes / per_col;
+  if (*jwin > cap) *jwin = cap < 32 ? 32 : (cap / 32) * 32;
+  return (size_t)(per_col * *jwin);
+}
+
+// reserved: bytes at the start of the scratch that hold the caller's operands
 template <class SR>
 static int launch_mm(gg_ctx* ctx, gg_mat* A, const SR& sr, int64_t k, const void* mask, int tmask,
-                     int64_t lo, int64_t hi) {
+                     int64_t lo, int64_t hi, size_t reserved = 0) {
   typedef typename SR::T T;
   const int64_t m = A->m;
   if (col1_sell_ok(A, sr, k, mask, lo)) return col1_sell(ctx, A, sr);
   GG_CHECK(build_mm_plan(ctx, A));
   const MMPlan* P = A->mmplan;
   int64_t jwin = k;
-  if (P->nseg > 0) {
-    const int64_t per_col = P->nseg * (int64_t)sizeof(T);
-    const int64_t cap = kMMPartialBytes / per_col;
-    if (jwin > cap) jwin = cap < 32 ? 32 : (cap / 32) * 32;
-    GG_CHECK(ensure_scratch(ctx, (size_t)(per_col * jwin)));
-  }
-  T* partials = static_cast<T*>(ctx->scratch);
+  const size_t pbytes = mm_partial_bytes(P, sizeof(T), k, &jwin);
+  if (pbytes > 0) GG_CHECK(ensure_scratch(ctx, reserved + pbytes));
+  T* partials = reinterpret_cast<T*>(static_cast<char*>(ctx->scratch) + reserved);
   const int64_t row_lo = lo > 0 ? lo - 1 : 0;
   const int64_t row_hi = lo > 0 ? hi : m;
   for (int64_t jlo = 0; jlo < k; jlo += jwin) {
@@ -712,6 +722,184 @@ static int launch_mm(gg_ctx* ctx, gg_mat* A, const SR& sr, int64_t k, const void
   return GG_OK;
 }
 
+// ---------------------------------------------------------------------------------
+// column-major operands
+// ---------------------------------------------------------------------------------
+// rows x k values of E, column-major with leading dimension ld, to row-major with leading
+// dimension kp >= k (columns past k filled with 0): 32 x 32 tiles, both sides coalesced
+template <typename E>
+__global__ void __launch_bounds__(256)
+    k_to_row_major(const E* __restrict__ src, int64_t ld, int64_t rows, int k, E* __restrict__ dst, int kp) {
+  __shared__ E tile[32][33];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  for (int64_t r0 = (int64_t)blockIdx.x * 32; r0 < rows; r0 += (int64_t)gridDim.x * 32) {
+    for (int c0 = 0; c0 < kp; c0 += 32) {
+#pragma unroll
+      for (int q = 0; q < 32; q += 8) {
+        const int c = c0 + ty + q;
+        tile[ty + q][tx] = c < k && r0 + tx < rows ? __ldcs(src + (int64_t)c * ld + r0 + tx) : E(0);
+      }
+      __syncthreads();
+#pragma unroll
+      for (int q = 0; q < 32; q += 8)
+        if (r0 + ty + q < rows && c0 + tx < kp) dst[(r0 + ty + q) * kp + c0 + tx] = tile[tx][ty + q];
+      __syncthreads();
+    }
+  }
+}
+
+// the rows the product wrote (range [row_lo, row_hi), mask) back to column-major
+__global__ void __launch_bounds__(256)
+    k_to_col_major_f32(const float* __restrict__ src, int kp, int64_t row_lo, int64_t row_hi, int k,
+                       float* __restrict__ dst, int64_t ld, const void* mask, int tmask) {
+  __shared__ float tile[32][33];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  for (int64_t r0 = row_lo + (int64_t)blockIdx.x * 32; r0 < row_hi; r0 += (int64_t)gridDim.x * 32) {
+    const int64_t r = r0 + tx;
+    const bool keep = r < row_hi && (!mask || !raw_is_zero(load_raw(mask, tmask, r), tmask));
+    for (int c0 = 0; c0 < k; c0 += 32) {
+#pragma unroll
+      for (int q = 0; q < 32; q += 8)
+        tile[ty + q][tx] = r0 + ty + q < row_hi && c0 + tx < kp
+                               ? __ldcs(src + (r0 + ty + q) * kp + c0 + tx) : 0.0f;
+      __syncthreads();
+#pragma unroll
+      for (int q = 0; q < 32; q += 8)
+        if (keep && c0 + ty + q < k) __stcs(dst + (int64_t)(c0 + ty + q) * ld + r, tile[tx][ty + q]);
+      __syncthreads();
+    }
+  }
+}
+
+template <typename E>
+static void to_row_major(gg_ctx* ctx, const void* src, int64_t ld, int64_t rows, int64_t k, void* dst,
+                         int64_t kp) {
+  int64_t g = (rows + 31) / 32;
+  const int64_t cap = (int64_t)ctx->num_sms * 8;
+  if (g > cap) g = cap;
+  if (g < 1) return;
+  k_to_row_major<E><<<(int)g, 256, 0, ctx->stream>>>(static_cast<const E*>(src), ld, rows, (int)k,
+                                                     static_cast<E*>(dst), (int)kp);
+  trace_count(ctx, 1);
+}
+
+// rows x k values, row-major with any leading dimension or alignment, to rows of kp (a
+// multiple of 4) values, and back: a warp per row
+__global__ void __launch_bounds__(256)
+    k_pad_rows_f32(const float* __restrict__ src, int64_t ld, int64_t rows, int k, float* __restrict__ dst,
+                   int kp) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rows;
+       r += ((int64_t)gridDim.x * blockDim.x) >> 5)
+    for (int c = lane; c < kp; c += 32) dst[r * kp + c] = c < k ? __ldcs(src + r * ld + c) : 0.0f;
+}
+__global__ void __launch_bounds__(256)
+    k_unpad_rows_f32(const float* __restrict__ src, int kp, int64_t row_lo, int64_t row_hi, int k,
+                     float* __restrict__ dst, int64_t ld) {
+  const int lane = threadIdx.x & 31;
+  for (int64_t r = row_lo + (((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5); r < row_hi;
+       r += ((int64_t)gridDim.x * blockDim.x) >> 5)
+    for (int c = lane; c < k; c += 32) __stcs(dst + r * ld + c, __ldcs(src + r * kp + c));
+}
+
+// Products below this many (entry, column) pairs take the operands where they lie: the
+// extra launches cost more than the gathers of operands that L1 holds.  Above, us, where
+// they lie / transposed (R-MAT, rows x columns): 300 x 4 - / 30, 1000 x 4 148 / 50, 10000 x 32 277 / 61,
+// 100000 x 32 1447 / 85, 2^20 x 32 13574 / 634; a row-major 100000 x 31 190 / 87 padded
+// to 32 columns.
+static const int64_t kMMTranspose = 1 << 10;
+// scratch for the transposed operands of one pass; wider products run in passes
+static const int64_t kMMTransposeBytes = (int64_t)5 << 28;
+
+// columns of a pass when every column takes per_col bytes, a multiple of 4
+static int64_t mm_pass_columns(int64_t k, int64_t per_col) {
+  int64_t w = kMMTransposeBytes / (per_col > 0 ? per_col : 1);
+  if (w > 32) w &= ~(int64_t)31;
+  w &= ~(int64_t)3;
+  if (w < 4) w = 4;
+  return w < k ? w : k;
+}
+
+// Float32 plus-times on operands the float4 kernels cannot read (column-major, or
+// row-major rows that are not whole 16-byte groups): both through row-major scratch.
+// GG_ERR_OOM (nothing launched): the caller takes them where they lie.
+static int spmm_staged_f32(gg_ctx* ctx, gg_mat* A, SRPlusTimesF32MM sr, int64_t k, int layout,
+                           const void* mask, int tmask, int64_t lo, int64_t hi) {
+  GG_CHECK(build_mm_plan(ctx, A));
+  const int64_t m = A->m, n = A->n;
+  const int64_t w = mm_pass_columns(k, (n + m) * (int64_t)sizeof(float));
+  const int64_t wp = (w + 3) & ~(int64_t)3;
+  const size_t bbytes = ((size_t)n * wp * sizeof(float) + 255) & ~(size_t)255;
+  const size_t cbytes = ((size_t)m * wp * sizeof(float) + 255) & ~(size_t)255;
+  int64_t jwin = 0;
+  GG_CHECK(ensure_scratch(ctx, bbytes + cbytes + mm_partial_bytes(A->mmplan, sizeof(float), wp, &jwin)));
+  const float* B = sr.x;
+  float* Cm = sr.y;
+  const int64_t ldb = sr.ldb, ldc = sr.ldc;
+  const bool col = layout == GG_COL_MAJOR;
+  float* Bt = static_cast<float*>(ctx->scratch);
+  float* Ct = reinterpret_cast<float*>(static_cast<char*>(ctx->scratch) + bbytes);
+  const int64_t row_lo = lo > 0 ? lo - 1 : 0, row_hi = lo > 0 ? hi : m;
+  sr.x = Bt;
+  sr.y = Ct;
+  for (int64_t j0 = 0; j0 < k; j0 += w) {
+    const int64_t kn = k - j0 < w ? k - j0 : w, kp = (kn + 3) & ~(int64_t)3;
+    sr.ldb = sr.ldc = kp;
+    if (col) {
+      to_row_major<float>(ctx, B + j0 * ldb, ldb, n, kn, Bt, kp);
+    } else {
+      k_pad_rows_f32<<<grid_mm(ctx, n), 256, 0, ctx->stream>>>(B + j0, ldb, n, (int)kn, Bt, (int)kp);
+      trace_count(ctx, 1);
+    }
+    GG_CHECK(launch_mm(ctx, A, sr, kp, mask, tmask, lo, hi, bbytes + cbytes));
+    const int64_t nrows = row_hi - row_lo;
+    if (nrows <= 0) continue;
+    if (col) {
+      int64_t g = (nrows + 31) / 32;
+      if (g > (int64_t)ctx->num_sms * 8) g = (int64_t)ctx->num_sms * 8;
+      k_to_col_major_f32<<<(int)g, 256, 0, ctx->stream>>>(Ct, (int)kp, row_lo, row_hi, (int)kn,
+                                                         Cm + j0 * ldc, ldc, mask, tmask);
+    } else {
+      k_unpad_rows_f32<<<grid_mm(ctx, nrows), 256, 0, ctx->stream>>>(Ct, (int)kp, row_lo, row_hi, (int)kn,
+                                                                    Cm + j0, ldc);
+    }
+    trace_count(ctx, 1);
+    GG_CUDA(cudaGetLastError());
+  }
+  return GG_OK;
+}
+
+// other semirings: B through row-major scratch, C where it lies
+template <class SR>
+static int spmm_colmajor(gg_ctx* ctx, gg_mat* A, SR sr, int64_t k, const void* mask, int tmask,
+                         int64_t lo, int64_t hi) {
+  typedef typename SR::T T;
+  GG_CHECK(build_mm_plan(ctx, A));
+  const int64_t n = A->n;
+  const int esz = dtype_size(sr.tx);
+  const int64_t w = mm_pass_columns(k, n * esz);
+  const size_t bbytes = ((size_t)n * w * esz + 255) & ~(size_t)255;
+  int64_t jwin = 0;
+  GG_CHECK(ensure_scratch(ctx, bbytes + mm_partial_bytes(A->mmplan, sizeof(T), w, &jwin)));
+  const char* B = static_cast<const char*>(sr.x);
+  const int64_t ldb = sr.ldb;
+  sr.x = ctx->scratch;
+  sr.layout = GG_ROW_MAJOR;
+  for (int64_t j0 = 0; j0 < k; j0 += w) {
+    const int64_t kn = k - j0 < w ? k - j0 : w;
+    const char* Bj = B + j0 * ldb * esz;
+    switch (esz) {
+      case 1: to_row_major<uint8_t>(ctx, Bj, ldb, n, kn, ctx->scratch, kn); break;
+      case 4: to_row_major<uint32_t>(ctx, Bj, ldb, n, kn, ctx->scratch, kn); break;
+      default: to_row_major<uint64_t>(ctx, Bj, ldb, n, kn, ctx->scratch, kn); break;
+    }
+    sr.ldb = kn;
+    sr.col0 = j0;
+    GG_CHECK(launch_mm(ctx, A, sr, kn, mask, tmask, lo, hi, bbytes));
+  }
+  return GG_OK;
+}
+
 template <int TC>
 static int spmm_generic(gg_ctx* ctx, gg_mat* A, int mul, int add, int accum, void* Cm, int tcm,
                         int64_t ldc, const void* B, int tb, int64_t ldb, int64_t k, int layout,
@@ -732,6 +920,11 @@ static int spmm_generic(gg_ctx* ctx, gg_mat* A, int mul, int add, int accum, voi
   sr.ldb = ldb;
   sr.ldc = ldc;
   sr.layout = layout;
+  sr.layout_c = layout;
+  if (layout == GG_COL_MAJOR && A->nnz * k >= kMMTranspose) {
+    const int rc = spmm_colmajor(ctx, A, sr, k, mask, tmask, lo, hi);
+    if (rc != GG_ERR_OOM) return rc;
+  }
   return launch_mm(ctx, A, sr, k, mask, tmask, lo, hi);
 }
 
@@ -745,15 +938,22 @@ int spmm_dispatch(gg_ctx* ctx, gg_mat* A, int tc, int mul, int add, int accum, v
     ldb = 1;
     ldc = 1;
   }
-  if (layout == GG_ROW_MAJOR && A->dtype == GG_FLOAT32 && tb == GG_FLOAT32 && tcm == GG_FLOAT32 &&
-      mul == GG_OP_MUL && add == GG_OP_ADD && accum == GG_OP_SECOND) {
+  if (A->dtype == GG_FLOAT32 && tb == GG_FLOAT32 && tcm == GG_FLOAT32 && mul == GG_OP_MUL &&
+      add == GG_OP_ADD && accum == GG_OP_SECOND) {
     SRPlusTimesF32MM sr;
     sr.nz = static_cast<const float*>(A->nzval);
     sr.x = static_cast<const float*>(B);
     sr.y = static_cast<float*>(Cm);
     sr.ldb = ldb;
     sr.ldc = ldc;
-    return launch_mm(ctx, A, sr, k, mask, tmask, lo, hi);
+    // row-major CSR products without a mask have the float4 kernels to gain from whole rows
+    const bool pad = layout == GG_ROW_MAJOR && A->format == GG_FMT_CSR && !mask && k > 1 &&
+                     !ShortRowsMM<SRPlusTimesF32MM>::ok(sr, 0, k, nullptr);
+    if ((layout == GG_COL_MAJOR || pad) && A->nnz * k >= kMMTranspose) {
+      const int rc = spmm_staged_f32(ctx, A, sr, k, layout, mask, tmask, lo, hi);
+      if (rc != GG_ERR_OOM) return rc;
+    }
+    if (layout == GG_ROW_MAJOR) return launch_mm(ctx, A, sr, k, mask, tmask, lo, hi);
   }
   switch (tc) {
     case GG_BOOL: return spmm_generic<GG_BOOL>(ctx, A, mul, add, accum, Cm, tcm, ldc, B, tb, ldb, k, layout, mask, tmask, lo, hi);
