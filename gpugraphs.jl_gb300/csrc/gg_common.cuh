@@ -635,6 +635,7 @@ int sell_slice_widths(gg_ctx* ctx, const int32_t* rowptr, const int32_t* perm, i
                       int64_t ns, int32_t* width);
 int sell_fill(gg_ctx* ctx, const gg_mat* csr, gg_mat* S);
 int sell_resorted(gg_ctx* ctx, const gg_mat* A, gg_mat** out);
+int sort_entries_by_value(gg_ctx* ctx, const gg_mat* A, int32_t* col, void* nz);
 int rank_columns(gg_ctx* ctx, const int32_t* cnt, int64_t n, int64_t top, int32_t* inv,
                  int32_t* rank, int64_t* top_sum);
 }  // namespace gg

@@ -51,8 +51,10 @@ struct GraphAux {
   int64_t max_in_deg = -1;  // largest row of the view (-1: not computed yet)
   double avg_w = -1.0;      // mean stored weight in the distance type (-1: not yet)
   // shortest-path pull rounds of large CSR handles: SELL-32 copy of A_T with rows
-  // sorted by length (coalesced column / weight loads, a lane per row)
+  // sorted by length (coalesced column / weight loads, a lane per row), every row's
+  // entries by ascending weight when pull_sorted
   gg_mat* pull_sell = nullptr;
+  bool pull_sorted = false;
 };
 
 void free_graph_aux(gg_mat* A) {
@@ -415,7 +417,11 @@ __device__ __forceinline__ bool bit_of(const unsigned* bm, int32_t v) {
 struct Counters {
   unsigned long long nf, mf, level, status;
   unsigned long long nh;  // frontier hubs deferred to the piece kernel
-  unsigned long long pad[3];
+  unsigned long long pad;
+  // shortest paths: smallest distance written in the round, as ~(its bits) and folded
+  // with max, so that the cleared word means "none noted"
+  unsigned long long low;
+  unsigned long long pad2;
 };
 
 // Frontier vertices with more than kPushHub out-edges are not walked by one warp:
@@ -1310,7 +1316,7 @@ static int bfs_run(gg_ctx* ctx, gg_mat* A, int32_t s, int which, int32_t* dist,
       if (frontier_is_bitmap) {
         const int64_t nwords = (n + 31) / 32;
         k_bitmap_to_queue<<<gridsz(ctx, nwords), 256, 0, ctx->stream>>>(sc.fb[cur], nwords, sc.q[cur],
-                                                                        &sc.ctr->pad[0]);
+                                                                        &sc.ctr->pad);
       }
       const bool hubs = P.max_deg > kPushHub;
       k_bfs_push<<<gridsz(ctx, nf * 32), 256, 0, ctx->stream>>>(
@@ -1411,12 +1417,46 @@ template <typename T> __device__ __forceinline__ T relax_add(T w, T d) {
 // relax the out-edges [kb, ke) of one frontier vertex at distance du, the whole warp:
 // 128 edges per step with their columns, weights and then distances in flight together;
 // improved targets join the next frontier once (bitmap inq_next)
+template <typename T> __device__ __forceinline__ unsigned long long dist_bits(T d);
+template <> __device__ __forceinline__ unsigned long long dist_bits<int32_t>(int32_t d) { return (unsigned)d; }
+template <> __device__ __forceinline__ unsigned long long dist_bits<int64_t>(int64_t d) { return (unsigned long long)d; }
+template <> __device__ __forceinline__ unsigned long long dist_bits<float>(float d) { return __float_as_uint(d); }
+template <> __device__ __forceinline__ unsigned long long dist_bits<double>(double d) {
+  return (unsigned long long)__double_as_longlong(d);
+}
+template <typename T> static T dist_of_bits(unsigned long long b) {
+  T d;
+  if (sizeof(T) == 4) {
+    const uint32_t w = (uint32_t)b;
+    memcpy(&d, &w, 4);
+  } else {
+    memcpy(&d, &b, 8);
+  }
+  return d;
+}
+// what a push or pull round found, added to the counters once per warp at its end
+template <typename T>
+struct RoundSums {
+  unsigned long long edges = 0;  // out-edges of the vertices that joined the next frontier
+  T low = Lim<T>::max();         // smallest distance written
+  __device__ __forceinline__ void flush(Counters* ctr) {
+    warp_add(edges, &ctr->mf);
+    unsigned long long b = ~dist_bits<T>(low);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const unsigned long long t = __shfl_xor_sync(kFullG, b, o);
+      b = t > b ? t : b;
+    }
+    if ((threadIdx.x & 31) == 0 && b != ~dist_bits<T>(Lim<T>::max())) atomicMax(&ctr->low, b);
+  }
+};
+
 template <typename T>
 __device__ __forceinline__ void sssp_push_range(const int32_t* __restrict__ prow,
                                                 const int32_t* __restrict__ pcol,
                                                 const T* __restrict__ pw, int32_t kb, int32_t ke,
                                                 T du, T* dist, unsigned* inq_next, WarpQueue& wq,
-                                                unsigned long long& edges) {
+                                                RoundSums<T>& sum) {
   const int lane = threadIdx.x & 31;
   for (int32_t base = kb; base < ke; base += 32 * kPushStep) {
     int32_t w[kPushStep];
@@ -1435,7 +1475,8 @@ __device__ __forceinline__ void sssp_push_range(const int32_t* __restrict__ prow
       if (cand[t] < dw[t] && cand[t] < atomic_min_t(dist + w[t], cand[t])) {
         const unsigned bit = 1u << (w[t] & 31);
         add = !(atomicOr(inq_next + (w[t] >> 5), bit) & bit);
-        if (add) edges += (unsigned long long)(__ldg(prow + w[t] + 1) - __ldg(prow + w[t]));
+        sum.low = cand[t] < sum.low ? cand[t] : sum.low;
+        if (add) sum.edges += (unsigned long long)(__ldg(prow + w[t] + 1) - __ldg(prow + w[t]));
       }
       wq.push(add, w[t]);
     }
@@ -1450,7 +1491,7 @@ __global__ void __launch_bounds__(256)
                 unsigned* inq_cur, unsigned* inq_next, int32_t* qn, Counters* ctr, int32_t* hq) {
   __shared__ int32_t stage[8][WarpQueue::kCap];
   WarpQueue wq(stage[threadIdx.x >> 5], qn, &ctr->nf);
-  unsigned long long edges = 0;
+  RoundSums<T> sum;
   const int lane = threadIdx.x & 31;
   for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < nf;
        i += ((int64_t)gridDim.x * blockDim.x) >> 5) {
@@ -1461,10 +1502,10 @@ __global__ void __launch_bounds__(256)
       if (lane == 0) hq[atomicAdd(&ctr->nh, 1ull)] = u;
       continue;
     }
-    sssp_push_range<T>(prow, pcol, pw, k0, k1, ld_cg(dist + u), dist, inq_next, wq, edges);
+    sssp_push_range<T>(prow, pcol, pw, k0, k1, ld_cg(dist + u), dist, inq_next, wq, sum);
   }
   wq.flush();
-  warp_add(edges, &ctr->mf);
+  sum.flush(ctr);
 }
 
 template <typename T>
@@ -1480,7 +1521,7 @@ __global__ void __launch_bounds__(256)
   if (nh == 0) return;
   const int64_t npieces = hoff[nh];
   WarpQueue wq(stage[threadIdx.x >> 5], qn, &ctr->nf);
-  unsigned long long edges = 0;
+  RoundSums<T> sum;
   int64_t h = 0;
   for (int64_t q = gw; q < npieces; q += nw) {
     h = hub_of(hoff, nh, q, h);
@@ -1488,10 +1529,10 @@ __global__ void __launch_bounds__(256)
     const int32_t k1 = prow[u + 1];
     const int32_t kb = prow[u] + (int32_t)(q - hoff[h]) * kPushPiece;
     const int32_t ke = kb + kPushPiece < k1 ? kb + kPushPiece : k1;
-    sssp_push_range<T>(prow, pcol, pw, kb, ke, ld_cg(dist + u), dist, inq_next, wq, edges);
+    sssp_push_range<T>(prow, pcol, pw, kb, ke, ld_cg(dist + u), dist, inq_next, wq, sum);
   }
   wq.flush();
-  warp_add(edges, &ctr->mf);
+  sum.flush(ctr);
 }
 
 // single-CTA rounds while the frontier is small (mirror of k_bfs_small)
@@ -1876,7 +1917,7 @@ __global__ void __launch_bounds__(256)
                 unsigned* chg_next, int32_t* qn, Counters* ctr, const int32_t* __restrict__ prow) {
   __shared__ int32_t stage[8][WarpQueue::kCap];
   WarpQueue wq(stage[threadIdx.x >> 5], qn, &ctr->nf);
-  unsigned long long edges = 0;
+  RoundSums<T> sum;
   const int lane = threadIdx.x & 31;
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < n; base += stride) {
@@ -1916,11 +1957,14 @@ __global__ void __launch_bounds__(256)
     }
     const unsigned word = __ballot_sync(kFullG, changed);
     if (lane == 0 && base + threadIdx.x - lane < n) chg_next[v >> 5] = word;
-    if (changed) edges += (unsigned long long)(prow[v + 1] - prow[v]);
+    if (changed) {
+      sum.edges += (unsigned long long)(prow[v + 1] - prow[v]);
+      sum.low = best < sum.low ? best : sum.low;
+    }
     wq.push(changed, (int32_t)v);
   }
   wq.flush();
-  warp_add(edges, &ctr->mf);
+  sum.flush(ctr);
 }
 
 // rows of 33..kHubDegB in-edges of a pull round (the hub plan's mid list, longest
@@ -1935,7 +1979,7 @@ __global__ void __launch_bounds__(256)
                     const int32_t* __restrict__ mid, int64_t nmid) {
   __shared__ int32_t stage[8][WarpQueue::kCap];
   WarpQueue wq(stage[threadIdx.x >> 5], qn, &ctr->nf);
-  unsigned long long edges = 0;
+  RoundSums<T> sum;
   const int lane = threadIdx.x & 31;
   // warps numbered block-major: the longest groups go to different SMs
   const int64_t gw = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
@@ -2027,11 +2071,14 @@ __global__ void __launch_bounds__(256)
       changed = true;
       atomicOr(chg_next + (myv >> 5), 1u << (myv & 31));
     }
-    if (changed) edges += (unsigned long long)(prow[myv + 1] - prow[myv]);
+    if (changed) {
+      sum.edges += (unsigned long long)(prow[myv + 1] - prow[myv]);
+      sum.low = mine < sum.low ? mine : sum.low;
+    }
     wq.push(changed, myv);
   }
   wq.flush();
-  warp_add(edges, &ctr->mf);
+  sum.flush(ctr);
 }
 
 // hub rows of the pull round: one warp per piece of the matrix's hub plan (rows of
@@ -2080,6 +2127,13 @@ __global__ void __launch_bounds__(256)
 // through L1 (a value lowered by another SM may be seen late: any distance read is an
 // upper bound of the fixpoint, and a vertex lowered in this round joins the next
 // frontier, so any order reaches the same fixpoint) and lowered in place.
+//
+// With the copy's entries by ascending weight a row stops at the first weight w with
+// w + dlow >= its best distance so far (dlow: the smallest distance written in the
+// previous round, so no source that changed lies below it; sums of non-negative values
+// only grow, rounding included): what follows cannot improve it.  On R-MAT scale 22 with
+// weights 1..255 most rows end within one or two groups of 8: a round takes 116 to 234 us
+// instead of 443.
 // ---------------------------------------------------------------------------------
 static const int kPullSellThreads = 512;
 // a round pulls when the frontier's out-edges exceed nnz / kPullSellDiv
@@ -2089,19 +2143,15 @@ static const int kPullSellThreads = 512;
 static const int64_t kPullSellDiv = GG_PULL_SELL_DIV;
 
 template <typename T>
-__device__ __forceinline__ void pull_lower(int64_t srow, int64_t m, const int32_t* __restrict__ perm,
-                                           T cand, T* dist, unsigned* inq_next, WarpQueue& wq,
-                                           unsigned long long& edges,
+__device__ __forceinline__ void pull_lower(int32_t v, T cand, T cur, T* dist, unsigned* inq_next,
+                                           WarpQueue& wq, RoundSums<T>& sum,
                                            const int32_t* __restrict__ prow) {
   bool improved = false;
-  int32_t v = 0;
-  if (srow < m && cand != Lim<T>::max()) {
-    v = __ldg(perm + srow) - 1;
-    if (cand < ld_cg(dist + v) && cand < atomic_min_t(dist + v, cand)) {
-      const unsigned bit = 1u << (v & 31);
-      improved = !(atomicOr(inq_next + (v >> 5), bit) & bit);
-      if (improved) edges += (unsigned long long)(__ldg(prow + v + 1) - __ldg(prow + v));
-    }
+  if (cand < cur && cand < atomic_min_t(dist + v, cand)) {
+    const unsigned bit = 1u << (v & 31);
+    improved = !(atomicOr(inq_next + (v >> 5), bit) & bit);
+    sum.low = cand < sum.low ? cand : sum.low;
+    if (improved) sum.edges += (unsigned long long)(__ldg(prow + v + 1) - __ldg(prow + v));
   }
   wq.push(improved, v);
 }
@@ -2111,16 +2161,20 @@ __global__ void __launch_bounds__(kPullSellThreads)
     k_sssp_pull_sell(const int32_t* __restrict__ colval, const void* __restrict__ nz, int tv,
                      const int32_t* __restrict__ perm, int64_t m, const int4* __restrict__ pitems,
                      int64_t nitems, T* dist, unsigned* inq_next, int32_t* qn, Counters* ctr,
-                     const int32_t* __restrict__ prow) {
+                     const int32_t* __restrict__ prow, bool sorted, T dlow) {
   __shared__ int32_t stage[kPullSellThreads / 32][WarpQueue::kCap];
   WarpQueue wq(stage[threadIdx.x >> 5], qn, &ctr->nf);
-  unsigned long long edges = 0;
+  RoundSums<T> sum;
   const int lane = threadIdx.x & 31;
   const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+  // the next item's descriptor and row ids are loaded while this one runs
+  auto row_at = [&](int64_t srow) -> int32_t { return srow < m ? __ldg(perm + srow) - 1 : -1; };
   int4 dn = gw < nitems ? __ldg(pitems + gw) : make_int4(0, 0, 0, -1);
+  int32_t vn = gw < nitems ? row_at((int64_t)dn.y + lane) : -1;
   for (int64_t it = gw; it < nitems; it += nw) {
     const int4 d = dn;  // first position, first stored row, columns (or -slices), partial
+    const int32_t v0 = vn;
     if (it + nw < nitems) dn = __ldg(pitems + it + nw);
     if (d.z < 0) {
       // group of -d.z narrow slices (widths in 4-bit fields of d.w), <= 8 columns in all
@@ -2139,58 +2193,67 @@ __global__ void __launch_bounds__(kPullSellThreads)
         }
       }
       int u0 = 0;
+      int32_t v = v0;
       for (int t = 0; t < ns; ++t) {
         const int w = (int)((widths >> (4 * t)) & 15u);
+        const int32_t vt = v;
+        if (t + 1 < ns) v = row_at((int64_t)d.y + (t + 1) * 32 + lane);
         T best = Lim<T>::max();
 #pragma unroll
         for (int u = 0; u < kNarrowCols; ++u)
           if (u >= u0 && u < u0 + w && c[u] < best) best = c[u];
         u0 += w;
-        pull_lower(d.y + t * 32 + lane, m, perm, best, dist, inq_next, wq, edges, prow);
+        if (w > 0) {
+          const T cur = best != Lim<T>::max() && vt >= 0 ? ld_cg(dist + vt) : Lim<T>::min();
+          pull_lower<T>(vt, best, cur, dist, inq_next, wq, sum, prow);
+        }
       }
+      if (it + nw < nitems) vn = row_at((int64_t)dn.y + lane);
       continue;
     }
-    const int64_t srow = (int64_t)d.y + lane;
-    T best = Lim<T>::max();
-    if (srow < m) {
-      // the next 8 columns / weights are loaded (streamed past L1) while the current
-      // 8 distances are gathered
-      int32_t col[8];
-      T w[8];
+    // the first 8 columns / weights, then (streamed past L1) the next 8 while the current
+    // 8 distances are gathered
+    int32_t col[8];
+    T w[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const int64_t pos = (int64_t)d.x + lane + (int64_t)u * 32;
+      col[u] = u < d.z ? __ldcs(colval + pos) : -1;
+      w[u] = u < d.z ? view_weight<T>(nz, tv, pos) : Lim<T>::max();
+    }
+    const T cur = v0 >= 0 ? ld_cg(dist + v0) : Lim<T>::min();
+    if (it + nw < nitems) vn = row_at((int64_t)dn.y + lane);
+    T best = cur;
+    for (int32_t j = 0; j < d.z; j += 8) {
+      // (a row's padding comes last: column -1)
+      const bool live = col[0] > 0 && (!sorted || relax_add(w[0], dlow) < best);
+      if (!__any_sync(kFullG, live)) break;
+      int32_t cn[8];
+      T wn[8];
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
-        const int64_t pos = (int64_t)d.x + lane + (int64_t)u * 32;
-        col[u] = u < d.z ? __ldcs(colval + pos) : -1;
-        w[u] = u < d.z ? view_weight<T>(nz, tv, pos) : Lim<T>::max();
+        const int64_t pos = (int64_t)d.x + lane + (int64_t)(j + 8 + u) * 32;
+        cn[u] = j + 8 + u < d.z ? __ldcs(colval + pos) : -1;
+        wn[u] = j + 8 + u < d.z ? view_weight<T>(nz, tv, pos) : Lim<T>::max();
       }
-      for (int32_t j = 0; j < d.z; j += 8) {
-        int32_t cn[8];
-        T wn[8];
+      T dv[8];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const int64_t pos = (int64_t)d.x + lane + (int64_t)(j + 8 + u) * 32;
-          cn[u] = j + 8 + u < d.z ? __ldcs(colval + pos) : -1;
-          wn[u] = j + 8 + u < d.z ? view_weight<T>(nz, tv, pos) : Lim<T>::max();
-        }
-        T dv[8];
+      for (int u = 0; u < 8; ++u) dv[u] = live && col[u] > 0 ? ld_l1(dist + (col[u] - 1)) : Lim<T>::max();
 #pragma unroll
-        for (int u = 0; u < 8; ++u) dv[u] = col[u] > 0 ? ld_l1(dist + (col[u] - 1)) : Lim<T>::max();
+      for (int u = 0; u < 8; ++u) {
+        const T cand = relax_add(w[u], dv[u]);
+        best = cand < best ? cand : best;
+      }
 #pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          const T cand = relax_add(w[u], dv[u]);
-          best = cand < best ? cand : best;
-        }
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-          col[u] = cn[u];
-          w[u] = wn[u];
-        }
+      for (int u = 0; u < 8; ++u) {
+        col[u] = cn[u];
+        w[u] = wn[u];
       }
     }
-    pull_lower(srow, m, perm, best, dist, inq_next, wq, edges, prow);
+    pull_lower<T>(v0, best, cur, dist, inq_next, wq, sum, prow);
   }
   wq.flush();
-  warp_add(edges, &ctr->mf);
+  sum.flush(ctr);
 }
 
 // the SELL-32 copy (rows sorted by length) and its work plan, built on first use
@@ -2198,13 +2261,33 @@ static int ensure_pull_sell(gg_ctx* ctx, gg_mat* A) {
   GraphAux* g = A->aux;
   if (g->pull_sell) return GG_OK;
   gg_mat* S = nullptr;
-  GG_CHECK(gg_sell_create(ctx, A, 32, A->m, &S));
+  // the entries of every row by ascending weight (1- and 4-byte types, and where the sort's
+  // buffers fit), then the copy of that
+  bool sorted = false;
+  if (g->nonneg && dtype_size(A->dtype) <= 4 && A->nnz > 0) {
+    gg_mat T;  // a view: rowptr is A's
+    T.m = A->m;
+    T.n = A->n;
+    T.nnz = A->nnz;
+    T.dtype = A->dtype;
+    T.device = A->device;
+    T.rowptr = A->rowptr;
+    cudaError_t e = cudaMalloc((void**)&T.colval, A->nnz * sizeof(int32_t));
+    if (e == cudaSuccess) e = cudaMalloc(&T.nzval, A->nnz * dtype_size(A->dtype));
+    if (e != cudaSuccess) (void)cudaGetLastError();
+    if (e == cudaSuccess && sort_entries_by_value(ctx, A, T.colval, T.nzval) == GG_OK)
+      sorted = gg_sell_create(ctx, &T, 32, A->m, &S) == GG_OK;
+    cudaFree(T.colval);
+    cudaFree(T.nzval);
+  }
+  if (!sorted) GG_CHECK(gg_sell_create(ctx, A, 32, A->m, &S));
   int rc = build_sell_plan(ctx, S);
   if (rc != GG_OK) {
     gg_mat_destroy(S);
     return rc;
   }
   g->pull_sell = S;
+  g->pull_sorted = sorted;
   return GG_OK;
 }
 
@@ -2314,6 +2397,7 @@ static int sssp_fixpoint(gg_ctx* ctx, gg_mat* A, T* d, int64_t* rounds_out) {
   const int32_t small_cap = kSmallCap;
   // large CSR handles pull over a SELL-32 copy (built at the first pull round)
   const bool sell_pull = A->format == GG_FMT_CSR && n >= (1 << 16);
+  T dlow = T(0);  // no distance below it was written in the previous round
   while (nf > 0) {
     if (rounds > max_rounds) return set_error(GG_ERR_NOT_CONVERGED, "shortest_path did not converge");
     if (nf <= small_cap && mf <= (int64_t)kSmallEdges) {
@@ -2326,6 +2410,7 @@ static int sssp_fixpoint(gg_ctx* ctx, gg_mat* A, T* d, int64_t* rounds_out) {
       GG_CUDA(cudaStreamSynchronize(ctx->stream));
       nf = (int64_t)h->nf;
       rounds += (int64_t)h->level;
+      dlow = T(0);
       // the remaining frontier is in q[cur]; its membership bits are in fb[cur] when
       // status == 0, else in fb[cur ^ 1] -- then swap roles so bits and queue agree
       // out-edges of the remaining frontier (counted by the kernel), for the direction
@@ -2349,7 +2434,7 @@ static int sssp_fixpoint(gg_ctx* ctx, gg_mat* A, T* d, int64_t* rounds_out) {
         k_sssp_pull_sell<T><<<ctx->num_sms * (2048 / kPullSellThreads), kPullSellThreads, 0,
                               ctx->stream>>>(S->colval, S->nzval, S->dtype, S->perm, S->m,
                                              SP->pitems, SP->npitems, d, sc.fb[cur ^ 1],
-                                             sc.q[cur ^ 1], sc.ctr, P.rowptr);
+                                             sc.q[cur ^ 1], sc.ctr, P.rowptr, g->pull_sorted, dlow);
       // the consumed membership bitmap becomes the next round's target: clear it
       GG_CUDA(cudaMemsetAsync(sc.fb[cur], 0, ((n + 31) / 32) * sizeof(unsigned), ctx->stream));
       GG_CUDA(cudaGetLastError());
@@ -2357,6 +2442,7 @@ static int sssp_fixpoint(gg_ctx* ctx, gg_mat* A, T* d, int64_t* rounds_out) {
       GG_CUDA(cudaStreamSynchronize(ctx->stream));
       nf = (int64_t)h->nf;
       mf = (int64_t)h->mf;
+      dlow = h->low ? dist_of_bits<T>(~h->low) : T(0);
       cur ^= 1;
       continue;
     }
@@ -2380,6 +2466,7 @@ static int sssp_fixpoint(gg_ctx* ctx, gg_mat* A, T* d, int64_t* rounds_out) {
       GG_CUDA(cudaStreamSynchronize(ctx->stream));
       nf = (int64_t)h->nf;
       mf = (int64_t)h->mf;
+      dlow = h->low ? dist_of_bits<T>(~h->low) : T(0);
       cur ^= 1;
       continue;
     }
@@ -2398,6 +2485,7 @@ static int sssp_fixpoint(gg_ctx* ctx, gg_mat* A, T* d, int64_t* rounds_out) {
     GG_CUDA(cudaStreamSynchronize(ctx->stream));
     nf = (int64_t)h->nf;
     mf = (int64_t)h->mf;
+    dlow = h->low ? dist_of_bits<T>(~h->low) : T(0);
     cur ^= 1;
   }
   if (rounds_out) *rounds_out += rounds;

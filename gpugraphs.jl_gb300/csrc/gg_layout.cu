@@ -133,6 +133,29 @@ int sell_slice_widths(gg_ctx* ctx, const int32_t* rowptr, const int32_t* perm, i
 // slice of p is searched from the one of the thread's previous place.
 static const int kFillTile = 4096;  // places per block step
 
+// the last of n segments s with ptr[s] - 1 <= p (ptr ascending, 1-based, p inside): searched
+// on from the thread's previous segment, usually one of the next few
+struct SegmentCursor {
+  int64_t s = 0;
+  bool first = true;
+  __device__ __forceinline__ void seek(const int32_t* __restrict__ ptr, int64_t n, int64_t p) {
+    if (!first && (int64_t)ptr[s + 1] - 1 > p) return;
+    int64_t lo = first ? 0 : s + 1, hi = n - 1;
+    if (!first)
+      for (int64_t step = 1; lo + step < n; step *= 2)
+        if ((int64_t)ptr[lo + step] - 1 > p) {
+          hi = lo + step - 1;
+          break;
+        }
+    while (lo < hi) {
+      const int64_t mid = (lo + hi + 1) >> 1;
+      if ((int64_t)ptr[mid] - 1 <= p) lo = mid; else hi = mid - 1;
+    }
+    s = lo;
+    first = false;
+  }
+};
+
 template <typename V>
 __global__ void __launch_bounds__(256)
     k_sell_fill(int64_t m, int32_t C, int64_t ns, int64_t nst, const int32_t* __restrict__ rowptr,
@@ -141,24 +164,10 @@ __global__ void __launch_bounds__(256)
                 int32_t* s_colval, V* s_nz) {
   for (int64_t tile = (int64_t)blockIdx.x * kFillTile; tile < nst; tile += (int64_t)gridDim.x * kFillTile) {
     const int64_t end = tile + kFillTile < nst ? tile + kFillTile : nst;
-    int64_t s = 0;
-    bool first = true;
+    SegmentCursor at;
     for (int64_t p = tile + threadIdx.x; p < end; p += blockDim.x) {
-      if (first || (int64_t)slice_ptr[s + 1] - 1 <= p) {  // last slice with slice_ptr[s] - 1 <= p
-        int64_t lo = first ? 0 : s + 1, hi = ns - 1;
-        if (!first)  // usually one of the next few
-          for (int64_t step = 1; lo + step < ns; step *= 2)
-            if ((int64_t)slice_ptr[lo + step] - 1 > p) {
-              hi = lo + step - 1;
-              break;
-            }
-        while (lo < hi) {
-          const int64_t mid = (lo + hi + 1) >> 1;
-          if ((int64_t)slice_ptr[mid] - 1 <= p) lo = mid; else hi = mid - 1;
-        }
-        s = lo;
-        first = false;
-      }
+      at.seek(slice_ptr, ns, p);
+      const int64_t s = at.s;
       const int32_t rel = (int32_t)(p - ((int64_t)slice_ptr[s] - 1));
       const int32_t j = rel / C, o = rel - j * C;
       const int64_t t = s * C + o;
@@ -325,6 +334,96 @@ int sell_resorted(gg_ctx* ctx, const gg_mat* A, gg_mat** out) {
   }
   *out = S;
   return GG_OK;
+}
+
+// ---------------------------------------------------------------------------------
+// a CSR matrix's entries by ascending value within each row
+// ---------------------------------------------------------------------------------
+// ordering bits of a non-negative value: -0.0 (which counts as non-negative, and adds as
+// +0.0 does) becomes +0.0
+__device__ __forceinline__ uint32_t value_key(uint8_t v) { return v; }
+__device__ __forceinline__ uint32_t value_key(uint32_t v) { return v == 0x80000000u ? 0u : v; }
+
+template <typename V>
+__global__ void k_value_max(const V* __restrict__ nz, int64_t nnz, unsigned* out) {
+  uint32_t mx = 0;
+  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < nnz;
+       k += (int64_t)gridDim.x * blockDim.x)
+    mx = max(mx, value_key(nz[k]));
+  mx = __reduce_max_sync(0xffffffffu, mx);
+  if ((threadIdx.x & 31) == 0 && mx) atomicMax(out, mx);
+}
+
+template <typename V>
+__global__ void __launch_bounds__(256)
+    k_entry_keys(int64_t m, int64_t nnz, const int32_t* __restrict__ rowptr, const V* __restrict__ nz,
+                 int vbits, uint64_t* __restrict__ key) {
+  for (int64_t tile = (int64_t)blockIdx.x * kFillTile; tile < nnz; tile += (int64_t)gridDim.x * kFillTile) {
+    const int64_t end = tile + kFillTile < nnz ? tile + kFillTile : nnz;
+    SegmentCursor at;
+    for (int64_t p = tile + threadIdx.x; p < end; p += blockDim.x) {
+      at.seek(rowptr, m, p);
+      key[p] = ((uint64_t)at.s << vbits) | value_key(nz[p]);
+    }
+  }
+}
+
+template <typename V>
+__global__ void k_key_values(const uint64_t* __restrict__ key, int64_t nnz, int vbits, V* __restrict__ nz) {
+  const uint64_t low = (1ull << vbits) - 1;
+  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < nnz;
+       k += (int64_t)gridDim.x * blockDim.x)
+    nz[k] = (V)(key[k] & low);
+}
+
+template <typename V>
+static int sort_entries_t(gg_ctx* ctx, const gg_mat* A, int32_t* col, V* nz) {
+  const int64_t m = A->m, nnz = A->nnz;
+  cudaStream_t st = ctx->stream;
+  const V* src = static_cast<const V*>(A->nzval);
+  unsigned h = 0;
+  uint64_t *key = nullptr, *key2 = nullptr;
+  void* tmp = nullptr;
+  size_t tmp_bytes = 0;
+  cudaError_t e = cudaMemsetAsync(ctx->d_flags, 0, sizeof(unsigned), st);
+  if (e == cudaSuccess) {
+    k_value_max<V><<<grid_of(ctx, nnz), 256, 0, st>>>(src, nnz, ctx->d_flags);
+    e = cudaMemcpyAsync(ctx->h_flags, ctx->d_flags, sizeof(unsigned), cudaMemcpyDeviceToHost, st);
+  }
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  h = ctx->h_flags[0];
+  const int vbits = bits_of(h), bits = vbits + bits_of((uint64_t)(m > 0 ? m - 1 : 0));
+  if (e == cudaSuccess) e = cudaMallocAsync((void**)&key, nnz * sizeof(uint64_t), st);
+  if (e == cudaSuccess) e = cudaMallocAsync((void**)&key2, nnz * sizeof(uint64_t), st);
+  if (e == cudaSuccess) {
+    int64_t g = (nnz + kFillTile - 1) / kFillTile;
+    if (g > (int64_t)ctx->num_sms * 8) g = (int64_t)ctx->num_sms * 8;
+    k_entry_keys<V><<<(int)g, 256, 0, st>>>(m, nnz, A->rowptr, src, vbits, key);
+    e = cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, key, key2, A->colval, col, nnz, 0,
+                                        bits > 0 ? bits : 1, st);
+  }
+  if (e == cudaSuccess) e = cudaMallocAsync(&tmp, tmp_bytes > 0 ? tmp_bytes : 1, st);
+  if (e == cudaSuccess)
+    e = cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, key, key2, A->colval, col, nnz, 0,
+                                        bits > 0 ? bits : 1, st);
+  if (e == cudaSuccess) {
+    k_key_values<V><<<grid_of(ctx, nnz), 256, 0, st>>>(key2, nnz, vbits, nz);
+    e = cudaGetLastError();
+  }
+  if (key) cudaFreeAsync(key, st);
+  if (key2) cudaFreeAsync(key2, st);
+  if (tmp) cudaFreeAsync(tmp, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e != cudaSuccess) return cuda_error(e, "entry order");
+  return GG_OK;
+}
+
+// A CSR handle's entries ordered by value within each row (values non-negative, 1 or 4
+// bytes: their bits order as they do) into col / nz (device, nnz each); rowptr as A's
+int sort_entries_by_value(gg_ctx* ctx, const gg_mat* A, int32_t* col, void* nz) {
+  if (A->nnz == 0) return GG_OK;
+  if (dtype_size(A->dtype) == 1) return sort_entries_t<uint8_t>(ctx, A, col, static_cast<uint8_t*>(nz));
+  return sort_entries_t<uint32_t>(ctx, A, col, static_cast<uint32_t*>(nz));
 }
 
 __global__ void k_iota(int32_t* p, int64_t n) {

@@ -126,3 +126,44 @@ def test_many_graphs_in_bands(dtype):
     for _ in range(2):
         for got, A, s in zip(mg.split(mg.sssp(src)), gs, src):
             assert torch.equal(got, G.shortest_path(A, s))
+
+
+@pytest.mark.parametrize("dtype", [np.bool_, np.int32, np.float32, np.float64, np.int64])
+@pytest.mark.parametrize("kind", ["spread", "zeros", "equal", "infinite"])
+def test_pull_rounds_stop_at_weights(dtype, kind):
+    """Shortest paths through pull rounds whose rows are scanned by ascending weight:
+    zero weights (-0.0 among them), equal ones, nine decades, +Inf, and hub rows of
+    several chunks; distances equal Dijkstra's bit for bit, from several sources."""
+    n = 70001
+    rng = np.random.default_rng(11)
+    r = rng.integers(0, n, 9 * n)
+    c = np.where(rng.random(9 * n) < 0.3, rng.integers(0, 40, 9 * n), rng.integers(0, n, 9 * n))
+    lo, hi = np.minimum(r, c), np.maximum(r, c)
+    key = np.unique((lo * n + hi)[lo != hi])
+    w = {"spread": np.floor(10.0 ** rng.uniform(0, 6, len(key))),
+         "zeros": rng.integers(0, 3, len(key)) * 7.0,
+         "equal": np.full(len(key), 3.0),
+         "infinite": rng.integers(1, 50, len(key)).astype(float)}[kind]
+    lo, hi = key // n, key % n
+    rows, cols = np.concatenate([lo, hi]), np.concatenate([hi, lo])
+    order = np.lexsort((cols, rows))
+    vals = np.concatenate([w, w])[order]
+    if kind == "zeros" and np.issubdtype(dtype, np.floating):
+        vals = np.where(vals == 0, -0.0, vals)
+    if kind == "infinite" and np.issubdtype(dtype, np.floating):
+        edge = np.minimum(rows, cols)[order] * n + np.maximum(rows, cols)[order]
+        vals = np.where(edge % 5 == 0, np.inf, vals)
+    rp = np.ones(n + 1, np.int32)
+    rp[1:] += np.cumsum(np.bincount(rows, minlength=n)).astype(np.int32)
+    cv, nz = (cols[order] + 1).astype(np.int32), vals.astype(dtype)
+    assert np.diff(rp).max() > 1000
+    A = G.SparseGPUMatrixCSR(n, n, rp, cv, nz)
+    for s in (1, 35000):
+        got = G.shortest_path(A, s).cpu().numpy()
+        if dtype in (np.bool_, np.int32, np.float32):
+            assert (got == O.sssp_dijkstra(n, rp, cv, nz, s, symmetric=True)).all()
+        else:  # whole numbers below 2^24: the 64-bit types' distances are the Float32 ones
+            ref = O.sssp_dijkstra(n, rp, cv, nz.astype(np.float32), s, symmetric=True).astype(np.float64)
+            exact = ref < 2 ** 24
+            far = got.astype(np.float64) if dtype == np.float64 else np.where(got == np.iinfo(dtype).max, np.inf, got.astype(np.float64))
+            assert (far[exact] == ref[exact]).all() and np.array_equal(np.isinf(far), np.isinf(ref))
