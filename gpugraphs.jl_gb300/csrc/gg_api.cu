@@ -225,8 +225,8 @@ int gg_init(int device, gg_ctx** out) {
   gg_ctx* c = new gg_ctx();
   c->device = device;
   cudaError_t e = cudaDeviceGetAttribute(&c->num_sms, cudaDevAttrMultiProcessorCount, device);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&c->d_flags, 64 * sizeof(unsigned));
-  if (e == cudaSuccess) e = cudaMallocHost((void**)&c->h_flags, 64 * sizeof(unsigned));
+  if (e == cudaSuccess) e = cudaMalloc((void**)&c->d_flags, kFlagWords * sizeof(unsigned));
+  if (e == cudaSuccess) e = cudaMallocHost((void**)&c->h_flags, kFlagWords * sizeof(unsigned));
   if (e == cudaSuccess) e = cudaMalloc((void**)&c->d_err, sizeof(unsigned));
   if (e == cudaSuccess) e = cudaMemset(c->d_err, 0, sizeof(unsigned));
   if (e != cudaSuccess) {

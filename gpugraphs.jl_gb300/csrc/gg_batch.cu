@@ -7,7 +7,12 @@
 //    vertex, one bottom-up level per launch; column q equals
 //    bfs_distances(A_T, sources[q]).
 //  * gg_sssp_batch: 32 sources per group, one relaxation round per launch; column q
-//    equals shortest_path(A_T, sources[q]).
+//    equals shortest_path(A_T, sources[q]).  Large graphs relax light edges first: most
+//    distances settle over the lighter half-mean weights, a quarter of the edges when
+//    weights are even, and the heavy ones are then visited a few times instead of in
+//    every round.
+#include <string.h>
+
 #include <algorithm>
 #include <vector>
 
@@ -176,13 +181,22 @@ __global__ void k_bs_seed(T* D, const int64_t* src, int64_t S, unsigned* changed
   }
 }
 
-// vertex-major 32-column block -> caller's column-major dist
+// vertex-major 32-column block -> caller's column-major dist, 32 x 32 tiles through
+// shared memory (both sides coalesced: 265 -> 43 us for 2^20 vertices)
 template <typename T>
-__global__ void k_bs_out(const T* D, int64_t n, int64_t S, T* dist, int64_t ld) {
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n * S;
-       t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t q = t / n, v = t - q * n;
-    dist[q * ld + v] = D[v * 32 + q];
+__global__ void __launch_bounds__(256)
+    k_bs_out(const T* __restrict__ D, int64_t n, int64_t S, T* __restrict__ dist, int64_t ld) {
+  __shared__ T tile[32][33];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  for (int64_t v0 = (int64_t)blockIdx.x * 32; v0 < n; v0 += (int64_t)gridDim.x * 32) {
+#pragma unroll
+    for (int q = 0; q < 32; q += 8)
+      if (v0 + ty + q < n) tile[ty + q][tx] = __ldcs(D + (v0 + ty + q) * 32 + tx);
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 32; q += 8)
+      if (v0 + tx < n && ty + q < S) __stcs(dist + (int64_t)(ty + q) * ld + v0 + tx, tile[tx][ty + q]);
+    __syncthreads();
   }
 }
 
@@ -202,16 +216,34 @@ __global__ void k_ms_degsum(const int32_t* __restrict__ cq, const unsigned long 
   if ((threadIdx.x & 31) == 0 && s) atomicAdd(out, s);
 }
 
-static const int kBsStreams = 8;  // 32-source groups run at once (8 x 32 bytes of ctx->h_flags)
-// with the SELL-32 full rounds a round is restricted to the marked vertices while the
-// out-edges of the changed vertices stay below nnz / kBsSellRestrict
-#ifndef GG_BS_SELL_RESTRICT
-#define GG_BS_SELL_RESTRICT 16
-#endif
-static const int64_t kBsSellRestrict = GG_BS_SELL_RESTRICT;
+static const int kBsStreams = 8;  // 32-source groups run at once (8 x 64 bytes of ctx->h_flags)
+static_assert(kBsStreams * 16 <= kFlagWords, "counters of the groups");
+// With row rounds (k_ms_round_rows) a round is restricted to the marked vertices while
+// the out-edges of the changed vertices stay below nnz / kBsRowRestrict; the column masks
+// of in-neighbours are looked at once fewer than n x kBsCheck pairs dropped; the light
+// phase ends once fewer than n x kBsLightEnd did.
+// (256 sources on R-MAT scale 20, ms: check at n x 16 / 8 / 3 / 1 37.2 / 36.3 / 34.9 / 34.4;
+// light phase ending at n x 4 / 1 / 0.25 37.0 / 36.3 / 37.0; restricted below nnz / 16 / 32 /
+// 64 36.3 / 35.8 / 35.7.)
+static const int64_t kBsRowRestrict = 16;
+static const int64_t kBsCheck = 1;
+static const double kBsLightEnd = 1.0;
+// light edges: at most this multiple of the mean weight (0 / 0.25 / 0.5 / 1: 40.3 / 35.3 /
+// 36.3 / 37.0 ms); graphs of a smaller mean degree skip the phase (their light edges
+// leave them in pieces)
+static const double kBsCap = 0.5;
+static const int64_t kBsLightDegree = 16;
+
+// the row rounds' view of the graph; rows.col is nullptr where there is none
+struct BsRows {
+  MsRows rows = {};
+  double cap = -1.0;  // light edges' largest weight, < 0: no light phase
+};
 
 // Work buffers of one batched shortest-path call.  ctr: [0] vertices changed this
-// round, [1] / [2] lengths of the changed queues cq[0] / cq[1], [3] marked vertices.
+// round, [1] / [2] lengths of the changed queues cq[0] / cq[1], [3] marked vertices, then
+// the out-edges of the changed ones, [4] hubs being marked, [5] pairs that dropped, [6]
+// smallest distance written (MsSums).
 template <typename T>
 struct BsWork {
   T* D;
@@ -240,6 +272,11 @@ struct BsRun {
   T* dist = nullptr;
   int cur = 0;
   bool restricted = false, done = false;
+  // light phase: heavy edges are being left out (light), some were (owed: every row has to
+  // be visited once more before the result is final)
+  bool light = false, owed = false;
+  int64_t pairs = 0;  // (vertex, column) pairs that dropped in the last round
+  T dlow = T(0);      // no distance below it was written in the last round
 };
 
 template <typename T>
@@ -279,11 +316,12 @@ static int bs_start(gg_ctx* ctx, int64_t n, BsRun<T>& R) {
   k_bs_init<T><<<(int)gb, 256, 0, R.st>>>(R.w.D, n, R.dsrc, R.S, R.w.c[0]);
   k_bs_seed<T><<<1, 64, 0, R.st>>>(R.w.D, R.dsrc, R.S, R.w.c[0], R.w.cq[0]);
   GG_CUDA(cudaGetLastError());
-  R.h[0] = 0;
+  for (int i = 0; i < 8; ++i) R.h[i] = 0;
   R.h[1] = (unsigned long long)R.S;
-  R.h[2] = 0;
-  R.h[3] = 0;
-  GG_CUDA(cudaMemcpyAsync(R.w.ctr, R.h, 4 * sizeof(unsigned long long), cudaMemcpyHostToDevice, R.st));
+  GG_CUDA(cudaMemcpyAsync(R.w.ctr, R.h, 8 * sizeof(unsigned long long), cudaMemcpyHostToDevice, R.st));
+  R.pairs = R.S;
+  R.dlow = T(0);
+  R.owed = false;
   R.nchanged = R.S;
   R.mchanged = -1;  // unknown before the first round
   return GG_OK;
@@ -302,7 +340,7 @@ static int bs_degsum(gg_ctx* ctx, const int32_t* prow, const int32_t* cq,
 // one round of group R, enqueued on its stream; the counters land in R.h
 template <typename T>
 static int bs_issue(gg_ctx* ctx, int64_t n, int64_t nnz, const BatchGraph& g, const HubPlan* hp,
-                    const int32_t* prow, const int32_t* pcol, const gg_mat* sell, BsRun<T>& R) {
+                    const int32_t* prow, const int32_t* pcol, const BsRows& br, BsRun<T>& R) {
   int64_t gb = (n * 32 + 255) / 256;
   if (gb > (int64_t)ctx->num_sms * 8) gb = (int64_t)ctx->num_sms * 8;
   int64_t pb = (hp->npiece * 32 + 255) / 256;
@@ -317,45 +355,58 @@ static int bs_issue(gg_ctx* ctx, int64_t n, int64_t nnz, const BatchGraph& g, co
   GG_CUDA(cudaMemsetAsync(w.ctr, 0, sizeof(unsigned long long), R.st));
   GG_CUDA(cudaMemsetAsync(ncq_nxt, 0, sizeof(unsigned long long), R.st));
   GG_CUDA(cudaMemsetAsync(w.c[cur ^ 1], 0, (size_t)n * sizeof(unsigned), R.st));
-  // with the SELL-32 full rounds (about half the vertex rounds' cost) a round is
-  // restricted to the marked vertices only while the changed ones are fewer
-  R.restricted = (sell && R.mchanged >= 0) ? R.mchanged * kBsSellRestrict < nnz
-                                            : R.nchanged * avg_deg * 4 < nnz;
+  GG_CUDA(cudaMemsetAsync(w.ctr + 5, 0, 2 * sizeof(unsigned long long), R.st));
+  const MsSums sums{w.ctr + 5, w.ctr + 6};
+  const bool by_row = sizeof(T) == 4 && br.rows.col != nullptr;
+  R.restricted = (by_row && R.mchanged >= 0) ? R.mchanged * kBsRowRestrict < nnz
+                                             : R.nchanged * avg_deg * 4 < nnz;
+  bool settle = false;  // this round visits every row over every edge
+  if (by_row && R.light && R.owed && (R.restricted || (double)R.pairs < kBsLightEnd * (double)n)) {
+    R.light = R.owed = R.restricted = false;
+    settle = true;
+  }
   if (R.restricted) {
     GG_CUDA(cudaMemsetAsync(w.mark, 0, ((n + 31) / 32) * sizeof(unsigned), R.st));
     GG_CUDA(cudaMemsetAsync(w.ctr + 3, 0, sizeof(unsigned long long), R.st));
     GG_CUDA(launch_ms_mark(R.st, ctx->num_sms, R.nchanged, prow, pcol, w.cq[cur], ncq_cur, w.mark,
                            w.vlist, w.ctr + 3, w.mhq, w.ctr + 4, w.mhoff));
     k_ms_round<T><<<(int)gcap, 256, 0, R.st>>>(n, g, w.D, w.c[cur], w.c[cur ^ 1], w.ctr, nullptr,
-                                               w.vlist, w.ctr + 3, w.cq[cur ^ 1], ncq_nxt);
-  } else if (sell) {
-    // every vertex over the SELL-32 copy (hubs included, as chunks of their rows)
+                                               w.vlist, w.ctr + 3, w.cq[cur ^ 1], ncq_nxt, sums);
+  } else if (by_row) {
+    // every row, hubs in pieces
     if constexpr (sizeof(T) == 4) {
-      const size_t smem = kMsSellWarps * sizeof(MsSellWarpSmem<T>);
-      k_ms_round_sell<T><<<ctx->num_sms * 4, kMsSellWarps * 32, smem, R.st>>>(
-          sell->colval, sell->nzval, sell->dtype, sell->perm, sell->m, sell->sellplan->pitems,
-          sell->sellplan->npitems, w.D, w.c[cur], w.c[cur ^ 1], w.ctr, nullptr, w.cq[cur ^ 1],
-          ncq_nxt);
+      int64_t rb = ((br.rows.nitems + br.rows.nshort + 3) / 4 + 7) / 8;
+      if (rb > (int64_t)ctx->num_sms * kMsRowBlocks) rb = (int64_t)ctx->num_sms * kMsRowBlocks;
+      if (rb < 1) rb = 1;
+      const T cap = R.light ? static_cast<T>(br.cap) : Lim<T>::max();
+      const T dlow = settle ? T(0) : R.dlow;
+      if (R.light) R.owed = true;
+      if (!settle && R.pairs < kBsCheck * n)
+        k_ms_round_rows<T, true><<<(int)rb, 256, 0, R.st>>>(br.rows, w.D, w.c[cur], w.c[cur ^ 1], w.ctr,
+                                                            nullptr, w.cq[cur ^ 1], ncq_nxt, sums, dlow, cap);
+      else
+        k_ms_round_rows<T, false><<<(int)rb, 256, 0, R.st>>>(br.rows, w.D, w.c[cur], w.c[cur ^ 1], w.ctr,
+                                                             nullptr, w.cq[cur ^ 1], ncq_nxt, sums, dlow, cap);
       GG_CUDA(cudaGetLastError());
       GG_CHECK(bs_degsum(ctx, prow, w.cq[cur ^ 1], ncq_nxt, w.ctr, R.st));
-      GG_CUDA(cudaMemcpyAsync(R.h, w.ctr, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, R.st));
+      GG_CUDA(cudaMemcpyAsync(R.h, w.ctr, 8 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, R.st));
       return GG_OK;
     }
   } else {
     // every non-hub vertex, in the plan's order: the long rows first, spread over the warps
     k_ms_round<T><<<(int)gb, 256, 0, R.st>>>(n, g, w.D, w.c[cur], w.c[cur ^ 1], w.ctr, nullptr,
-                                             hp->order, hp->d_norder, w.cq[cur ^ 1], ncq_nxt);
+                                             hp->order, hp->d_norder, w.cq[cur ^ 1], ncq_nxt, sums);
   }
   GG_CUDA(cudaGetLastError());
   if (hp->npiece > 0) {
     k_ms_round_hub<T><<<(int)pb, 256, 0, R.st>>>(g, hp->pieces, hp->npiece, hp->hubs, w.D,
                                                  w.c[cur], w.c[cur ^ 1], w.ctr, nullptr,
                                                  R.restricted ? w.mark : nullptr, w.cq[cur ^ 1],
-                                                 ncq_nxt);
+                                                 ncq_nxt, sums);
     GG_CUDA(cudaGetLastError());
   }
   GG_CHECK(bs_degsum(ctx, prow, w.cq[cur ^ 1], ncq_nxt, w.ctr, R.st));
-  GG_CUDA(cudaMemcpyAsync(R.h, w.ctr, 4 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, R.st));
+  GG_CUDA(cudaMemcpyAsync(R.h, w.ctr, 8 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, R.st));
   return GG_OK;
 }
 
@@ -368,16 +419,16 @@ static int sssp_batch_t(gg_ctx* ctx, gg_mat* A, const BatchGraph& g, const int64
   const int32_t* pcol = nullptr;
   GG_CHECK(push_view(ctx, A, &prow, &pcol));
   const HubPlan* hp = A->hubplan;
-  // full rounds over the SELL-32 copy of large CSR graphs (4-byte distances: a warp
-  // keeps 32 rows x 32 columns of minima in registers)
-  const gg_mat* sell = nullptr;
+  // rounds over every row of CSR graphs with 4-byte distances: rows by ascending weight
+  // (where they fit), the SpMM plan's work lists
+  BsRows br;
   if constexpr (sizeof(T) == 4) {
-    const int prc = pull_sell_copy(ctx, A, &sell);
-    if (prc == GG_ERR_OOM) sell = nullptr;  // no room for the copy: vertex rounds only
-    else GG_CHECK(prc);
-    if (sell)
-      GG_CUDA(cudaFuncSetAttribute(k_ms_round_sell<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)(kMsSellWarps * sizeof(MsSellWarpSmem<T>))));
+    double mean_w = 0.0;
+    GG_CHECK(ms_rows_of(ctx, A, &br.rows, &mean_w));
+    if (br.rows.col) {
+      const double cap = kBsCap * mean_w;
+      if ((int64_t)A->nnz >= kBsLightDegree * n && cap > 0.0 && cap < (double)Lim<T>::max() / 2) br.cap = cap;
+    }
   }
   // a hub may enter a changed queue once per piece
   const int64_t qcap = n + hp->npiece + 64;
@@ -400,7 +451,7 @@ static int sssp_batch_t(gg_ctx* ctx, gg_mat* A, const BatchGraph& g, const int64
       rc = set_error(GG_ERR_CUDA, "stream creation failed");
       break;
     }
-    R.h = hbase + 4 * i;
+    R.h = hbase + 8 * i;
     if (cudaStreamWaitEvent(R.st, ready, 0) != cudaSuccess) rc = set_error(GG_ERR_CUDA, "stream wait");
     if (rc == GG_OK) rc = bs_alloc<T>(R.w, n, qcap, R.st);
     R.done = true;  // not started
@@ -415,6 +466,7 @@ static int sssp_batch_t(gg_ctx* ctx, gg_mat* A, const BatchGraph& g, const int64
     R.cur = 0;
     R.r = 0;
     R.done = false;
+    R.light = br.cap >= 0.0;
     ++next_group;
     return bs_start<T>(ctx, n, R);
   };
@@ -425,7 +477,7 @@ static int sssp_batch_t(gg_ctx* ctx, gg_mat* A, const BatchGraph& g, const int64
   while (active && rc == GG_OK) {
     active = false;
     for (auto& R : runs)
-      if (!R.done && rc == GG_OK) rc = bs_issue<T>(ctx, n, nnz, g, hp, prow, pcol, sell, R);
+      if (!R.done && rc == GG_OK) rc = bs_issue<T>(ctx, n, nnz, g, hp, prow, pcol, br, R);
     for (auto& R : runs) {
       if (R.done || rc != GG_OK) continue;
       if (cudaStreamSynchronize(R.st) != cudaSuccess) {
@@ -434,7 +486,7 @@ static int sssp_batch_t(gg_ctx* ctx, gg_mat* A, const BatchGraph& g, const int64
       }
       if (rounds) *rounds += 1;
       ++R.r;
-      if (R.h[0] == 0) {  // converged: write the group out, take the next one
+      if (R.h[0] == 0 && !R.owed) {  // converged: write the group out, take the next one
         k_bs_out<T><<<(int)gb, 256, 0, R.st>>>(R.w.D, n, R.S, R.dist, ld);
         R.done = true;
         rc = start_next(R);
@@ -443,6 +495,10 @@ static int sssp_batch_t(gg_ctx* ctx, gg_mat* A, const BatchGraph& g, const int64
       } else {
         R.nchanged = (int64_t)R.h[1 + (R.cur ^ 1)];
         R.mchanged = (int64_t)R.h[3];
+        R.pairs = (int64_t)R.h[5];
+        const unsigned low = ~(unsigned)R.h[6];
+        if (sizeof(T) == 4 && R.h[6]) memcpy(&R.dlow, &low, 4);
+        else R.dlow = T(0);
         R.cur ^= 1;
       }
       if (!R.done) active = true;

@@ -376,7 +376,7 @@ struct MMPlan {
   // CSR: the rows of at most 32 entries (the short-row kernel's), longest first, so
   // the four rows a warp takes have about the same length
   int32_t* short_rows = nullptr;
-  int64_t nshort = 0;
+  int64_t nshort = 0, nlive = 0;  // nlive: the leading ones that hold an entry
 };
 static const int kSegMM = 256;
 
@@ -502,6 +502,10 @@ static const int kSegNnz = 4096;
 
 }  // namespace gg
 
+namespace gg {
+static const int kFlagWords = 128;  // words of gg_ctx::d_flags / h_flags
+}
+
 struct gg_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -610,6 +614,7 @@ gg_mat* sell_for_spmv(gg_ctx* ctx, gg_mat* A);
 int spmv_typed(gg_ctx* ctx, gg_mat* A, int tc, int mul, int add, int accum, void* y, int ty,
                const void* x, int tx, const void* mask, int tmask, int64_t lo, int64_t hi, bool* done);
 int build_row_blocks(gg_ctx* ctx, gg_mat* A);
+int build_mm_plan(gg_ctx* ctx, gg_mat* A);  // gg_spmm.cu
 int build_sell_plan(gg_ctx* ctx, gg_mat* A);
 int launch_col1_sell(gg_ctx* ctx, gg_mat* A, const float* x, float* y);  // gg_spmv.cu
 int build_hub_plan(gg_ctx* ctx, gg_mat* A, const int32_t* rowptr, int64_t n);  // gg_batch.cu

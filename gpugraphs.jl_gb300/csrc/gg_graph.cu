@@ -55,12 +55,19 @@ struct GraphAux {
   // entries by ascending weight when pull_sorted
   gg_mat* pull_sell = nullptr;
   bool pull_sorted = false;
+  // CSR handles, batched shortest paths: the entries of every row by ascending weight
+  // (rowptr is the handle's), built on first use
+  int32_t* srt_col = nullptr;
+  void* srt_w = nullptr;
+  bool srt_failed = false;  // did not fit
 };
 
 void free_graph_aux(gg_mat* A) {
   GraphAux* g = A->aux;
   if (!g) return;
   if (g->pull_sell) gg_mat_destroy(g->pull_sell);
+  cudaFree(g->srt_col);
+  cudaFree(g->srt_w);
   if (g->owns_view) {
     cudaFree(g->vrowptr);
     cudaFree(g->vcolval);
@@ -1871,17 +1878,6 @@ __global__ void __launch_bounds__(kNfThreads, 1)
   }
 }
 
-template <typename T>
-__global__ void k_sum_weights(const T* __restrict__ w, int64_t nnz, double* out) {
-  double s = 0.0;
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < nnz;
-       k += (int64_t)gridDim.x * blockDim.x)
-    s += (double)w[k];
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(kFullG, s, o);
-  if ((threadIdx.x & 31) == 0) atomicAdd(out, s);
-}
-
 // ---------------------------------------------------------------------------------
 // pull rounds for large frontiers: every vertex takes the minimum over its in-edges
 // from vertices that changed in the previous round (membership bitmap chg), in place.
@@ -1898,6 +1894,16 @@ __device__ __forceinline__ T view_weight(const void* nz, int tv, int64_t k) {
     case GG_FLOAT32: return static_cast<T>(static_cast<const float*>(nz)[k]);
   }
   return static_cast<T>(static_cast<const double*>(nz)[k]);
+}
+
+__global__ void k_sum_weights(const void* __restrict__ nz, int tv, int64_t nnz, double* out) {
+  double s = 0.0;
+  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < nnz;
+       k += (int64_t)gridDim.x * blockDim.x)
+    s += view_weight<double>(nz, tv, k);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(kFullG, s, o);
+  if ((threadIdx.x & 31) == 0) atomicAdd(out, s);
 }
 
 template <typename T>
@@ -2256,6 +2262,20 @@ __global__ void __launch_bounds__(kPullSellThreads)
   sum.flush(ctr);
 }
 
+// mean stored weight (as the distance type holds it), once per matrix
+static int mean_weight(gg_ctx* ctx, gg_mat* A) {
+  GraphAux* g = A->aux;
+  double* dsum = reinterpret_cast<double*>(ctx->d_flags + 2);
+  GG_CUDA(cudaMemsetAsync(dsum, 0, sizeof(double), ctx->stream));
+  k_sum_weights<<<gridsz(ctx, A->nnz), 256, 0, ctx->stream>>>(g->vnz, A->dtype, A->nnz, dsum);
+  GG_CUDA(cudaGetLastError());
+  GG_CUDA(cudaMemcpyAsync(ctx->h_flags + 2, dsum, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+  GG_CUDA(cudaStreamSynchronize(ctx->stream));
+  const double sum = *reinterpret_cast<const double*>(ctx->h_flags + 2);
+  g->avg_w = A->nnz > 0 ? sum / (double)A->nnz : 1.0;
+  return GG_OK;
+}
+
 // the SELL-32 copy (rows sorted by length) and its work plan, built on first use
 static int ensure_pull_sell(gg_ctx* ctx, gg_mat* A) {
   GraphAux* g = A->aux;
@@ -2291,14 +2311,35 @@ static int ensure_pull_sell(gg_ctx* ctx, gg_mat* A) {
   return GG_OK;
 }
 
-// The SELL-32 copy (rows sorted by length, with its work items) of the shortest-path
-// pull rounds, built on first use; nullptr for SELL handles and CSR handles of fewer
-// than 65536 rows.
-int pull_sell_copy(gg_ctx* ctx, gg_mat* A, const gg_mat** out) {
-  *out = nullptr;
-  if (A->format != GG_FMT_CSR || A->m < (1 << 16) || !A->aux) return GG_OK;
-  GG_CHECK(ensure_pull_sell(ctx, A));
-  *out = A->aux->pull_sell;
+// The rows of a CSR handle with their entries by ascending weight, for the batched
+// shortest paths (rowptr is A's); *col stays nullptr where there are none: SELL handles,
+// 8-byte or negative weights, no room.
+int weight_sorted_rows(gg_ctx* ctx, gg_mat* A, const int32_t** col, const void** w, double* mean_w) {
+  *col = nullptr;
+  *w = nullptr;
+  *mean_w = 0.0;
+  if (A->format != GG_FMT_CSR || !A->aux || !A->aux->nonneg || dtype_size(A->dtype) > 4 || A->nnz == 0)
+    return GG_OK;
+  GraphAux* g = A->aux;
+  if (!g->srt_col && !g->srt_failed) {
+    cudaError_t e = cudaMalloc((void**)&g->srt_col, A->nnz * sizeof(int32_t));
+    if (e == cudaSuccess) e = cudaMalloc(&g->srt_w, A->nnz * dtype_size(A->dtype));
+    int rc = e == cudaSuccess ? sort_entries_by_value(ctx, A, g->srt_col, g->srt_w)
+                              : cuda_error(e, "weight-sorted rows");
+    if (rc != GG_OK) {
+      cudaFree(g->srt_col);
+      cudaFree(g->srt_w);
+      g->srt_col = nullptr;
+      g->srt_w = nullptr;
+      g->srt_failed = true;
+      if (rc != GG_ERR_OOM) return rc;
+    }
+  }
+  if (!g->srt_col) return GG_OK;
+  if (g->avg_w < 0) GG_CHECK(mean_weight(ctx, A));
+  *col = g->srt_col;
+  *w = g->srt_w;
+  *mean_w = g->avg_w;
   return GG_OK;
 }
 
@@ -2358,18 +2399,7 @@ static int sssp_fixpoint(gg_ctx* ctx, gg_mat* A, T* d, int64_t* rounds_out) {
   const bool coop_ok = P.max_deg <= kCoopMaxDeg && n >= (1 << 16);
   if (coop_ok && nf > 0) {
     // hub-free graph: the whole search in one near-far ordered persistent launch
-    if (g->avg_w < 0) {
-      double* dsum = nullptr;
-      GG_CUDA(cudaMallocAsync((void**)&dsum, sizeof(double), ctx->stream));
-      GG_CUDA(cudaMemsetAsync(dsum, 0, sizeof(double), ctx->stream));
-      k_sum_weights<T><<<gridsz(ctx, P.nnz), 256, 0, ctx->stream>>>(static_cast<const T*>(P.w), P.nnz,
-                                                                    dsum);
-      double hs = 0.0;
-      GG_CUDA(cudaMemcpyAsync(&hs, dsum, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-      GG_CUDA(cudaStreamSynchronize(ctx->stream));
-      cudaFree(dsum);
-      g->avg_w = P.nnz > 0 ? hs / (double)P.nnz : 1.0;
-    }
+    if (g->avg_w < 0) GG_CHECK(mean_weight(ctx, A));
     double dd = g->avg_w * kNearFarScale;
     if (!(dd > 0.0)) dd = 1.0;
     T delta = static_cast<T>(dd);

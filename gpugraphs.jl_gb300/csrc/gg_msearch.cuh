@@ -16,6 +16,7 @@
 //    is that of shortest_path's Jacobi rounds (src/algorithms/shortest_path.jl:61-80).
 #pragma once
 
+#include "gg_queue.cuh"
 #include "gg_semiring.cuh"
 
 namespace gg {
@@ -25,7 +26,8 @@ int graph_view(gg_ctx* ctx, gg_mat* A, const int32_t** rp, const int32_t** cv, c
 int build_hub_plan(gg_ctx* ctx, gg_mat* A, const int32_t* rowptr, int64_t n);  // gg_batch.cu
 int push_view(gg_ctx* ctx, gg_mat* A, const int32_t** prow, const int32_t** pcol);  // gg_graph.cu
 int sssp_prepare(gg_ctx* ctx, gg_mat* A);  // gg_graph.cu
-int pull_sell_copy(gg_ctx* ctx, gg_mat* A, const gg_mat** out);  // gg_graph.cu
+int weight_sorted_rows(gg_ctx* ctx, gg_mat* A, const int32_t** col, const void** w,
+                       double* mean_w);  // gg_graph.cu
 
 namespace {
 
@@ -267,19 +269,22 @@ __device__ __forceinline__ bool bs_pull(const BatchGraph& g, const T* D,
                                         const unsigned* __restrict__ chg, const unsigned* chg_cur,
                                         int64_t k0, int64_t k1, int lane, T& best) {
   bool any = false;
-  for (int64_t kb = k0; kb < k1; kb += 32) {
-    const int64_t kk = kb + lane;
-    int32_t u = -1;
-    unsigned cm = 0;
-    T wl = T(0);
-    if (kk < k1) {
-      const int32_t c = __ldg(g.colval + kk) - 1;
-      cm = __ldcg(chg + c) | __ldcg(chg_cur + c);
-      if (cm) {
-        u = c;
-        wl = b_weight<T>(g.nz, g.tv, kk);
-      }
-    }
+  // columns and masks of 128 edges in flight (few of a late round's neighbours changed: a
+  // 2048-edge hub piece was 64 chains of two round trips)
+  for (int64_t kb4 = k0; kb4 < k1; kb4 += 128) {
+   int32_t c4[4];
+   unsigned m4[4];
+#pragma unroll
+   for (int t = 0; t < 4; ++t)
+     c4[t] = kb4 + t * 32 + lane < k1 ? __ldg(g.colval + kb4 + t * 32 + lane) - 1 : -1;
+#pragma unroll
+   for (int t = 0; t < 4; ++t) m4[t] = c4[t] >= 0 ? (__ldcg(chg + c4[t]) | __ldcg(chg_cur + c4[t])) : 0u;
+#pragma unroll
+   for (int t4 = 0; t4 < 4; ++t4) {
+    const int64_t kk = kb4 + t4 * 32 + lane;
+    const unsigned cm = m4[t4];
+    const int32_t u = cm ? c4[t4] : -1;
+    const T wl = cm ? b_weight<T>(g.nz, g.tv, kk) : T(0);
     unsigned act = __ballot_sync(kFullB, u >= 0);
     // changed in-neighbours 8 at a time: their rows of D are read together, so a warp
     // keeps up to 8 reads in flight (the minimum does not depend on the order)
@@ -308,6 +313,7 @@ __device__ __forceinline__ bool bs_pull(const BatchGraph& g, const T* D,
         }
       }
     }
+   }
   }
   return any;
 }
@@ -323,6 +329,28 @@ __device__ __forceinline__ void ms_changed(int64_t v, unsigned cols, unsigned* c
   if (cq) cq[atomicAdd(ncq, 1ull)] = (int32_t)v;
 }
 
+template <typename T> __device__ __forceinline__ unsigned ms_dist_bits(T d) {
+  if constexpr (sizeof(T) == 4) return *reinterpret_cast<const unsigned*>(&d);
+  return 0u;  // (8-byte distances: not noted)
+}
+
+// what a round's kernels found beside the changed vertices: (vertex, column) pairs that
+// dropped, and the smallest distance written, kept as ~(its bits) under max so that the
+// cleared word means none (4-byte distances, which order as their bits do).  Null
+// pointers: not wanted.
+struct MsSums {
+  unsigned long long* pairs;
+  unsigned long long* low;
+  template <typename T>
+  __device__ __forceinline__ void add(unsigned long long n, T d) const {  // the whole warp
+    if (!pairs) return;
+    warp_add(n, pairs);
+    const unsigned b = __reduce_max_sync(kFullB, ~ms_dist_bits<T>(d));
+    if ((threadIdx.x & 31) == 0 && b != ~ms_dist_bits<T>(Lim<T>::max()))
+      atomicMax(low, (unsigned long long)b);
+  }
+};
+
 // one round: warp per vertex v (every vertex, or the marked ones in vlist[0, *nlist)),
 // lane = source column; pull from in-neighbours that changed last round, lower D[v]
 // in place, flag v when any column dropped (chg_next is cleared before the round).
@@ -332,9 +360,11 @@ __global__ void __launch_bounds__(256)
     k_ms_round(int64_t n, BatchGraph g, T* D, const unsigned* __restrict__ chg,
                unsigned* chg_next, unsigned long long* count, unsigned* drop,
                const int32_t* __restrict__ vlist, const unsigned long long* nlist, int32_t* cq,
-               unsigned long long* ncq) {
+               unsigned long long* ncq, MsSums sums) {
   const int lane = threadIdx.x & 31;
   unsigned dropped_cols = 0;
+  unsigned long long pairs = 0;
+  T low = Lim<T>::max();
   const int64_t total = vlist ? (int64_t)*((volatile const unsigned long long*)nlist) : n;
   const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -363,6 +393,8 @@ __global__ void __launch_bounds__(256)
         if (best < *dv) {
           *dv = best;
           dropped = true;
+          low = best < low ? best : low;
+          ++pairs;
         }
       }
       const unsigned b = __ballot_sync(kFullB, dropped);
@@ -382,6 +414,7 @@ __global__ void __launch_bounds__(256)
     }
   }
   if (drop && lane == 0 && dropped_cols) atomicOr(drop, dropped_cols);
+  sums.add<T>(pairs, low);
 }
 
 // marking for a frontier-restricted round: the out-neighbours of the changed vertices
@@ -540,179 +573,197 @@ template <> __device__ __forceinline__ double b_atomic_min<double>(double* p, do
   return __longlong_as_double(atomicMin((long long*)p, __double_as_longlong(v)));
 }
 
-// Full round over the SELL-32 copy of the graph (4-byte distance types): a warp takes
-// one work item of the copy's plan (a chunk of up to kSellChunk entry columns of a
-// slice, or a group of narrow slices), i.e. 32 rows.  Entry columns are read 4 at a
-// time (lane = row): in-neighbours, their changed-column masks and weights, all loads
-// independent; the entries whose in-neighbour changed last round go to a per-warp
-// queue in shared memory (6 KB per warp with the minima, so 4 CTAs of 8 warps fit an
-// SM: the round waits on its loads, and 32 warps hide more of that than 24 did).  The queue is then drained 16 entries at a time, 4 entries
-// per warp instruction (8 lanes per entry, 4 source columns per lane, 16-byte loads of
-// D): 16 rows of D in flight per warp, candidates folded with shared-memory atomic min
-// into the warp's 32 x 32 minima.  The vertex-per-warp round waits on
-// one vertex's chain of loads at a time instead.  Rows are lowered in place with atomic
-// min (a long row's chunks are separate items; min is exact in any order, so the
-// fixpoint is unchanged), and a vertex enters the next changed queue once, by the warp
-// whose atomic OR first set a bit of it.
-static const int kMsSellWarps = 8;
-static const int kMsSellQ = 4 * 32;  // queue entries of one 4-column step
-static const int kMsSellBatch = 16;  // queue entries a warp drains per step (4 at once)
-
-template <typename T>
-struct MsSellWarpSmem {
-  T acc[32 * 32];       // row l, column q at l * 32 + q
-  int4 q[kMsSellQ];     // (in-neighbour, weight bits, changed columns, row)
+// Round over every row (4-byte distances, rows with their entries by ascending weight):
+// 8 lanes take a row of up to kSegMM entries or a piece of a longer one, 4 source columns a
+// lane with their minima in registers, four rows of about one length a warp (the SpMM
+// plan's lists).  An entry costs a 16-byte load of D and four add-min instructions a
+// lane; 8 entries' loads are in flight, the next 8 columns and weights behind them.
+//  * A row ends at the first weight w with w + dlow >= the largest of its 32 minima, or
+//    w > cap: sums of non-negative values only grow, and no distance below dlow was written
+//    in the previous round, so an unchanged or pruned entry cannot lower it.  cap < max
+//    leaves heavy entries out altogether; a later round must then visit every row with
+//    dlow = 0 and no cap before the result is final.
+//  * kCheck: entries whose in-neighbour did not change in the previous round are left out
+//    by its column mask (worth its gather once few of the pairs drop).
+// Whole rows have one writer; pieces lower their row by atomic min.  Any order of
+// relaxations reaches the same fixpoint.
+// Against the round it replaces (a warp per 32-row SELL item, changed entries through a
+// shared-memory queue, 19.5 warp instructions an entry, all entries): 800 -> 250 us on R-MAT
+// scale 20, 32 Int32 columns; 256 sources 57.5 -> 25.5 ms.  Now bound by issue (41%) and
+// the row lists' dependent loads.
+struct MsRows {
+  const int32_t* rowptr;  // 1-based
+  const int32_t* col;     // 1-based, entries of a row by ascending weight
+  const void* w;
+  int tv;
+  const int4* items;      // rows of more than 32 entries and pieces: (row, first, end, piece or -1)
+  int64_t nitems;
+  const int32_t* short_rows;  // rows of 1..32 entries
+  int64_t nshort;
 };
 
-template <typename T>
-__device__ __forceinline__ int ms_bits(T w);
-template <> __device__ __forceinline__ int ms_bits<int32_t>(int32_t w) { return w; }
-template <> __device__ __forceinline__ int ms_bits<float>(float w) { return __float_as_int(w); }
-template <typename T>
-__device__ __forceinline__ T ms_unbits(int b);
-template <> __device__ __forceinline__ int32_t ms_unbits<int32_t>(int b) { return b; }
-template <> __device__ __forceinline__ float ms_unbits<float>(int b) { return __int_as_float(b); }
-
-template <typename T>
-__device__ __forceinline__ void ms_sell_slice(const int32_t* __restrict__ colval, const void* nz,
-                                              int tv, int64_t pos0, int width, int64_t row0,
-                                              int64_t m, const int32_t* __restrict__ perm, T* D,
-                                              const unsigned* __restrict__ chg, unsigned* chg_next,
-                                              unsigned long long* count, int32_t* cq,
-                                              unsigned long long* ncq, int lane,
-                                              MsSellWarpSmem<T>& sm, unsigned& dropped_cols) {
-#pragma unroll 4
-  for (int l = 0; l < 32; ++l) sm.acc[l * 32 + lane] = Lim<T>::max();
-  for (int j0 = 0; j0 < width; j0 += kMsSellQ / 32) {
-    int32_t c[kMsSellQ / 32];
-    unsigned cm[kMsSellQ / 32];
-    T wv[kMsSellQ / 32];
-#pragma unroll
-    for (int k = 0; k < kMsSellQ / 32; ++k) {
-      c[k] = j0 + k < width ? __ldcs(colval + pos0 + (int64_t)(j0 + k) * 32 + lane) : -1;
-      wv[k] = j0 + k < width ? b_weight<T>(nz, tv, pos0 + (int64_t)(j0 + k) * 32 + lane) : T(0);
-    }
-#pragma unroll
-    for (int k = 0; k < kMsSellQ / 32; ++k)
-      cm[k] = c[k] > 0 ? (__ldcg(chg + (c[k] - 1)) | __ldcg(chg_next + (c[k] - 1))) : 0u;
-    __syncwarp();  // the previous step's queue has been drained
-    int nq = 0;
-#pragma unroll
-    for (int k = 0; k < kMsSellQ / 32; ++k) {
-      const unsigned b = __ballot_sync(kFullB, cm[k] != 0);
-      if (cm[k]) sm.q[nq + __popc(b & ((1u << lane) - 1u))] = make_int4(c[k] - 1, ms_bits<T>(wv[k]), (int)cm[k], lane);
-      nq += __popc(b);
-    }
-    __syncwarp();
-    // 4 queue entries per warp step: lanes 8e .. 8e + 7 take entry e, 4 source columns
-    // each (16-byte loads of D); kMsSellBatch / 4 steps' loads in flight.  Two entries
-    // of one step may share a row, so the minima are folded with shared-memory atomic
-    // min (distances are non-negative: floats order like their bit patterns).
-    const int es = lane >> 3, cq4 = (lane & 7) * 4;
-    for (int e0 = 0; e0 < nq; e0 += kMsSellBatch) {
-      T dv[kMsSellBatch / 4][4];
-      int4 qe[kMsSellBatch / 4];
-#pragma unroll
-      for (int b = 0; b < kMsSellBatch / 4; ++b) {
-        const int e = e0 + b * 4 + es;
-        qe[b] = e < nq ? sm.q[e] : make_int4(0, 0, 0, 0);
-        const unsigned bits = ((unsigned)qe[b].z >> cq4) & 15u;
-        dv[b][0] = dv[b][1] = dv[b][2] = dv[b][3] = Lim<T>::max();
-        if (bits) {
-          const T* row = D + (int64_t)qe[b].x * 32 + cq4;
-          if constexpr (sizeof(T) == 4) {
-            const int4 r4 = __ldcg(reinterpret_cast<const int4*>(row));
-            if (bits & 1u) dv[b][0] = ms_unbits<T>(r4.x);
-            if (bits & 2u) dv[b][1] = ms_unbits<T>(r4.y);
-            if (bits & 4u) dv[b][2] = ms_unbits<T>(r4.z);
-            if (bits & 8u) dv[b][3] = ms_unbits<T>(r4.w);
-          }
-        }
-      }
-#pragma unroll
-      for (int b = 0; b < kMsSellBatch / 4; ++b) {
-        if (e0 + b * 4 + es < nq) {
-          const T w = ms_unbits<T>(qe[b].y);
-          int* a = reinterpret_cast<int*>(sm.acc + qe[b].w * 32 + cq4);
-          const int4 cur = *reinterpret_cast<const int4*>(a);  // may be stale: atomics decide
-          const int cv[4] = {cur.x, cur.y, cur.z, cur.w};
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const int cb = ms_bits<T>(b_relax(w, dv[b][k]));
-            if (cb < cv[k]) atomicMin(a + k, cb);
-          }
-        }
-      }
-    }
-  }
-  __syncwarp();
-  // lower the rows 8 at a time: their D rows read together, the drops sent as atomic
-  // min without waiting (a column counts as dropped when the minimum is below the value
-  // read; another warp lowering it further in the meantime changed it as well), and
-  // the changed-column bookkeeping of the 8 rows done by lanes 0..7 at once
-  const int32_t vl = row0 + lane < m ? __ldg(perm + row0 + lane) - 1 : -1;
-  for (int l0 = 0; l0 < 32; l0 += 8) {
-    T best[8], cur[8];
-    int32_t v[8];
-#pragma unroll
-    for (int t = 0; t < 8; ++t) {
-      v[t] = __shfl_sync(kFullB, vl, l0 + t);
-      best[t] = sm.acc[(l0 + t) * 32 + lane];
-      cur[t] = (v[t] >= 0 && best[t] != Lim<T>::max()) ? __ldcg(D + (int64_t)v[t] * 32 + lane)
-                                                        : Lim<T>::max();
-    }
-    unsigned mine = 0;
-    int32_t myv = -1;
-#pragma unroll
-    for (int t = 0; t < 8; ++t) {
-      const bool dropped = best[t] < cur[t];
-      if (dropped) b_atomic_min<T>(D + (int64_t)v[t] * 32 + lane, best[t]);
-      const unsigned b = __ballot_sync(kFullB, dropped);
-      dropped_cols |= b;
-      if (lane == t) {
-        mine = b;
-        myv = v[t];
-      }
-    }
-    if (mine && myv >= 0 && atomicOr(chg_next + myv, mine) == 0u) {
-      atomicAdd(count, 1ull);
-      if (cq) cq[atomicAdd(ncq, 1ull)] = myv;
-    }
-  }
-  __syncwarp();
+// the row rounds' view of A (CSR handles with 1- or 4-byte values; out->col stays nullptr
+// for others and where the sorted rows do not fit) and the mean weight
+static inline int ms_rows_of(gg_ctx* ctx, gg_mat* A, MsRows* out, double* mean_w) {
+  *out = MsRows{};
+  GG_CHECK(weight_sorted_rows(ctx, A, &out->col, &out->w, mean_w));
+  if (!out->col) return GG_OK;
+  GG_CHECK(build_mm_plan(ctx, A));
+  const MMPlan* P = A->mmplan;
+  out->rowptr = A->rowptr;
+  out->tv = A->dtype;
+  out->items = P->items;
+  out->nitems = P->nitems;
+  out->short_rows = P->short_rows;
+  out->nshort = P->nlive;
+  return GG_OK;
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kMsSellWarps * 32, 4)
-    k_ms_round_sell(const int32_t* __restrict__ colval, const void* __restrict__ nz, int tv,
-                    const int32_t* __restrict__ perm, int64_t m, const int4* __restrict__ pitems,
-                    int64_t nitems, T* D, const unsigned* __restrict__ chg, unsigned* chg_next,
-                    unsigned long long* count, unsigned* drop, int32_t* cq,
-                    unsigned long long* ncq) {
-  extern __shared__ __align__(16) unsigned char ms_smem[];
-  unsigned dropped_cols = 0;  // source columns that dropped anywhere (drop, when given)
-  const int lane = threadIdx.x & 31;
-  MsSellWarpSmem<T>& sm = reinterpret_cast<MsSellWarpSmem<T>*>(ms_smem)[threadIdx.x >> 5];
-  const int64_t gw = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  int4 dn = gw < nitems ? __ldg(pitems + gw) : make_int4(0, 0, 0, 0);
-  for (int64_t it = gw; it < nitems; it += nw) {
-    const int4 d = dn;  // first position, first stored row, columns (or -slices), partial
-    if (it + nw < nitems) dn = __ldg(pitems + it + nw);
-    if (d.z < 0) {  // -d.z narrow slices, widths in 4-bit fields of d.w
-      int64_t pos = d.x;
-      for (int t = 0; t < -d.z; ++t) {
-        const int w = (int)(((uint32_t)d.w >> (4 * t)) & 15u);
-        ms_sell_slice<T>(colval, nz, tv, pos, w, (int64_t)d.y + t * 32, m, perm, D, chg, chg_next,
-                         count, cq, ncq, lane, sm, dropped_cols);
-        pos += (int64_t)w * 32;
-      }
-    } else {
-      ms_sell_slice<T>(colval, nz, tv, d.x, d.z, d.y, m, perm, D, chg, chg_next, count, cq, ncq,
-                       lane, sm, dropped_cols);
+template <typename T> __device__ __forceinline__ T ms_unbits(int b);
+template <> __device__ __forceinline__ int32_t ms_unbits<int32_t>(int b) { return b; }
+template <> __device__ __forceinline__ float ms_unbits<float>(int b) { return __int_as_float(b); }
+// min(best, w + d) on non-negative values; a sum past Int32 (an unreached d among them)
+// stays above every distance
+__device__ __forceinline__ int32_t ms_relax(int32_t best, int32_t w, int32_t d) {
+  return (int32_t)__viaddmin_u32((unsigned)w, (unsigned)d, (unsigned)best);
+}
+__device__ __forceinline__ float ms_relax(float best, float w, float d) {
+  return fminf(best, __fadd_rn(w, d));
+}
+
+// 4 entries of a row with their D rows in flight and 40 warps an SM: 8 entries with 24 / 32
+// warps 35.5 / 33.0 ms, 4 with 32 / 40 / 48 (spills) 32.5 / 31.9 / 37.1 ms (256 sources,
+// R-MAT scale 20)
+static const int kMsRowStep = 4;
+static const int kMsRowBlocks = 5;  // CTAs of 256 threads an SM
+
+template <typename T, bool kCheck>
+__global__ void __launch_bounds__(256, kMsRowBlocks)
+    k_ms_round_rows(MsRows g, T* D, const unsigned* __restrict__ chg, unsigned* chg_next,
+                    unsigned long long* count, unsigned* drop, int32_t* cq, unsigned long long* ncq,
+                    MsSums sums, T dlow, T cap) {
+  __shared__ int32_t stage[8][WarpQueue::kCap];
+  const int lane = threadIdx.x & 31, sub = lane & 7, lead = lane & ~7;
+  const unsigned gmask = 0xffu << lead;
+  WarpQueue wq(stage[threadIdx.x >> 5], cq, ncq);
+  unsigned dropped_cols = 0;
+  unsigned long long pairs = 0, changed = 0;
+  T low = Lim<T>::max();
+  const T far_t = Lim<T>::max();
+  const int far = *reinterpret_cast<const int*>(&far_t);
+  const int64_t total = g.nitems + g.nshort;
+  // warps numbered across the blocks first: the longest rows go to different SMs
+  const int64_t gw = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+  const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
+  for (int64_t id0 = gw * 4; id0 < total; id0 += nw * 4) {
+    const int64_t id = id0 + (lane >> 3);
+    int32_t v = -1, k = 0, k1 = 0;
+    bool piece = false;
+    if (id < g.nitems) {
+      const int4 d = __ldg(g.items + id);
+      v = d.x;
+      k = d.y;
+      k1 = d.z;
+      piece = d.w >= 0;
+    } else if (id < total) {
+      v = __ldg(g.short_rows + (id - g.nitems));
+      k = __ldg(g.rowptr + v) - 1;
+      k1 = __ldg(g.rowptr + v + 1) - 1;
     }
+    int32_t c = k + sub < k1 ? __ldg(g.col + k + sub) : 0;
+    T w = k + sub < k1 ? b_weight<T>(g.w, g.tv, k + sub) : Lim<T>::max();
+    T* row = D + (int64_t)(v < 0 ? 0 : v) * 32 + sub * 4;
+    T cur[4], best[4];
+    {
+      const int4 r = v >= 0 ? __ldcg(reinterpret_cast<const int4*>(row)) : make_int4(0, 0, 0, 0);
+      cur[0] = ms_unbits<T>(r.x);
+      cur[1] = ms_unbits<T>(r.y);
+      cur[2] = ms_unbits<T>(r.z);
+      cur[3] = ms_unbits<T>(r.w);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) best[q] = cur[q];
+    for (; __any_sync(kFullB, k < k1); k += 8) {
+      // the largest of the row's minima so far, and the entries it still admits
+      T top = best[0] > best[1] ? best[0] : best[1];
+      const T t2 = best[2] > best[3] ? best[2] : best[3];
+      top = t2 > top ? t2 : top;
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) {
+        const T t = __shfl_xor_sync(kFullB, top, o);
+        top = t > top ? t : top;
+      }
+      const bool in = c > 0 && b_relax(w, dlow) < top && w <= cap;
+      if (!in) c = 0;
+      const unsigned any = __ballot_sync(kFullB, in);
+      if (!(any & gmask)) k = k1;  // ascending weights: nothing of the row is left
+      if (!any) break;
+      const int32_t kn = k + 8 + sub;
+      const int32_t cn = kn < k1 ? __ldg(g.col + kn) : 0;
+      const T wn = kn < k1 ? b_weight<T>(g.w, g.tv, kn) : Lim<T>::max();
+      unsigned m = ~0u;
+      if (kCheck) m = c > 0 ? __ldg(chg + (c - 1)) : 0u;
+#pragma unroll
+      for (int h = 0; h < 8; h += kMsRowStep) {
+        int4 dv[kMsRowStep];
+#pragma unroll
+        for (int u = 0; u < kMsRowStep; ++u) {
+          const int32_t cu = __shfl_sync(kFullB, c, lead + h + u);
+          bool need = cu > 0;
+          if constexpr (kCheck) {
+            const unsigned mu = __shfl_sync(kFullB, m, lead + h + u);  // every lane takes part
+            need = need && ((mu >> (sub * 4)) & 15u);
+          }
+          dv[u] = need ? __ldcg(reinterpret_cast<const int4*>(D + (int64_t)(cu - 1) * 32 + sub * 4))
+                       : make_int4(far, far, far, far);
+        }
+#pragma unroll
+        for (int u = 0; u < kMsRowStep; ++u) {
+          const T wu = __shfl_sync(kFullB, w, lead + h + u);
+          best[0] = ms_relax(best[0], wu, ms_unbits<T>(dv[u].x));
+          best[1] = ms_relax(best[1], wu, ms_unbits<T>(dv[u].y));
+          best[2] = ms_relax(best[2], wu, ms_unbits<T>(dv[u].z));
+          best[3] = ms_relax(best[3], wu, ms_unbits<T>(dv[u].w));
+        }
+      }
+      c = cn;
+      w = wn;
+    }
+    unsigned bits = 0;
+    if (v >= 0) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (best[q] < cur[q] && (!piece || best[q] < b_atomic_min<T>(row + q, best[q]))) {
+          bits |= 1u << q;
+          low = best[q] < low ? best[q] : low;
+        }
+      if (bits && !piece)
+        __stcg(reinterpret_cast<int4*>(row), *reinterpret_cast<const int4*>(best));
+      pairs += __popc(bits);
+    }
+    unsigned cols = bits << (sub * 4);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) cols |= __shfl_xor_sync(kFullB, cols, o);
+    dropped_cols |= cols;
+    bool fresh = false;  // first to flag the row this round
+    if (sub == 0 && cols) {
+      if (piece) {
+        fresh = atomicOr(chg_next + v, cols) == 0u;
+      } else {
+        chg_next[v] = cols;
+        fresh = true;
+      }
+    }
+    changed += fresh;
+    wq.push(fresh, v);
   }
-  if (drop && lane == 0 && dropped_cols) atomicOr(drop, dropped_cols);
+  wq.flush();
+  warp_add(changed, count);
+  if (drop) {
+    dropped_cols = __reduce_or_sync(kFullB, dropped_cols);
+    if (lane == 0 && dropped_cols) atomicOr(drop, dropped_cols);
+  }
+  sums.add<T>(pairs, low);
 }
 
 // hub pieces: one warp per piece, atomic min into the hub's 32 columns
@@ -722,9 +773,12 @@ __global__ void __launch_bounds__(256)
     k_ms_round_hub(BatchGraph g, const int4* __restrict__ pieces, int64_t npiece,
                    const int32_t* __restrict__ hubs, T* D, const unsigned* __restrict__ chg,
                    unsigned* chg_next, unsigned long long* count, unsigned* drop,
-                   const unsigned* __restrict__ mark, int32_t* cq, unsigned long long* ncq) {
+                   const unsigned* __restrict__ mark, int32_t* cq, unsigned long long* ncq,
+                   MsSums sums) {
   const int lane = threadIdx.x & 31;
   unsigned dropped_cols = 0;
+  unsigned long long pairs = 0;
+  T low = Lim<T>::max();
   for (int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < npiece;
        i += ((int64_t)gridDim.x * blockDim.x) >> 5) {
     const int4 p = pieces[i];
@@ -736,12 +790,17 @@ __global__ void __launch_bounds__(256)
     if (any) {
       T* dv = D + v * 32 + lane;
       if (best < *dv) dropped = best < b_atomic_min<T>(dv, best);
+      if (dropped) {
+        low = best < low ? best : low;
+        ++pairs;
+      }
     }
     const unsigned b = __ballot_sync(kFullB, dropped);
     dropped_cols |= b;
     if (lane == 0 && b) ms_changed(v, b, chg_next, count, cq, ncq);
   }
   if (drop && lane == 0 && dropped_cols) atomicOr(drop, dropped_cols);
+  sums.add<T>(pairs, low);
 }
 
 }  // namespace

@@ -54,6 +54,7 @@ struct Request {
 
 struct SrvGraph {
   BatchGraph g;
+  MsRows rows = {};  // rows by ascending weight for the shortest-path executors
   bool nonneg;
   int64_t n;
 };
@@ -452,17 +453,9 @@ static int exec_admit(gg_server* S, int gi, Executor& E, std::vector<Request>& w
   return k;
 }
 
-// shared memory of the SELL-32 full rounds (more than the default 48 KB per CTA)
-template <typename T>
-static int sell_round_attr() {
-  GG_CUDA(cudaFuncSetAttribute(k_ms_round_sell<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                               (int)(kMsSellWarps * sizeof(MsSellWarpSmem<T>))));
-  return GG_OK;
-}
-
 template <typename T>
 static void ss_round(gg_server* S, Executor& E, const SrvGraph& sg, const HubPlan* hp,
-                     int64_t nnz, const gg_mat* sell) {
+                     int64_t nnz, const MsRows& rows) {
   cudaStream_t st = E.ectx.stream;
   const int64_t n = sg.n;
   T* D = static_cast<T*>(E.D);
@@ -472,35 +465,38 @@ static void ss_round(gg_server* S, Executor& E, const SrvGraph& sg, const HubPla
   cudaMemsetAsync(ncq_nxt, 0, sizeof(unsigned long long), st);
   const int64_t avg_deg = n > 0 ? (nnz + n - 1) / n : 1;
   // few changed vertices: visit only their out-neighbours (same fixpoint)
-  const bool restricted = E.nchanged * avg_deg * (sell ? 32 : 4) < nnz;
+  const bool by_row = sizeof(T) == 4 && rows.col != nullptr;
+  const bool restricted = E.nchanged * avg_deg * (by_row ? 32 : 4) < nnz;
+  const MsSums none{nullptr, nullptr};
   if (restricted) {
     cudaMemsetAsync(E.mark, 0, ((n + 31) / 32) * sizeof(unsigned), st);
     cudaMemsetAsync(E.d_cnt + 3, 0, sizeof(unsigned long long), st);
     launch_ms_mark(st, S->own.num_sms, E.nchanged, E.prow, E.pcol, E.cq[cur], ncq_cur, E.mark,
                    E.vlist, E.d_cnt + 3, E.mhq, E.d_cnt + 4, E.mhoff);
     k_ms_round<T><<<grid_s(S, n * 32), 256, 0, st>>>(n, sg.g, D, E.c0, E.c1, E.d_cnt, E.d_amask,
-                                                      E.vlist, E.d_cnt + 3, E.cq[cur ^ 1], ncq_nxt);
+                                                      E.vlist, E.d_cnt + 3, E.cq[cur ^ 1], ncq_nxt,
+                                                      none);
   } else {
     if constexpr (sizeof(T) == 4) {
-      if (sell) {
-        // every vertex over the graph's SELL-32 copy (hubs as chunks of their rows), as
-        // the batched rounds do
-        k_ms_round_sell<T><<<S->own.num_sms * 4, kMsSellWarps * 32,
-                             kMsSellWarps * sizeof(MsSellWarpSmem<T>), st>>>(
-            sell->colval, sell->nzval, sell->dtype, sell->perm, sell->m, sell->sellplan->pitems,
-            sell->sellplan->npitems, D, E.c0, E.c1, E.d_cnt, E.d_amask, E.cq[cur ^ 1], ncq_nxt);
+      if (by_row) {
+        // every row by ascending weight, hubs in pieces, as the batched rounds do; queries
+        // join at any tick, so no distance bounds the next round's and no edge is left out
+        int64_t rb = ((rows.nitems + rows.nshort + 3) / 4 + 7) / 8;
+        const int64_t gcap = (int64_t)S->own.num_sms * kMsRowBlocks;
+        k_ms_round_rows<T, true><<<(int)(rb < gcap ? (rb > 0 ? rb : 1) : gcap), 256, 0, st>>>(
+            rows, D, E.c0, E.c1, E.d_cnt, E.d_amask, E.cq[cur ^ 1], ncq_nxt, none, T(0), Lim<T>::max());
         return;
       }
     }
     // every non-hub vertex in the plan's order (long rows first, spread over the warps)
     k_ms_round<T><<<grid_s(S, n * 32), 256, 0, st>>>(n, sg.g, D, E.c0, E.c1, E.d_cnt, E.d_amask,
                                                       hp->order, hp->d_norder, E.cq[cur ^ 1],
-                                                      ncq_nxt);
+                                                      ncq_nxt, none);
   }
   if (hp->npiece > 0)
     k_ms_round_hub<T><<<grid_s(S, hp->npiece * 32), 256, 0, st>>>(
         sg.g, hp->pieces, hp->npiece, hp->hubs, D, E.c0, E.c1, E.d_cnt, E.d_amask,
-        restricted ? E.mark : nullptr, E.cq[cur ^ 1], ncq_nxt);
+        restricted ? E.mark : nullptr, E.cq[cur ^ 1], ncq_nxt, none);
 }
 
 // one tick of an executor, enqueued on its stream, followed by its event
@@ -533,13 +529,12 @@ static int exec_tick(gg_server* S, int gi, Executor& E) {
     GG_CUDA(cudaMemsetAsync(E.d_amask, 0, 4, st));  // dropped columns of this round
     GG_CUDA(cudaMemsetAsync(E.c1, 0, (size_t)n * sizeof(unsigned), st));
     const int64_t nnz = S->graphs[gi]->nnz;
-    const gg_mat* sell = nullptr;  // built when the graph was added (sssp_prepare)
-    GG_CHECK(pull_sell_copy(&S->own, S->graphs[gi], &sell));
+    const MsRows& rows = sg.rows;  // built when the graph was added
     switch (E.dtype) {
-      case GG_INT32: ss_round<int32_t>(S, E, sg, hp, nnz, sell); break;
-      case GG_INT64: ss_round<int64_t>(S, E, sg, hp, nnz, nullptr); break;
-      case GG_FLOAT32: ss_round<float>(S, E, sg, hp, nnz, sell); break;
-      default: ss_round<double>(S, E, sg, hp, nnz, nullptr); break;
+      case GG_INT32: ss_round<int32_t>(S, E, sg, hp, nnz, rows); break;
+      case GG_INT64: ss_round<int64_t>(S, E, sg, hp, nnz, rows); break;
+      case GG_FLOAT32: ss_round<float>(S, E, sg, hp, nnz, rows); break;
+      default: ss_round<double>(S, E, sg, hp, nnz, rows); break;
     }
     std::swap(E.c0, E.c1);
     GG_CUDA(cudaMemcpyAsync(E.h_result, E.d_amask, 4, cudaMemcpyDeviceToHost, st));
@@ -886,11 +881,8 @@ int gg_server_add_graph(gg_server* S, const gg_mat* A_T, int* graph_id) {
     if (rc == GG_OK && nonneg && n > 0) {
       const int64_t one = 1;
       rc = sssp_prepare(&S->own, A);
-      // the full rounds of the shortest-path executors run over the SELL-32 copy
-      if (rc == GG_OK)
-        rc = sell_round_attr<int32_t>();
-      if (rc == GG_OK)
-        rc = sell_round_attr<float>();
+      double mean_w = 0.0;
+      if (rc == GG_OK) rc = ms_rows_of(&S->own, A, &g.rows, &mean_w);
       if (rc == GG_OK)
         rc = gg_sssp(&S->own, A, &one, 1, tmp, nullptr, A->dtype == GG_BOOL ? GG_INT32 : A->dtype,
                      n, nullptr);

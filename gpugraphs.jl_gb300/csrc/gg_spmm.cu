@@ -523,10 +523,11 @@ static int grid_mm(gg_ctx* ctx, int64_t warps) {
 }
 
 // long-row pieces, built once per matrix from rowptr (CSR) or slice_ptr (SELL)
-static int build_mm_plan(gg_ctx* ctx, gg_mat* A) {
+int build_mm_plan(gg_ctx* ctx, gg_mat* A) {
   if (A->mmplan) return GG_OK;
   std::vector<int4> segs, items;
   std::vector<int32_t> first, rows, short_rows;
+  int64_t nlive = 0;
   if (A->format == GG_FMT_CSR) {
     const int64_t m = A->m;
     std::vector<int32_t> rp(m + 1);
@@ -544,6 +545,7 @@ static int build_mm_plan(gg_ctx* ctx, gg_mat* A) {
       for (int64_t r = 0; r < m; ++r) {
         const int64_t L = rp[r + 1] - rp[r];
         if (L <= kShortMM) short_rows[cnt[kShortMM - L]++] = (int32_t)r;
+        if (L > 0 && L <= kShortMM) ++nlive;
       }
     }
     for (int64_t r = 0; r < m; ++r) {
@@ -597,6 +599,7 @@ static int build_mm_plan(gg_ctx* ctx, gg_mat* A) {
   up((void**)&P->rows, rows.data(), rows.size() * sizeof(int32_t));
   up((void**)&P->items, items.data(), (size_t)P->nitems * sizeof(int4));
   P->nshort = (int64_t)short_rows.size();
+  P->nlive = nlive;
   up((void**)&P->short_rows, short_rows.data(), short_rows.size() * sizeof(int32_t));
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
   if (e != cudaSuccess) {
