@@ -15,7 +15,8 @@
 //    semiring, software pipelined (next block's loads in flight during the current
 //    block's gathers), A streamed past L1, long segments read with 128-bit loads.
 //    Used for CSR matrices of fewer than 65536 rows; larger ones run plus-times on a
-//    SELL-32 copy with rows sorted by length (built once per matrix).
+//    SELL-32 copy with rows sorted by length (built once per matrix), by the
+//    fixed-semiring kernel of gg_spmv_typed.cu or by k_sell_hot32 below.
 //  * k_csr_first_hit<TC>: add == GPUGraphs_any with a mask on CSR: the first stored
 //    column whose x is nonzero (any_dense_masked_csr_spmv_kernel!, CSR.jl:147-171).
 //  * k_sell<SR>: one thread per (stored SELL row, chunk of <= 128 slice columns)
@@ -1200,6 +1201,20 @@ gg_mat* sell_for_spmv(gg_ctx* ctx, gg_mat* A) {
   return A->sell_copy;
 }
 
+// Float32 plus-times of A on SELL-32 arrays S (A itself or its copy), without a mask or
+// accumulator: the fixed-semiring kernel (gg_spmv_typed.cu), which refolds NaN rows itself
+// and folds narrow slices entry by entry.  Skewed columns of a handle with tuned choices
+// keep the kernel that was tuned, and so do those of more than kTypedPlainRows rows, where
+// its hub phase pays.  k_sell_hot32 (with its combine and refold passes) / fixed-semiring
+// kernel, us: R-MAT scale 17 56 / 41, 20 112 / 92, 22 339 / 336, 23 789 / 773, 24 1628 /
+// 1647; flat columns (k_sell): ER with 16.8 M entries 79 / 67, a 1024 x 1024 grid 26 / 14.
+static const int64_t kTypedPlainRows = (int64_t)3 << 22;
+static bool typed_plain(const gg_mat* A, const gg_mat* S) {
+  if (S->slice_size != 32) return false;
+  if (!S->colperm->enabled) return true;
+  return A->tuned_spmv == 0 && S->sell_variant == 0 && S->hot_cols == 0 && S->m < kTypedPlainRows;
+}
+
 // dispatch of gg_spmv after validation (gg_api.cu); tc = accumulator type
 int spmv_dispatch(gg_ctx* ctx, gg_mat* A, int tc, int mul, int add, int accum, void* y, int ty,
                   const void* x, int tx, const void* mask, int tmask, int64_t lo, int64_t hi) {
@@ -1240,20 +1255,23 @@ int spmv_dispatch(gg_ctx* ctx, gg_mat* A, int tc, int mul, int add, int accum, v
         A->sell_copy->hot_cols = A->hot_cols;
       }
       A->last_layout = 2;
-      // columns without skew: the fixed-semiring kernel, which keeps the stop at +Inf
-      // itself (ER, 16.8 M entries: 79 us with k_sell and the refold pass, 67 us; a
-      // 1024 x 1024 grid 26 and 14 us)
       GG_CHECK(build_colperm(ctx, A->sell_copy));
-      if (!A->sell_copy->colperm->enabled && A->sell_copy->slice_size == 32) {
+      if (typed_plain(A, A->sell_copy)) {
         bool done = false;
         return spmv_typed(ctx, A, tc, mul, add, accum, y, ty, x, tx, mask, tmask, lo, hi, &done);
       }
+      A->sell_copy->tuned_spmv = A->tuned_spmv;  // the copy's own dispatch keeps a tuned kernel
       GG_CHECK(spmv_dispatch(ctx, A->sell_copy, tc, mul, add, accum, y, ty, x, tx, mask, tmask,
                              lo, hi));
       return launch_refold_nan_rows(ctx, A, sr.x, sr.y);
     }
     GG_CHECK(build_colperm(ctx, A));
     const int32_t* colval = A->colval;
+    if (A->format == GG_FMT_SELL && typed_plain(A, A)) {
+      A->last_layout = 2;
+      bool done = false;
+      return spmv_typed(ctx, A, tc, mul, add, accum, y, ty, x, tx, mask, tmask, lo, hi, &done);
+    }
     if (A->colperm->enabled) {
       k_gather_x<<<grid_for(ctx, A->n, 256), 256, 0, ctx->stream>>>(
           static_cast<const float*>(x), A->colperm->inv, A->n, A->colperm->xr);
@@ -1267,10 +1285,6 @@ int spmv_dispatch(gg_ctx* ctx, gg_mat* A, int tc, int mul, int add, int accum, v
     }
     A->last_layout = 2;
     if (A->colperm->enabled) return launch_sell_hot(ctx, A, sr, colval);
-    if (A->slice_size == 32) {
-      bool done = false;
-      return spmv_typed(ctx, A, tc, mul, add, accum, y, ty, x, tx, mask, tmask, lo, hi, &done);
-    }
     return launch_sell(ctx, A, sr, nullptr, 0, 0, 0, colval);
   }
   bool done = false;

@@ -180,6 +180,9 @@ __global__ void __launch_bounds__(kHot ? kTypedHotThreads : 256, kHot ? 1 : 4)
                    int64_t nitems, typename SR::T* partials, int hot, TypedFilter flt) {
   typedef typename SR::T T;
   constexpr int U = sizeof(T) == 8 ? 4 : 8;  // entries of a row in flight
+  // whether a warp looks for an early end: Bool sums end at the first true, a SELL handle's
+  // own slices may be padded (a CSR's copy is not: rows of one length share a slice)
+  constexpr bool kEarly = SR::kType == GG_BOOL || !SR::kHasAbsorbCheck;
   extern __shared__ __align__(16) unsigned char typed_smem[];
   const T* sx = reinterpret_cast<const T*>(typed_smem);
   if (kHot) {
@@ -285,8 +288,10 @@ __global__ void __launch_bounds__(kHot ? kTypedHotThreads : 256, kHot ? 1 : 4)
 #pragma unroll
       for (int u = 0; u < U; ++u) acc = sr.step(acc, c[u] > 0 ? sr.mul(a[u], xv[u]) : sr.neutral());
       // a row's padding comes last, and nothing follows the absorbing value
-      if (c[U - 1] <= 0 || sr.is_absorb(acc)) live = false;
-      if (!__any_sync(kFull, live)) break;
+      if (kEarly) {
+        if (c[U - 1] <= 0 || sr.is_absorb(acc)) live = false;
+        if (!__any_sync(kFull, live)) break;
+      }
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         c[u] = cn[u];
@@ -308,41 +313,84 @@ __global__ void __launch_bounds__(kHot ? kTypedHotThreads : 256, kHot ? 1 : 4)
   }
 }
 
-// Rows of the slices cut into chunks: a CTA per slice, warp w takes chunks w, w + 8, ...
-// (lane = row: one line per chunk), then warp 0 adds the warps' shares in order.  A CSR
-// row whose chunks end NaN is folded again in storage order with the stop (kStop).
+// Rows of the slices cut into chunks (lane = row: one line per chunk).  Wide slices: a CTA
+// each, four shares a warp and a tree over the 32 shares.  Slices of at most kNarrowChunks:
+// a warp each, the chunks' loads in flight together.  Both add in the order of
+// k_sell_combine (share l has the chunks c = l mod 32; share l joins l + 16, then l + 8, 4,
+// 2, 1).  A CSR row whose chunks end NaN is folded again in storage order with the stop.
+template <class SR>
+__device__ __forceinline__ typename SR::T tree8(const SR& sr, const typename SR::T (&v)[8]) {
+  static_assert(kNarrowChunks == 8, "tree over eight values");
+  const typename SR::T a = sr.step(v[0], v[4]), b = sr.step(v[1], v[5]);
+  const typename SR::T c = sr.step(v[2], v[6]), d = sr.step(v[3], v[7]);
+  return sr.step(sr.step(a, c), sr.step(b, d));
+}
+
+template <class SR>
+__device__ __forceinline__ void typed_finish(const SR& sr, typename SR::T acc, bool live, int32_t r1,
+                                             int lane, const int32_t* __restrict__ rowptr,
+                                             const int32_t* __restrict__ colval) {
+  unsigned bad = SR::kRefold ? __ballot_sync(kFull, live && acc != acc) : 0u;
+  while (bad) {
+    const int b = __ffs(bad) - 1;
+    bad &= bad - 1;
+    const typename SR::T v =
+        warp_refold_row(sr, rowptr, colval, (int64_t)__shfl_sync(kFull, r1, b) - 1, lane);
+    if (lane == b) acc = v;
+  }
+  if (live) sr.write((int64_t)r1 - 1, acc);
+}
+
 template <class SR>
 __global__ void __launch_bounds__(256)
     k_sell32_typed_combine(SR sr, const int32_t* __restrict__ perm, int64_t m,
-                           const int4* __restrict__ multi, int64_t nmulti,
+                           const int4* __restrict__ wide, int64_t nwide,
+                           const int4* __restrict__ narrow, int64_t nnarrow,
                            const typename SR::T* __restrict__ partials, TypedFilter flt,
                            const int32_t* __restrict__ rowptr, const int32_t* __restrict__ colval) {
   typedef typename SR::T T;
   __shared__ T part[8][32];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int64_t q = blockIdx.x; q < nmulti; q += gridDim.x) {
-    const int4 d = multi[q];  // slice, first partial, chunks
-    const int64_t srow = (int64_t)d.x * 32 + lane;
-    int64_t r1 = srow + 1;
-    bool live = srow < m;
-    if (live && perm) r1 = __ldg(perm + srow);
-    if (live) live = flt.keep(r1);
-    T acc = sr.neutral();
-    if (live)
-      for (int c = warp; c < d.z; c += 8) acc = sr.step(acc, partials[(int64_t)(d.y + c) * 32 + lane]);
-    part[warp][lane] = acc;
+  auto row_at = [&](int32_t slice) -> int32_t {  // 1-based, 0: not wanted
+    const int64_t srow = (int64_t)slice * 32 + lane;
+    if (srow >= m) return 0;
+    const int32_t r1 = perm ? __ldg(perm + srow) : (int32_t)(srow + 1);
+    return flt.keep(r1) ? r1 : 0;
+  };
+  const int64_t nblk = nwide + (nnarrow + 7) / 8;
+  for (int64_t q = blockIdx.x; q < nblk; q += gridDim.x) {
+    if (q >= nwide) {
+      const int64_t i = (q - nwide) * 8 + warp;
+      if (i >= nnarrow) continue;
+      const int4 d = narrow[i];  // slice, first partial, chunks
+      T p[kNarrowChunks];
+#pragma unroll
+      for (int c = 0; c < kNarrowChunks; ++c)
+        p[c] = c < d.z ? partials[(int64_t)(d.y + c) * 32 + lane] : sr.neutral();
+      const int32_t r1 = row_at(d.x);
+      typed_finish(sr, tree8(sr, p), r1 > 0, r1, lane, rowptr, colval);
+      continue;
+    }
+    const int4 d = wide[q];
+    const int32_t r1 = row_at(d.x);
+    T acc[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) acc[k] = sr.neutral();
+    for (int c = warp; c < d.z; c += 32) {
+      T v[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        v[k] = c + 8 * k < d.z ? partials[(int64_t)(d.y + c + 8 * k) * 32 + lane] : sr.neutral();
+#pragma unroll
+      for (int k = 0; k < 4; ++k) acc[k] = sr.step(acc[k], v[k]);
+    }
+    part[warp][lane] = sr.step(sr.step(acc[0], acc[2]), sr.step(acc[1], acc[3]));
     __syncthreads();
     if (warp == 0) {
-      const int nshare = d.z < 8 ? d.z : 8;
-      for (int w = 1; w < nshare; ++w) acc = sr.step(acc, part[w][lane]);
-      unsigned bad = SR::kRefold ? __ballot_sync(kFull, live && acc != acc) : 0u;
-      while (bad) {
-        const int b = __ffs(bad) - 1;
-        bad &= bad - 1;
-        const T v = warp_refold_row(sr, rowptr, colval, __shfl_sync(kFull, r1, b) - 1, lane);
-        if (lane == b) acc = v;
-      }
-      if (live) sr.write(r1 - 1, acc);
+      T v[8];
+#pragma unroll
+      for (int w = 0; w < 8; ++w) v[w] = part[w][lane];
+      typed_finish(sr, tree8(sr, v), r1 > 0, r1, lane, rowptr, colval);
     }
     __syncthreads();
   }
@@ -350,9 +398,19 @@ __global__ void __launch_bounds__(256)
 
 template <typename T>
 __global__ void k_gather_typed(const T* __restrict__ x, const int32_t* __restrict__ inv, int64_t n, T* xr) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-       i += (int64_t)gridDim.x * blockDim.x)
-    xr[i] = __ldg(x + inv[i]);
+  // four ranks of a thread in flight
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += 4 * stride) {
+    int32_t c[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) c[u] = i + u * stride < n ? __ldg(inv + i + u * stride) : 0;
+    T v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) v[u] = __ldg(x + c[u]);
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (i + u * stride < n) xr[i + u * stride] = v[u];
+  }
 }
 
 // S: the SELL-32 arrays; A: the CSR handle they were made of (nullptr for a SELL handle).
@@ -396,10 +454,10 @@ static int launch_sell32_typed(gg_ctx* ctx, gg_mat* S, const gg_mat* A, SR sr, c
   }
   if (P->nmulti > 0 && e == cudaSuccess) {
     if (A) sr.nz = static_cast<const T*>(A->nzval);
-    const int64_t cap = (int64_t)ctx->num_sms * 8;
-    k_sell32_typed_combine<SR><<<(int)(P->nmulti < cap ? P->nmulti : cap), 256, 0, ctx->stream>>>(
-        sr, perm, S->m, P->multi, P->nmulti, partials, flt, A ? A->rowptr : nullptr,
-        A ? A->colval : nullptr);
+    const int64_t cap = (int64_t)ctx->num_sms * 8, nblk = P->nwide + (P->nnarrow + 7) / 8;
+    k_sell32_typed_combine<SR><<<(int)(nblk < cap ? nblk : cap), 256, 0, ctx->stream>>>(
+        sr, perm, S->m, P->wide, P->nwide, P->narrow, P->nnarrow, partials, flt,
+        A ? A->rowptr : nullptr, A ? A->colval : nullptr);
     trace_count(ctx, 1);
   }
   if (e == cudaSuccess) e = cudaGetLastError();
