@@ -4,6 +4,7 @@ Device arrays are torch CUDA tensors (torch is used for device memory and stream
 only).  Each device gets one library context; every call binds the caller's current
 torch stream, so work is ordered with the caller's own kernels like the reference's
 KernelAbstractions launches are ordered on the backend's stream."""
+import contextlib
 import ctypes
 
 import numpy as np
@@ -22,6 +23,7 @@ NP2CODE = {np.dtype(np.bool_): BOOL, np.dtype(np.int32): INT32, np.dtype(np.int6
 CODE2NP = {v: k for k, v in NP2CODE.items()}
 
 _ctx = {}
+_HERE = contextlib.nullcontext()
 
 
 def lib():
@@ -42,9 +44,22 @@ def ctx(device=None):
         check(L.gg_init(device, ctypes.byref(h)), L)
         c = h
         _ctx[device] = c
-    stream = torch.cuda.current_stream(device).cuda_stream
-    check(L.gg_set_stream(c, ctypes.c_void_p(stream)), L)
+    if not torch.cuda.is_initialized():
+        torch.cuda.init()
+    # the stream's address alone: a torch Stream object of every call would be thrown away
+    rc = L.gg_set_stream(c, torch._C._cuda_getCurrentRawStream(device))
+    if rc:
+        check(rc, L)
     return c
+
+
+def on_device(device):
+    """Context manager under which `device` is the current one.  Small calls are bound by
+    the host, and most are made with their device current already: torch.cuda.device would
+    then switch to it and back for nothing."""
+    if torch.cuda.current_device() == device.index:
+        return _HERE
+    return torch.cuda.device(device)
 
 
 def dtype_code(t):

@@ -37,7 +37,7 @@ def gpu_ewise_(z, x, y, op, mask=None):
         raise ArgumentError("All inputs must be on the same backend")
     mask, mcode = _mask_args(mask, z.numel(), z.device)
     L = core.lib()
-    with torch.cuda.device(z.device):
+    with core.on_device(z.device):
         c = core.ctx(z.device)
         check(L.gg_ewise(c, op_code(op), core.ptr(z), core.dtype_code(z), core.ptr(x),
                          core.dtype_code(x), core.ptr(y), core.dtype_code(y), z.numel(),
@@ -69,7 +69,7 @@ def gpu_apply_(z, x, s, op, bind_first=False, s_dtype=None, mask=None):
     buf, scode = _scalar(s, s_dtype, x.dtype)
     mask, mcode = _mask_args(mask, z.numel(), z.device)
     L = core.lib()
-    with torch.cuda.device(z.device):
+    with core.on_device(z.device):
         c = core.ctx(z.device)
         check(L.gg_apply(c, op_code(op), core.ptr(z), core.dtype_code(z), core.ptr(x),
                          core.dtype_code(x), buf.ctypes.data_as(ctypes.c_void_p), scode,
@@ -85,7 +85,7 @@ def gpu_reduce(x, add):
     code = core.dtype_code(x)
     out = np.zeros(1, dtype=core.CODE2NP[code])
     L = core.lib()
-    with torch.cuda.device(x.device):
+    with core.on_device(x.device):
         c = core.ctx(x.device)
         check(L.gg_reduce(c, op_code(add), core.ptr(x), code, x.numel(),
                           out.ctypes.data_as(ctypes.c_void_p)), L)

@@ -42,17 +42,18 @@ def gpu_spmv_(C, A, B, mul=GPUGraphs_mul, add=GPUGraphs_add, accum=GPUGraphs_sec
         raise ArgumentError("A must be a SparseGPUMatrixCSR, SparseGPUMatrixCSC or SparseGPUMatrixSELL")
     if not isinstance(B, torch.Tensor) or not isinstance(C, torch.Tensor):
         raise ArgumentError("All inputs must be on the same backend")
-    if A.size(2) != B.numel():
-        raise DimensionMismatch("Matrix dimensions must agree")
-    if C.shape[0] != A.size(1):
+    nb, nc = B.numel(), C.numel()
+    if A.n != nb or C.shape[0] != A.m:
         raise DimensionMismatch("Matrix dimensions must agree")
     tv, tx, ty = A.dtype_code, core.dtype_code(B), core.dtype_code(C)
     if core.promote_code(tv, tx) != ty:
         raise ArgumentError("Result type must be able to hold the result of the multiplication")
+    dev = A.device
     for t, name in ((B, "B"), (C, "C")):
-        core.device_vector(t, name)
-        if t.device != A.device:
+        if not t.is_cuda or t.device != dev:
             raise ArgumentError("All inputs must be on the same backend")
+        if not t.is_contiguous():
+            raise ArgumentError("%s must be contiguous" % name)
     mcode, mlen, mp = 0, 0, None
     if mask is not None:
         if not isinstance(mask, torch.Tensor) or mask.dim() != 1:
@@ -67,10 +68,11 @@ def gpu_spmv_(C, A, B, mul=GPUGraphs_mul, add=GPUGraphs_add, accum=GPUGraphs_sec
     L = core.lib()
     # a CSC matrix is the CSR storage of its transpose: its product is the transposed SpMV
     fn = L.gg_spmv_t if isinstance(A, SparseGPUMatrixCSC) else L.gg_spmv
-    with torch.cuda.device(A.device):
-        c = core.ctx(A.device)
-        check(fn(c, A.handle, op_code(mul), op_code(add), op_code(accum), core.ptr(C), ty,
-                 C.numel(), core.ptr(B), tx, B.numel(), mp, mcode, mlen, lo, hi), L)
+    with core.on_device(dev):
+        rc = fn(core.ctx(dev), A.handle, op_code(mul), op_code(add), op_code(accum), C.data_ptr(),
+                ty, nc, B.data_ptr(), tx, nb, mp, mcode, mlen, lo, hi)
+        if rc:
+            check(rc, L)
     return None
 
 
@@ -123,7 +125,7 @@ def gpu_spmm_(C, A, B, mul=GPUGraphs_mul, add=GPUGraphs_add, accum=GPUGraphs_sec
         mcode, mlen, mp = core.dtype_code(mask), mask.numel(), core.ptr(mask)
     lo, hi = _range_bounds(range)
     L = core.lib()
-    with torch.cuda.device(A.device):
+    with core.on_device(A.device):
         c = core.ctx(A.device)
         check(L.gg_spmm(c, A.handle, op_code(mul), op_code(add), op_code(accum), core.ptr(C),
                         core.dtype_code(C), C.shape[0], ldc, core.ptr(B), core.dtype_code(B),
@@ -155,7 +157,7 @@ def gpu_spmspv_(C, A, B, mul=GPUGraphs_mul, add=GPUGraphs_add, accum=GPUGraphs_s
     out = torch.empty(max(A.size(1), 1), dtype=torch.int32, device=A.device)
     cnt = ctypes.c_int64(0)
     L = core.lib()
-    with torch.cuda.device(A.device):
+    with core.on_device(A.device):
         c = core.ctx(A.device)
         check(L.gg_spmspv(c, A.handle, op_code(mul), op_code(add), op_code(accum), core.ptr(C), ty,
                           C.numel(), core.ptr(B.nzind), core.ptr(B.nzval), tx, B.nnz(), B.n,
@@ -190,7 +192,7 @@ def gpu_spmv_rows_(C, A, B, rows, mul=GPUGraphs_mul, add=GPUGraphs_add, accum=GP
         rows = torch.as_tensor(rows, dtype=torch.int32)
     rows = rows.to(device=A.device, dtype=torch.int32).contiguous()
     L = core.lib()
-    with torch.cuda.device(A.device):
+    with core.on_device(A.device):
         c = core.ctx(A.device)
         check(L.gg_spmv_rows(c, A.handle, op_code(mul), op_code(add), op_code(accum), core.ptr(C),
                              ty, C.numel(), core.ptr(B), tx, B.numel(), core.ptr(rows),
