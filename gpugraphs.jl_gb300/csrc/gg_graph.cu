@@ -1212,7 +1212,13 @@ static int bfs_run(gg_ctx* ctx, gg_mat* A, int32_t s, int which, int32_t* dist,
   bool frontier_is_bitmap = false, pull = false;  // a pull level leaves a bitmap, no queue
   const int64_t total_edges = P.nnz;
   // hub-free graphs (grids, meshes) run medium frontiers in the persistent kernel
-  const bool coop_ok = P.max_deg <= kCoopMaxDeg && n >= (1 << 16);
+  // Hub-free graphs with few entries a vertex, whose levels are many and narrow, run in the
+  // cluster and grid-wide persistent kernels: 70 x 33 grid 240 to 193 us, 250 x 250 grid
+  // 1324 to 883, ER with 6 entries a vertex and 10^4 / 10^6 vertices 246 to 94 and 415 to
+  // 335.  With more entries the frontier is most of the graph within a few levels, and
+  // separate pull launches are faster: ER with 32 entries a vertex and 60000 / 10^6 / 4 10^6
+  // vertices, persistent 236 / 539 / 822 us, separate 140 / 231 / 359.
+  const bool coop_ok = P.max_deg <= kCoopMaxDeg && n >= 2048 && P.nnz <= 6 * n;
   const int32_t small_cap = coop_ok ? kCoopLo : kSmallCap;
   const long long coop_hi = n / 24 > kCoopLo ? n / 24 : kCoopLo;
   CoopCtl* hc = reinterpret_cast<CoopCtl*>(ctx->h_flags);
@@ -2343,6 +2349,17 @@ int weight_sorted_rows(gg_ctx* ctx, gg_mat* A, const int32_t** col, const void**
   return GG_OK;
 }
 
+// Whether the pull rounds of A (its out-edge view is there) run over the SELL-32 copy:
+// large CSR handles, and smaller ones with hubs.  R-MAT with 9000 / 16384 / 45000
+// vertices: 949 / 1451 / 1584 us by the push and hub rounds, 306 / 319 / 350 over the copy;
+// the first search, which builds it, 1.53 / 2.37 / 2.92 and 1.70 / 2.08 / 2.53 ms, hence
+// the line.  Without hubs the gain (ER, 60000 vertices: 510 to 352 us) would take seven
+// searches to pay for a copy that takes 1.1 ms.
+static bool pulls_over_copy(const gg_mat* A) {
+  if (A->format != GG_FMT_CSR) return false;
+  return A->m >= (1 << 16) || (A->m >= 12288 && A->aux->push[2].max_deg > kPushHub);
+}
+
 // Builds, ahead of any concurrent use, every analysis a shortest-path search of A may
 // build on first use: the out-edge view with weights, the hub plan and (large CSR
 // handles) the SELL-32 copy of the pull rounds.  The serving loop calls it when a
@@ -2359,9 +2376,16 @@ int sssp_prepare(gg_ctx* ctx, gg_mat* A) {
     g->max_in_deg = ctx->h_flags[0];
   }
   if (g->max_in_deg > 32) GG_CHECK(build_hub_plan(ctx, A, g->vrowptr, A->m));
-  if (A->format == GG_FMT_CSR && A->m >= (1 << 16)) GG_CHECK(ensure_pull_sell(ctx, A));
+  if (pulls_over_copy(A)) GG_CHECK(ensure_pull_sell(ctx, A));
   return GG_OK;
 }
+
+// Hub-free graphs of at least this many vertices are searched by the near-far kernel, with
+// a CTA for every kNearFarCta vertices up to one an SM (the frontier of a small graph fills
+// few CTAs, and a barrier among few is shorter).  Single-CTA rounds / near-far, us:
+// 33 x 31 grid 263 / 269 (one CTA an SM), 70 x 33 546 / 420, 70 x 70 775 / 542 (590 with
+// one CTA an SM), 128 x 128 1292 / 904, 250 x 250 4497 / 1875.
+static const int64_t kNearFarRows = 2048, kNearFarCta = 256;
 
 template <typename T>
 static int sssp_fixpoint(gg_ctx* ctx, gg_mat* A, T* d, int64_t* rounds_out) {
@@ -2396,7 +2420,7 @@ static int sssp_fixpoint(gg_ctx* ctx, gg_mat* A, T* d, int64_t* rounds_out) {
     GG_CHECK(build_hub_plan(ctx, A, g->vrowptr, n));
     hp = A->hubplan;
   }
-  const bool coop_ok = P.max_deg <= kCoopMaxDeg && n >= (1 << 16);
+  const bool coop_ok = P.max_deg <= kCoopMaxDeg && n >= kNearFarRows;
   if (coop_ok && nf > 0) {
     // hub-free graph: the whole search in one near-far ordered persistent launch
     if (g->avg_w < 0) GG_CHECK(mean_weight(ctx, A));
@@ -2414,7 +2438,9 @@ static int sssp_fixpoint(gg_ctx* ctx, gg_mat* A, T* d, int64_t* rounds_out) {
     long long max_steps = 8 * (long long)n + 1024;
     void* args[] = {&P.rowptr, &P.colval, &pw, &qa, &qb, &sc.hq, &sc.q2, &sc.q3, &d, &ia, &ib,
                     &sc.visited, &ncc, &delta, &max_steps};
-    GG_CUDA(cudaLaunchCooperativeKernel((const void*)k_sssp_nearfar<T>, dim3(ctx->num_sms),
+    const int64_t want = n / kNearFarCta;
+    const int ctas = (int)(want < ctx->num_sms ? want : ctx->num_sms);
+    GG_CUDA(cudaLaunchCooperativeKernel((const void*)k_sssp_nearfar<T>, dim3(ctas),
                                         dim3(kNfThreads), args, 0, ctx->stream));
     NfCtl hn;
     GG_CUDA(cudaMemcpyAsync(&hn, ncc, sizeof(NfCtl), cudaMemcpyDeviceToHost, ctx->stream));
@@ -2426,7 +2452,7 @@ static int sssp_fixpoint(gg_ctx* ctx, gg_mat* A, T* d, int64_t* rounds_out) {
   }
   const int32_t small_cap = kSmallCap;
   // large CSR handles pull over a SELL-32 copy (built at the first pull round)
-  const bool sell_pull = A->format == GG_FMT_CSR && n >= (1 << 16);
+  const bool sell_pull = pulls_over_copy(A);
   T dlow = T(0);  // no distance below it was written in the previous round
   while (nf > 0) {
     if (rounds > max_rounds) return set_error(GG_ERR_NOT_CONVERGED, "shortest_path did not converge");
