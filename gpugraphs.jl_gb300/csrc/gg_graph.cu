@@ -55,6 +55,7 @@ struct GraphAux {
   // entries by ascending weight when pull_sorted
   gg_mat* pull_sell = nullptr;
   bool pull_sorted = false;
+  bool no_pull_sell = false;  // a graph below 65536 vertices whose copy did not fit
   // CSR handles, batched shortest paths: the entries of every row by ascending weight
   // (rowptr is the handle's), built on first use
   int32_t* srt_col = nullptr;
@@ -436,6 +437,12 @@ struct Counters {
 // pieces of kPushPiece edges spread over all warps.  A piece is four steps of a warp
 // (bfs_push_range); with 2048 / 1024 one vertex below the line held its warp for 67 us.
 static const int kPushHub = 512;
+
+// Whether push rounds have the two hub launches at all: in a graph of under 2^20 edges a
+// warp is through with at most 2048 of them before the launches would be.
+static bool defer_hubs(const PushCSR& P) {
+  return P.max_deg > (P.nnz < (1 << 20) ? 4 * kPushHub : kPushHub);
+}
 static const int kPushPiece = 512;
 
 __global__ void k_bfs_init(int32_t s, unsigned* visited, int32_t* dist, int32_t* q) {
@@ -566,6 +573,8 @@ __global__ void __launch_bounds__(256)
   warp_add(edges, &ctr->mf);
 }
 
+static const int64_t kPullQueueRows = 1 << 16;
+
 // bottom-up level: thread per vertex; an unvisited vertex joins when one of its
 // in-neighbours (A_T row) is in the frontier bitmap over an active edge.  In-edges are
 // tested four at a time (one 32-byte sector of columns, then four bitmap words, in
@@ -574,12 +583,13 @@ __global__ void __launch_bounds__(256)
 // it then (k_bitmap_to_queue).  With a queue written by every level (two same-address
 // atomics per warp, a million in one level of R-MAT scale 24) and one in-edge at a time
 // the three pull levels of a scale-24 search took 2130 us; the whole search went from
-// 3.00 to 0.66 ms.
+// 3.00 to 0.66 ms.  Small graphs (kPullQueueRows) pass a queue: the conversion's launch
+// costs more than a few appends (R-MAT, 3000 vertices: 152 us with it, 138 without).
 template <bool kOddOnly>
 __global__ void __launch_bounds__(256)
     k_bfs_pull(int64_t n, const int32_t* __restrict__ rp, const int32_t* __restrict__ cv,
                const void* nz, int tv, const unsigned* __restrict__ fb, unsigned* visited,
-               int32_t* dist, int32_t level, unsigned* fbn, Counters* ctr,
+               int32_t* dist, int32_t level, unsigned* fbn, int32_t* queue, Counters* ctr,
                const int32_t* __restrict__ prow) {
   __shared__ unsigned long long s_nf, s_mf;
   if (threadIdx.x == 0) s_nf = s_mf = 0;
@@ -614,6 +624,12 @@ __global__ void __launch_bounds__(256)
       const int64_t word = v >> 5;  // the warp's 32 vertices share one bitmap word
       visited[word] = vw | bal;
       fbn[word] = bal;
+    }
+    if (queue && bal) {  // the same for the whole warp
+      unsigned long long at = 0;
+      if (lane == 0) at = atomicAdd(&ctr->pad, (unsigned long long)__popc(bal));
+      at = __shfl_sync(kFullG, at, 0) + __popc(bal & ((1u << lane) - 1u));
+      if (found) queue[at] = (int32_t)v;
     }
   }
   warp_add(joined, &s_nf);
@@ -1211,6 +1227,7 @@ static int bfs_run(gg_ctx* ctx, gg_mat* A, int32_t s, int which, int32_t* dist,
   int cur = 0;
   bool frontier_is_bitmap = false, pull = false;  // a pull level leaves a bitmap, no queue
   const int64_t total_edges = P.nnz;
+  const bool pull_queue = n < kPullQueueRows;
   // hub-free graphs (grids, meshes) run medium frontiers in the persistent kernel
   // Hub-free graphs with few entries a vertex, whose levels are many and narrow, run in the
   // cluster and grid-wide persistent kernels: 70 x 33 grid 240 to 193 us, 250 x 250 grid
@@ -1287,6 +1304,17 @@ static int bfs_run(gg_ctx* ctx, gg_mat* A, int32_t s, int which, int32_t* dist,
       }
       continue;
     }
+    if (pull && nf * 24 < n && nf <= small_cap && mf <= (int64_t)kSmallEdges) {
+      // the pull levels are over and one CTA can take the rest: no push level in between
+      const int64_t nwords = (n + 31) / 32;
+      if (!pull_queue) {
+        GG_CUDA(cudaMemsetAsync(sc.ctr, 0, sizeof(Counters), ctx->stream));
+        k_bitmap_to_queue<<<gridsz(ctx, nwords), 256, 0, ctx->stream>>>(sc.fb[cur], nwords, sc.q[cur],
+                                                                        &sc.ctr->pad);
+        GG_CUDA(cudaGetLastError());
+      }
+      pull = frontier_is_bitmap = false;
+    }
     if (!pull && nf <= small_cap && mf <= (int64_t)kSmallEdges) {
       k_bfs_small<<<1, kSmallThreads, kSmallSmem, ctx->stream>>>(
           P.rowptr, P.colval, sc.q[cur], (int32_t)nf, (int32_t)level, small_cap, sc.visited, dist,
@@ -1319,19 +1347,19 @@ static int bfs_run(gg_ctx* ctx, gg_mat* A, int32_t s, int which, int32_t* dist,
       if (odd_only)
         k_bfs_pull<true><<<gridsz(ctx, n), 256, 0, ctx->stream>>>(
             n, g->vrowptr, g->vcolval, g->vnz, A->dtype, sc.fb[cur], sc.visited, dist,
-            (int32_t)level, sc.fb[cur ^ 1], sc.ctr, P.rowptr);
+            (int32_t)level, sc.fb[cur ^ 1], pull_queue ? sc.q[cur ^ 1] : nullptr, sc.ctr, P.rowptr);
       else
         k_bfs_pull<false><<<gridsz(ctx, n), 256, 0, ctx->stream>>>(
             n, g->vrowptr, g->vcolval, g->vnz, A->dtype, sc.fb[cur], sc.visited, dist,
-            (int32_t)level, sc.fb[cur ^ 1], sc.ctr, P.rowptr);
+            (int32_t)level, sc.fb[cur ^ 1], pull_queue ? sc.q[cur ^ 1] : nullptr, sc.ctr, P.rowptr);
       frontier_is_bitmap = true;
     } else {
-      if (frontier_is_bitmap) {
+      if (frontier_is_bitmap && !pull_queue) {
         const int64_t nwords = (n + 31) / 32;
         k_bitmap_to_queue<<<gridsz(ctx, nwords), 256, 0, ctx->stream>>>(sc.fb[cur], nwords, sc.q[cur],
                                                                         &sc.ctr->pad);
       }
-      const bool hubs = P.max_deg > kPushHub;
+      const bool hubs = defer_hubs(P);
       k_bfs_push<<<gridsz(ctx, nf * 32), 256, 0, ctx->stream>>>(
           P.rowptr, P.colval, sc.q[cur], nf, (int32_t)level, sc.visited, dist, sc.q[cur ^ 1], sc.ctr,
           hubs ? sc.hq : nullptr);
@@ -2357,7 +2385,16 @@ int weight_sorted_rows(gg_ctx* ctx, gg_mat* A, const int32_t** col, const void**
 // searches to pay for a copy that takes 1.1 ms.
 static bool pulls_over_copy(const gg_mat* A) {
   if (A->format != GG_FMT_CSR) return false;
-  return A->m >= (1 << 16) || (A->m >= 12288 && A->aux->push[2].max_deg > kPushHub);
+  return A->m >= (1 << 16) ||
+         (A->m >= 12288 && A->aux->push[2].max_deg > kPushHub && !A->aux->no_pull_sell);
+}
+
+// Builds the copy; the smaller graphs go without where it does not fit.
+static int pull_copy(gg_ctx* ctx, gg_mat* A) {
+  const int rc = ensure_pull_sell(ctx, A);
+  if (rc == GG_OK || A->m >= (1 << 16)) return rc;
+  A->aux->no_pull_sell = true;
+  return GG_OK;
 }
 
 // Builds, ahead of any concurrent use, every analysis a shortest-path search of A may
@@ -2376,7 +2413,7 @@ int sssp_prepare(gg_ctx* ctx, gg_mat* A) {
     g->max_in_deg = ctx->h_flags[0];
   }
   if (g->max_in_deg > 32) GG_CHECK(build_hub_plan(ctx, A, g->vrowptr, A->m));
-  if (pulls_over_copy(A)) GG_CHECK(ensure_pull_sell(ctx, A));
+  if (pulls_over_copy(A)) GG_CHECK(pull_copy(ctx, A));
   return GG_OK;
 }
 
@@ -2452,7 +2489,7 @@ static int sssp_fixpoint(gg_ctx* ctx, gg_mat* A, T* d, int64_t* rounds_out) {
   }
   const int32_t small_cap = kSmallCap;
   // large CSR handles pull over a SELL-32 copy (built at the first pull round)
-  const bool sell_pull = pulls_over_copy(A);
+  bool sell_pull = pulls_over_copy(A);
   T dlow = T(0);  // no distance below it was written in the previous round
   while (nf > 0) {
     if (rounds > max_rounds) return set_error(GG_ERR_NOT_CONVERGED, "shortest_path did not converge");
@@ -2482,8 +2519,11 @@ static int sssp_fixpoint(gg_ctx* ctx, gg_mat* A, T* d, int64_t* rounds_out) {
     ++rounds;
     GG_CUDA(cudaMemsetAsync(sc.ctr, 0, sizeof(Counters), ctx->stream));
     if (sell_pull && mf * kPullSellDiv > P.nnz) {
+      GG_CHECK(pull_copy(ctx, A));
+      sell_pull = g->pull_sell != nullptr;
+    }
+    if (sell_pull && mf * kPullSellDiv > P.nnz) {
       // large frontier: pull round over the SELL-32 copy, every in-edge
-      GG_CHECK(ensure_pull_sell(ctx, A));
       const gg_mat* S = g->pull_sell;
       const SellPlan* SP = S->sellplan;
       if (SP->npitems > 0)
@@ -2526,7 +2566,7 @@ static int sssp_fixpoint(gg_ctx* ctx, gg_mat* A, T* d, int64_t* rounds_out) {
       cur ^= 1;
       continue;
     }
-    const bool hubs = P.max_deg > kPushHub;
+    const bool hubs = defer_hubs(P);
     k_sssp_push<T><<<gridsz(ctx, nf * 32), 256, 0, ctx->stream>>>(
         P.rowptr, P.colval, static_cast<const T*>(P.w), sc.q[cur], nf, d, sc.fb[cur],
         sc.fb[cur ^ 1], sc.q[cur ^ 1], sc.ctr, hubs ? sc.hq : nullptr);
