@@ -444,10 +444,11 @@ def run_spmv_rmat(args, scale=22):
                         "+ k_hubwin / k_hw_combine (the %d hub rows folded from shared-memory "
                         "column windows)" % G.spmv_hub_rows(A))
     else:
-        kernel_label = ({"registers": "k_sell_hot32", "bulk_copy": "k_sell_tma32",
-                         "hub_windows": "k_sell_hot32"}[
-            args.sell_variant or "registers"]
-            + " (SELL-32 copy sorted by row length, relabelled columns)")
+        tuned = args.sell_variant or args.hot_cols or args.layout == "sell"
+        by_default = "k_sell32_typed" if n < (3 << 22) else "k_sell_hot32"
+        kernel_label = ((("k_sell_tma32" if args.sell_variant == "bulk_copy" else "k_sell_hot32")
+                         if tuned else by_default)
+                        + " (SELL-32 copy sorted by row length, relabelled columns)")
     # parity of this run's own output, every row, after the timed region
     parity = {}
     if rank == 0 and not args.no_parity:

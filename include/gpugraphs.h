@@ -202,10 +202,14 @@ int gg_mat_values_changed(gg_ctx* ctx, gg_mat* A);
  * such a column are not written.  Checks of _validate_args (src/spmv/CSR.jl:358-408)
  * return GG_ERR_DIMENSION / GG_ERR_TYPE.
  * Device memory: the first call of a kind builds its analysis on the handle, kept until
- * gg_mat_destroy or gg_mat_values_changed.  The first plus-times Float32 call on a CSR
- * handle of at least 65536 rows builds a SELL-32 copy of the matrix with rows sorted by
- * length and relabelled columns: about 12 bytes per stored entry plus 16 per row, i.e.
- * more than the CSR itself (about 1.6 GB at R-MAT scale 22, 6.5 GB at scale 24).  Other
+ * gg_mat_destroy or gg_mat_values_changed.  The first call with one element type and a
+ * common semiring (mul / add, add or safe_add / min, band or land / bor or lor) on a CSR
+ * handle of at least 65536 rows, or on a SELL handle with more than a quarter of padding, builds
+ * a SELL-32 copy of the matrix with rows sorted by length and relabelled columns: about
+ * 8 bytes per stored entry more than the values take, plus 16 per row, i.e. more than the
+ * CSR itself (4-byte values: about 1.6 GB at R-MAT scale 22, 6.5 GB at scale 24); the
+ * semirings of a handle share it.  Where it does not fit, semirings other than Float32
+ * plus-times run on the handle's own arrays.  Other
  * first calls add row-block descriptors (16 bytes per block of up to 256 entries).
  * Later calls allocate nothing and are asynchronous.
  */
@@ -220,6 +224,11 @@ int gg_spmv(gg_ctx* ctx, const gg_mat* A, int mul, int add, int accum, void* y, 
  * B is b_rows x k, C is c_rows x k, both in `layout` with leading dimensions ldb/ldc
  * (elements).  Mask / range select rows as in gg_spmv.  Shape checks return
  * GG_ERR_ASSERTION like the reference's @assert.
+ * Column-major operands, and row-major Float32 ones whose width is not a multiple of
+ * four, are transposed or padded through the context's scratch where that takes at most
+ * 1.25 GiB.  The scratch grows on demand, so a call that is to be captured in a CUDA
+ * graph is made once before, and a larger call on the context afterwards may move the
+ * scratch that a captured one uses.
  */
 int gg_spmm(gg_ctx* ctx, const gg_mat* A, int mul, int add, int accum, void* C, int c_dtype,
             int64_t c_rows, int64_t ldc, const void* B, int b_dtype, int64_t b_rows,
@@ -406,10 +415,10 @@ int gg_bfs_levels_batch(gg_ctx* ctx, const gg_mat* A_T, const int64_t* sources, 
  * round.  Needs non-negative weights (GG_ERR_UNSUPPORTED otherwise; gg_sssp then
  * runs the reference's Jacobi rounds).  gg_sssp routes several sources here.
  * Memory: a 32-column distance block (n x 32 elements) per group of 32 sources, up to
- * 8 groups at once; for CSR graphs of at least 65536 vertices with 4-byte distances
- * the rounds over every vertex also use the SELL-32 copy of A_T that single-source
- * gg_sssp builds (about the size of the CSR), built by the first call that needs it
- * (when it does not fit, those rounds run vertex by vertex instead).
+ * 8 groups at once; for CSR graphs with 4-byte distances the rounds over every vertex
+ * also use a copy of the entries by ascending weight in each row (8 bytes per entry),
+ * built by the first call that needs it (when it does not fit, those rounds run vertex
+ * by vertex instead).
  */
 int gg_sssp_batch(gg_ctx* ctx, const gg_mat* A_T, const int64_t* sources, int64_t S, void* dist,
                   int dist_dtype, int64_t ld, int64_t* rounds_out);
@@ -479,8 +488,7 @@ int gg_multigraph_info(const gg_multigraph* mg, int64_t* ngraphs, int64_t* total
  * x, y: concatenated device vectors of total_n entries.  Asynchronous. */
 int gg_multigraph_spmv(gg_ctx* ctx, const gg_multigraph* mg, const float* x, float* y);
 /* One BFS per graph (sources[g], 1-based within graph g, host array) in one
- * persistent cooperative launch captured in a CUDA graph (re-captured when dist
- * changes).  dist: concatenated Int32 device vector, levels as bfs_distances of
+ * persistent cooperative launch captured in a CUDA graph.  dist: concatenated Int32 device vector, levels as bfs_distances of
  * each graph with rows of A_T used as out-edges (exact for symmetric graphs; a
  * floating-point graph is searched over its Bool pattern, every stored entry an
  * edge), typemax(Int32) when unreached.  Synchronous; GG_ERR_TIMEOUT if the grid barrier's
@@ -494,7 +502,8 @@ int gg_multigraph_bfs(gg_ctx* ctx, gg_multigraph* mg, const int64_t* sources, in
  * for symmetric graphs).  dist: concatenated device vector of dist_dtype (Int32 for
  * Bool graphs, else the graphs' type), typemax / +Inf when unreached.  Needs
  * non-negative weights (GG_ERR_UNSUPPORTED otherwise).  Synchronous; GG_ERR_TIMEOUT
- * if the grid barrier's bounded wait ran out.  rounds_out: rounds run. */
+ * if the grid barrier's bounded wait ran out.  rounds_out: steps run (large sets take
+ * the vertices of one distance band after another, several steps a band). */
 int gg_multigraph_sssp(gg_ctx* ctx, gg_multigraph* mg, const int64_t* sources, void* dist,
                        int dist_dtype, int64_t* rounds_out);
 
