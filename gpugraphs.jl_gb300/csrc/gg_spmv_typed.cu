@@ -376,13 +376,17 @@ __global__ void __launch_bounds__(256)
     T acc[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) acc[k] = sr.neutral();
-    for (int c = warp; c < d.z; c += 32) {
-      T v[4];
+    // chunks of a warp in flight (a hub's slice has a thousand and more).  4 / 16, us:
+    // or-and scale 20 88.8 / 82.6, min-plus Int32 scale 21 177.6 / 172.9, Float64 scale 20
+    // 203.7 / 204.8
+    constexpr int kFly = sizeof(T) == 8 ? 4 : 16;
+    for (int c = warp; c < d.z; c += 8 * kFly) {
+      T v[kFly];
 #pragma unroll
-      for (int k = 0; k < 4; ++k)
+      for (int k = 0; k < kFly; ++k)
         v[k] = c + 8 * k < d.z ? partials[(int64_t)(d.y + c + 8 * k) * 32 + lane] : sr.neutral();
 #pragma unroll
-      for (int k = 0; k < 4; ++k) acc[k] = sr.step(acc[k], v[k]);
+      for (int k = 0; k < kFly; ++k) acc[k & 3] = sr.step(acc[k & 3], v[k]);
     }
     part[warp][lane] = sr.step(sr.step(acc[0], acc[2]), sr.step(acc[1], acc[3]));
     __syncthreads();
