@@ -429,7 +429,7 @@ struct Counters {
   // shortest paths: smallest distance written in the round, as ~(its bits) and folded
   // with max, so that the cleared word means "none noted"
   unsigned long long low;
-  unsigned long long pad2;
+  unsigned long long odd_start;  // shortest paths: a start distance with a sign bit, or NaN
 };
 
 // Frontier vertices with more than kPushHub out-edges are not walked by one warp:
@@ -1438,12 +1438,16 @@ template <> __device__ __forceinline__ int32_t atomic_min_t<int32_t>(int32_t* p,
 template <> __device__ __forceinline__ int64_t atomic_min_t<int64_t>(int64_t* p, int64_t v) {
   return (int64_t)atomicMin((long long*)p, (long long)v);
 }
-// non-negative floats order like their bit patterns
+// Floats order like their bit patterns read as signed integers, except that negative ones
+// (a caller's start) order the other way among themselves, as their unsigned bits do.
 template <> __device__ __forceinline__ float atomic_min_t<float>(float* p, float v) {
-  return __int_as_float(atomicMin((int*)p, __float_as_int(v)));
+  const int b = __float_as_int(v);
+  return __int_as_float(b >= 0 ? atomicMin((int*)p, b) : (int)atomicMax((unsigned*)p, (unsigned)b));
 }
 template <> __device__ __forceinline__ double atomic_min_t<double>(double* p, double v) {
-  return __longlong_as_double(atomicMin((long long*)p, __double_as_longlong(v)));
+  const long long b = __double_as_longlong(v);
+  return __longlong_as_double(b >= 0 ? atomicMin((long long*)p, b)
+                                     : (long long)atomicMax((unsigned long long*)p, (unsigned long long)b));
 }
 
 template <typename T> __device__ __forceinline__ T ld_cg(const T* p) { return __ldcg(p); }
@@ -1724,20 +1728,29 @@ __global__ void __launch_bounds__(1024)
   }
 }
 
-// frontier = every vertex whose start distance is finite
+// frontier = every vertex whose start distance is finite.  Start distances below zero (-0.0
+// among them) or NaN are noted: a caller may start from any values, and the bounds that
+// searches end early by hold from non-negative ones only.
+template <typename T> __device__ __forceinline__ bool odd_start(T d) { return d < T(0); }
+template <> __device__ __forceinline__ bool odd_start<float>(float d) { return !(d >= 0.0f) || signbit(d); }
+template <> __device__ __forceinline__ bool odd_start<double>(double d) { return !(d >= 0.0) || signbit(d); }
 template <typename T>
 __global__ void __launch_bounds__(256) k_sssp_seed(int64_t n, const T* dist, unsigned* inq, int32_t* q, Counters* ctr) {
   __shared__ int32_t stage[8][WarpQueue::kCap];
   WarpQueue wq(stage[threadIdx.x >> 5], q, &ctr->nf);
   const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+  bool odd = false;
   for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < n; base += stride) {
     const int64_t v = base + threadIdx.x;
-    const bool fin = v < n && dist[v] != Lim<T>::max();
+    const T d = v < n ? dist[v] : Lim<T>::max();
+    const bool fin = d != Lim<T>::max();
+    odd |= odd_start<T>(d);
     const unsigned bal = __ballot_sync(kFullG, fin);
     if ((threadIdx.x & 31) == 0 && bal) inq[v >> 5] = bal;
     wq.push(fin, (int32_t)v);
   }
   wq.flush();
+  if (odd) ctr->odd_start = 1;
 }
 
 template <typename T>
@@ -1798,7 +1811,7 @@ __global__ void __launch_bounds__(kNfThreads, 1)
     k_sssp_nearfar(const int32_t* __restrict__ prow, const int32_t* __restrict__ pcol,
                    const T* __restrict__ pw, int32_t* qa, int32_t* qb, int32_t* fa, int32_t* fb,
                    int32_t* fz, T* dist, unsigned* inq_a, unsigned* inq_b, unsigned* infar,
-                   NfCtl* cc, T delta, long long max_steps) {
+                   NfCtl* cc, T delta, long long max_steps, bool look_first) {
   __shared__ StepLists S;
   const int lane = threadIdx.x & 31;
   const int64_t gw = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
@@ -1883,7 +1896,8 @@ __global__ void __launch_bounds__(kNfThreads, 1)
             w = __ldg(pcol + k);
             const T cand = relax_add(__ldg(pw + k), du);
             // lowered by the atomic alone: one L2 round trip on the step's critical path
-            if (cand < atomic_min_t(dist + w, cand)) {
+            // (look_first: a NaN start's bits would give way to it)
+            if ((!look_first || cand < ld_cg(dist + w)) && cand < atomic_min_t(dist + w, cand)) {
               const unsigned bit = 1u << (w & 31);
               if (cand < thr) near_add = !(atomicOr(inxt + (w >> 5), bit) & bit);
               else far_add = !(atomicOr(infar + (w >> 5), bit) & bit);
@@ -2171,7 +2185,8 @@ __global__ void __launch_bounds__(256)
 // With the copy's entries by ascending weight a row stops at the first weight w with
 // w + dlow >= its best distance so far (dlow: the smallest distance written in the
 // previous round, so no source that changed lies below it; sums of non-negative values
-// only grow, rounding included): what follows cannot improve it.  On R-MAT scale 22 with
+// only grow, rounding included): what follows cannot improve it.  A caller's start with
+// a negative distance, whose bits dlow does not order, scans whole rows.  On R-MAT scale 22 with
 // weights 1..255 most rows end within one or two groups of 8: a round takes 116 to 234 us
 // instead of 443.
 // ---------------------------------------------------------------------------------
@@ -2441,6 +2456,7 @@ static int sssp_fixpoint(gg_ctx* ctx, gg_mat* A, T* d, int64_t* rounds_out) {
   GG_CUDA(cudaMemcpyAsync(h, sc.ctr, sizeof(Counters), cudaMemcpyDeviceToHost, ctx->stream));
   GG_CUDA(cudaStreamSynchronize(ctx->stream));
   int64_t nf = (int64_t)h->nf, rounds = 0, mf = 0;
+  bool odd = h->odd_start != 0;
   int cur = 0;
   const int64_t max_rounds = n + 1;  // Bellman-Ford bound for non-negative weights
   if (g->max_in_deg < 0) {
@@ -2474,7 +2490,7 @@ static int sssp_fixpoint(gg_ctx* ctx, gg_mat* A, T* d, int64_t* rounds_out) {
     const T* pw = static_cast<const T*>(P.w);
     long long max_steps = 8 * (long long)n + 1024;
     void* args[] = {&P.rowptr, &P.colval, &pw, &qa, &qb, &sc.hq, &sc.q2, &sc.q3, &d, &ia, &ib,
-                    &sc.visited, &ncc, &delta, &max_steps};
+                    &sc.visited, &ncc, &delta, &max_steps, &odd};
     const int64_t want = n / kNearFarCta;
     const int ctas = (int)(want < ctx->num_sms ? want : ctx->num_sms);
     GG_CUDA(cudaLaunchCooperativeKernel((const void*)k_sssp_nearfar<T>, dim3(ctas),
@@ -2530,7 +2546,8 @@ static int sssp_fixpoint(gg_ctx* ctx, gg_mat* A, T* d, int64_t* rounds_out) {
         k_sssp_pull_sell<T><<<ctx->num_sms * (2048 / kPullSellThreads), kPullSellThreads, 0,
                               ctx->stream>>>(S->colval, S->nzval, S->dtype, S->perm, S->m,
                                              SP->pitems, SP->npitems, d, sc.fb[cur ^ 1],
-                                             sc.q[cur ^ 1], sc.ctr, P.rowptr, g->pull_sorted, dlow);
+                                             sc.q[cur ^ 1], sc.ctr, P.rowptr,
+                                             g->pull_sorted && !odd, dlow);
       // the consumed membership bitmap becomes the next round's target: clear it
       GG_CUDA(cudaMemsetAsync(sc.fb[cur], 0, ((n + 31) / 32) * sizeof(unsigned), ctx->stream));
       GG_CUDA(cudaGetLastError());
