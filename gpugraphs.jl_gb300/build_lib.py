@@ -33,6 +33,7 @@ def nvcc():
 
 def _deps():
     return (glob.glob(os.path.join(SRC, "*.cu")) + glob.glob(os.path.join(SRC, "*.cuh")) +
+            glob.glob(os.path.join(SRC, "*.h")) +
             [os.path.join(INCLUDE, "gpugraphs.h"), os.path.abspath(__file__)])
 
 

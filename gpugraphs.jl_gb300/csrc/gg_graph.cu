@@ -21,6 +21,7 @@
 //    Negative or NaN weights run the reference's Jacobi rounds (min-plus SpMV).
 #include <vector>
 
+#include "gg_band.h"
 #include "gg_queue.cuh"
 #include "gg_semiring.cuh"
 #include "gg_tma.cuh"
@@ -2477,10 +2478,7 @@ static int sssp_fixpoint(gg_ctx* ctx, gg_mat* A, T* d, int64_t* rounds_out) {
   if (coop_ok && nf > 0) {
     // hub-free graph: the whole search in one near-far ordered persistent launch
     if (g->avg_w < 0) GG_CHECK(mean_weight(ctx, A));
-    double dd = g->avg_w * kNearFarScale;
-    if (!(dd > 0.0)) dd = 1.0;
-    T delta = static_cast<T>(dd);
-    if (!(delta > T(0))) delta = T(1);
+    T delta = band_width<T>(g->avg_w * kNearFarScale);
     NfCtl* ncc = reinterpret_cast<NfCtl*>(sc.cc);
     k_nf_init<<<1, 1, 0, ctx->stream>>>(ncc, nf, barrier_polls(ctx));
     int32_t* qa = sc.q[cur];

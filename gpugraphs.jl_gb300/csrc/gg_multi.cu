@@ -26,6 +26,7 @@
 #include <algorithm>
 #include <vector>
 
+#include "gg_band.h"
 #include "gg_queue.cuh"
 #include "gg_semiring.cuh"
 
@@ -638,11 +639,8 @@ static int mg_sssp_capture(gg_ctx* ctx, gg_multigraph* M) {
   if (per_sm < 1) return set_error(GG_ERR_CUDA, "k_mg_sssp cannot be resident");
   const int grid = ctx->num_sms * per_sm;  // every block resident: the barrier is safe
   const double nnz = M->total_nnz > 0 ? (double)M->total_nnz : 1.0;
-  double dd = kMgBand * (M->sum_w / nnz) / (nnz / (double)(M->total_n > 0 ? M->total_n : 1));
-  if (!(dd > 0.0)) dd = 1.0;
-  if (dd > (double)Lim<T>::max() / 4) dd = (double)Lim<T>::max() / 4;
-  T delta = static_cast<T>(dd);
-  if (!(delta > T(0))) delta = T(1);
+  T delta = band_width<T>(kMgBand * (M->sum_w / nnz) /
+                           (nnz / (double)(M->total_n > 0 ? M->total_n : 1)));
   if (M->total_nnz < kMgBandNnz) delta = Lim<T>::max();
   cudaStream_t cs = nullptr;
   GG_CUDA(cudaStreamCreateWithFlags(&cs, cudaStreamNonBlocking));

@@ -6,6 +6,7 @@ import pytest
 import torch
 
 import gpugraphs as G
+from oracle import oracle as O
 from test_graph_gpu import _reference_inplace
 from test_search_queue_gpu import _graph
 
@@ -60,3 +61,19 @@ def test_hub_free_graphs(n, dtype):
     rp, cv, nz = _graph(n, r, c, dtype, seed=4)
     dist0, next0 = _starts(n, dtype, n, -60, 60)
     _check(n, rp, cv, nz, n // 2, dist0, next0)
+
+
+@pytest.mark.parametrize("dtype,scale", [(np.int32, 10**8), (np.int64, 10**17), (np.float32, 1e30)])
+@pytest.mark.parametrize("n", [2048, 5000])
+def test_heavy_weights(n, scale, dtype):
+    """Mean weights whose multiple, the near-far band, is past the distance type."""
+    rng = np.random.default_rng(n)
+    v = np.arange(n)
+    r, c = np.concatenate([v] * 6), np.concatenate([rng.permutation(n) for _ in range(6)])
+    keep = r != c
+    rp, cv, nz = _graph(n, r[keep], c[keep], dtype, seed=9)
+    nz = (np.minimum(nz, 4) * dtype(scale)).astype(dtype)
+    A = G.SparseGPUMatrixCSR(n, n, rp, cv, nz)
+    ref, _ = O.sssp(n, rp, cv, nz, [1, n])
+    for q, s in enumerate((1, n)):
+        assert (G.shortest_path(A, s).cpu().numpy() == ref[:, q]).all()
