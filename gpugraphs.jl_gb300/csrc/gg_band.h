@@ -1,4 +1,4 @@
-// gg_band.h -- band width of the near-far shortest-path searches (plain C++).
+// gg_band.h -- bands of the near-far shortest-path searches (plain C++).
 #pragma once
 
 #include <limits>
@@ -17,5 +17,11 @@ inline T band_width(double want) {
   const T width = static_cast<T>(want);
   return width > T(0) ? width : T(1);
 }
+
+// Empty bands in a row (each twice as wide as the one before) that a search takes before it
+// gives up: more than the doublings from the smallest Float64 to the largest.  A gap between
+// two distances takes about log2(gap / width) of them, which no count of vertices bounds
+// (1400 short paths 2^52 apart take some 45000), so they do not count as steps.
+static const int kEmptyBandRun = 2200;
 
 }  // namespace gg

@@ -1787,7 +1787,8 @@ __global__ void k_changed_copy(int64_t n, const T* next, T* dist, unsigned* flag
 // On high-diameter graphs with spread weights this avoids most of the repeated
 // relaxations of plain rounds.  The fixpoint is the same (min over paths of the
 // left-folded sums; every improved vertex is relaxed again eventually).  Grid
-// barriers are bounded (coop_leader_sync); the number of steps is bounded by max_steps.
+// barriers are bounded (coop_leader_sync).  Steps that relax something are bounded by
+// max_steps, a run of empty bands by kEmptyBandRun.
 struct NfCtl {
   unsigned long long cnt[3];  // near queue lengths, rotating as in CoopCtl
   unsigned long long fcnt[3];  // far list lengths (three lists in rotation)
@@ -1829,6 +1830,8 @@ __global__ void __launch_bounds__(kNfThreads, 1)
   int fc = 0;
   T thr = delta, width = delta;
   bool was_change = false;
+  long long empty = 0;  // bands that moved nothing, so far
+  int run = 0;          // the latest ones in a row
   if (threadIdx.x == 0) {
     S.n[0] = S.n[1] = 0;
     S.len = (long long)*((volatile unsigned long long*)&cc->cnt[2]);
@@ -1840,10 +1843,13 @@ __global__ void __launch_bounds__(kNfThreads, 1)
     const long long nf = S.len, nfar = S.flen;
     const int fn = fc == 2 ? 0 : fc + 1;
     const bool band = nf == 0;
-    if (st >= max_steps || (band && nfar == 0)) {
+    run = band && was_change ? run + 1 : 0;
+    empty += run > 0;
+    const bool out = st - empty >= max_steps || run > kEmptyBandRun;
+    if (out || (band && nfar == 0)) {
       if (blockIdx.x == 0 && threadIdx.x == 0) {
         cc->steps_out = st;
-        cc->status = st >= max_steps ? 2 : 1;
+        cc->status = out ? 2 : 1;
       }
       return;
     }

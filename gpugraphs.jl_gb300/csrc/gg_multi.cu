@@ -301,13 +301,18 @@ __global__ void __launch_bounds__(kMgThreads, 3)
   T thr = delta, width = delta;
   int64_t band = 0;
   bool was_change = false;
+  int64_t empty = 0;  // bands that moved nothing, so far
+  int run = 0;        // the latest ones in a row
   long long nf = (long long)*((volatile unsigned long long*)ctr), nfar = 0;
   for (int64_t step = 1;; ++step) {
     const int r = (int)(step % 3);
-    if ((nf == 0 && nfar == 0) || step > max_steps) {
+    run = nf == 0 && was_change ? run + 1 : 0;
+    empty += run > 0;
+    const bool out = step - empty > max_steps || run > kEmptyBandRun;
+    if ((nf == 0 && nfar == 0) || out) {
       if (blockIdx.x == 0 && threadIdx.x == 0) {
         bar[3] = (unsigned)(step - 1);
-        if (step > max_steps) atomicExch(bar + 2, 2u);  // still improving
+        if (out) atomicExch(bar + 2, 2u);  // still improving
       }
       return;
     }

@@ -6,6 +6,7 @@ import pytest
 import torch
 
 import gpugraphs as G
+from gpugraphs.multigraph import MultiGraph
 from oracle import oracle as O
 from test_graph_gpu import _reference_inplace
 from test_search_queue_gpu import _graph
@@ -77,3 +78,33 @@ def test_heavy_weights(n, scale, dtype):
     ref, _ = O.sssp(n, rp, cv, nz, [1, n])
     for q, s in enumerate((1, n)):
         assert (G.shortest_path(A, s).cpu().numpy() == ref[:, q]).all()
+
+
+@pytest.mark.parametrize("dtype", [np.int64, np.float64])
+def test_starts_far_apart(dtype):
+    """1400 paths of three vertices whose starts lie 2^52 apart: the gaps take more empty
+    bands than eight a vertex (the first round, a product, reaches the middle vertices)."""
+    n = 4200
+    v = np.arange(0, n, 3)
+    rp, cv, nz = _graph(n, np.concatenate([v, v + 1]), np.concatenate([v + 1, v + 2]), dtype)
+    nz[:] = 1
+    top = np.inf if dtype == np.float64 else np.iinfo(dtype).max
+    dist0 = np.full(n, top, dtype)
+    dist0[::3] = np.arange(n // 3).astype(dtype) * dtype(2**52)
+    _check(n, rp, cv, nz, 1, dist0, dist0.copy())
+
+
+def test_far_apart_in_many_graphs():
+    """A dense graph of light edges beside a path of heavy ones: the path's steps are far
+    wider than the common band."""
+    n, m, p, w = 2000, 1 << 25, 6000, 2**40
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    rowptr = (torch.arange(n + 1, device="cuda") * m // n + 1).to(torch.int32)
+    cols = (torch.randint(0, n, (m,), generator=gen, device="cuda") + 1).to(torch.int32)
+    dense = G.SparseGPUMatrixCSR(n, n, rowptr, cols, torch.ones(m, dtype=torch.int64, device="cuda"))
+    v = np.arange(p - 1)
+    rp, cv, nz = _graph(p, v, v + 1, np.int64)
+    nz[:] = w
+    d = MultiGraph([dense, G.SparseGPUMatrixCSR(p, p, rp, cv, nz)]).sssp([1, 1]).cpu().numpy()
+    assert (d[n:] == np.arange(p) * w).all()
+    assert d[0] == 0 and set(d[1:n]) == {1}
