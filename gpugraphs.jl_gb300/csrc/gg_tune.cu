@@ -19,6 +19,8 @@
 
 namespace gg {
 
+static const int kVariantBuiltIn = 3;  // gg_tune_result::sell_variant: the built-in rule's kernel
+
 static int time_median(gg_ctx* ctx, double* ms_out, int (*fn)(void*), void* arg) {
   cudaEvent_t e0, e1;
   GG_CUDA(cudaEventCreate(&e0));
@@ -220,8 +222,11 @@ static int tune_spmv(gg_ctx* ctx, gg_mat* A, gg_tune_result* out) {
     if (L) {
       out->slice_size = L->slice_size;
       out->sigma = L->sigma;
-      out->sell_variant = L->sell_variant;
-      out->hot_cols = L->hot_cols > 0 ? L->hot_cols : 32768;
+      // without earlier choices on the handle the built-in rule picked the kernel that was
+      // timed: applying the result leaves it to the rule again
+      const bool rule = A->sell_variant == 0 && A->hot_cols == 0;
+      out->sell_variant = rule ? kVariantBuiltIn : L->sell_variant;
+      out->hot_cols = rule ? 0 : (L->hot_cols > 0 ? L->hot_cols : 32768);
     } else {
       out->block_rows = kBlockRows;
     }
@@ -330,7 +335,7 @@ extern "C" int gg_tune_apply(gg_ctx* ctx, gg_mat* A, const gg_tune_result* choic
     GG_CHECK(gg_sell_create(ctx, A, choice->slice_size, choice->sigma, &S));
     if (A->sell_copy) gg_mat_destroy(A->sell_copy);
     A->sell_copy = S;
-    A->tuned_spmv = 2;
+    A->tuned_spmv = choice->sell_variant == kVariantBuiltIn ? 0 : 2;
     A->block_rows = 0;
   } else if (choice->spmv_kernel == 3) {
     if (A->format != GG_FMT_CSR) return set_error(GG_ERR_ARGUMENT, "window tiles need a CSR handle");
@@ -342,7 +347,10 @@ extern "C" int gg_tune_apply(gg_ctx* ctx, gg_mat* A, const gg_tune_result* choic
     return set_error(GG_ERR_ARGUMENT, "spmv_kernel must be 0, 1, 2 or 3");
   }
   if (cpl) A->mm_cpl = cpl;
-  if (choice->sell_variant >= 0 && choice->sell_variant <= 2) {
+  if (choice->sell_variant == kVariantBuiltIn) {
+    A->sell_variant = A->hot_cols = 0;
+    if (A->sell_copy) A->sell_copy->sell_variant = A->sell_copy->hot_cols = 0;
+  } else if (choice->sell_variant >= 0 && choice->sell_variant <= 2) {
     A->sell_variant = choice->sell_variant;
     if (A->sell_copy) A->sell_copy->sell_variant = choice->sell_variant;
   }

@@ -20,10 +20,10 @@ class TuneResult(ctypes.Structure):
                 ("candidates", ctypes.c_int), ("sell_variant", ctypes.c_int),
                 ("hot_cols", ctypes.c_int)]
 
-# SELL-32 plus-times kernels: register loads (the built-in choice), the matrix stream
-# staged by bulk copies, register loads with the hub rows folded from shared-memory
-# column windows where dense enough
-SELL_VARIANTS = ("registers", "bulk_copy", "hub_windows")
+# SELL-32 plus-times kernels: register loads, the matrix stream staged by bulk copies,
+# register loads with the hub rows folded from shared-memory column windows where dense
+# enough, and whichever kernel the built-in rule picks
+SELL_VARIANTS = ("registers", "bulk_copy", "hub_windows", "built_in")
 KERNELS = {1: "csr_row_blocks", 2: "sell", 3: "window_tiles"}
 
 

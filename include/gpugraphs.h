@@ -523,8 +523,9 @@ typedef struct gg_tune_result {
   int sell_variant;        /* SELL-32 plus-times kernel: 0 = register loads, 1 = matrix
                               stream staged in shared memory by bulk copies, 2 = register
                               loads with the hub rows folded from shared-memory column
-                              windows where dense enough (gg_spmv_hub_rows) (-1 in
-                              gg_tune_apply: leave as is) */
+                              windows where dense enough (gg_spmv_hub_rows), 3 = the
+                              kernel the built-in rule picks (-1 in gg_tune_apply:
+                              leave as is) */
   int hot_cols;            /* most frequent x values staged in shared memory by the register
                               kernel (0: built-in 32768; at most 53248) */
 } gg_tune_result;

@@ -1,0 +1,51 @@
+"""Tuned choices and the kernels that then run: what another handle gets from a choice, and
+what the order of calls must not change.  Kernels are told apart by their launch counts."""
+import numpy as np
+import pytest
+import torch
+
+import gpugraphs as G
+from gpugraphs import generators as gen
+from gpugraphs import tuning
+from gpugraphs.tracing import launch_trace
+
+pytestmark = pytest.mark.gpu
+
+
+def product(A, x):
+    """(launches, result) of a Float32 plus-times product; the first call builds its layout."""
+    y = torch.zeros(A.m, dtype=torch.float32, device="cuda")
+    G.gpu_spmv_(y, A, x)
+    with launch_trace() as t:
+        G.gpu_spmv_(y, A, x)
+    return t.launches, y
+
+
+@pytest.mark.parametrize("sigma", [0, 64])
+def test_applied_choice_runs_the_kernel_that_was_timed(sigma):
+    """On a CSR handle and on a padded SELL handle, whose sorted copy a choice must not bar."""
+    def handle():
+        A = gen.rmat(20 if sigma == 0 else 18, 16, seed=9, wkind=gen.W_U01_F32)
+        return G.SparseGPUMatrixSELL(A, 32, sigma) if sigma else A
+    A, B = handle(), handle()
+    x = torch.rand(A.n, device="cuda")
+    res = tuning.autotune(A)
+    tuning.apply(B, res)
+    (la, ya), (lb, yb) = product(A, x), product(B, x)
+    assert la == lb and torch.equal(ya, yb)
+
+
+@pytest.mark.parametrize("sigma", [0, 64])
+def test_built_in_choice_undoes_a_tuned_one(sigma):
+    A = gen.rmat(18, 16, seed=9, wkind=gen.W_U01_F32)
+    if sigma:
+        A = G.SparseGPUMatrixSELL(A, 32, sigma)
+    x = torch.rand(A.n, device="cuda")
+    la, ya = product(A, x)
+    tuning.apply(A, {"spmv_kernel": "sell", "slice_size": 32, "sigma": sigma or A.m,
+                     "sell_variant": "bulk_copy", "hot_cols": 16384})
+    assert product(A, x)[0] != la
+    tuning.apply(A, {"spmv_kernel": "sell", "slice_size": 32, "sigma": sigma or A.m,
+                     "sell_variant": "built_in"})
+    lb, yb = product(A, x)
+    assert la == lb and torch.equal(ya, yb)
