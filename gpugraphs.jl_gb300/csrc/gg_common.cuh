@@ -610,6 +610,7 @@ int spmv_dispatch(gg_ctx* ctx, gg_mat* A, int tc, int mul, int add, int accum, v
                   const void* x, int tx, const void* mask, int tmask, int64_t lo, int64_t hi);
 // the SELL matrix a product of SELL handle A runs on: its sorted copy or A (gg_spmv.cu)
 gg_mat* sell_for_spmv(gg_ctx* ctx, gg_mat* A);
+int ensure_sell_copy(gg_ctx* ctx, gg_mat* A);  // gg_spmv.cu
 // products of the common semirings with fixed operators and type (gg_spmv_typed.cu)
 int spmv_typed(gg_ctx* ctx, gg_mat* A, int tc, int mul, int add, int accum, void* y, int ty,
                const void* x, int tx, const void* mask, int tmask, int64_t lo, int64_t hi, bool* done);

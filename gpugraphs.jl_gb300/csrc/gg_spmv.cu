@@ -1054,14 +1054,20 @@ __global__ void k_col1_combine(const int4* __restrict__ multi, int64_t nmulti,
   }
 }
 
+// The SELL-32 copy of CSR handle A (rows sorted by length), whichever product needs it
+// first, with the tuned choices that were applied to A before.
+int ensure_sell_copy(gg_ctx* ctx, gg_mat* A) {
+  if (A->sell_copy) return GG_OK;
+  GG_CHECK(gg_sell_create(ctx, A, 32, A->m, &A->sell_copy));
+  A->sell_copy->sell_variant = A->sell_variant;
+  A->sell_copy->hot_cols = A->hot_cols;
+  return GG_OK;
+}
+
 // y = A x, one column, for a CSR handle of >= 65536 rows (gg_spmm with k == 1); the
 // relabelled x and the piece partials live in the context's scratch arena
 int launch_col1_sell(gg_ctx* ctx, gg_mat* A, const float* x, float* y) {
-  if (!A->sell_copy) {
-    GG_CHECK(gg_sell_create(ctx, A, 32, A->m, &A->sell_copy));
-    A->sell_copy->sell_variant = A->sell_variant;
-    A->sell_copy->hot_cols = A->hot_cols;
-  }
+  GG_CHECK(ensure_sell_copy(ctx, A));
   gg_mat* S = A->sell_copy;
   GG_CHECK(build_colperm(ctx, S));
   GG_CHECK(build_col1_plan(ctx, S));
@@ -1249,11 +1255,7 @@ int spmv_dispatch(gg_ctx* ctx, gg_mat* A, int tc, int mul, int add, int accum, v
       // plus-times over a large CSR runs on a SELL-32 copy with rows sorted by length
       // (built once; gg_tune may pick another C and sigma): slices of equal-length
       // rows give every thread the same work
-      if (!A->sell_copy) {
-        GG_CHECK(gg_sell_create(ctx, A, 32, A->m, &A->sell_copy));
-        A->sell_copy->sell_variant = A->sell_variant;  // choices applied before the copy
-        A->sell_copy->hot_cols = A->hot_cols;
-      }
+      GG_CHECK(ensure_sell_copy(ctx, A));
       A->last_layout = 2;
       GG_CHECK(build_colperm(ctx, A->sell_copy));
       if (typed_plain(A, A->sell_copy)) {

@@ -487,7 +487,7 @@ static int spmv_typed_t(gg_ctx* ctx, gg_mat* A, int accum, void* y, const void* 
   const SRTyped<TC, MUL, ADD, true> sr{static_cast<const T*>(A->nzval), static_cast<const T*>(x),
                                        static_cast<T*>(y), accum};
   if (lo == 0 && A->m >= kTypedCopyRows && !A->no_sell_copy) {
-    if (!A->sell_copy && gg_sell_create(ctx, A, 32, A->m, &A->sell_copy) != GG_OK) {
+    if (ensure_sell_copy(ctx, A) != GG_OK) {
       A->sell_copy = nullptr;  // no room for the copy, or past its index range: row blocks
       A->no_sell_copy = true;
     }

@@ -49,3 +49,25 @@ def test_built_in_choice_undoes_a_tuned_one(sigma):
                      "sell_variant": "built_in"})
     lb, yb = product(A, x)
     assert la == lb and torch.equal(ya, yb)
+
+
+@pytest.mark.parametrize("first", ["plain", "masked", "minplus", "spmm1"])
+def test_choice_outlives_whichever_product_comes_first(first):
+    """A kernel chosen before the copy exists runs, whatever product makes the copy."""
+    A = gen.rmat(17, 16, seed=9, wkind=gen.W_U01_F32)
+    x = torch.rand(A.n, device="cuda")
+    built_in, _ = product(A, x)
+    B = gen.rmat(17, 16, seed=9, wkind=gen.W_U01_F32)
+    tuning.apply(B, {"sell_variant": "bulk_copy"})
+    y = torch.zeros(B.m, device="cuda")
+    if first == "masked":
+        G.gpu_spmv_(y, B, x, mask=torch.ones(B.m, dtype=torch.bool, device="cuda"))
+    elif first == "minplus":
+        G.gpu_spmv_(y, B, x, mul=G.GPUGraphs_safe_add, add=G.GPUGraphs_min)
+    elif first == "spmm1":
+        G.gpu_spmm_(y.view(-1, 1), B, x.view(-1, 1))
+    tuned, yb = product(B, x)
+    C = gen.rmat(17, 16, seed=9, wkind=gen.W_U01_F32)
+    tuning.apply(C, {"sell_variant": "bulk_copy"})
+    ref, yc = product(C, x)
+    assert tuned == ref != built_in and torch.equal(yb, yc)
