@@ -614,6 +614,7 @@ int ensure_sell_copy(gg_ctx* ctx, gg_mat* A);  // gg_spmv.cu
 // products of the common semirings with fixed operators and type (gg_spmv_typed.cu)
 int spmv_typed(gg_ctx* ctx, gg_mat* A, int tc, int mul, int add, int accum, void* y, int ty,
                const void* x, int tx, const void* mask, int tmask, int64_t lo, int64_t hi, bool* done);
+int spmv_typed_on_copy(gg_ctx* ctx, gg_mat* A, const float* x, float* y);
 int build_row_blocks(gg_ctx* ctx, gg_mat* A);
 int build_mm_plan(gg_ctx* ctx, gg_mat* A);  // gg_spmm.cu
 int build_sell_plan(gg_ctx* ctx, gg_mat* A);

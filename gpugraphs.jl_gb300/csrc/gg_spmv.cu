@@ -1258,10 +1258,7 @@ int spmv_dispatch(gg_ctx* ctx, gg_mat* A, int tc, int mul, int add, int accum, v
       GG_CHECK(ensure_sell_copy(ctx, A));
       A->last_layout = 2;
       GG_CHECK(build_colperm(ctx, A->sell_copy));
-      if (typed_plain(A, A->sell_copy)) {
-        bool done = false;
-        return spmv_typed(ctx, A, tc, mul, add, accum, y, ty, x, tx, mask, tmask, lo, hi, &done);
-      }
+      if (typed_plain(A, A->sell_copy)) return spmv_typed_on_copy(ctx, A, sr.x, sr.y);
       A->sell_copy->tuned_spmv = A->tuned_spmv;  // the copy's own dispatch keeps a tuned kernel
       GG_CHECK(spmv_dispatch(ctx, A->sell_copy, tc, mul, add, accum, y, ty, x, tx, mask, tmask,
                              lo, hi));

@@ -497,6 +497,14 @@ static int spmv_typed_t(gg_ctx* ctx, gg_mat* A, int accum, void* y, const void* 
   return launch_rowblock(ctx, A, sr, mask, tmask, lo, hi);
 }
 
+// y = A x (Float32 plus-times, every row) on the SELL-32 copy that CSR handle A has: made by
+// the built-in rule or, at any size, by a tuned choice
+int spmv_typed_on_copy(gg_ctx* ctx, gg_mat* A, const float* x, float* y) {
+  const SRTyped<GG_FLOAT32, GG_OP_MUL, GG_OP_ADD, true> sr{static_cast<const float*>(A->nzval), x, y,
+                                                          GG_OP_SECOND};
+  return launch_sell32_typed(ctx, A->sell_copy, A, sr, TypedFilter{nullptr, 0, 0, 0});
+}
+
 template <int TC>
 static int spmv_typed_num(gg_ctx* ctx, gg_mat* A, int mul, int add, int accum, void* y, const void* x,
                           const void* mask, int tmask, int64_t lo, int64_t hi, bool* done) {

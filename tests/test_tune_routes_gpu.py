@@ -71,3 +71,22 @@ def test_choice_outlives_whichever_product_comes_first(first):
     tuning.apply(C, {"sell_variant": "bulk_copy"})
     ref, yc = product(C, x)
     assert tuned == ref != built_in and torch.equal(yb, yc)
+
+
+@pytest.mark.parametrize("m", [3000, 65535, 65536])
+def test_chosen_copy_runs_at_every_size(m):
+    """A SELL-32 layout chosen for a matrix below 65536 rows: a hub's row comes in chunks of
+    128 entries, folded by a second launch that row blocks do not make."""
+    rng = np.random.default_rng(m)
+    deg = rng.integers(1, 9, m)
+    deg[7] = 2000
+    rp = np.concatenate([[1], 1 + np.cumsum(deg)]).astype(np.int32)
+    cv = rng.integers(1, m + 1, rp[-1] - 1).astype(np.int32)
+    nz = rng.random(len(cv), dtype=np.float32)
+    A = G.SparseGPUMatrixCSR(m, m, rp, cv, nz)
+    tuning.apply(A, {"spmv_kernel": "sell", "slice_size": 32, "sigma": m})
+    x = torch.rand(m, device="cuda")
+    launches, y = product(A, x)
+    assert launches == 2 and G.spmv_layout(A) == "sell"
+    ref = np.add.reduceat(nz.astype(np.float64) * x.cpu().numpy()[cv - 1], rp[:-1] - 1)
+    np.testing.assert_allclose(y.cpu().numpy(), ref, rtol=1e-5)
