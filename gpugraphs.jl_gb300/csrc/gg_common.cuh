@@ -9,6 +9,7 @@
 #include <stdint.h>
 
 #include <string>
+#include <vector>
 
 #include "../../include/gpugraphs.h"
 
@@ -377,8 +378,12 @@ struct MMPlan {
   // the four rows a warp takes have about the same length
   int32_t* short_rows = nullptr;
   int64_t nshort = 0, nlive = 0;  // nlive: the leading ones that hold an entry
+  // CSR, host: entries before every kMMBlockRows-th row, and the longest row from there to
+  // the next (what a row range holds)
+  std::vector<int32_t> block_entry, block_longest;
 };
 static const int kSegMM = 256;
+static const int kMMBlockRows = 32;
 
 // Hub vertices of a graph's CSR view for the batched searches: rows longer than
 // kHubDegB entries, cut into pieces of kHubPieceB entries (0-based positions in

@@ -526,7 +526,7 @@ static int grid_mm(gg_ctx* ctx, int64_t warps) {
 int build_mm_plan(gg_ctx* ctx, gg_mat* A) {
   if (A->mmplan) return GG_OK;
   std::vector<int4> segs, items;
-  std::vector<int32_t> first, rows, short_rows;
+  std::vector<int32_t> first, rows, short_rows, block_entry, block_longest;
   int64_t nlive = 0;
   if (A->format == GG_FMT_CSR) {
     const int64_t m = A->m;
@@ -550,6 +550,11 @@ int build_mm_plan(gg_ctx* ctx, gg_mat* A) {
     }
     for (int64_t r = 0; r < m; ++r) {
       const int64_t k0 = rp[r] - 1, k1 = rp[r + 1] - 1;
+      if (r % kMMBlockRows == 0) {
+        block_entry.push_back((int32_t)k0);
+        block_longest.push_back(0);
+      }
+      block_longest.back() = std::max(block_longest.back(), (int32_t)(k1 - k0));
       if (k1 - k0 > kShortMM && k1 - k0 <= kSegMM) items.push_back(make_int4((int)r, (int)k0, (int)k1, -1));
       if (k1 - k0 <= kSegMM) continue;
       rows.push_back((int32_t)r);
@@ -600,6 +605,9 @@ int build_mm_plan(gg_ctx* ctx, gg_mat* A) {
   up((void**)&P->items, items.data(), (size_t)P->nitems * sizeof(int4));
   P->nshort = (int64_t)short_rows.size();
   P->nlive = nlive;
+  block_entry.push_back((int32_t)A->nnz);
+  P->block_entry = std::move(block_entry);
+  P->block_longest = std::move(block_longest);
   up((void**)&P->short_rows, short_rows.data(), short_rows.size() * sizeof(int32_t));
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
   if (e != cudaSuccess) {
@@ -760,6 +768,7 @@ __global__ void __launch_bounds__(256)
   for (int64_t r0 = row_lo + (int64_t)blockIdx.x * 32; r0 < row_hi; r0 += (int64_t)gridDim.x * 32) {
     const int64_t r = r0 + tx;
     const bool keep = r < row_hi && (!mask || !raw_is_zero(load_raw(mask, tmask, r), tmask));
+    if (!__any_sync(0xffffffffu, keep)) continue;  // the same for every warp: lane = row
     for (int c0 = 0; c0 < k; c0 += 32) {
 #pragma unroll
       for (int q = 0; q < 32; q += 8)
@@ -807,10 +816,59 @@ __global__ void __launch_bounds__(256)
 
 // Products below this many (entry, column) pairs take the operands where they lie: the
 // extra launches cost more than the gathers of operands that L1 holds.  Above, us, where
-// they lie / transposed (R-MAT, rows x columns): 300 x 4 - / 30, 1000 x 4 148 / 50, 10000 x 32 277 / 61,
+// they lie / transposed (R-MAT, rows x columns): 1000 x 4 148 / 50, 10000 x 32 277 / 61,
 // 100000 x 32 1447 / 85, 2^20 x 32 13574 / 634; a row-major 100000 x 31 190 / 87 padded
 // to 32 columns.
 static const int64_t kMMTranspose = 1 << 10;
+
+// entries of the selected rows (to whole blocks of kMMBlockRows; SELL: by the mean), and
+// the longest row among them (SELL: 0; the largest int past 2^17 rows of a range)
+static void mm_selected(const gg_mat* A, int64_t lo, int64_t hi, int64_t* entries, int32_t* longest) {
+  *entries = A->nnz;
+  *longest = INT32_MAX;
+  if (lo <= 0) return;
+  const MMPlan* P = A->mmplan;
+  if (A->format != GG_FMT_CSR) {
+    *entries = (int64_t)((double)A->nnz * (double)(hi - lo + 1) / (double)A->m);
+    *longest = 0;
+    return;
+  }
+  const int64_t b0 = (lo - 1) / kMMBlockRows, b1 = (hi - 1) / kMMBlockRows + 1;
+  *entries = P->block_entry[b1] - P->block_entry[b0];
+  if (b1 - b0 > 4096) return;
+  *longest = *std::max_element(P->block_longest.begin() + b0, P->block_longest.begin() + b1);
+}
+
+// Whether the gathers of e entries from a column-major Float32 B cost more than rewriting all
+// n rows of it, in us: a row's entries are a chain of dependent lines (0.45 us each, up to a
+// piece of kSegMM), the launch as a whole pays 0.4 ns an entry plus 25 ps a value; the rewrite
+// takes 25 ps a row plus 0.65 a value and two launches, 5 us.  Where it lies / transposed, us,
+// 2^20 rows: ER, 32 entries a row, 1000 rows x 32 columns 68 / 89, 3000 rows 122 / 92, 3000 x 2
+// 55 / 73, 10000 x 2 86 / 77; R-MAT, 100 rows x 32 62 / 105, 1000 rows, a hub among them,
+// 224 / 138.
+static bool staging_pays_f32(int64_t e, int32_t longest, int64_t n, int64_t k) {
+  const double chain = 0.45 * std::min(longest, (int32_t)kSegMM);
+  const double all = (double)e * (4e-4 + 2.5e-5 * (double)k);
+  return std::max(chain, all) >= 5.0 + (double)n * (25e-6 + 0.65e-6 * (double)k);
+}
+
+// Row-major rows that are no whole 16-byte groups: what the aligned kernels save on the rows
+// and the entries against padding B, unpadding C and two launches, in us.  Where they lie /
+// padded, us, 31 columns: ER 2^20 10^5 rows 131 / 180, 3 10^5 325 / 295, all 1066 / 682; R-MAT scale
+// 20, the first 3000 rows (2.8 n entries) 160 / 261, 30000 (7.1 n) 351 / 304, all 1781 / 701; scale
+// 16, 3000 rows 62 / 87, 30000 115 / 90, all 160 / 94; 7 columns: ER 10^5 rows 95 / 133,
+// 3 10^5 232 / 194.
+static bool padding_pays_f32(int64_t rows, int64_t e, int64_t n, int64_t k) {
+  const double saved = (double)rows * (3e-4 + 7e-6 * (double)k) + (double)e * 1.8e-5;
+  return saved >= 15.0 + (double)n * (45e-6 + 0.8e-6 * (double)k);
+}
+
+// Other semirings and types, whose gathers are a smaller part of an entry's cost: Int32
+// min-plus where it lies / transposed, us: ER 2^20 x 32, 10^4 rows (0.15 n entries) 100 / 123, 30000
+// (0.46 n) 260 / 221, all 8266 / 4522; x 8, 30000 rows 143 / 186, 3 10^5 (4.6 n) 1205 / 1177; R-MAT
+// scale 20 x 32, 30000 rows (0.26 n) 383 / 389, 10^5 (0.6 n) 865 / 702.
+static bool staging_pays(int64_t e, int64_t n, int64_t k) { return e * k >= 14 * n; }
+
 // scratch for the transposed operands of one pass; wider products run in passes
 static const int64_t kMMTransposeBytes = (int64_t)5 << 28;
 
@@ -828,12 +886,13 @@ static int64_t mm_pass_columns(int64_t k, int64_t per_col) {
 // GG_ERR_OOM (nothing launched): the caller takes them where they lie.
 static int spmm_staged_f32(gg_ctx* ctx, gg_mat* A, SRPlusTimesF32MM sr, int64_t k, int layout,
                            const void* mask, int tmask, int64_t lo, int64_t hi) {
-  GG_CHECK(build_mm_plan(ctx, A));
-  const int64_t m = A->m, n = A->n;
-  const int64_t w = mm_pass_columns(k, (n + m) * (int64_t)sizeof(float));
+  const int64_t n = A->n;
+  const int64_t row_lo = lo > 0 ? lo - 1 : 0, row_hi = lo > 0 ? hi : A->m;
+  const int64_t nrows = row_hi - row_lo;  // C is staged for these alone
+  const int64_t w = mm_pass_columns(k, (n + nrows) * (int64_t)sizeof(float));
   const int64_t wp = (w + 3) & ~(int64_t)3;
   const size_t bbytes = ((size_t)n * wp * sizeof(float) + 255) & ~(size_t)255;
-  const size_t cbytes = ((size_t)m * wp * sizeof(float) + 255) & ~(size_t)255;
+  const size_t cbytes = ((size_t)nrows * wp * sizeof(float) + 255) & ~(size_t)255;
   int64_t jwin = 0;
   GG_CHECK(ensure_scratch(ctx, bbytes + cbytes + mm_partial_bytes(A->mmplan, sizeof(float), wp, &jwin)));
   const float* B = sr.x;
@@ -842,12 +901,12 @@ static int spmm_staged_f32(gg_ctx* ctx, gg_mat* A, SRPlusTimesF32MM sr, int64_t 
   const bool col = layout == GG_COL_MAJOR;
   float* Bt = static_cast<float*>(ctx->scratch);
   float* Ct = reinterpret_cast<float*>(static_cast<char*>(ctx->scratch) + bbytes);
-  const int64_t row_lo = lo > 0 ? lo - 1 : 0, row_hi = lo > 0 ? hi : m;
   sr.x = Bt;
-  sr.y = Ct;
   for (int64_t j0 = 0; j0 < k; j0 += w) {
     const int64_t kn = k - j0 < w ? k - j0 : w, kp = (kn + 3) & ~(int64_t)3;
     sr.ldb = sr.ldc = kp;
+    float* const C0 = Ct - row_lo * kp;  // where row 0 would be
+    sr.y = C0;
     if (col) {
       to_row_major<float>(ctx, B + j0 * ldb, ldb, n, kn, Bt, kp);
     } else {
@@ -855,15 +914,13 @@ static int spmm_staged_f32(gg_ctx* ctx, gg_mat* A, SRPlusTimesF32MM sr, int64_t 
       trace_count(ctx, 1);
     }
     GG_CHECK(launch_mm(ctx, A, sr, kp, mask, tmask, lo, hi, bbytes + cbytes));
-    const int64_t nrows = row_hi - row_lo;
-    if (nrows <= 0) continue;
     if (col) {
       int64_t g = (nrows + 31) / 32;
       if (g > (int64_t)ctx->num_sms * 8) g = (int64_t)ctx->num_sms * 8;
-      k_to_col_major_f32<<<(int)g, 256, 0, ctx->stream>>>(Ct, (int)kp, row_lo, row_hi, (int)kn,
+      k_to_col_major_f32<<<(int)g, 256, 0, ctx->stream>>>(C0, (int)kp, row_lo, row_hi, (int)kn,
                                                          Cm + j0 * ldc, ldc, mask, tmask);
     } else {
-      k_unpad_rows_f32<<<grid_mm(ctx, nrows), 256, 0, ctx->stream>>>(Ct, (int)kp, row_lo, row_hi, (int)kn,
+      k_unpad_rows_f32<<<grid_mm(ctx, nrows), 256, 0, ctx->stream>>>(C0, (int)kp, row_lo, row_hi, (int)kn,
                                                                     Cm + j0, ldc);
     }
     trace_count(ctx, 1);
@@ -877,7 +934,6 @@ template <class SR>
 static int spmm_colmajor(gg_ctx* ctx, gg_mat* A, SR sr, int64_t k, const void* mask, int tmask,
                          int64_t lo, int64_t hi) {
   typedef typename SR::T T;
-  GG_CHECK(build_mm_plan(ctx, A));
   const int64_t n = A->n;
   const int esz = dtype_size(sr.tx);
   const int64_t w = mm_pass_columns(k, n * esz);
@@ -924,9 +980,15 @@ static int spmm_generic(gg_ctx* ctx, gg_mat* A, int mul, int add, int accum, voi
   sr.ldc = ldc;
   sr.layout = layout;
   sr.layout_c = layout;
-  if (layout == GG_COL_MAJOR && A->nnz * k >= kMMTranspose) {
-    const int rc = spmm_colmajor(ctx, A, sr, k, mask, tmask, lo, hi);
-    if (rc != GG_ERR_OOM) return rc;
+  if (layout == GG_COL_MAJOR) {
+    GG_CHECK(build_mm_plan(ctx, A));
+    int64_t e = 0;
+    int32_t longest = 0;
+    mm_selected(A, lo, hi, &e, &longest);
+    if (A->nnz * k >= kMMTranspose && staging_pays(e, A->n, k)) {
+      const int rc = spmm_colmajor(ctx, A, sr, k, mask, tmask, lo, hi);
+      if (rc != GG_ERR_OOM) return rc;
+    }
   }
   return launch_mm(ctx, A, sr, k, mask, tmask, lo, hi);
 }
@@ -952,9 +1014,17 @@ int spmm_dispatch(gg_ctx* ctx, gg_mat* A, int tc, int mul, int add, int accum, v
     // row-major CSR products without a mask have the float4 kernels to gain from whole rows
     const bool pad = layout == GG_ROW_MAJOR && A->format == GG_FMT_CSR && !mask && k > 1 &&
                      !ShortRowsMM<SRPlusTimesF32MM>::ok(sr, 0, k, nullptr);
-    if ((layout == GG_COL_MAJOR || pad) && A->nnz * k >= kMMTranspose) {
-      const int rc = spmm_staged_f32(ctx, A, sr, k, layout, mask, tmask, lo, hi);
-      if (rc != GG_ERR_OOM) return rc;
+    if (layout == GG_COL_MAJOR || pad) {
+      GG_CHECK(build_mm_plan(ctx, A));
+      int64_t e = 0;
+      int32_t longest = 0;
+      mm_selected(A, lo, hi, &e, &longest);
+      const bool pays = pad ? padding_pays_f32(lo > 0 ? hi - lo + 1 : A->m, e, A->n, k)
+                            : staging_pays_f32(e, longest, A->n, k);
+      if (A->nnz * k >= kMMTranspose && pays) {
+        const int rc = spmm_staged_f32(ctx, A, sr, k, layout, mask, tmask, lo, hi);
+        if (rc != GG_ERR_OOM) return rc;
+      }
     }
     if (layout == GG_ROW_MAJOR) return launch_mm(ctx, A, sr, k, mask, tmask, lo, hi);
   }
