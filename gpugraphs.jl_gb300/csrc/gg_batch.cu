@@ -161,11 +161,14 @@ static int bb_group(gg_ctx* ctx, int64_t n, const BatchGraph& g, const HubPlan* 
 // ---------------------------------------------------------------------------------
 // batched shortest paths: 32 source columns, lane = source
 // ---------------------------------------------------------------------------------
+// Columns past the group's S sources start at 0, the smallest distance: nothing lowers them,
+// and a row's largest minimum, by which the row rounds end it early, is that of the sources.
+// With every column at the maximum a row of a smaller group was always visited to its end.
 template <typename T>
-__global__ void k_bs_init(T* D, int64_t n, const int64_t* src, int64_t S, unsigned* changed) {
+__global__ void k_bs_init(T* D, int64_t n, int64_t S, unsigned* changed) {
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n * 32;
        t += (int64_t)gridDim.x * blockDim.x)
-    D[t] = Lim<T>::max();
+    D[t] = (t & 31) < S ? Lim<T>::max() : T(0);
   for (int64_t v = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; v < n;
        v += (int64_t)gridDim.x * blockDim.x)
     changed[v] = 0;
@@ -313,7 +316,7 @@ template <typename T>
 static int bs_start(gg_ctx* ctx, int64_t n, BsRun<T>& R) {
   int64_t gb = (n * 32 + 255) / 256;
   if (gb > (int64_t)ctx->num_sms * 8) gb = (int64_t)ctx->num_sms * 8;
-  k_bs_init<T><<<(int)gb, 256, 0, R.st>>>(R.w.D, n, R.dsrc, R.S, R.w.c[0]);
+  k_bs_init<T><<<(int)gb, 256, 0, R.st>>>(R.w.D, n, R.S, R.w.c[0]);
   k_bs_seed<T><<<1, 64, 0, R.st>>>(R.w.D, R.dsrc, R.S, R.w.c[0], R.w.cq[0]);
   GG_CUDA(cudaGetLastError());
   for (int i = 0; i < 8; ++i) R.h[i] = 0;
