@@ -467,6 +467,10 @@ int gg_mat_values_changed(gg_ctx* ctx, gg_mat* A) {
   GG_CUDA(cudaSetDevice(ctx->device));
   GG_CUDA(cudaStreamSynchronize(ctx->stream));
   free_derived(A);
+  // a padded SELL handle's sorted copy costs about eight of the products it speeds up:
+  // values that lasted for fewer do without one the next time
+  if (A->products > 0) A->values_churn = A->products < kCopyProducts;
+  A->products = 0;
   return GG_OK;
 }
 

@@ -508,6 +508,7 @@ static const int kSegNnz = 4096;
 }  // namespace gg
 
 namespace gg {
+static const int64_t kCopyProducts = 8;
 static const int kFlagWords = 128;  // words of gg_ctx::d_flags / h_flags
 }
 
@@ -589,6 +590,10 @@ struct gg_mat {
   // whose own slices are mostly padding
   gg_mat* sell_copy = nullptr;
   bool no_sell_copy = false;  // the copy could not be made (memory, index range)
+  // padded SELL handles: products since the values last changed, and whether they change
+  // too often for a copy (sell_for_spmv)
+  int64_t products = 0;
+  bool values_churn = false;  // set by gg_mat_values_changed
   gg_mat* tr_copy = nullptr;    // CSR handles: CSR storage of the transpose (gg_spmv_t)
   int64_t max_row_len = -1;
   // tuned choices (gg_tune): plus-times SpMV kernel (0 = built-in rule, 1 = CSR row

@@ -481,7 +481,8 @@ static int spmv_typed_t(gg_ctx* ctx, gg_mat* A, int accum, void* y, const void* 
   if (A->format == GG_FMT_SELL) {
     const SRTyped<TC, MUL, ADD, false> sr{static_cast<const T*>(A->nzval), static_cast<const T*>(x),
                                           static_cast<T*>(y), accum};
-    if (A->slice_size == 32) return launch_sell32_typed(ctx, A, nullptr, sr, flt);
+    // (relabelled columns are a layout of their own: not for values that change often)
+    if (A->slice_size == 32 && !A->values_churn) return launch_sell32_typed(ctx, A, nullptr, sr, flt);
     return launch_sell(ctx, A, sr, mask, tmask, lo, hi);
   }
   const SRTyped<TC, MUL, ADD, true> sr{static_cast<const T*>(A->nzval), static_cast<const T*>(x),

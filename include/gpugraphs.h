@@ -184,7 +184,8 @@ int gg_mat_arrays(const gg_mat* A, void** ptr, void** colval, void** nzval, void
  * Drops everything the library derived from the handle's values on first use (the
  * SELL-32 and transposed copies, graph analyses, plans); call it after writing to the
  * arrays gg_mat_arrays returns (setindex!, src/storage/CSR.jl:166-180).  Waits for the
- * context's stream first.
+ * context's stream first.  A padded SELL handle whose values lasted for fewer than eight
+ * products gets no sorted copy (gg_spmv) for the next ones.
  */
 int gg_mat_values_changed(gg_ctx* ctx, gg_mat* A);
 
