@@ -548,13 +548,17 @@ int build_mm_plan(gg_ctx* ctx, gg_mat* A) {
         if (L > 0 && L <= kShortMM) ++nlive;
       }
     }
+    block_entry.reserve(m / kMMBlockRows + 2);
+    block_longest.reserve(m / kMMBlockRows + 1);
+    for (int64_t r0 = 0; r0 < m; r0 += kMMBlockRows) {
+      const int64_t r1 = r0 + kMMBlockRows < m ? r0 + kMMBlockRows : m;
+      int32_t longest = 0;
+      for (int64_t r = r0; r < r1; ++r) longest = std::max(longest, rp[r + 1] - rp[r]);
+      block_entry.push_back(rp[r0] - 1);
+      block_longest.push_back(longest);
+    }
     for (int64_t r = 0; r < m; ++r) {
       const int64_t k0 = rp[r] - 1, k1 = rp[r + 1] - 1;
-      if (r % kMMBlockRows == 0) {
-        block_entry.push_back((int32_t)k0);
-        block_longest.push_back(0);
-      }
-      block_longest.back() = std::max(block_longest.back(), (int32_t)(k1 - k0));
       if (k1 - k0 > kShortMM && k1 - k0 <= kSegMM) items.push_back(make_int4((int)r, (int)k0, (int)k1, -1));
       if (k1 - k0 <= kSegMM) continue;
       rows.push_back((int32_t)r);
