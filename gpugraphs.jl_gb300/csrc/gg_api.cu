@@ -33,7 +33,33 @@ int cuda_error(cudaError_t e, const char* what) {
   return set_error(code, "%s: %s", what, cudaGetErrorString(e));
 }
 
+static bool capturing(gg_ctx* ctx) {
+  cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(ctx->stream, &s) == cudaSuccess) return s != cudaStreamCaptureStatusNone;
+  (void)cudaGetLastError();  // the legacy stream while another stream is being captured
+  return true;
+}
+
+int order_before(gg_ctx* ctx, StreamOrder& o) {
+  if (!o.used || o.last == ctx->stream || capturing(ctx)) return GG_OK;
+  GG_CUDA(cudaStreamWaitEvent(ctx->stream, o.event, 0));
+  return GG_OK;
+}
+
+int order_after(gg_ctx* ctx, StreamOrder& o) {
+  if (capturing(ctx)) return GG_OK;
+  if (!o.event) GG_CUDA(cudaEventCreateWithFlags(&o.event, cudaEventDisableTiming));
+  GG_CUDA(cudaEventRecord(o.event, ctx->stream));
+  o.last = ctx->stream;
+  o.used = true;
+  return GG_OK;
+}
+
+// The context's one scratch arena, for the current call.  The synchronous searches end
+// before another call can start; gg_spmm records its use.
 int ensure_scratch(gg_ctx* ctx, size_t bytes) {
+  GG_CHECK(order_before(ctx, ctx->scratch_order));
+  ctx->scratch_used = true;
   if (ctx->scratch_bytes >= bytes) return GG_OK;
   if (ctx->scratch) {
     GG_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -195,6 +221,7 @@ static void free_mat_storage(gg_mat* A) {
   cudaFree(A->perm);
   cudaFree(A->iperm);
   free_derived(A);
+  if (A->order.event) cudaEventDestroy(A->order.event);
 }
 
 static int blocks_for(gg_ctx* ctx, int64_t work) {
@@ -247,6 +274,7 @@ int gg_destroy(gg_ctx* ctx) {
   cudaFree(ctx->d_flags);
   cudaFreeHost(ctx->h_flags);
   cudaFree(ctx->d_err);
+  if (ctx->scratch_order.event) cudaEventDestroy(ctx->scratch_order.event);
   if (ctx->trace_ev) {
     for (int i = 0; i < 2 * kTraceMax; ++i) cudaEventDestroy(ctx->trace_ev[i]);
     delete[] ctx->trace_ev;
@@ -549,8 +577,11 @@ int gg_spmm(gg_ctx* ctx, const gg_mat* A, int mul, int add, int accum, void* C, 
   if (!C || (A->n > 0 && !B)) return set_error(GG_ERR_ARGUMENT, "NULL matrix");
   if (range_lo != 0 && range_lo > range_hi) return GG_OK;
   GG_CUDA(cudaSetDevice(ctx->device));
-  return spmm_dispatch(ctx, const_cast<gg_mat*>(A), tc, mul, add, accum, C, c_dtype, ldc, B, b_dtype,
-                       ldb, k, layout, mask, mask_dtype, range_lo, range_hi);
+  ctx->scratch_used = false;
+  const int rc = spmm_dispatch(ctx, const_cast<gg_mat*>(A), tc, mul, add, accum, C, c_dtype, ldc, B,
+                               b_dtype, ldb, k, layout, mask, mask_dtype, range_lo, range_hi);
+  const int rc2 = ctx->scratch_used ? order_after(ctx, ctx->scratch_order) : GG_OK;
+  return rc != GG_OK ? rc : rc2;
 }
 
 }  // extern "C"

@@ -508,6 +508,16 @@ static const int kSegNnz = 4096;
 }  // namespace gg
 
 namespace gg {
+// Orders the asynchronous users of one workspace over streams: the calls that use it record
+// an event after their launches (about 1 us of host time), and a call on another stream
+// waits for it first.  The event is recorded with the call, so a stream may be destroyed
+// afterwards.  Under capture nothing is recorded or waited for: who replays a graph orders
+// it against other calls.
+struct StreamOrder {
+  cudaEvent_t event = nullptr;
+  cudaStream_t last = nullptr;
+  bool used = false;
+};
 static const int64_t kCopyProducts = 8;
 static const int kFlagWords = 128;  // words of gg_ctx::d_flags / h_flags
 }
@@ -519,6 +529,8 @@ struct gg_ctx {
   // scratch arena, grown on demand, freed by gg_destroy
   void* scratch = nullptr;
   size_t scratch_bytes = 0;
+  gg::StreamOrder scratch_order;
+  bool scratch_used = false;  // by the current gg_spmm call
   unsigned int* d_flags = nullptr;  // small device word array for status flags
   unsigned int* h_flags = nullptr;  // pinned mirror
   unsigned int* d_err = nullptr;    // set by kernels whose bounded waits ran out
@@ -592,6 +604,7 @@ struct gg_mat {
   bool no_sell_copy = false;  // the copy could not be made (memory, index range)
   // padded SELL handles: products since the values last changed, and whether they change
   // too often for a copy (sell_for_spmv)
+  gg::StreamOrder order;  // products that use buffers of the handle's plans
   int64_t products = 0;
   bool values_churn = false;  // set by gg_mat_values_changed
   gg_mat* tr_copy = nullptr;    // CSR handles: CSR storage of the transpose (gg_spmv_t)
@@ -613,6 +626,8 @@ struct gg_mat {
 
 namespace gg {
 int ensure_scratch(gg_ctx* ctx, size_t bytes);
+int order_before(gg_ctx* ctx, StreamOrder& o);  // before a workspace is touched (gg_api.cu)
+int order_after(gg_ctx* ctx, StreamOrder& o);   // after the last launch that touches it
 void free_graph_aux(gg_mat* A);
 int compute_type(int tv, int tx, int mul);
 int check_semiring(int tv, int tx, int ty, int mul, int add, int accum, int* tc_out);

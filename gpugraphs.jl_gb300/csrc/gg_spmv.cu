@@ -1223,8 +1223,7 @@ static bool typed_plain(const gg_mat* A, const gg_mat* S) {
   return A->tuned_spmv == 0 && S->sell_variant == 0 && S->hot_cols == 0 && S->m < kTypedPlainRows;
 }
 
-// dispatch of gg_spmv after validation (gg_api.cu); tc = accumulator type
-int spmv_dispatch(gg_ctx* ctx, gg_mat* A, int tc, int mul, int add, int accum, void* y, int ty,
+static int spmv_run(gg_ctx* ctx, gg_mat* A, int tc, int mul, int add, int accum, void* y, int ty,
                   const void* x, int tx, const void* mask, int tmask, int64_t lo, int64_t hi) {
   if (A->m == 0) return GG_OK;
   const bool plain = (mask == nullptr && lo == 0);
@@ -1232,7 +1231,7 @@ int spmv_dispatch(gg_ctx* ctx, gg_mat* A, int tc, int mul, int add, int accum, v
     gg_mat* S = sell_for_spmv(ctx, A);
     if (S != A) {
       A->last_layout = 2;
-      return spmv_dispatch(ctx, S, tc, mul, add, accum, y, ty, x, tx, mask, tmask, lo, hi);
+      return spmv_run(ctx, S, tc, mul, add, accum, y, ty, x, tx, mask, tmask, lo, hi);
     }
   }
   if (plain && A->dtype == GG_FLOAT32 && tx == GG_FLOAT32 && ty == GG_FLOAT32 &&
@@ -1262,8 +1261,7 @@ int spmv_dispatch(gg_ctx* ctx, gg_mat* A, int tc, int mul, int add, int accum, v
       GG_CHECK(build_colperm(ctx, A->sell_copy));
       if (typed_plain(A, A->sell_copy)) return spmv_typed_on_copy(ctx, A, sr.x, sr.y);
       A->sell_copy->tuned_spmv = A->tuned_spmv;  // the copy's own dispatch keeps a tuned kernel
-      GG_CHECK(spmv_dispatch(ctx, A->sell_copy, tc, mul, add, accum, y, ty, x, tx, mask, tmask,
-                             lo, hi));
+      GG_CHECK(spmv_run(ctx, A->sell_copy, tc, mul, add, accum, y, ty, x, tx, mask, tmask, lo, hi));
       return launch_refold_nan_rows(ctx, A, sr.x, sr.y);
     }
     GG_CHECK(build_colperm(ctx, A));
@@ -1298,6 +1296,21 @@ int spmv_dispatch(gg_ctx* ctx, gg_mat* A, int tc, int mul, int add, int accum, v
     case GG_FLOAT32: return spmv_generic<GG_FLOAT32>(ctx, A, mul, add, accum, y, ty, x, tx, mask, tmask, lo, hi);
     default: return spmv_generic<GG_FLOAT64>(ctx, A, mul, add, accum, y, ty, x, tx, mask, tmask, lo, hi);
   }
+}
+
+// whether products of A write buffers that its plans own: a reordered x, partial results
+static bool has_workspace(const gg_mat* A) {
+  return A->sell_copy || (A->colperm && A->colperm->enabled) || (A->blocks && A->blocks->nsegs > A->blocks->nlong) ||
+         (A->sellplan && A->sellplan->nmulti > 0) || A->winplan || A->hubwin;
+}
+
+// dispatch of gg_spmv after validation (gg_api.cu); tc = accumulator type
+int spmv_dispatch(gg_ctx* ctx, gg_mat* A, int tc, int mul, int add, int accum, void* y, int ty,
+                  const void* x, int tx, const void* mask, int tmask, int64_t lo, int64_t hi) {
+  GG_CHECK(order_before(ctx, A->order));
+  const int rc = spmv_run(ctx, A, tc, mul, add, accum, y, ty, x, tx, mask, tmask, lo, hi);
+  const int rc2 = has_workspace(A) ? order_after(ctx, A->order) : GG_OK;
+  return rc != GG_OK ? rc : rc2;
 }
 
 }  // namespace gg

@@ -17,7 +17,10 @@
  *  - Work is enqueued on the context's stream (gg_set_stream; default: the legacy
  *    default stream) and is asynchronous unless stated otherwise, like the
  *    reference's KernelAbstractions launches (callers synchronize before reading).
- *  - A context may be used from one host thread at a time.
+ *  - A context may be used from one host thread at a time.  Its calls may go to several
+ *    streams: those that share a workspace (the context's scratch arena; the buffers of one
+ *    matrix's plans) wait for one another on the device, others overlap.  Replays of
+ *    captured graphs are not seen: who replays one orders it against other calls.
  */
 #ifndef GPUGRAPHS_H
 #define GPUGRAPHS_H
