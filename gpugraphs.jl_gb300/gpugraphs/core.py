@@ -30,6 +30,17 @@ def lib():
     return _lib.load()
 
 
+def _raw_stream_of():
+    """Function from a device index to the address of torch's current stream there.  The
+    private call makes no Stream object that every library call would throw away; a torch
+    without it takes the public way."""
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    return raw or (lambda device: torch.cuda.current_stream(device).cuda_stream)
+
+
+_raw_stream = _raw_stream_of()
+
+
 def ctx(device=None):
     """Library context of `device` (default: torch's current device), bound to the
     current torch stream."""
@@ -46,8 +57,7 @@ def ctx(device=None):
         _ctx[device] = c
     if not torch.cuda.is_initialized():
         torch.cuda.init()
-    # the stream's address alone: a torch Stream object of every call would be thrown away
-    rc = L.gg_set_stream(c, torch._C._cuda_getCurrentRawStream(device))
+    rc = L.gg_set_stream(c, _raw_stream(device))
     if rc:
         check(rc, L)
     return c
