@@ -845,17 +845,15 @@ __global__ void __launch_bounds__(1024)
 // <= kCoopMaxDeg) while the frontier is medium-sized: one launch runs level after
 // level over all SMs with a grid barrier in between, instead of one launch and one
 // host round trip per level.  The barrier's wait is bounded (by default 2^26 polls of
-// 100 ns, about 7 s; gg_set_wait_limit sets another count): when it runs out, the
-// kernel records an error, every block returns, and the call reports GG_ERR_TIMEOUT.  Queue counters rotate over three words so that the counter being
-// zeroed is never the one being read or appended.
+// about 0.18 us, some 12 s; gg_set_wait_limit sets another count): when it runs out, the
+// kernel records an error, every block returns, and the call reports GG_ERR_TIMEOUT.
+// Queue counters rotate over three words so that the counter being zeroed is never the
+// one being read or appended.
 // ---------------------------------------------------------------------------------
 static const int kCoopMaxDeg = 64;
 static const int kCoopLo = 1024;   // the single-CTA kernel takes smaller frontiers
 static const int kCoopThreads = 1024;
-#ifndef GG_NF_THREADS
-#define GG_NF_THREADS 512
-#endif
-static const int kNfThreads = GG_NF_THREADS;  // near-far searches
+static const int kNfThreads = 512;  // near-far searches
 static const double kNearFarScale = 32.0;  // near-far band width = this x the mean weight
 
 struct CoopCtl {

@@ -577,7 +577,7 @@ template <> __device__ __forceinline__ double b_atomic_min<double>(double* p, do
 // 8 lanes take a row of up to kSegMM entries or a piece of a longer one, 4 source columns a
 // lane with their minima in registers, four rows of about one length a warp (the SpMM
 // plan's lists).  An entry costs a 16-byte load of D and four add-min instructions a
-// lane; 8 entries' loads are in flight, the next 8 columns and weights behind them.
+// lane; 4 entries' loads are in flight, the next 8 columns and weights behind them.
 //  * A row ends at the first weight w with w + dlow >= the largest of its 32 minima, or
 //    w > cap: sums of non-negative values only grow, and no distance below dlow was written
 //    in the previous round, so an unchanged or pruned entry cannot lower it.  cap < max
@@ -589,8 +589,8 @@ template <> __device__ __forceinline__ double b_atomic_min<double>(double* p, do
 // relaxations reaches the same fixpoint.
 // Against the round it replaces (a warp per 32-row SELL item, changed entries through a
 // shared-memory queue, 19.5 warp instructions an entry, all entries): 800 -> 250 us on R-MAT
-// scale 20, 32 Int32 columns; 256 sources 57.5 -> 25.5 ms.  Now bound by issue (41%) and
-// the row lists' dependent loads.
+// scale 20, 32 Int32 columns; 256 sources 57.5 -> 25.5 ms.  A round alone takes 260 us:
+// issue 55%, 45% of the warp slots, L2 20%, DRAM 18%, most stalls on the rows of D.
 struct MsRows {
   const int32_t* rowptr;  // 1-based
   const int32_t* col;     // 1-based, entries of a row by ascending weight

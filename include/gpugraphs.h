@@ -123,11 +123,11 @@ int gg_stream_sync(gg_ctx* ctx);
  * reference counterpart: the reference's host loops wait on nothing on the device).
  * It bounds the grid barriers of the persistent kernels (cooperative BFS and
  * shortest-path phases of hub-free graphs, the near-far search, the many-graph BFS /
- * shortest paths; each poll sleeps ~100 ns) and the bulk-copy waits of the staged
+ * shortest paths; a poll takes about 0.18 us) and the bulk-copy waits of the staged
  * SpMV kernels.  A wait that runs out records an error; every block returns, and the
  * call (or, for asynchronous SpMV calls, the next gg_stream_sync) returns
  * GG_ERR_TIMEOUT with partial results.  The context stays usable.  polls = 0
- * restores the built-in limits (2^26 barrier polls, about 7 s; 2^22 copy polls);
+ * restores the built-in limits (2^26 barrier polls, about 12 s; 2^22 copy polls);
  * values above 2^32 - 1 are clamped. */
 int gg_set_wait_limit(gg_ctx* ctx, uint64_t polls);
 
@@ -229,8 +229,10 @@ int gg_spmv(gg_ctx* ctx, const gg_mat* A, int mul, int add, int accum, void* y, 
  * (elements).  Mask / range select rows as in gg_spmv.  Shape checks return
  * GG_ERR_ASSERTION like the reference's @assert.
  * Column-major operands, and row-major Float32 ones whose width is not a multiple of
- * four, are transposed or padded through the context's scratch where that takes at most
- * 1.25 GiB.  The scratch grows on demand, so a call that is to be captured in a CUDA
+ * four, are transposed or padded through the context's scratch where the entries of the
+ * selected range make up for it (a mask's rows are not counted), in passes of at most
+ * 1.25 GiB of operands but never fewer than four columns; where the scratch cannot grow,
+ * they are taken where they lie.  The scratch grows on demand, so a call that is to be captured in a CUDA
  * graph is made once before, and a larger call on the context afterwards may move the
  * scratch that a captured one uses.
  */
