@@ -1437,6 +1437,14 @@ template <> __device__ __forceinline__ int32_t atomic_min_t<int32_t>(int32_t* p,
 template <> __device__ __forceinline__ int64_t atomic_min_t<int64_t>(int64_t* p, int64_t v) {
   return (int64_t)atomicMin((long long*)p, (long long)v);
 }
+// by the bits alone: non-negative floats order like them
+template <typename T> __device__ __forceinline__ T atomic_min_bits(T* p, T v) { return atomic_min_t<T>(p, v); }
+template <> __device__ __forceinline__ float atomic_min_bits<float>(float* p, float v) {
+  return __int_as_float(atomicMin((int*)p, __float_as_int(v)));
+}
+template <> __device__ __forceinline__ double atomic_min_bits<double>(double* p, double v) {
+  return __longlong_as_double(atomicMin((long long*)p, __double_as_longlong(v)));
+}
 // Floats order like their bit patterns read as signed integers, except that negative ones
 // (a caller's start) order the other way among themselves, as their unsigned bits do.
 template <> __device__ __forceinline__ float atomic_min_t<float>(float* p, float v) {
@@ -1730,9 +1738,9 @@ __global__ void __launch_bounds__(1024)
 // frontier = every vertex whose start distance is finite.  Start distances below zero (-0.0
 // among them) or NaN are noted: a caller may start from any values, and the bounds that
 // searches end early by hold from non-negative ones only.
-template <typename T> __device__ __forceinline__ bool odd_start(T d) { return d < T(0); }
-template <> __device__ __forceinline__ bool odd_start<float>(float d) { return !(d >= 0.0f) || signbit(d); }
-template <> __device__ __forceinline__ bool odd_start<double>(double d) { return !(d >= 0.0) || signbit(d); }
+template <typename T> __device__ __forceinline__ bool is_odd(T d) { return d < T(0); }
+template <> __device__ __forceinline__ bool is_odd<float>(float d) { return !(d >= 0.0f) || signbit(d); }
+template <> __device__ __forceinline__ bool is_odd<double>(double d) { return !(d >= 0.0) || signbit(d); }
 template <typename T>
 __global__ void __launch_bounds__(256) k_sssp_seed(int64_t n, const T* dist, unsigned* inq, int32_t* q, Counters* ctr) {
   __shared__ int32_t stage[8][WarpQueue::kCap];
@@ -1743,7 +1751,7 @@ __global__ void __launch_bounds__(256) k_sssp_seed(int64_t n, const T* dist, uns
     const int64_t v = base + threadIdx.x;
     const T d = v < n ? dist[v] : Lim<T>::max();
     const bool fin = d != Lim<T>::max();
-    odd |= odd_start<T>(d);
+    odd |= is_odd<T>(d);
     const unsigned bal = __ballot_sync(kFullG, fin);
     if ((threadIdx.x & 31) == 0 && bal) inq[v >> 5] = bal;
     wq.push(fin, (int32_t)v);
@@ -1806,12 +1814,12 @@ __global__ void k_nf_init(NfCtl* cc, long long nf0, unsigned polls) {
   cc->status = 0;
 }
 
-template <typename T>
+template <typename T, bool kOddStart>
 __global__ void __launch_bounds__(kNfThreads, 1)
     k_sssp_nearfar(const int32_t* __restrict__ prow, const int32_t* __restrict__ pcol,
                    const T* __restrict__ pw, int32_t* qa, int32_t* qb, int32_t* fa, int32_t* fb,
                    int32_t* fz, T* dist, unsigned* inq_a, unsigned* inq_b, unsigned* infar,
-                   NfCtl* cc, T delta, long long max_steps, bool look_first) {
+                   NfCtl* cc, T delta, long long max_steps) {
   __shared__ StepLists S;
   const int lane = threadIdx.x & 31;
   const int64_t gw = (int64_t)(threadIdx.x >> 5) * gridDim.x + blockIdx.x;
@@ -1828,8 +1836,7 @@ __global__ void __launch_bounds__(kNfThreads, 1)
   int fc = 0;
   T thr = delta, width = delta;
   bool was_change = false;
-  long long empty = 0;  // bands that moved nothing, so far
-  int run = 0;          // the latest ones in a row
+  int run = 0;  // the latest bands in a row that moved nothing; max_steps grows by them
   if (threadIdx.x == 0) {
     S.n[0] = S.n[1] = 0;
     S.len = (long long)*((volatile unsigned long long*)&cc->cnt[2]);
@@ -1841,13 +1848,10 @@ __global__ void __launch_bounds__(kNfThreads, 1)
     const long long nf = S.len, nfar = S.flen;
     const int fn = fc == 2 ? 0 : fc + 1;
     const bool band = nf == 0;
-    run = band && was_change ? run + 1 : 0;
-    empty += run > 0;
-    const bool out = st - empty >= max_steps || run > kEmptyBandRun;
-    if (out || (band && nfar == 0)) {
+    if (st >= max_steps || (band && nfar == 0)) {
       if (blockIdx.x == 0 && threadIdx.x == 0) {
         cc->steps_out = st;
-        cc->status = out ? 2 : 1;
+        cc->status = st >= max_steps ? 2 : 1;
       }
       return;
     }
@@ -1860,6 +1864,8 @@ __global__ void __launch_bounds__(kNfThreads, 1)
       // frontier (counted and marked like a normal step's output), the others move to
       // the next far list
       // (an empty band doubles the next one, so gaps between the distances cost few steps)
+      run = was_change ? run + 1 : 0;
+      max_steps = run > kEmptyBandRun ? 0 : max_steps + was_change;
       width = !was_change ? delta : (width < Lim<T>::max() / 2 ? w_add(width, width) : width);
       was_change = true;
       thr = thr > Lim<T>::max() - width ? Lim<T>::max() : w_add(thr, width);
@@ -1901,8 +1907,10 @@ __global__ void __launch_bounds__(kNfThreads, 1)
             w = __ldg(pcol + k);
             const T cand = relax_add(__ldg(pw + k), du);
             // lowered by the atomic alone: one L2 round trip on the step's critical path
-            // (look_first: a NaN start's bits would give way to it)
-            if ((!look_first || cand < ld_cg(dist + w)) && cand < atomic_min_t(dist + w, cand)) {
+            // (kOddStart: the bits of NaN and of negative floats would give way to it)
+            const bool lower = kOddStart ? cand < ld_cg(dist + w) && cand < atomic_min_t(dist + w, cand)
+                                         : cand < atomic_min_bits(dist + w, cand);
+            if (lower) {
               const unsigned bit = 1u << (w & 31);
               if (cand < thr) near_add = !(atomicOr(inxt + (w >> 5), bit) & bit);
               else far_add = !(atomicOr(infar + (w >> 5), bit) & bit);
@@ -2492,11 +2500,11 @@ static int sssp_fixpoint(gg_ctx* ctx, gg_mat* A, T* d, int64_t* rounds_out) {
     const T* pw = static_cast<const T*>(P.w);
     long long max_steps = 8 * (long long)n + 1024;
     void* args[] = {&P.rowptr, &P.colval, &pw, &qa, &qb, &sc.hq, &sc.q2, &sc.q3, &d, &ia, &ib,
-                    &sc.visited, &ncc, &delta, &max_steps, &odd};
+                    &sc.visited, &ncc, &delta, &max_steps};
     const int64_t want = n / kNearFarCta;
     const int ctas = (int)(want < ctx->num_sms ? want : ctx->num_sms);
-    GG_CUDA(cudaLaunchCooperativeKernel((const void*)k_sssp_nearfar<T>, dim3(ctas),
-                                        dim3(kNfThreads), args, 0, ctx->stream));
+    const void* kernel = odd ? (const void*)k_sssp_nearfar<T, true> : (const void*)k_sssp_nearfar<T, false>;
+    GG_CUDA(cudaLaunchCooperativeKernel(kernel, dim3(ctas), dim3(kNfThreads), args, 0, ctx->stream));
     NfCtl hn;
     GG_CUDA(cudaMemcpyAsync(&hn, ncc, sizeof(NfCtl), cudaMemcpyDeviceToHost, ctx->stream));
     GG_CUDA(cudaStreamSynchronize(ctx->stream));
