@@ -25,6 +25,22 @@ def _host_array(a, dtype=None):
     return np.ascontiguousarray(a)
 
 
+class _Owner:
+    """A library handle, destroyed with the last of the matrix and the tensors over its arrays.
+    Those refer to this object and not to the matrix, which refers to them: a cycle through a
+    tensor's storage is none that the garbage collector can see."""
+
+    def __init__(self, h):
+        self.h = h
+
+    def __del__(self):
+        if core._lib._lib is not None:
+            try:
+                core.lib().gg_mat_destroy(self.h)
+            except Exception:
+                pass
+
+
 class AbstractSparseGPUMatrix:
     """Common interface of the device sparse matrices (src/storage/GPUGraphsMatrix.jl)."""
 
@@ -49,14 +65,8 @@ class AbstractSparseGPUMatrix:
         """length(A) = m * n (src/storage/CSR.jl:144)."""
         return self.m * self.n
 
-    def __del__(self):
-        h = getattr(self, "_h", None)
-        if h is not None and core._lib._lib is not None:
-            try:
-                core.lib().gg_mat_destroy(h)
-            except Exception:
-                pass
-            self._h = None
+    def _own(self, h):
+        self._h, self._owner = h, _Owner(h)
 
     def _info(self):
         L = core.lib()
@@ -125,12 +135,12 @@ class SparseGPUMatrixCSR(AbstractSparseGPUMatrix):
             h = ctypes.c_void_p()
             check(L.gg_csr_create(c, int(m), int(n), int(len(colval)), *args, code,
                                   1 if on_dev else 0, ctypes.byref(h)), L)
-        self._h = h
+        self._own(h)
         self.device = dev
         p, cv_, nz_, _ = self._info()
-        self.rowptr = core.wrap_device(self, p, self.m + 1, core.INT32, dev)
-        self.colval = core.wrap_device(self, cv_, self._nnz, core.INT32, dev)
-        self.nzval = core.wrap_device(self, nz_, self._nnz, self.dtype_code, dev)
+        self.rowptr = core.wrap_device(self._owner, p, self.m + 1, core.INT32, dev)
+        self.colval = core.wrap_device(self._owner, cv_, self._nnz, core.INT32, dev)
+        self.nzval = core.wrap_device(self._owner, nz_, self._nnz, self.dtype_code, dev)
 
     # ---- reference constructors ----
     @classmethod
@@ -271,14 +281,14 @@ class SparseGPUMatrixSELL(AbstractSparseGPUMatrix):
             L = core.lib()
             h = ctypes.c_void_p()
             check(L.gg_sell_create(c, A.handle, int(slice_size), int(sigma), ctypes.byref(h)), L)
-        self._h = h
+        self._own(h)
         self.device = dev
         self.sigma = int(sigma)
         p, cv, nz, pm = self._info()
-        self.slice_ptr = core.wrap_device(self, p, self.nslices + 1, core.INT32, dev)
-        self.colval = core.wrap_device(self, cv, self.n_stored, core.INT32, dev)
-        self.nzval = core.wrap_device(self, nz, self.n_stored, self.dtype_code, dev)
-        self.perm = core.wrap_device(self, pm, self.m, core.INT32, dev)
+        self.slice_ptr = core.wrap_device(self._owner, p, self.nslices + 1, core.INT32, dev)
+        self.colval = core.wrap_device(self._owner, cv, self.n_stored, core.INT32, dev)
+        self.nzval = core.wrap_device(self._owner, nz, self.n_stored, self.dtype_code, dev)
+        self.perm = core.wrap_device(self._owner, pm, self.m, core.INT32, dev)
 
     def __getitem__(self, ij):
         """A[i, j] (1-based).  Walks the slice holding row i (the reference's
