@@ -274,6 +274,7 @@ int gg_destroy(gg_ctx* ctx) {
   cudaFree(ctx->d_flags);
   cudaFreeHost(ctx->h_flags);
   cudaFree(ctx->d_err);
+  cudaFree(ctx->mm_choice);
   if (ctx->scratch_order.event) cudaEventDestroy(ctx->scratch_order.event);
   if (ctx->trace_ev) {
     for (int i = 0; i < 2 * kTraceMax; ++i) cudaEventDestroy(ctx->trace_ev[i]);

@@ -531,6 +531,7 @@ struct gg_ctx {
   size_t scratch_bytes = 0;
   gg::StreamOrder scratch_order;
   bool scratch_used = false;  // by the current gg_spmm call
+  unsigned int* mm_choice = nullptr;  // masked SpMM: 8 words (k_mask_choice), made on first use
   unsigned int* d_flags = nullptr;  // small device word array for status flags
   unsigned int* h_flags = nullptr;  // pinned mirror
   unsigned int* d_err = nullptr;    // set by kernels whose bounded waits ran out

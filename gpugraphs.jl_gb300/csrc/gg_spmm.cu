@@ -95,6 +95,14 @@ __device__ __forceinline__ void fold_csr(const SR& sr, const int32_t* __restrict
   }
 }
 
+// A launch that is wanted for one outcome of a device-side choice only (k_mask_choice): the
+// others end at once.
+struct MMGate {
+  const unsigned* word = nullptr;
+  unsigned want = 0;
+  __device__ __forceinline__ bool closed() const { return word && __ldg(word) != want; }
+};
+
 // CSR: items [0, nseg) are pieces of rows longer than kSegMM (their partials go to
 // partials[slot * jn + j - jlo]); items [nseg, nseg + nrows) are the rows of
 // [row_lo, row_lo + nrows), one warp per row, lane per dense column (CPL columns per
@@ -104,8 +112,9 @@ __global__ void __launch_bounds__(256)
     k_csr_spmm(SR sr, const int32_t* __restrict__ rowptr, const int32_t* __restrict__ colval,
                int64_t row_lo, int64_t nrows, int64_t jlo, int64_t jn, const void* mask, int tmask,
                const int4* __restrict__ segs, int64_t nseg, typename SR::T* partials,
-               int32_t skip_le) {
+               int32_t skip_le, MMGate gate) {
   typedef typename SR::T T;
+  if (gate.closed()) return;
   const int lane = threadIdx.x & 31;
   const int64_t w0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -162,7 +171,9 @@ __global__ void __launch_bounds__(256)
     k_sell_spmm(SR sr, const int32_t* __restrict__ slice_ptr, const int32_t* __restrict__ colval,
                 const int32_t* __restrict__ perm, int64_t C, int64_t s_lo, int64_t s_hi,
                 int64_t jlo, int64_t jn, int64_t range_lo, int64_t range_hi, const void* mask,
-                int tmask, const int4* __restrict__ segs, int64_t nseg, typename SR::T* partials) {
+                int tmask, const int4* __restrict__ segs, int64_t nseg, typename SR::T* partials,
+                MMGate gate) {
+  if (gate.closed()) return;
   const int lane = threadIdx.x & 31;
   const int64_t w0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -204,8 +215,9 @@ __global__ void __launch_bounds__(256)
     k_spmm_combine(SR sr, const int32_t* __restrict__ rows, const int32_t* __restrict__ first,
                    int64_t nlong, const int32_t* __restrict__ perm, bool sell, int64_t row_lo,
                    int64_t row_hi, int64_t jlo, int64_t jn, const void* mask, int tmask,
-                   const typename SR::T* __restrict__ partials) {
+                   const typename SR::T* __restrict__ partials, MMGate gate) {
   typedef typename SR::T T;
+  if (gate.closed()) return;
   const int lane = threadIdx.x & 31;
   const int64_t w0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -659,7 +671,7 @@ static size_t mm_partial_bytes(const MMPlan* P, size_t esz, int64_t k, int64_t* 
 // reserved: bytes at the start of the scratch that hold the caller's operands
 template <class SR>
 static int launch_mm(gg_ctx* ctx, gg_mat* A, const SR& sr, int64_t k, const void* mask, int tmask,
-                     int64_t lo, int64_t hi, size_t reserved = 0) {
+                     int64_t lo, int64_t hi, size_t reserved = 0, MMGate gate = MMGate()) {
   typedef typename SR::T T;
   const int64_t m = A->m;
   if (col1_sell_ok(A, sr, k, mask, lo)) return col1_sell(ctx, A, sr);
@@ -700,15 +712,15 @@ static int launch_mm(gg_ctx* ctx, gg_mat* A, const SR& sr, int64_t k, const void
       if (cpl == 4)
         k_csr_spmm<SR, 4><<<grid_mm(ctx, P->nseg + nrows), 256, 0, ctx->stream>>>(
             sr, A->rowptr, A->colval, row_lo, nrows, jlo, jn, mask, tmask, P->segs, P->nseg, partials,
-            skip);
+            skip, gate);
       else if (cpl == 2)
         k_csr_spmm<SR, 2><<<grid_mm(ctx, P->nseg + nrows), 256, 0, ctx->stream>>>(
             sr, A->rowptr, A->colval, row_lo, nrows, jlo, jn, mask, tmask, P->segs, P->nseg, partials,
-            skip);
+            skip, gate);
       else
         k_csr_spmm<SR, 1><<<grid_mm(ctx, P->nseg + nrows), 256, 0, ctx->stream>>>(
             sr, A->rowptr, A->colval, row_lo, nrows, jlo, jn, mask, tmask, P->segs, P->nseg, partials,
-            skip);
+            skip, gate);
       }
     } else {
       int64_t s_lo = 0, s_hi = m;
@@ -721,7 +733,7 @@ static int launch_mm(gg_ctx* ctx, gg_mat* A, const SR& sr, int64_t k, const void
       tr = trace_main_begin(ctx);
       k_sell_spmm<SR><<<grid_mm(ctx, P->nseg + s_hi - s_lo), 256, 0, ctx->stream>>>(
           sr, A->slice_ptr, A->colval, A->sigma > 1 ? A->perm : nullptr, A->slice_size, s_lo, s_hi,
-          jlo, jn, lo, hi, mask, tmask, P->segs, P->nseg, partials);
+          jlo, jn, lo, hi, mask, tmask, P->segs, P->nseg, partials, gate);
     }
     trace_main_end(ctx, tr);
     trace_count(ctx, 1);
@@ -730,7 +742,7 @@ static int launch_mm(gg_ctx* ctx, gg_mat* A, const SR& sr, int64_t k, const void
       trace_count(ctx, 1);
       k_spmm_combine<SR><<<grid_mm(ctx, P->nlong), 256, 0, ctx->stream>>>(
           sr, P->rows, P->first, P->nlong, A->sigma > 1 ? A->perm : nullptr,
-          A->format != GG_FMT_CSR, row_lo, row_hi, jlo, jn, mask, tmask, partials);
+          A->format != GG_FMT_CSR, row_lo, row_hi, jlo, jn, mask, tmask, partials, gate);
       GG_CUDA(cudaGetLastError());
     }
   }
@@ -744,7 +756,9 @@ static int launch_mm(gg_ctx* ctx, gg_mat* A, const SR& sr, int64_t k, const void
 // dimension kp >= k (columns past k filled with 0): 32 x 32 tiles, both sides coalesced
 template <typename E>
 __global__ void __launch_bounds__(256)
-    k_to_row_major(const E* __restrict__ src, int64_t ld, int64_t rows, int k, E* __restrict__ dst, int kp) {
+    k_to_row_major(const E* __restrict__ src, int64_t ld, int64_t rows, int k, E* __restrict__ dst, int kp,
+                   MMGate gate) {
+  if (gate.closed()) return;
   __shared__ E tile[32][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   for (int64_t r0 = (int64_t)blockIdx.x * 32; r0 < rows; r0 += (int64_t)gridDim.x * 32) {
@@ -766,7 +780,9 @@ __global__ void __launch_bounds__(256)
 // the rows the product wrote (range [row_lo, row_hi), mask) back to column-major
 __global__ void __launch_bounds__(256)
     k_to_col_major_f32(const float* __restrict__ src, int kp, int64_t row_lo, int64_t row_hi, int k,
-                       float* __restrict__ dst, int64_t ld, const void* mask, int tmask) {
+                       float* __restrict__ dst, int64_t ld, const void* mask, int tmask,
+                       MMGate gate) {
+  if (gate.closed()) return;
   __shared__ float tile[32][33];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   for (int64_t r0 = row_lo + (int64_t)blockIdx.x * 32; r0 < row_hi; r0 += (int64_t)gridDim.x * 32) {
@@ -789,13 +805,13 @@ __global__ void __launch_bounds__(256)
 
 template <typename E>
 static void to_row_major(gg_ctx* ctx, const void* src, int64_t ld, int64_t rows, int64_t k, void* dst,
-                         int64_t kp) {
+                         int64_t kp, MMGate gate) {
   int64_t g = (rows + 31) / 32;
   const int64_t cap = (int64_t)ctx->num_sms * 8;
   if (g > cap) g = cap;
   if (g < 1) return;
   k_to_row_major<E><<<(int)g, 256, 0, ctx->stream>>>(static_cast<const E*>(src), ld, rows, (int)k,
-                                                     static_cast<E*>(dst), (int)kp);
+                                                     static_cast<E*>(dst), (int)kp, gate);
   trace_count(ctx, 1);
 }
 
@@ -850,10 +866,10 @@ static void mm_selected(const gg_mat* A, int64_t lo, int64_t hi, int64_t* entrie
 // 2^20 rows: ER, 32 entries a row, 1000 rows x 32 columns 68 / 89, 3000 rows 122 / 92, 3000 x 2
 // 55 / 73, 10000 x 2 86 / 77; R-MAT, 100 rows x 32 62 / 105, 1000 rows, a hub among them,
 // 224 / 138.
-static bool staging_pays_f32(int64_t e, int32_t longest, int64_t n, int64_t k) {
-  const double chain = 0.45 * std::min(longest, (int32_t)kSegMM);
+__host__ __device__ static bool staging_pays_f32(int64_t e, int32_t longest, int64_t n, int64_t k) {
+  const double chain = 0.45 * (longest < kSegMM ? longest : kSegMM);
   const double all = (double)e * (4e-4 + 2.5e-5 * (double)k);
-  return std::max(chain, all) >= 5.0 + (double)n * (25e-6 + 0.65e-6 * (double)k);
+  return (chain > all ? chain : all) >= 5.0 + (double)n * (25e-6 + 0.65e-6 * (double)k);
 }
 
 // Row-major rows that are no whole 16-byte groups: what the aligned kernels save on the rows
@@ -871,7 +887,72 @@ static bool padding_pays_f32(int64_t rows, int64_t e, int64_t n, int64_t k) {
 // min-plus where it lies / transposed, us: ER 2^20 x 32, 10^4 rows (0.15 n entries) 100 / 123, 30000
 // (0.46 n) 260 / 221, all 8266 / 4522; x 8, 30000 rows 143 / 186, 3 10^5 (4.6 n) 1205 / 1177; R-MAT
 // scale 20 x 32, 30000 rows (0.26 n) 383 / 389, 10^5 (0.6 n) 865 / 702.
-static bool staging_pays(int64_t e, int64_t n, int64_t k) { return e * k >= 14 * n; }
+__host__ __device__ static bool staging_pays(int64_t e, int64_t n, int64_t k) { return e * k >= 14 * n; }
+
+// What a mask keeps of the m rows is known on the device alone, and the call does not wait
+// for it: this kernel counts the entries (rowptr; SELL: per_row of them a row) and writes 1 to
+// g[4] where rewriting B pays, else 0, and the launches of both ways follow, each with its
+// gate.  g: entries (64 bits), longest row, blocks done, choice; cleared before.
+__global__ void __launch_bounds__(256)
+    k_mask_choice(const int32_t* __restrict__ rowptr, double per_row, int64_t m, const void* mask,
+                  int tmask, int64_t n, int64_t k, bool f32, unsigned* g) {
+  unsigned long long* entries = reinterpret_cast<unsigned long long*>(g);
+  unsigned long long e = 0;
+  unsigned longest = 0;
+  for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < m;
+       r += (int64_t)gridDim.x * blockDim.x) {
+    if (raw_is_zero(load_raw(mask, tmask, r), tmask)) continue;
+    const unsigned len = rowptr ? (unsigned)(__ldg(rowptr + r + 1) - __ldg(rowptr + r)) : 1u;
+    e += len;
+    if (rowptr) longest = len > longest ? len : longest;
+  }
+  longest = __reduce_max_sync(kFullMM, longest);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(kFullMM, e, o);
+  if ((threadIdx.x & 31) == 0 && e) {
+    atomicAdd(entries, e);
+    if (longest) atomicMax(g + 2, longest);
+  }
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x != 0 || atomicAdd(g + 3, 1u) != gridDim.x - 1) return;
+  __threadfence();
+  e = *((volatile unsigned long long*)entries);
+  if (!rowptr) e = (unsigned long long)((double)e * per_row);
+  const int32_t top = (int32_t)*((volatile unsigned*)(g + 2));
+  g[4] = f32 ? staging_pays_f32((int64_t)e, top, n, k) : staging_pays((int64_t)e, n, k);
+}
+
+// Masks of products whose B takes at least this long to rewrite, in us, are counted: the
+// count and the launches that end at once cost about 8.
+static const double kMMMaskCost = 20.0;
+
+static bool mask_counts(const gg_mat* A, const void* mask, int64_t k) {
+  return mask && (double)A->n * (25e-6 + 0.65e-6 * (double)k) >= kMMMaskCost;
+}
+
+// *gate: the word that holds 1 where staging pays for the rows the mask keeps (nullptr: no
+// memory for it, not counted)
+static int count_mask(gg_ctx* ctx, const gg_mat* A, const void* mask, int tmask, int64_t k, bool f32,
+                      const unsigned** gate) {
+  *gate = nullptr;
+  GG_CHECK(ensure_scratch(ctx, 1));  // the word is ordered between streams as the scratch is
+  if (!ctx->mm_choice && cudaMalloc((void**)&ctx->mm_choice, 32) != cudaSuccess) {
+    (void)cudaGetLastError();
+    ctx->mm_choice = nullptr;
+    return GG_OK;
+  }
+  GG_CUDA(cudaMemsetAsync(ctx->mm_choice, 0, 32, ctx->stream));
+  int64_t g = (A->m + 255) / 256;
+  if (g > (int64_t)ctx->num_sms * 4) g = (int64_t)ctx->num_sms * 4;
+  k_mask_choice<<<(int)(g > 0 ? g : 1), 256, 0, ctx->stream>>>(
+      A->format == GG_FMT_CSR ? A->rowptr : nullptr, A->m > 0 ? (double)A->nnz / (double)A->m : 0.0,
+      A->m, mask, tmask, A->n, k, f32, ctx->mm_choice);
+  GG_CUDA(cudaGetLastError());
+  trace_count(ctx, 1);
+  *gate = ctx->mm_choice + 4;
+  return GG_OK;
+}
 
 // scratch for the transposed operands of one pass; wider products run in passes
 static const int64_t kMMTransposeBytes = (int64_t)5 << 28;
@@ -889,7 +970,7 @@ static int64_t mm_pass_columns(int64_t k, int64_t per_col) {
 // row-major rows that are not whole 16-byte groups): both through row-major scratch.
 // GG_ERR_OOM (nothing launched): the caller takes them where they lie.
 static int spmm_staged_f32(gg_ctx* ctx, gg_mat* A, SRPlusTimesF32MM sr, int64_t k, int layout,
-                           const void* mask, int tmask, int64_t lo, int64_t hi) {
+                           const void* mask, int tmask, int64_t lo, int64_t hi, MMGate gate) {
   const int64_t n = A->n;
   const int64_t row_lo = lo > 0 ? lo - 1 : 0, row_hi = lo > 0 ? hi : A->m;
   const int64_t nrows = row_hi - row_lo;  // C is staged for these alone
@@ -912,17 +993,17 @@ static int spmm_staged_f32(gg_ctx* ctx, gg_mat* A, SRPlusTimesF32MM sr, int64_t 
     float* const C0 = Ct - row_lo * kp;  // where row 0 would be
     sr.y = C0;
     if (col) {
-      to_row_major<float>(ctx, B + j0 * ldb, ldb, n, kn, Bt, kp);
+      to_row_major<float>(ctx, B + j0 * ldb, ldb, n, kn, Bt, kp, gate);
     } else {
       k_pad_rows_f32<<<grid_mm(ctx, n), 256, 0, ctx->stream>>>(B + j0, ldb, n, (int)kn, Bt, (int)kp);
       trace_count(ctx, 1);
     }
-    GG_CHECK(launch_mm(ctx, A, sr, kp, mask, tmask, lo, hi, bbytes + cbytes));
+    GG_CHECK(launch_mm(ctx, A, sr, kp, mask, tmask, lo, hi, bbytes + cbytes, gate));
     if (col) {
       int64_t g = (nrows + 31) / 32;
       if (g > (int64_t)ctx->num_sms * 8) g = (int64_t)ctx->num_sms * 8;
       k_to_col_major_f32<<<(int)g, 256, 0, ctx->stream>>>(C0, (int)kp, row_lo, row_hi, (int)kn,
-                                                         Cm + j0 * ldc, ldc, mask, tmask);
+                                                         Cm + j0 * ldc, ldc, mask, tmask, gate);
     } else {
       k_unpad_rows_f32<<<grid_mm(ctx, nrows), 256, 0, ctx->stream>>>(C0, (int)kp, row_lo, row_hi, (int)kn,
                                                                     Cm + j0, ldc);
@@ -936,7 +1017,7 @@ static int spmm_staged_f32(gg_ctx* ctx, gg_mat* A, SRPlusTimesF32MM sr, int64_t 
 // other semirings: B through row-major scratch, C where it lies
 template <class SR>
 static int spmm_colmajor(gg_ctx* ctx, gg_mat* A, SR sr, int64_t k, const void* mask, int tmask,
-                         int64_t lo, int64_t hi) {
+                         int64_t lo, int64_t hi, MMGate gate) {
   typedef typename SR::T T;
   const int64_t n = A->n;
   const int esz = dtype_size(sr.tx);
@@ -952,13 +1033,13 @@ static int spmm_colmajor(gg_ctx* ctx, gg_mat* A, SR sr, int64_t k, const void* m
     const int64_t kn = k - j0 < w ? k - j0 : w;
     const char* Bj = B + j0 * ldb * esz;
     switch (esz) {
-      case 1: to_row_major<uint8_t>(ctx, Bj, ldb, n, kn, ctx->scratch, kn); break;
-      case 4: to_row_major<uint32_t>(ctx, Bj, ldb, n, kn, ctx->scratch, kn); break;
-      default: to_row_major<uint64_t>(ctx, Bj, ldb, n, kn, ctx->scratch, kn); break;
+      case 1: to_row_major<uint8_t>(ctx, Bj, ldb, n, kn, ctx->scratch, kn, gate); break;
+      case 4: to_row_major<uint32_t>(ctx, Bj, ldb, n, kn, ctx->scratch, kn, gate); break;
+      default: to_row_major<uint64_t>(ctx, Bj, ldb, n, kn, ctx->scratch, kn, gate); break;
     }
     sr.ldb = kn;
     sr.col0 = j0;
-    GG_CHECK(launch_mm(ctx, A, sr, kn, mask, tmask, lo, hi, bbytes));
+    GG_CHECK(launch_mm(ctx, A, sr, kn, mask, tmask, lo, hi, bbytes, gate));
   }
   return GG_OK;
 }
@@ -966,7 +1047,7 @@ static int spmm_colmajor(gg_ctx* ctx, gg_mat* A, SR sr, int64_t k, const void* m
 template <int TC>
 static int spmm_generic(gg_ctx* ctx, gg_mat* A, int mul, int add, int accum, void* Cm, int tcm,
                         int64_t ldc, const void* B, int tb, int64_t ldb, int64_t k, int layout,
-                        const void* mask, int tmask, int64_t lo, int64_t hi) {
+                        const void* mask, int tmask, int64_t lo, int64_t hi, MMGate gate) {
   typedef typename CType<TC>::T T;
   SRGen<TC> sr;
   sr.mul = mul;
@@ -984,17 +1065,20 @@ static int spmm_generic(gg_ctx* ctx, gg_mat* A, int mul, int add, int accum, voi
   sr.ldc = ldc;
   sr.layout = layout;
   sr.layout_c = layout;
-  if (layout == GG_COL_MAJOR) {
+  if (layout == GG_COL_MAJOR && !gate.word) {
     GG_CHECK(build_mm_plan(ctx, A));
     int64_t e = 0;
     int32_t longest = 0;
     mm_selected(A, lo, hi, &e, &longest);
     if (A->nnz * k >= kMMTranspose && staging_pays(e, A->n, k)) {
-      const int rc = spmm_colmajor(ctx, A, sr, k, mask, tmask, lo, hi);
-      if (rc != GG_ERR_OOM) return rc;
+      const unsigned* choice = nullptr;
+      if (mask_counts(A, mask, k)) GG_CHECK(count_mask(ctx, A, mask, tmask, k, false, &choice));
+      const int rc = spmm_colmajor(ctx, A, sr, k, mask, tmask, lo, hi, MMGate{choice, 1});
+      if (rc == GG_OK && choice) gate = MMGate{choice, 0};
+      else if (rc != GG_ERR_OOM) return rc;
     }
   }
-  return launch_mm(ctx, A, sr, k, mask, tmask, lo, hi);
+  return launch_mm(ctx, A, sr, k, mask, tmask, lo, hi, 0, gate);
 }
 
 int spmm_dispatch(gg_ctx* ctx, gg_mat* A, int tc, int mul, int add, int accum, void* Cm, int tcm,
@@ -1007,6 +1091,7 @@ int spmm_dispatch(gg_ctx* ctx, gg_mat* A, int tc, int mul, int add, int accum, v
     ldb = 1;
     ldc = 1;
   }
+  MMGate gate;
   if (A->dtype == GG_FLOAT32 && tb == GG_FLOAT32 && tcm == GG_FLOAT32 && mul == GG_OP_MUL &&
       add == GG_OP_ADD && accum == GG_OP_SECOND) {
     SRPlusTimesF32MM sr;
@@ -1026,18 +1111,21 @@ int spmm_dispatch(gg_ctx* ctx, gg_mat* A, int tc, int mul, int add, int accum, v
       const bool pays = pad ? padding_pays_f32(lo > 0 ? hi - lo + 1 : A->m, e, A->n, k)
                             : staging_pays_f32(e, longest, A->n, k);
       if (A->nnz * k >= kMMTranspose && pays) {
-        const int rc = spmm_staged_f32(ctx, A, sr, k, layout, mask, tmask, lo, hi);
-        if (rc != GG_ERR_OOM) return rc;
+        const unsigned* choice = nullptr;
+        if (mask_counts(A, mask, k)) GG_CHECK(count_mask(ctx, A, mask, tmask, k, true, &choice));
+        const int rc = spmm_staged_f32(ctx, A, sr, k, layout, mask, tmask, lo, hi, MMGate{choice, 1});
+        if (rc == GG_OK && choice) gate = MMGate{choice, 0};
+        else if (rc != GG_ERR_OOM) return rc;
       }
     }
     if (layout == GG_ROW_MAJOR) return launch_mm(ctx, A, sr, k, mask, tmask, lo, hi);
   }
   switch (tc) {
-    case GG_BOOL: return spmm_generic<GG_BOOL>(ctx, A, mul, add, accum, Cm, tcm, ldc, B, tb, ldb, k, layout, mask, tmask, lo, hi);
-    case GG_INT32: return spmm_generic<GG_INT32>(ctx, A, mul, add, accum, Cm, tcm, ldc, B, tb, ldb, k, layout, mask, tmask, lo, hi);
-    case GG_INT64: return spmm_generic<GG_INT64>(ctx, A, mul, add, accum, Cm, tcm, ldc, B, tb, ldb, k, layout, mask, tmask, lo, hi);
-    case GG_FLOAT32: return spmm_generic<GG_FLOAT32>(ctx, A, mul, add, accum, Cm, tcm, ldc, B, tb, ldb, k, layout, mask, tmask, lo, hi);
-    default: return spmm_generic<GG_FLOAT64>(ctx, A, mul, add, accum, Cm, tcm, ldc, B, tb, ldb, k, layout, mask, tmask, lo, hi);
+    case GG_BOOL: return spmm_generic<GG_BOOL>(ctx, A, mul, add, accum, Cm, tcm, ldc, B, tb, ldb, k, layout, mask, tmask, lo, hi, gate);
+    case GG_INT32: return spmm_generic<GG_INT32>(ctx, A, mul, add, accum, Cm, tcm, ldc, B, tb, ldb, k, layout, mask, tmask, lo, hi, gate);
+    case GG_INT64: return spmm_generic<GG_INT64>(ctx, A, mul, add, accum, Cm, tcm, ldc, B, tb, ldb, k, layout, mask, tmask, lo, hi, gate);
+    case GG_FLOAT32: return spmm_generic<GG_FLOAT32>(ctx, A, mul, add, accum, Cm, tcm, ldc, B, tb, ldb, k, layout, mask, tmask, lo, hi, gate);
+    default: return spmm_generic<GG_FLOAT64>(ctx, A, mul, add, accum, Cm, tcm, ldc, B, tb, ldb, k, layout, mask, tmask, lo, hi, gate);
   }
 }
 

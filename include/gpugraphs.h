@@ -230,8 +230,9 @@ int gg_spmv(gg_ctx* ctx, const gg_mat* A, int mul, int add, int accum, void* y, 
  * GG_ERR_ASSERTION like the reference's @assert.
  * Column-major operands, and row-major Float32 ones whose width is not a multiple of
  * four, are transposed or padded through the context's scratch where the entries of the
- * selected range make up for it (a mask's rows are not counted), in passes of at most
- * 1.25 GiB of operands but never fewer than four columns; where the scratch cannot grow,
+ * selected range, or of the rows that a mask keeps (counted on the device for operands that
+ * take 20 us and more to rewrite), make up for it, in passes of at most 1.25 GiB of operands
+ * but never fewer than four columns; where the scratch cannot grow,
  * they are taken where they lie.  The scratch grows on demand, so a call that is to be captured in a CUDA
  * graph is made once before, and a larger call on the context afterwards may move the
  * scratch that a captured one uses.
