@@ -378,9 +378,9 @@ struct MMPlan {
   // the four rows a warp takes have about the same length
   int32_t* short_rows = nullptr;
   int64_t nshort = 0, nlive = 0;  // nlive: the leading ones that hold an entry
-  // CSR, host: entries before every kMMBlockRows-th row, and the longest row from there to
-  // the next (what a row range holds)
-  std::vector<int32_t> block_entry, block_longest;
+  // CSR, host: the row pointers, and the longest row of every kMMBlockRows rows where a row
+  // range has asked for it, else -1 (what a range holds)
+  std::vector<int32_t> host_rowptr, block_longest;
 };
 static const int kSegMM = 256;
 static const int kMMBlockRows = 32;

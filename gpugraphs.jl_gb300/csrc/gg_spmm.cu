@@ -538,11 +538,11 @@ static int grid_mm(gg_ctx* ctx, int64_t warps) {
 int build_mm_plan(gg_ctx* ctx, gg_mat* A) {
   if (A->mmplan) return GG_OK;
   std::vector<int4> segs, items;
-  std::vector<int32_t> first, rows, short_rows, block_entry, block_longest;
+  std::vector<int32_t> first, rows, short_rows, rp;
   int64_t nlive = 0;
   if (A->format == GG_FMT_CSR) {
     const int64_t m = A->m;
-    std::vector<int32_t> rp(m + 1);
+    rp.resize(m + 1);
     GG_CUDA(cudaMemcpyAsync(rp.data(), A->rowptr, (m + 1) * sizeof(int32_t),
                             cudaMemcpyDeviceToHost, ctx->stream));
     GG_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -557,17 +557,8 @@ int build_mm_plan(gg_ctx* ctx, gg_mat* A) {
       for (int64_t r = 0; r < m; ++r) {
         const int64_t L = rp[r + 1] - rp[r];
         if (L <= kShortMM) short_rows[cnt[kShortMM - L]++] = (int32_t)r;
-        if (L > 0 && L <= kShortMM) ++nlive;
       }
-    }
-    block_entry.reserve(m / kMMBlockRows + 2);
-    block_longest.reserve(m / kMMBlockRows + 1);
-    for (int64_t r0 = 0; r0 < m; r0 += kMMBlockRows) {
-      const int64_t r1 = r0 + kMMBlockRows < m ? r0 + kMMBlockRows : m;
-      int32_t longest = 0;
-      for (int64_t r = r0; r < r1; ++r) longest = std::max(longest, rp[r + 1] - rp[r]);
-      block_entry.push_back(rp[r0] - 1);
-      block_longest.push_back(longest);
+      nlive = cnt[kShortMM - 1];  // past the rows of one entry
     }
     for (int64_t r = 0; r < m; ++r) {
       const int64_t k0 = rp[r] - 1, k1 = rp[r + 1] - 1;
@@ -621,9 +612,7 @@ int build_mm_plan(gg_ctx* ctx, gg_mat* A) {
   up((void**)&P->items, items.data(), (size_t)P->nitems * sizeof(int4));
   P->nshort = (int64_t)short_rows.size();
   P->nlive = nlive;
-  block_entry.push_back((int32_t)A->nnz);
-  P->block_entry = std::move(block_entry);
-  P->block_longest = std::move(block_longest);
+  P->host_rowptr = std::move(rp);
   up((void**)&P->short_rows, short_rows.data(), short_rows.size() * sizeof(int32_t));
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
   if (e != cudaSuccess) {
@@ -841,22 +830,35 @@ __global__ void __launch_bounds__(256)
 // to 32 columns.
 static const int64_t kMMTranspose = 1 << 10;
 
-// entries of the selected rows (to whole blocks of kMMBlockRows; SELL: by the mean), and
-// the longest row among them (SELL: 0; the largest int past 2^17 rows of a range)
+// entries of the selected rows (SELL: by the mean), and the longest row of the blocks of
+// kMMBlockRows that hold them (SELL: 0; the largest int past 2^17 rows of a range).  A block is
+// looked through when a range first needs it: all of them in the plan cost a matrix of 2^20
+// rows 1.4 ms of its first product, whatever that selected.
 static void mm_selected(const gg_mat* A, int64_t lo, int64_t hi, int64_t* entries, int32_t* longest) {
   *entries = A->nnz;
   *longest = INT32_MAX;
   if (lo <= 0) return;
-  const MMPlan* P = A->mmplan;
+  MMPlan* P = A->mmplan;
   if (A->format != GG_FMT_CSR) {
     *entries = (int64_t)((double)A->nnz * (double)(hi - lo + 1) / (double)A->m);
     *longest = 0;
     return;
   }
+  const std::vector<int32_t>& rp = P->host_rowptr;
+  *entries = rp[hi] - rp[lo - 1];
   const int64_t b0 = (lo - 1) / kMMBlockRows, b1 = (hi - 1) / kMMBlockRows + 1;
-  *entries = P->block_entry[b1] - P->block_entry[b0];
   if (b1 - b0 > 4096) return;
-  *longest = *std::max_element(P->block_longest.begin() + b0, P->block_longest.begin() + b1);
+  if (P->block_longest.empty()) P->block_longest.assign((A->m + kMMBlockRows - 1) / kMMBlockRows, -1);
+  *longest = 0;
+  for (int64_t b = b0; b < b1; ++b) {
+    int32_t& L = P->block_longest[b];
+    if (L < 0) {
+      L = 0;
+      const int64_t r1 = (b + 1) * kMMBlockRows < A->m ? (b + 1) * kMMBlockRows : A->m;
+      for (int64_t r = b * kMMBlockRows; r < r1; ++r) L = std::max(L, rp[r + 1] - rp[r]);
+    }
+    *longest = std::max(*longest, L);
+  }
 }
 
 // Whether the gathers of e entries from a column-major Float32 B cost more than rewriting all
