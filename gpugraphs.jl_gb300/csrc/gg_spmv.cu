@@ -593,8 +593,8 @@ int build_colperm(gg_ctx* ctx, gg_mat* A) {
   const int64_t len = A->format == GG_FMT_CSR ? A->nnz : A->n_stored;
   if (n < (1 << 16) || A->nnz == 0) return GG_OK;
   int32_t *cnt = nullptr, *rank = nullptr;
-  cudaError_t e = cudaMallocAsync((void**)&cnt, n * sizeof(int32_t), ctx->stream);
-  if (e == cudaSuccess) e = cudaMallocAsync((void**)&rank, n * sizeof(int32_t), ctx->stream);
+  cudaError_t e = cudaMalloc((void**)&cnt, 2 * n * sizeof(int32_t));  // counts, ranks
+  if (e == cudaSuccess) rank = cnt + n;
   if (e == cudaSuccess) e = cudaMalloc((void**)&P->inv, n * sizeof(int32_t));
   if (e == cudaSuccess) e = cudaMemsetAsync(cnt, 0, n * sizeof(int32_t), ctx->stream);
   int rc = GG_OK;
@@ -619,9 +619,8 @@ int build_colperm(gg_ctx* ctx, gg_mat* A) {
       e = cudaGetLastError();
     }
   }
-  cudaFreeAsync(cnt, ctx->stream);
-  cudaFreeAsync(rank, ctx->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+  cudaFree(cnt);
   GG_CHECK(rc);
   if (e != cudaSuccess) return cuda_error(e, "column relabelling");
   P->enabled = skewed;
