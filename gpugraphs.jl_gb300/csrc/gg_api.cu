@@ -9,6 +9,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <numeric>
 #include <vector>
 
 #include "gg_common.cuh"
@@ -150,6 +151,32 @@ __global__ void k_invert_perm(int64_t m, const int32_t* perm, int32_t* iperm) {
   for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < m;
        t += (int64_t)gridDim.x * blockDim.x)
     iperm[perm[t] - 1] = (int32_t)t;
+}
+
+// Rows up to which gg_sell_create orders them on the host, with windows to sort and without:
+// the device's order is some ten launches, allocations and waits.  Device / host, us, sigma =
+// 1024 and 1: R-MAT, 256 rows 346 / 109 and 314 / 109, 4096 rows 418 / 309 and 416 / 268, 8192
+// rows 489 / 490 and 419 / 278, 32768 rows 522 / 1150 and 445 / 365; 128 x 128 grid 382 / 283
+// and 319 / 148.
+static const int64_t kHostOrderRows = 8192, kHostWidthRows = 32768;
+
+// the row order of a SELL-C-sigma layout (1-based) and the widest row of every slice
+static int order_rows_on_host(gg_ctx* ctx, const int32_t* rowptr, int64_t m, int64_t C, int64_t sigma,
+                              std::vector<int32_t>* perm, std::vector<int32_t>* width) {
+  std::vector<int32_t> rp(m + 1);
+  GG_CUDA(cudaMemcpyAsync(rp.data(), rowptr, (m + 1) * sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
+  GG_CUDA(cudaStreamSynchronize(ctx->stream));
+  perm->resize(m);
+  std::iota(perm->begin(), perm->end(), 1);
+  auto len = [&](int32_t r) { return rp[r] - rp[r - 1]; };
+  for (int64_t w0 = 0; w0 < m && sigma > 1; w0 += sigma)
+    std::stable_sort(perm->begin() + w0, perm->begin() + std::min(w0 + sigma, m),
+                     [&](int32_t a, int32_t b) { return len(a) > len(b); });
+  for (int64_t t = 0; t < m; ++t) {
+    int32_t& w = (*width)[t / C];
+    w = std::max(w, len((*perm)[t]));
+  }
+  return GG_OK;
 }
 
 static void free_mat_storage(gg_mat* A);
@@ -418,21 +445,26 @@ int gg_sell_create(gg_ctx* ctx, const gg_mat* csr, int64_t slice_size, int64_t s
   // slice height clamped to m (src/storage/SELL.jl:108)
   const int64_t C = slice_size < m ? slice_size : m;
   const int64_t ns = C > 0 ? (m + C - 1) / C : 0;
-  // row order and slice widths on the device; the slices' offsets (64 bits, checked
-  // against the Int32 range) here
+  // row order and slice widths on the device, or here for few rows; the slices' offsets
+  // (64 bits, checked against the Int32 range) here
   int32_t *perm = nullptr, *d_width = nullptr;
-  std::vector<int32_t> width(ns), sp(ns + 1);
+  std::vector<int32_t> width(ns), sp(ns + 1), host_perm;
   cudaError_t e = cudaMalloc((void**)&perm, (m > 0 ? m : 1) * sizeof(int32_t));
   if (e != cudaSuccess) return cuda_error(e, "gg_sell_create");
-  int rc = sort_rows_by_length(ctx, csr->rowptr, m, sigma, perm);
-  if (rc == GG_OK) {
-    e = cudaMallocAsync((void**)&d_width, (ns > 0 ? ns : 1) * sizeof(int32_t), ctx->stream);
+  int rc = GG_OK;
+  if (m <= (sigma > 1 ? kHostOrderRows : kHostWidthRows)) {
+    rc = order_rows_on_host(ctx, csr->rowptr, m, C, sigma, &host_perm, &width);
+    if (rc == GG_OK && m > 0)
+      e = cudaMemcpyAsync(perm, host_perm.data(), m * sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream);
+    if (e != cudaSuccess) rc = cuda_error(e, "gg_sell_create");
+  } else if ((rc = sort_rows_by_length(ctx, csr->rowptr, m, sigma, perm)) == GG_OK) {
+    e = cudaMalloc((void**)&d_width, (ns > 0 ? ns : 1) * sizeof(int32_t));
     if (e == cudaSuccess) rc = sell_slice_widths(ctx, csr->rowptr, perm, m, C, ns, d_width);
     if (e == cudaSuccess && rc == GG_OK && ns > 0)
       e = cudaMemcpyAsync(width.data(), d_width, ns * sizeof(int32_t), cudaMemcpyDeviceToHost,
                           ctx->stream);
-    cudaFreeAsync(d_width, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    cudaFree(d_width);
     if (e != cudaSuccess && rc == GG_OK) rc = cuda_error(e, "gg_sell_create");
   }
   sp[0] = 1;
