@@ -1216,10 +1216,13 @@ gg_mat* sell_for_spmv(gg_ctx* ctx, gg_mat* A) {
 // kernel, us: R-MAT scale 17 56 / 41, 20 112 / 92, 22 339 / 336, 23 789 / 773, 24 1628 /
 // 1647; flat columns (k_sell): ER with 16.8 M entries 79 / 67, a 1024 x 1024 grid 26 / 14.
 static const int64_t kTypedPlainRows = (int64_t)3 << 22;
-static bool typed_plain(const gg_mat* A, const gg_mat* S) {
-  if (S->slice_size != 32) return false;
-  if (!S->colperm->enabled) return true;
-  return A->tuned_spmv == 0 && S->sell_variant == 0 && S->hot_cols == 0 && S->m < kTypedPlainRows;
+static int typed_plain(gg_ctx* ctx, const gg_mat* A, gg_mat* S, bool* plain) {
+  *plain = S->slice_size == 32;
+  if (*plain && A->tuned_spmv == 0 && S->sell_variant == 0 && S->hot_cols == 0 && S->m < kTypedPlainRows)
+    return GG_OK;  // whatever the columns: they are not looked at
+  GG_CHECK(build_colperm(ctx, S));
+  *plain = *plain && !S->colperm->enabled;
+  return GG_OK;
 }
 
 static int spmv_run(gg_ctx* ctx, gg_mat* A, int tc, int mul, int add, int accum, void* y, int ty,
@@ -1257,15 +1260,18 @@ static int spmv_run(gg_ctx* ctx, gg_mat* A, int tc, int mul, int add, int accum,
       // rows give every thread the same work
       GG_CHECK(ensure_sell_copy(ctx, A));
       A->last_layout = 2;
-      GG_CHECK(build_colperm(ctx, A->sell_copy));
-      if (typed_plain(A, A->sell_copy)) return spmv_typed_on_copy(ctx, A, sr.x, sr.y);
+      bool typed = false;
+      GG_CHECK(typed_plain(ctx, A, A->sell_copy, &typed));
+      if (typed) return spmv_typed_on_copy(ctx, A, sr.x, sr.y);
       A->sell_copy->tuned_spmv = A->tuned_spmv;  // the copy's own dispatch keeps a tuned kernel
       GG_CHECK(spmv_run(ctx, A->sell_copy, tc, mul, add, accum, y, ty, x, tx, mask, tmask, lo, hi));
       return launch_refold_nan_rows(ctx, A, sr.x, sr.y);
     }
-    GG_CHECK(build_colperm(ctx, A));
+    bool typed = false;
+    if (A->format == GG_FMT_SELL) GG_CHECK(typed_plain(ctx, A, A, &typed));
+    else GG_CHECK(build_colperm(ctx, A));
     const int32_t* colval = A->colval;
-    if (A->format == GG_FMT_SELL && typed_plain(A, A)) {
+    if (typed) {
       A->last_layout = 2;
       bool done = false;
       return spmv_typed(ctx, A, tc, mul, add, accum, y, ty, x, tx, mask, tmask, lo, hi, &done);

@@ -162,6 +162,13 @@ struct SRTyped {
 // ---------------------------------------------------------------------------------
 static const int kTypedHotBytes = 128 << 10;
 static const int kTypedHotThreads = 1024;
+// Columns up to which x is gathered as it lies: L2 holds it, and ranking and relabelling the
+// columns (0.3 ms of the first product), reordering x and filling the shared part of every
+// SM cost more than they save.  With the shared part / without, us, R-MAT scale 16, 18, 20:
+// Int32 min-plus 54 / 32, 65 / 44, 106 / 98; Float64 min-plus 261 / 90, 284 / 178, 551 / 442
+// (its few full SMs wait for the FP64 pipe); masked or-and 51 / 30, 67 / 34, 81 / 49.  Scale
+// 21: Int32 177 / 198.
+static const int64_t kTypedHotCols = 1 << 20;
 
 struct TypedFilter {  // rows whose results are wanted (1-based range, 0 = all)
   const void* mask;
@@ -424,9 +431,9 @@ template <class SR>
 static int launch_sell32_typed(gg_ctx* ctx, gg_mat* S, const gg_mat* A, SR sr, const TypedFilter& flt) {
   typedef typename SR::T T;
   GG_CHECK(build_sell_plan(ctx, S));
-  GG_CHECK(build_colperm(ctx, S));
+  if (S->n > kTypedHotCols) GG_CHECK(build_colperm(ctx, S));
   const SellPlan* P = S->sellplan;
-  const bool hot_x = S->colperm->enabled;
+  const bool hot_x = S->n > kTypedHotCols && S->colperm->enabled;
   const int32_t* colval = hot_x ? S->colperm->colval_r : S->colval;
   const int32_t* perm = S->sigma > 1 ? S->perm : nullptr;
   const T* x = sr.x;  // sr keeps the caller's x for the refolds over A's own columns

@@ -209,10 +209,10 @@ int gg_mat_values_changed(gg_ctx* ctx, gg_mat* A);
  * gg_mat_destroy or gg_mat_values_changed.  The first call with one element type and a
  * common semiring (mul / add, add or safe_add / min, band or land / bor or lor) on a CSR
  * handle of at least 65536 rows, or on a SELL handle with more than a quarter of padding, builds
- * a SELL-32 copy of the matrix with rows sorted by length and relabelled columns: about
- * 8 bytes per stored entry more than the values take, plus 16 per row, i.e. more than the
- * CSR itself (4-byte values: about 1.6 GB at R-MAT scale 22, 6.5 GB at scale 24); the
- * semirings of a handle share it.  Where it does not fit, semirings other than Float32
+ * a SELL-32 copy of the matrix with rows sorted by length and, past 2^20 columns, relabelled
+ * columns: about 8 bytes per stored entry more than the values take (4 without relabelling),
+ * plus 16 per row, i.e. more than the CSR itself (4-byte values: about 1.6 GB at R-MAT scale
+ * 22, 6.5 GB at scale 24); the semirings of a handle share it.  Where it does not fit, semirings other than Float32
  * plus-times run on the handle's own arrays.  Other
  * first calls add row-block descriptors (16 bytes per block of up to 256 entries).
  * Later calls allocate nothing and are asynchronous.

@@ -18,7 +18,7 @@ def changed(A):
 
 @pytest.mark.parametrize("C", [8, 32])
 def test_copy_follows_how_long_values_last(C):
-    A = gen.rmat(17, 16, seed=3, wkind=gen.W_INT_1_255)
+    A = gen.rmat(21, 16, seed=3, wkind=gen.W_INT_1_255)  # columns enough for the relabelling
     S = G.SparseGPUMatrixSELL(A, C, 64)
     x = torch.randint(0, 5000, (A.n,), device="cuda", dtype=torch.int32)
     op = dict(mul=G.GPUGraphs_safe_add, add=G.GPUGraphs_min)
