@@ -34,7 +34,7 @@ int cuda_error(cudaError_t e, const char* what) {
   return set_error(code, "%s: %s", what, cudaGetErrorString(e));
 }
 
-static bool capturing(gg_ctx* ctx) {
+bool capturing(gg_ctx* ctx) {
   cudaStreamCaptureStatus s = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(ctx->stream, &s) == cudaSuccess) return s != cudaStreamCaptureStatusNone;
   (void)cudaGetLastError();  // the legacy stream while another stream is being captured
@@ -528,8 +528,8 @@ int gg_mat_values_changed(gg_ctx* ctx, gg_mat* A) {
   GG_CUDA(cudaSetDevice(ctx->device));
   GG_CUDA(cudaStreamSynchronize(ctx->stream));
   free_derived(A);
-  // a padded SELL handle's sorted copy costs about eight of the products it speeds up:
-  // values that lasted for fewer do without one the next time
+  // a sorted copy costs about eight of the products it speeds up: after values that lasted
+  // for fewer the next ones get theirs with the ninth product only
   if (A->products > 0) A->values_churn = A->products < kCopyProducts;
   A->products = 0;
   return GG_OK;

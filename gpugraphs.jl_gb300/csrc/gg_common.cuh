@@ -608,6 +608,7 @@ struct gg_mat {
   gg::StreamOrder order;  // products that use buffers of the handle's plans
   int64_t products = 0;
   bool values_churn = false;  // set by gg_mat_values_changed
+  bool copy_due() const { return !values_churn || products > gg::kCopyProducts; }
   gg_mat* tr_copy = nullptr;    // CSR handles: CSR storage of the transpose (gg_spmv_t)
   int64_t max_row_len = -1;
   // tuned choices (gg_tune): plus-times SpMV kernel (0 = built-in rule, 1 = CSR row
@@ -629,6 +630,7 @@ namespace gg {
 int ensure_scratch(gg_ctx* ctx, size_t bytes);
 int order_before(gg_ctx* ctx, StreamOrder& o);  // before a workspace is touched (gg_api.cu)
 int order_after(gg_ctx* ctx, StreamOrder& o);   // after the last launch that touches it
+bool capturing(gg_ctx* ctx);  // whether the context's stream is (gg_api.cu)
 void free_graph_aux(gg_mat* A);
 int compute_type(int tv, int tx, int mul);
 int check_semiring(int tv, int tx, int ty, int mul, int add, int accum, int* tc_out);

@@ -1190,7 +1190,7 @@ static int launch_refold_nan_rows(gg_ctx* ctx, const gg_mat* A, const float* x, 
 // every row keeps its entries' order and its chunks, only the padding goes.  Small
 // matrices, windows of the whole matrix already (such a copy itself, or a CSR handle's:
 // sorting again would change nothing), handles with tuned choices, copies that do not
-// fit and handles whose values change often keep their own arrays.
+// fit and values that have not lasted yet (gg_mat_values_changed) keep their own arrays.
 // Float64 plus-times on R-MAT scale 20, sigma = 1 / 1024: 1157 / 482 us on the handle's
 // own slices, 199 on the copy; Float32 460 / 217 us, 107.
 gg_mat* sell_for_spmv(gg_ctx* ctx, gg_mat* A) {
@@ -1198,8 +1198,8 @@ gg_mat* sell_for_spmv(gg_ctx* ctx, gg_mat* A) {
       A->sell_variant != 0 || A->hot_cols != 0)
     return A;
   ++A->products;
-  if (A->values_churn) return A;
   if (A->sell_copy) return A->sell_copy;
+  if (!A->copy_due() || (A->values_churn && capturing(ctx))) return A;
   if (sell_resorted(ctx, A, &A->sell_copy) != GG_OK) {
     A->sell_copy = nullptr;
     A->no_sell_copy = true;

@@ -488,13 +488,19 @@ static int spmv_typed_t(gg_ctx* ctx, gg_mat* A, int accum, void* y, const void* 
   if (A->format == GG_FMT_SELL) {
     const SRTyped<TC, MUL, ADD, false> sr{static_cast<const T*>(A->nzval), static_cast<const T*>(x),
                                           static_cast<T*>(y), accum};
-    // (relabelled columns are a layout of their own: not for values that change often)
-    if (A->slice_size == 32 && !A->values_churn) return launch_sell32_typed(ctx, A, nullptr, sr, flt);
+    // (relabelled columns are a layout of their own: not for values that may not last)
+    if (A->slice_size == 32 &&
+        (A->n <= kTypedHotCols || A->colperm || (A->copy_due() && !(A->values_churn && capturing(ctx)))))
+      return launch_sell32_typed(ctx, A, nullptr, sr, flt);
     return launch_sell(ctx, A, sr, mask, tmask, lo, hi);
   }
   const SRTyped<TC, MUL, ADD, true> sr{static_cast<const T*>(A->nzval), static_cast<const T*>(x),
                                        static_cast<T*>(y), accum};
-  if (lo == 0 && A->m >= kTypedCopyRows && !A->no_sell_copy) {
+  const bool large = lo == 0 && A->m >= kTypedCopyRows;
+  if (large) ++A->products;
+  // values that may not last get no copy; one that another product made is taken
+  if (large && !A->no_sell_copy &&
+      (A->sell_copy || (A->copy_due() && !(A->values_churn && capturing(ctx))))) {
     if (ensure_sell_copy(ctx, A) != GG_OK) {
       A->sell_copy = nullptr;  // no room for the copy, or past its index range: row blocks
       A->no_sell_copy = true;

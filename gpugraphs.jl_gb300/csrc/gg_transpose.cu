@@ -156,6 +156,9 @@ int gg_spmv_t(gg_ctx* ctx, const gg_mat* A_, int mul, int add, int accum, void* 
   if (range_lo != 0 && range_lo > range_hi) return GG_OK;
   GG_CUDA(cudaSetDevice(ctx->device));
   GG_CHECK(build_transpose(ctx, A));
+  // how long values last is known to the handle: the transposed copy goes with them
+  A->tr_copy->values_churn = A->values_churn;
+  A->tr_copy->products = A->products++;
   return spmv_dispatch(ctx, A->tr_copy, tc, mul, add, accum, y, y_dtype, x, x_dtype, mask,
                        mask_dtype, range_lo, range_hi);
 }

@@ -187,8 +187,9 @@ int gg_mat_arrays(const gg_mat* A, void** ptr, void** colval, void** nzval, void
  * Drops everything the library derived from the handle's values on first use (the
  * SELL-32 and transposed copies, graph analyses, plans); call it after writing to the
  * arrays gg_mat_arrays returns (setindex!, src/storage/CSR.jl:166-180).  Waits for the
- * context's stream first.  A padded SELL handle whose values lasted for fewer than eight
- * products gets no sorted copy (gg_spmv) for the next ones.
+ * context's stream first.  After values that lasted for fewer than eight products the
+ * sorted copy of a handle (gg_spmv, other than a CSR's Float32 plus-times) is made with the
+ * ninth product of the next ones, and not under capture.
  */
 int gg_mat_values_changed(gg_ctx* ctx, gg_mat* A);
 
@@ -215,7 +216,7 @@ int gg_mat_values_changed(gg_ctx* ctx, gg_mat* A);
  * 22, 6.5 GB at scale 24); the semirings of a handle share it.  Where it does not fit, semirings other than Float32
  * plus-times run on the handle's own arrays.  Other
  * first calls add row-block descriptors (16 bytes per block of up to 256 entries).
- * Later calls allocate nothing and are asynchronous.
+ * Later calls allocate nothing and are asynchronous (but see gg_mat_values_changed).
  */
 int gg_spmv(gg_ctx* ctx, const gg_mat* A, int mul, int add, int accum, void* y, int y_dtype,
             int64_t y_len, const void* x, int x_dtype, int64_t x_len, const void* mask,
