@@ -1228,13 +1228,15 @@ static int bfs_run(gg_ctx* ctx, gg_mat* A, int32_t s, int which, int32_t* dist,
   const int64_t total_edges = P.nnz;
   const bool pull_queue = n < kPullQueueRows;
   // hub-free graphs (grids, meshes) run medium frontiers in the persistent kernel
-  // Hub-free graphs with few entries a vertex, whose levels are many and narrow, run in the
-  // cluster and grid-wide persistent kernels: 70 x 33 grid 240 to 193 us, 250 x 250 grid
-  // 1324 to 883, ER with 6 entries a vertex and 10^4 / 10^6 vertices 246 to 94 and 415 to
-  // 335.  With more entries the frontier is most of the graph within a few levels, and
-  // separate pull launches are faster: ER with 32 entries a vertex and 60000 / 10^6 / 4 10^6
-  // vertices, persistent 236 / 539 / 822 us, separate 140 / 231 / 359.
-  const bool coop_ok = P.max_deg <= kCoopMaxDeg && n >= 2048 && P.nnz <= 6 * n;
+  // Hub-free graphs with few (searched) entries a vertex, whose levels are many and narrow,
+  // run in the cluster and grid-wide persistent kernels: 70 x 33 grid 240 to 193 us, 250 x
+  // 250 grid 1324 to 883, ER with 8 entries a vertex and 2^14 / 2^18 / 2^22 vertices 201 to
+  // 119, 359 to 290 and 624 to 507, with 8 odd ones of 16 (pull levels read all) 215 to 120,
+  // 354 to 300 and 828 to 667.  With more entries the frontier is most of the graph within a
+  // few levels, and separate pull launches are faster from 2^20 vertices: 12 entries 209 /
+  // 289 / 497 us for 2^16 / 2^20 / 2^22, persistent 217 / 321 / 561; 24 entries 174 / 269 /
+  // 472, persistent 229 / 380 / 595.
+  const bool coop_ok = P.max_deg <= kCoopMaxDeg && n >= 2048 && P.nnz <= 9 * n;
   const int32_t small_cap = coop_ok ? kCoopLo : kSmallCap;
   const long long coop_hi = n / 24 > kCoopLo ? n / 24 : kCoopLo;
   CoopCtl* hc = reinterpret_cast<CoopCtl*>(ctx->h_flags);
