@@ -243,10 +243,10 @@ struct BsRows {
   double cap = -1.0;  // light edges' largest weight, < 0: no light phase
 };
 
-// Work buffers of one batched shortest-path call.  ctr: [0] vertices changed this
-// round, [1] / [2] lengths of the changed queues cq[0] / cq[1], [3] marked vertices, then
-// the out-edges of the changed ones, [4] hubs being marked, [5] pairs that dropped, [6]
-// smallest distance written (MsSums).
+// Work buffers of one batched shortest-path call.  ctr: [0] / [5] lengths of the changed
+// queues cq[0] / cq[1], [1] vertices changed this round, [2] pairs that dropped, [3] smallest
+// distance written (MsSums), [4] out-edges of the changed vertices, [6] marked vertices, [7]
+// hubs being marked.  A round clears its queue's length and [1] to [4] in one go.
 template <typename T>
 struct BsWork {
   T* D;
@@ -320,7 +320,7 @@ static int bs_start(gg_ctx* ctx, int64_t n, BsRun<T>& R) {
   k_bs_seed<T><<<1, 64, 0, R.st>>>(R.w.D, R.dsrc, R.S, R.w.c[0], R.w.cq[0]);
   GG_CUDA(cudaGetLastError());
   for (int i = 0; i < 8; ++i) R.h[i] = 0;
-  R.h[1] = (unsigned long long)R.S;
+  R.h[0] = (unsigned long long)R.S;
   GG_CUDA(cudaMemcpyAsync(R.w.ctr, R.h, 8 * sizeof(unsigned long long), cudaMemcpyHostToDevice, R.st));
   R.pairs = R.S;
   R.dlow = T(0);
@@ -330,12 +330,10 @@ static int bs_start(gg_ctx* ctx, int64_t n, BsRun<T>& R) {
   return GG_OK;
 }
 
-// ctr[3] (the marked count, used inside a restricted round only) becomes the out-edge
-// count of this round's changed vertices once the round's kernels are done
+// the out-edges of this round's changed vertices into ctr[4], once its kernels are done
 static int bs_degsum(gg_ctx* ctx, const int32_t* prow, const int32_t* cq,
                      const unsigned long long* ncq, unsigned long long* ctr, cudaStream_t st) {
-  GG_CUDA(cudaMemsetAsync(ctr + 3, 0, sizeof(unsigned long long), st));
-  k_ms_degsum<<<ctx->num_sms * 4, 256, 0, st>>>(cq, ncq, prow, ctr + 3);
+  k_ms_degsum<<<ctx->num_sms * 4, 256, 0, st>>>(cq, ncq, prow, ctr + 4);
   GG_CUDA(cudaGetLastError());
   return GG_OK;
 }
@@ -353,14 +351,17 @@ static int bs_issue(gg_ctx* ctx, int64_t n, int64_t nnz, const BatchGraph& g, co
   const int64_t avg_deg = n > 0 ? (nnz + n - 1) / n : 1;
   BsWork<T>& w = R.w;
   const int cur = R.cur;
-  unsigned long long* ncq_cur = w.ctr + 1 + cur;
-  unsigned long long* ncq_nxt = w.ctr + 1 + (cur ^ 1);
-  GG_CUDA(cudaMemsetAsync(w.ctr, 0, sizeof(unsigned long long), R.st));
-  GG_CUDA(cudaMemsetAsync(ncq_nxt, 0, sizeof(unsigned long long), R.st));
+  unsigned long long* ncq_cur = w.ctr + 5 * cur;
+  unsigned long long* ncq_nxt = w.ctr + 5 * (cur ^ 1);
+  GG_CUDA(cudaMemsetAsync(w.ctr + (cur ^ 1), 0, 5 * sizeof(unsigned long long), R.st));
   GG_CUDA(cudaMemsetAsync(w.c[cur ^ 1], 0, (size_t)n * sizeof(unsigned), R.st));
-  GG_CUDA(cudaMemsetAsync(w.ctr + 5, 0, 2 * sizeof(unsigned long long), R.st));
-  const MsSums sums{w.ctr + 5, w.ctr + 6};
   const bool by_row = sizeof(T) == 4 && br.rows.col != nullptr;
+  // Thin graphs go without the sums: their rows are too short to end early, and the two atomics
+  // a warp were paid in every one of many rounds (300 x 300 grid, 40 / 256 sources, ms: 53.1 /
+  // 125.2 with them and four clears of the counters, 41.7 / 103.3 now; 600 x 600, 256 sources,
+  // 468, 623 by the vertex rounds before).  Then dlow is 0 and the masks are always looked at.
+  const bool thin = nnz < kMsThin * n;
+  const MsSums sums{thin ? nullptr : w.ctr + 2, thin ? nullptr : w.ctr + 3};
   R.restricted = (by_row && R.mchanged >= 0) ? R.mchanged * kBsRowRestrict < nnz
                                              : R.nchanged * avg_deg * 4 < nnz;
   bool settle = false;  // this round visits every row over every edge
@@ -370,11 +371,11 @@ static int bs_issue(gg_ctx* ctx, int64_t n, int64_t nnz, const BatchGraph& g, co
   }
   if (R.restricted) {
     GG_CUDA(cudaMemsetAsync(w.mark, 0, ((n + 31) / 32) * sizeof(unsigned), R.st));
-    GG_CUDA(cudaMemsetAsync(w.ctr + 3, 0, sizeof(unsigned long long), R.st));
+    GG_CUDA(cudaMemsetAsync(w.ctr + 6, 0, sizeof(unsigned long long), R.st));
     GG_CUDA(launch_ms_mark(R.st, ctx->num_sms, R.nchanged, prow, pcol, w.cq[cur], ncq_cur, w.mark,
-                           w.vlist, w.ctr + 3, w.mhq, w.ctr + 4, w.mhoff));
-    k_ms_round<T><<<(int)gcap, 256, 0, R.st>>>(n, g, w.D, w.c[cur], w.c[cur ^ 1], w.ctr, nullptr,
-                                               w.vlist, w.ctr + 3, w.cq[cur ^ 1], ncq_nxt, sums);
+                           w.vlist, w.ctr + 6, w.mhq, w.ctr + 7, w.mhoff));
+    k_ms_round<T><<<(int)gcap, 256, 0, R.st>>>(n, g, w.D, w.c[cur], w.c[cur ^ 1], w.ctr + 1, nullptr,
+                                               w.vlist, w.ctr + 6, w.cq[cur ^ 1], ncq_nxt, sums);
   } else if (by_row) {
     // every row, hubs in pieces
     if constexpr (sizeof(T) == 4) {
@@ -385,10 +386,10 @@ static int bs_issue(gg_ctx* ctx, int64_t n, int64_t nnz, const BatchGraph& g, co
       const T dlow = settle ? T(0) : R.dlow;
       if (R.light) R.owed = true;
       if (!settle && R.pairs < kBsCheck * n)
-        k_ms_round_rows<T, true><<<(int)rb, 256, 0, R.st>>>(br.rows, w.D, w.c[cur], w.c[cur ^ 1], w.ctr,
+        k_ms_round_rows<T, true><<<(int)rb, 256, 0, R.st>>>(br.rows, w.D, w.c[cur], w.c[cur ^ 1], w.ctr + 1,
                                                             nullptr, w.cq[cur ^ 1], ncq_nxt, sums, dlow, cap);
       else
-        k_ms_round_rows<T, false><<<(int)rb, 256, 0, R.st>>>(br.rows, w.D, w.c[cur], w.c[cur ^ 1], w.ctr,
+        k_ms_round_rows<T, false><<<(int)rb, 256, 0, R.st>>>(br.rows, w.D, w.c[cur], w.c[cur ^ 1], w.ctr + 1,
                                                              nullptr, w.cq[cur ^ 1], ncq_nxt, sums, dlow, cap);
       GG_CUDA(cudaGetLastError());
       GG_CHECK(bs_degsum(ctx, prow, w.cq[cur ^ 1], ncq_nxt, w.ctr, R.st));
@@ -397,13 +398,13 @@ static int bs_issue(gg_ctx* ctx, int64_t n, int64_t nnz, const BatchGraph& g, co
     }
   } else {
     // every non-hub vertex, in the plan's order: the long rows first, spread over the warps
-    k_ms_round<T><<<(int)gb, 256, 0, R.st>>>(n, g, w.D, w.c[cur], w.c[cur ^ 1], w.ctr, nullptr,
+    k_ms_round<T><<<(int)gb, 256, 0, R.st>>>(n, g, w.D, w.c[cur], w.c[cur ^ 1], w.ctr + 1, nullptr,
                                              hp->order, hp->d_norder, w.cq[cur ^ 1], ncq_nxt, sums);
   }
   GG_CUDA(cudaGetLastError());
   if (hp->npiece > 0) {
     k_ms_round_hub<T><<<(int)pb, 256, 0, R.st>>>(g, hp->pieces, hp->npiece, hp->hubs, w.D,
-                                                 w.c[cur], w.c[cur ^ 1], w.ctr, nullptr,
+                                                 w.c[cur], w.c[cur ^ 1], w.ctr + 1, nullptr,
                                                  R.restricted ? w.mark : nullptr, w.cq[cur ^ 1],
                                                  ncq_nxt, sums);
     GG_CUDA(cudaGetLastError());
@@ -489,18 +490,18 @@ static int sssp_batch_t(gg_ctx* ctx, gg_mat* A, const BatchGraph& g, const int64
       }
       if (rounds) *rounds += 1;
       ++R.r;
-      if (R.h[0] == 0 && !R.owed) {  // converged: write the group out, take the next one
+      if (R.h[1] == 0 && !R.owed) {  // converged: write the group out, take the next one
         k_bs_out<T><<<(int)gb, 256, 0, R.st>>>(R.w.D, n, R.S, R.dist, ld);
         R.done = true;
         rc = start_next(R);
       } else if (R.r > n + 1) {
         rc = set_error(GG_ERR_NOT_CONVERGED, "batched shortest paths did not converge");
       } else {
-        R.nchanged = (int64_t)R.h[1 + (R.cur ^ 1)];
-        R.mchanged = (int64_t)R.h[3];
-        R.pairs = (int64_t)R.h[5];
-        const unsigned low = ~(unsigned)R.h[6];
-        if (sizeof(T) == 4 && R.h[6]) memcpy(&R.dlow, &low, 4);
+        R.nchanged = (int64_t)R.h[5 * (R.cur ^ 1)];
+        R.mchanged = (int64_t)R.h[4];
+        R.pairs = (int64_t)R.h[2];
+        const unsigned low = ~(unsigned)R.h[3];
+        if (sizeof(T) == 4 && R.h[3]) memcpy(&R.dlow, &low, 4);
         else R.dlow = T(0);
         R.cur ^= 1;
       }

@@ -584,13 +584,16 @@ template <> __device__ __forceinline__ double b_atomic_min<double>(double* p, do
 //    leaves heavy entries out altogether; a later round must then visit every row with
 //    dlow = 0 and no cap before the result is final.
 //  * kCheck: entries whose in-neighbour did not change in the previous round are left out
-//    by its column mask (worth its gather once few of the pairs drop).
+//    by its column mask (worth its gather once few of the pairs drop).  On thin graphs what
+//    has dropped in this round so far counts too, as in bs_pull: a tenth fewer of the many
+//    rounds of a grid.
 // Whole rows have one writer; pieces lower their row by atomic min.  Any order of
 // relaxations reaches the same fixpoint.
 // Against the round it replaces (a warp per 32-row SELL item, changed entries through a
 // shared-memory queue, 19.5 warp instructions an entry, all entries): 800 -> 250 us on R-MAT
 // scale 20, 32 Int32 columns; 256 sources 57.5 -> 25.5 ms.  A round alone takes 260 us:
 // issue 55%, 45% of the warp slots, L2 20%, DRAM 18%, most stalls on the rows of D.
+static const int64_t kMsThin = 8;
 struct MsRows {
   const int32_t* rowptr;  // 1-based
   const int32_t* col;     // 1-based, entries of a row by ascending weight
@@ -600,6 +603,7 @@ struct MsRows {
   int64_t nitems;
   const int32_t* short_rows;  // rows of 1..32 entries
   int64_t nshort;
+  bool thin;                  // fewer than kMsThin entries a row in the mean
 };
 
 // the row rounds' view of A (CSR handles with 1- or 4-byte values; out->col stays nullptr
@@ -616,6 +620,7 @@ static inline int ms_rows_of(gg_ctx* ctx, gg_mat* A, MsRows* out, double* mean_w
   out->nitems = P->nitems;
   out->short_rows = P->short_rows;
   out->nshort = P->nlive;
+  out->thin = A->nnz < kMsThin * A->m;
   return GG_OK;
 }
 
@@ -702,7 +707,10 @@ __global__ void __launch_bounds__(256, kMsRowBlocks)
       const int32_t cn = kn < k1 ? __ldg(g.col + kn) : 0;
       const T wn = kn < k1 ? b_weight<T>(g.w, g.tv, kn) : Lim<T>::max();
       unsigned m = ~0u;
-      if (kCheck) m = c > 0 ? __ldg(chg + (c - 1)) : 0u;
+      if (kCheck) {
+        m = c > 0 ? __ldg(chg + (c - 1)) : 0u;
+        if (g.thin && c > 0) m |= __ldcg(chg_next + (c - 1));
+      }
 #pragma unroll
       for (int h = 0; h < 8; h += kMsRowStep) {
         int4 dv[kMsRowStep];
