@@ -223,13 +223,17 @@ __global__ void __launch_bounds__(kHot ? kTypedHotThreads : 256, kHot ? 1 : 4)
         const int64_t srow = (int64_t)d.y + t * 32 + lane;
         return srow < m ? (perm ? __ldg(perm + srow) : (int32_t)(srow + 1)) : 0;
       };
-      if (flt.lo > 0) {  // a row range: groups outside it are passed over
-        bool any = false;
-        for (int t = 0; t < ns; ++t) {
-          const int32_t r = row_at(t);
-          any |= r >= flt.lo && r <= flt.hi;
+      // a row range: groups outside it are passed over (SELL handles alone: ranges of a CSR
+      // take the row blocks, and with the check its scale 22 product took 338 us, not 329)
+      if constexpr (!SR::kHasAbsorbCheck) {
+        if (flt.lo > 0) {
+          bool any = false;
+          for (int t = 0; t < ns; ++t) {
+            const int32_t r = row_at(t);
+            any |= r >= flt.lo && r <= flt.hi;
+          }
+          if (!__any_sync(kFull, any)) continue;
         }
-        if (!__any_sync(kFull, any)) continue;
       }
       int32_t c[kNarrowCols];
       T p[kNarrowCols];
