@@ -12,9 +12,9 @@
 //  * SELL-32 handles: k_sell32_typed on their own arrays; other slice heights: k_sell.
 // Rows fold in storage order within chunks of kSellChunk entries, as everywhere.
 // Measured, us before -> now: Int32 min-plus R-MAT 21 422 -> 178; masked Bool or-and
-// R-MAT 20 307 -> 85; Float64 plus-times R-MAT 20 608 -> 225 (bound by the FP64 pipe: a
-// multiply and an add per entry, 100 us), on a SELL-32 handle with sigma 1024 975 -> 199;
-// masked Float32 plus-times R-MAT 20 328 -> 108; Int32 min-plus on a 2^20-vertex ER graph
+// R-MAT 20 307 -> 43; Float64 plus-times R-MAT 20 608 -> 169 (bound by the FP64 pipe: a
+// multiply and an add per entry, 100 us), on a SELL-32 handle with sigma 1024 975 -> 152;
+// masked Float32 plus-times R-MAT 20 328 -> 81; Int32 min-plus on a 2^20-vertex ER graph
 // 102 -> 70 and a 1024 x 1024 grid 28 -> 17.
 #include "gg_spmv_kernels.cuh"
 
