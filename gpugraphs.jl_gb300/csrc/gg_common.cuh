@@ -603,9 +603,9 @@ struct gg_mat {
   // whose own slices are mostly padding
   gg_mat* sell_copy = nullptr;
   bool no_sell_copy = false;  // the copy could not be made (memory, index range)
-  // padded SELL handles: products since the values last changed, and whether they change
-  // too often for a copy (sell_for_spmv)
   gg::StreamOrder order;  // products that use buffers of the handle's plans
+  // products since the values last changed, and whether they change too often for a sorted
+  // copy or relabelled columns (sell_for_spmv, spmv_typed_t)
   int64_t products = 0;
   bool values_churn = false;  // set by gg_mat_values_changed
   bool copy_due() const { return !values_churn || products > gg::kCopyProducts; }
